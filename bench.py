@@ -302,8 +302,9 @@ def run_ours(args):
     sim.profile_begin()
     sim.step(48)
     kprof = sim.profile_end()
-    # roofline of the dominant kernel, the bulk streaming kernel (one launch
-    # per step over every particle): its algorithmic bytes per particle are
+    # roofline of the bulk streaming kernel (one launch per stretch of steps
+    # over every particle, which it takes through all of them): its algorithmic
+    # bytes per particle and launch are
     # the stream's state read and positions written -- FP64: positions 3 x 8
     # and velocities 3 x 8 read, positions 3 x 8 written = 72 B; FP32: two
     # float4 read, one written = 48 B (the 32-byte FP64 velocity record
@@ -340,7 +341,7 @@ def run_ours(args):
                        timed="whole collision cycles: the requested steps rounded up to a multiple of 12"),
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "traffic": traffic,
-                     "kernel": "k_stream_fast" if precision == G.FP64 else "k_stream_f",
+                     "kernel": "k_stream_bulk" if precision == G.FP64 else "k_stream_bulk_f",
                      "bytes_per_particle": bpp, "units_per_launch": ns, "peak_kind": kind,
                      "kernel_ms_avg": bulk_avg_ms,
                      "step_bytes_per_particle_step": step_bpp,

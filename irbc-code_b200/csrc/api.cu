@@ -26,6 +26,18 @@ namespace irbc {
 std::atomic<int64_t> g_launches{0};
 }
 
+namespace {
+// Host copy of the membrane (set-up, and the patches of the membrane kernel).
+struct HostMesh {
+  int nv = 0, ne = 0, nt = 0;
+  std::vector<double> x, y, z, vx, vy, vz;
+  std::vector<int> ix, iy;
+  std::vector<int> e1, e2, es1, es2, iedge, t1, t2, t3;
+  std::vector<double> l0, kappap, tarea, cmx, cmy, cmz;
+  double Sarea0 = 0, Volume0 = 0, theta0 = 0, center[3] = {0, 0, 0};
+};
+}  // namespace
+
 struct irbc_handle {
   uint64_t uid = 0;        // unique for the life of the process (a freed handle's address can return)
   void* rec = nullptr;     // device staging of irbc_record_async
@@ -38,19 +50,18 @@ struct irbc_handle {
   cudaStream_t st2 = nullptr;  // membrane kernels, run beside the solvent ones (== st with one stream)
   cudaStream_t st2_own = nullptr;  // the side stream this handle created
   int mem_mode = 1;                // membrane step: 1 wide kernels, 2 one block, 3 one cluster
+  HostMesh host_mesh;              // topology only
   FastBufs fb;
   bool fp32 = false;           // solvent held in sf (float4) between exchanges
   SolventF sf;
-  int snap_buf = 0;            // which snapshot the next streaming step reads
-  bool snap_ready = false;     // snapshot/triangle prep of the next step done
-  cudaEvent_t ev_snap = nullptr, ev_mem = nullptr, ev_coll = nullptr, ev_str[2] = {nullptr, nullptr};
+  cudaEvent_t ev_mem = nullptr, ev_coll = nullptr;
   cudaEvent_t ev_vbin = nullptr;
   uint64_t* ebase = nullptr;   // device: the draw epoch base of the current call (DevParams::ebase)
   int64_t ebase_val = 0;       // its value as last written
   // captured step sequences (irbc_step): one per starting configuration
   struct StepGraph {
     cudaGraphExec_t exec = nullptr;
-    int colsteps0 = 0, parity = 0;
+    int colsteps0 = 0;
     double wallspeed = 0;
     int64_t launches = 0, collisions = 0;
   };
@@ -149,16 +160,6 @@ void free_membrane(Membrane& m) {
     dfree(*p);
   dfree(m.vkey);
 }
-
-// Host copy of the membrane used during set-up.
-struct HostMesh {
-  int nv = 0, ne = 0, nt = 0;
-  std::vector<double> x, y, z, vx, vy, vz;
-  std::vector<int> ix, iy;
-  std::vector<int> e1, e2, es1, es2, iedge, t1, t2, t3;
-  std::vector<double> l0, kappap, tarea, cmx, cmy, cmz;
-  double Sarea0 = 0, Volume0 = 0, theta0 = 0, center[3] = {0, 0, 0};
-};
 
 inline void hcp(const double A[], const double B[], double C[]) {
   C[0] = (A[1] * B[2]) - (B[1] * A[2]);
@@ -293,41 +294,239 @@ int down(irbc_handle* h, T* v, const T* d, int64_t n) {
 }
 
 void free_fast(FastBufs& f) {
-  for (int b = 0; b < 2; ++b) {
-    for (double** q : {&f.snap[b].x, &f.snap[b].y, &f.snap[b].z, &f.snap[b].vx, &f.snap[b].vy, &f.snap[b].vz})
-      dfree(*q);
-    dfree(f.pre[b]);
-  }
-  dfree(f.slot); dfree(f.gstart); dfree(f.gidx); dfree(f.vd); dfree(f.vw); dfree(f.vX);
+  for (double** q : {&f.snap.x, &f.snap.y, &f.snap.z, &f.snap.vx, &f.snap.vy, &f.snap.vz, &f.slot, &f.a4, &f.fac,
+                     &f.ux, &f.uy, &f.vX, &f.vS})
+    dfree(*q);
+  for (int** q : {&f.gstart, &f.gidx, &f.vd, &f.pidx, &f.st1, &f.st2, &f.st3}) dfree(*q);
+  dfree(f.pre);
+  dfree(f.bands);
+  dfree(f.patch.hdr);
+  dfree(f.patch.blob);
+  f.patch = PatchPlan{};
 }
 
 // per-vertex force slots in the order force_calculate_dt adds the terms:
 // slots 4i..4i+3 of edge i (l1 WLC, l1 POW, l2 WLC, l2 POW), 9 per triangle
-// after 4E (alpha, alphad per corner, then the three volume terms), 4 per
-// dihedral after 4E+9T (l1, l4, l2, l3)
+// after 4E (the area pair per corner, then the three volume terms), 4 per
+// dihedral after 4E+9T (l1, l4, l2, l3).  A vertex's entries: both slots of
+// each edge; the first slot of its corner and the volume slot of each
+// triangle; the slot of each dihedral; gstart[3 v + k] is where kind k starts.
 void build_gather(const HostMesh& M, const std::vector<int>& start, const std::vector<int>& inc,
                   std::vector<int>& gstart, std::vector<int>& gidx) {
   const int base_t = 4 * M.ne, base_d = 4 * M.ne + 9 * M.nt;
-  gstart.assign(M.nv + 1, 0);
+  gstart.assign(3 * (size_t)M.nv + 1, 0);
   gidx.clear();
   for (int v = 0; v < M.nv; ++v) {
-    gstart[v] = (int)gidx.size();
-    for (int q = start[v]; q < start[v + 1]; ++q) {
-      int e = inc[q];
-      int kind = (e >> 30) & 3, role = (e >> 27) & 7, item = e & ((1 << 27) - 1);
-      if (kind == 0) {
-        gidx.push_back(4 * item + 2 * role);
-        gidx.push_back(4 * item + 2 * role + 1);
-      } else if (kind == 1) {
-        gidx.push_back(base_t + 9 * item + 2 * role);
-        gidx.push_back(base_t + 9 * item + 2 * role + 1);
-        gidx.push_back(base_t + 9 * item + 6 + role);
-      } else {
-        gidx.push_back(base_d + 4 * item + role);
+    int q = start[v];
+    for (int k = 0; k < 3; ++k) {
+      gstart[3 * (size_t)v + k] = (int)gidx.size();
+      for (; q < start[v + 1] && ((inc[q] >> 30) & 3) == k; ++q) {
+        int e = inc[q];
+        int role = (e >> 27) & 7, item = e & ((1 << 27) - 1);
+        if (k == 0) {
+          gidx.push_back(4 * item + 2 * role);
+          gidx.push_back(4 * item + 2 * role + 1);
+        } else if (k == 1) {
+          gidx.push_back(base_t + 9 * item + 2 * role);
+          gidx.push_back(base_t + 9 * item + 6 + role);
+        } else {
+          gidx.push_back(base_d + 4 * item + role);
+        }
       }
     }
   }
-  gstart[M.nv] = (int)gidx.size();
+  gstart[3 * (size_t)M.nv] = (int)gidx.size();
+}
+
+// the vertices ordered so that every run of them is a connected patch where
+// the mesh allows it: each half of a bisection is the nearer half, by edges,
+// to a vertex far from the others; `part` weights of the runs
+void bisect(const std::vector<std::vector<int>>& nb, std::vector<int>& v, size_t lo, size_t hi,
+            const std::vector<double>& w, size_t p0, size_t p1, std::vector<size_t>& cut) {
+  if (p1 - p0 < 2) return;
+  std::vector<int> at(nb.size(), -1);
+  auto bfs = [&](int from) {
+    for (size_t q = lo; q < hi; ++q) at[v[q]] = 0;  // 0: in this set, not reached
+    std::vector<int> out;
+    size_t next = lo;
+    for (int start = from; out.size() < hi - lo;) {
+      at[start] = 1;
+      out.push_back(start);
+      for (size_t q = out.size() - 1; q < out.size(); ++q)
+        for (int u : nb[out[q]])
+          if (at[u] == 0) { at[u] = 1; out.push_back(u); }
+      while (next < hi && at[v[next]] != 0) ++next;  // a part of its own
+      if (next < hi) start = v[next];
+    }
+    for (size_t q = lo; q < hi; ++q) at[v[q]] = -1;
+    return out;
+  };
+  if (hi > lo) {
+    const int far = bfs(v[lo]).back();
+    const std::vector<int> order = bfs(far);
+    std::copy(order.begin(), order.end(), v.begin() + lo);
+  }
+  const size_t pm = (p0 + p1) / 2;
+  double wl = 0, wa = 0;
+  for (size_t q = p0; q < p1; ++q) { wa += w[q]; if (q < pm) wl += w[q]; }
+  const size_t mid = lo + (size_t)std::llround((double)(hi - lo) * (wa > 0 ? wl / wa : 0.5));
+  cut[pm] = mid;
+  bisect(nb, v, lo, mid, w, p0, pm, cut);
+  bisect(nb, v, mid, hi, w, pm, p1, cut);
+}
+
+// The mesh split into patches for a cluster of nc blocks, the tables of each
+// block (segment.cuh) in `blob`.  Returns false when a block would not hold
+// its patch.  own: the vertices in patch order.
+bool build_patches(const HostMesh& M, const std::vector<int>& start, const std::vector<int>& inc, int nc, bool tree,
+                   PatchPlan& P, std::vector<PatchHdr>& hdr, std::vector<unsigned char>& blob, std::vector<int>& own) {
+  // The summing warps: in reference order the sums take half of two blocks'
+  // warps, the warp tree one of four (the others for the tail); those blocks'
+  // patches are smaller by as much (and by the room that many terms take).
+  P = PatchPlan{};
+  P.nc = nc;
+  P.sw = tree ? 4 : 8;
+  std::vector<double> w(nc, 1.0);
+  w[0] = w[1] = tree && M.nt <= 2048 ? 0.85 : 0.5;
+  std::vector<std::vector<int>> nb(M.nv);
+  for (int i = 0; i < M.ne; ++i) { nb[M.e1[i]].push_back(M.e2[i]); nb[M.e2[i]].push_back(M.e1[i]); }
+  own.resize(M.nv);
+  for (int v = 0; v < M.nv; ++v) own[v] = v;
+  std::vector<size_t> cut(nc + 1, 0);
+  cut[nc] = M.nv;
+  bisect(nb, own, 0, M.nv, w, 0, nc, cut);
+  std::vector<int> place(M.nv), owner(M.nv);
+  for (int b = 0; b < nc; ++b) {
+    for (size_t q = cut[b]; q < cut[b + 1]; ++q) { place[own[q]] = (int)(q - cut[b]); owner[own[q]] = b; }
+    if (cut[b + 1] - cut[b] > (size_t)kPatchOwn) return false;
+  }
+  hdr.assign(nc, PatchHdr{});
+  blob.clear();
+  struct Tables {
+    std::vector<PatchTri> tri;
+    std::vector<PatchEdge> edge;
+    std::vector<PatchDih> dih;
+    std::vector<unsigned short> ent, eend;
+    std::vector<PatchSend> send;
+  };
+  std::vector<Tables> tab(nc);
+  for (int b = 0; b < nc; ++b) {
+    PatchHdr& h = hdr[b];
+    Tables& t = tab[b];
+    h.base = (int)cut[b];
+    h.no = (int)(cut[b + 1] - cut[b]);
+    std::vector<int> slot(M.nv, -1), it(M.ne, -1), itt(M.nt, -1), itd(M.ne, -1);
+    int nl = h.no;
+    auto local = [&](int v) -> unsigned short {
+      if (owner[v] == b) return (unsigned short)place[v];
+      if (slot[v] < 0) {
+        slot[v] = nl++;
+        tab[owner[v]].send.push_back({(unsigned short)place[v], (unsigned short)slot[v], (unsigned short)b, 0});
+      }
+      return (unsigned short)slot[v];
+    };
+    int ne = 0, nt = 0, nd = 0;
+    for (int q = 0; q < h.no; ++q) {
+      const int v = own[cut[b] + q];
+      t.ent.push_back((unsigned short)ne);
+      t.ent.push_back((unsigned short)nt);
+      t.ent.push_back((unsigned short)nd);
+      for (int u = start[v]; u < start[v + 1]; ++u) {
+        const int e = inc[u], kind = (e >> 30) & 3, role = (e >> 27) & 7, item = e & ((1 << 27) - 1);
+        if (kind == 0) {
+          if (it[item] < 0) {
+            it[item] = (int)t.edge.size();
+            t.edge.push_back({{local(M.e1[item]), local(M.e2[item])}, {0, 0}, M.l0[item], M.kappap[item]});
+          }
+          t.eend.push_back((unsigned short)(2 * it[item] + role));
+          ++ne;
+        } else if (kind == 1) {
+          if (itt[item] < 0) {
+            itt[item] = (int)t.tri.size();
+            t.tri.push_back({{local(M.t1[item]), local(M.t2[item]), local(M.t3[item])}, {kNoEntry, kNoEntry, kNoEntry},
+                             owner[M.t1[item]] == b ? item : -1, M.tarea[item]});
+          }
+          t.tri[itt[item]].d[role] = (unsigned short)nt++;
+        } else {
+          if (itd[item] < 0) {
+            int l2, l3;
+            if (M.iedge[item] == -1) { l3 = M.e1[item]; l2 = M.e2[item]; } else { l2 = M.e1[item]; l3 = M.e2[item]; }
+            itd[item] = (int)t.dih.size();
+            t.dih.push_back({{local(M.es1[item]), local(M.es2[item]), local(l2), local(l3)},
+                             {kNoEntry, kNoEntry, kNoEntry, kNoEntry}});
+          }
+          t.dih[itd[item]].d[role] = (unsigned short)nd++;
+        }
+      }
+    }
+    for (int q : {ne, nt, nd}) t.ent.push_back((unsigned short)q);
+    if (std::max({nl, 2 * (int)t.edge.size(), nt, nd}) >= kNoEntry) return false;
+    h.nl = nl; h.ntri = (int)t.tri.size(); h.ned = (int)t.edge.size(); h.ndih = (int)t.dih.size();
+    h.ne = ne; h.nt = nt; h.nd = nd;
+    P.nl = std::max(P.nl, nl);
+  }
+  for (int b = 0; b < nc; ++b) {
+    PatchHdr& h = hdr[b];
+    const Tables& t = tab[b];
+    h.nsend = (int)t.send.size();
+    h.blob = (int)blob.size();
+    auto put = [&](const void* d, size_t bytes) {
+      const int at = (int)blob.size() - h.blob;
+      blob.insert(blob.end(), (const unsigned char*)d, (const unsigned char*)d + bytes);
+      blob.resize((blob.size() + 15) / 16 * 16);
+      return at;
+    };
+    h.own = put(own.data() + cut[b], sizeof(int) * h.no);
+    h.tri = put(t.tri.data(), sizeof(PatchTri) * t.tri.size());
+    h.edge = put(t.edge.data(), sizeof(PatchEdge) * t.edge.size());
+    h.dih = put(t.dih.data(), sizeof(PatchDih) * t.dih.size());
+    h.ent = put(t.ent.data(), sizeof(unsigned short) * t.ent.size());
+    h.eend = put(t.eend.data(), sizeof(unsigned short) * t.eend.size());
+    h.send = put(t.send.data(), sizeof(PatchSend) * t.send.size());
+    h.bytes = (int)blob.size() - h.blob;
+  }
+  patch_layout(P, hdr.data(), M.nt);
+  return P.smem <= kSegSmemMax;
+}
+
+// the patches of the handle's mesh and membrane form; without them (one or
+// eight blocks asked for, or a mesh that does not fit) the snapshots keep the
+// vertices' order
+int upload_patches(irbc_handle* h) {
+  FastBufs& f = h->fb;
+  const HostMesh& M = h->host_mesh;
+  dfree(f.patch.hdr);
+  dfree(f.patch.blob);
+  f.patch = PatchPlan{};
+  std::vector<int> start, inc, own(M.nv);
+  for (int v = 0; v < M.nv; ++v) own[v] = v;
+  if (h->mem_mode == 1) {
+    build_incidence(M, start, inc);
+    // eight blocks, or sixteen (a non-portable size) where eight do not hold
+    // their patches and the device can run such a cluster.  Fewer blocks than
+    // eight take two rounds of items a phase: 21 against 15 us a step on the
+    // 600-vertex mesh with four
+    for (int nc : {8, 16}) {
+      PatchPlan P;
+      std::vector<PatchHdr> hdr;
+      std::vector<unsigned char> blob;
+      std::vector<int> order;
+      if (!build_patches(M, start, inc, nc, h->dp.tree_sums != 0, P, hdr, blob, order)) continue;
+      if (!cluster_fits(nc, P.smem)) continue;
+      CK(dalloc(&P.hdr, nc));
+      CK(dalloc(&P.blob, (int64_t)blob.size()));
+      if (up(h, P.hdr, hdr) || up(h, P.blob, blob)) return IRBC_ERR_CUDA;
+      f.patch = P;
+      own = order;
+      break;
+    }
+  }
+  std::vector<int> place(M.nv), c1(M.nt), c2(M.nt), c3(M.nt);
+  for (int q = 0; q < M.nv; ++q) place[own[q]] = q;
+  for (int j = 0; j < M.nt; ++j) { c1[j] = place[M.t1[j]]; c2[j] = place[M.t2[j]]; c3[j] = place[M.t3[j]]; }
+  if (up(h, f.pidx, place) || up(h, f.st1, c1) || up(h, f.st2, c2) || up(h, f.st3, c3)) return IRBC_ERR_CUDA;
+  CK(cudaStreamSynchronize(h->st));  // the copies' sources are local
+  return 0;
 }
 
 void invalidate_graphs(irbc_handle* h);
@@ -339,7 +538,6 @@ int upload_mesh(irbc_handle* h, const HostMesh& M) {
   invalidate_graphs(h);
   free_membrane(m);
   free_fast(h->fb);
-  h->snap_ready = false;
   m.nv = M.nv; m.ne = M.ne; m.nt = M.nt;
   for (double** p : {&m.x, &m.y, &m.z, &m.vx, &m.vy, &m.vz, &m.fx, &m.fy, &m.fz, &m.poff, &m.pon})
     CK(dalloc(p, M.nv));
@@ -358,19 +556,24 @@ int upload_mesh(irbc_handle* h, const HostMesh& M) {
   if (up(h, m.inc_start, start) || up(h, m.inc, inc)) return IRBC_ERR_CUDA;
   {
     FastBufs& f = h->fb;
-    for (int b = 0; b < 2; ++b) {
-      for (double** q : {&f.snap[b].x, &f.snap[b].y, &f.snap[b].z, &f.snap[b].vx, &f.snap[b].vy, &f.snap[b].vz})
-        CK(dalloc(q, M.nv));
-      CK(dalloc(&f.pre[b], M.nt));
-      f.snap[b].t1 = m.t1; f.snap[b].t2 = m.t2; f.snap[b].t3 = m.t3;
-    }
+    for (double** q : {&f.snap.x, &f.snap.y, &f.snap.z, &f.snap.vx, &f.snap.vy, &f.snap.vz})
+      CK(dalloc(q, (int64_t)kSegMax * M.nv));
+    CK(dalloc(&f.pre, (int64_t)kSegMax * M.nt));
+    CK(dalloc(&f.bands, (int64_t)kSegMax * M.nt));
+    CK(dalloc(&f.pidx, M.nv));
+    for (int** q : {&f.st1, &f.st2, &f.st3}) CK(dalloc(q, M.nt));
+    f.snap.t1 = f.st1; f.snap.t2 = f.st2; f.snap.t3 = f.st3;
     std::vector<int> gstart, gidx;
     build_gather(M, start, inc, gstart, gidx);
     CK(dalloc(&f.slot, 3 * (int64_t)(8 * M.ne + 9 * M.nt)));
-    CK(dalloc(&f.gstart, M.nv + 1));
+    CK(dalloc(&f.a4, M.nt));
+    CK(dalloc(&f.fac, 2));
+    CK(dalloc(&f.ux, M.nv));
+    CK(dalloc(&f.uy, M.nv));
+    CK(dalloc(&f.vS, 3 * (int64_t)M.nv));
+    CK(dalloc(&f.gstart, 3 * (int64_t)M.nv + 1));
     CK(dalloc(&f.gidx, (int64_t)gidx.size()));
     CK(dalloc(&f.vd, M.nv));
-    CK(dalloc(&f.vw, M.nv));
     CK(dalloc(&f.vX, 3 * (int64_t)M.nv));
     if (up(h, f.gstart, gstart) || up(h, f.gidx, gidx)) return IRBC_ERR_CUDA;
   }
@@ -385,9 +588,12 @@ int upload_mesh(irbc_handle* h, const HostMesh& M) {
   // does inside its bending loop (Src/memfuncs.cpp:401)
   h->dp.cth0 = cos(M.theta0 * h->P.Pi / 180.0);
   h->dp.sth0 = sin(M.theta0 * h->P.Pi / 180.0);
-  h->have_mesh = true;
+  h->host_mesh = M;
   h->fb.one_block = h->mem_mode == 2 && one_block_fits(h->dp);
   h->fb.cluster = h->mem_mode == 3;
+  const int rc = upload_patches(h);
+  if (rc) return rc;
+  h->have_mesh = true;
   return 0;
 }
 
@@ -486,18 +692,17 @@ struct ProfScope {
 // the streaming kernels; in a profiling window the bulk kernel alone is
 // bracketed by a pair of events of its own
 // returns the number of kernels it launched
-int stream_any(irbc_handle* h, int buf, cudaStream_t st, cudaEvent_t snap = nullptr) {
+int stream_any(irbc_handle* h, int H, cudaStream_t st, cudaEvent_t snap = nullptr) {
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (h->prof && !h->capturing) {
     h->ev_marks.push_back({PROF_STREAM_BULK, h->ev_used, h->ev_used + 1});
     e0 = next_event(h);
     e1 = next_event(h);
   }
-  // the staging capacity follows the longest list; captured steps keep the
-  // largest, so that a replay stays valid after the lists grow
+  // the capacity follows the longest list; captured steps keep the largest, so
+  // that a replay stays valid after the lists grow
   h->fb.hcap = (h->graphs_on || h->capturing) ? kHeavyList : heavy_cap(h->c.lmax);
-  if (h->fp32) return fast_stream_f(h->dp, h->sf, h->c, h->fb, buf, st, e0, e1, snap);
-  return fast_stream(h->dp, h->s, h->c, h->fb, buf, st, e0, e1, snap);
+  return fast_stream(h->dp, h->s, h->fp32 ? &h->sf : nullptr, h->c, h->fb, H, st, e0, e1, snap);
 }
 
 }  // namespace
@@ -520,10 +725,11 @@ extern "C" int64_t irbc_footprint_bytes(const irbc_params* p, int32_t nv, int32_
   int64_t nx = (int64_t)(p->Lx / p->a), ny = (int64_t)(p->Ly / p->a), nz = (int64_t)(p->Lz / p->a) + 1;
   int64_t C = nx * ny * nz;
   int64_t ns = p->Ns;
-  int64_t b = ns * (2 * (3 * 8 + 32 + 2 * 4) + 4 * 4);  // two buffer sets + key/slot/perm/stream queue
+  int64_t b = ns * (2 * (3 * 8 + 32 + 2 * 4) + 4 * 4 + 1);  // two buffer sets + key/slot/perm/stream queue
   if (p->precision == IRBC_FP32) b += ns * (2 * 32 + 2 * 4);  // float4 sets + cell ids
-  b += C * (7 * 4) + (C + 1) * 4 * 3;                // cell counts/ranks + cell and llist starts
+  b += C * (7 * 4 + 1) + (C + 1) * 4 * 3;            // cell counts/ranks/flags + cell and llist starts
   b += (int64_t)nv * (12 * 8 + 8 * 4 + kMaxPairs * 12) + (int64_t)ne * 40 + (int64_t)nt * 80;
+  b += kSegMax * ((int64_t)nv * 48 + (int64_t)nt * 97);  // a stretch's snapshots and triangle records
   b += 2 * (int64_t)(4 * p->Lx * 4 * p->Ly) * 16;    // ligands
   b += 2 * C * 4 * 8;                                 // llist entries (typical)
   return b;
@@ -569,8 +775,7 @@ extern "C" int irbc_create(const irbc_params* p, irbc_handle** out) {
       return IRBC_ERR_CUDA;
     }
     h->st2_own = h->st2;
-    for (cudaEvent_t* e : {&h->ev_snap, &h->ev_mem, &h->ev_coll, &h->ev_str[0], &h->ev_str[1], &h->ev_vbin,
-                           &h->ev_health})
+    for (cudaEvent_t* e : {&h->ev_mem, &h->ev_coll, &h->ev_vbin, &h->ev_health})
       cudaEventCreateWithFlags(e, cudaEventDisableTiming);
   }
   {
@@ -616,6 +821,8 @@ extern "C" int irbc_create(const irbc_params* p, irbc_handle** out) {
   h->dp.health = h->health;
   A(cudaHostAlloc((void**)&h->health_host, sizeof(int), cudaHostAllocDefault));
   A(dalloc(&h->fb.queue, s.n));
+  A(dalloc(&h->fb.qk, s.n));
+  A(dalloc(&c.flag, c.n));
   A(dalloc(&h->fb.qn, 4));
   if (p->precision == IRBC_FP32) {
     h->fp32 = true;
@@ -626,6 +833,7 @@ extern "C" int irbc_create(const irbc_params* p, irbc_handle** out) {
   }
   if (rc) { irbc_destroy(h); return create_failed(rc, "device allocation"); }
   cudaMemsetAsync(c.lstart, 0, sizeof(int) * (c.n + 1), h->st);
+  cudaMemsetAsync(c.flag, 2, c.n, h->st);
   cudaMemsetAsync(h->m.ligi, 0, sizeof(int) * h->dp.nlig, h->st);
   cudaMemsetAsync(h->m.sc, 0, sizeof(MemScalars), h->st);
   cudaMemsetAsync(h->ebase, 0, sizeof(uint64_t), h->st);
@@ -648,12 +856,12 @@ extern "C" void irbc_destroy(irbc_handle* h) {
   if (h->st2_own) cudaStreamSynchronize(h->st2_own);
   invalidate_graphs(h);
   free_fast(h->fb);
-  dfree(h->fb.queue); dfree(h->fb.qn); dfree(h->fb.bcnt); dfree(h->fb.bucket); dfree(h->fb.border);
+  dfree(h->fb.queue); dfree(h->fb.qk); dfree(h->c.flag); dfree(h->fb.qn); dfree(h->fb.bcnt); dfree(h->fb.bucket); dfree(h->fb.border);
   dfree(h->fb.arng);
   if (h->rec) cudaFree(h->rec);
   for (float4** q : {&h->sf.pos, &h->sf.vel, &h->sf.pos2, &h->sf.vel2}) dfree(*q);
   dfree(h->sf.pid); dfree(h->sf.pid2);
-  for (cudaEvent_t e : {h->ev_snap, h->ev_mem, h->ev_coll, h->ev_str[0], h->ev_str[1], h->ev_vbin, h->ev_health})
+  for (cudaEvent_t e : {h->ev_mem, h->ev_coll, h->ev_vbin, h->ev_health})
     if (e) cudaEventDestroy(e);
   dfree(h->health);
   if (h->health_host) cudaFreeHost(h->health_host);
@@ -1126,9 +1334,8 @@ extern "C" int irbc_collide(irbc_handle* h, int64_t epoch) {
 }
 extern "C" int irbc_stream(irbc_handle* h) {
   if (!h || !h->have_mesh) return IRBC_ERR_ARG;
-  fast_snap_prep(h->dp, h->m, h->fb, 0, h->st);
-  g_launches += 2 + stream_any(h, 0, h->st);
-  h->snap_ready = false;
+  fast_snap_prep(h->dp, h->m, h->fb, h->st);
+  g_launches += 2 + stream_any(h, 1, h->st);
   CK(cudaGetLastError());
   return 0;
 }
@@ -1177,25 +1384,19 @@ extern "C" int irbc_step_part1(irbc_handle* h) {
     g_launches += collide_any(h, 0, h->st);
     h->colsteps = 0;
   }
-  const int buf = (int)(s & 1);
-  {
-    ProfScope ps(h, PROF_MEMBRANE);
-    g_launches += fast_kick_prep(h->dp, h->m, h->fb, buf, h->st);
-  }
   if (h->upd == h->uplist) {
     int rc = do_llist(h);
     if (rc) return rc;
     h->upd = 0;
   }
   {
-    ProfScope ps(h, PROF_STREAM);
-    g_launches += stream_any(h, buf, h->st);
+    ProfScope ps(h, PROF_MEMBRANE);
+    g_launches += launch_membrane(h->dp, h->m, h->fb, 0, 1, SEG_FIRST, h->st);
   }
   {
-    ProfScope ps(h, PROF_MEMBRANE);
-    g_launches += fast_drift_va(h->dp, h->m, h->st, true);
+    ProfScope ps(h, PROF_STREAM);
+    g_launches += stream_any(h, 1, h->st);
   }
-  h->snap_ready = false;
   CK(cudaGetLastError());
   return 0;
 }
@@ -1208,7 +1409,7 @@ extern "C" int irbc_step_part2(irbc_handle* h) {
   CK(set_epoch_base(h, (uint64_t)s));
   {
     ProfScope ps(h, PROF_MEMBRANE);
-    g_launches += fast_forces_tail(h->dp, h->m, h->fb, 0, 0, (int)((s + 1) & 1), h->st, false);
+    g_launches += launch_membrane(h->dp, h->m, h->fb, 0, 1, SEG_SECOND, h->st);
   }
   if (h->filecc == h->P.out_every) { h->filec += 1; h->filecc = 0; }
   h->step = s + 1;
@@ -1216,79 +1417,84 @@ extern "C" int irbc_step_part2(irbc_handle* h) {
   return 0;
 }
 
-// One timestep of the pipelined schedule: step s streams the solvent
-// (h->st) while the membrane drifts, computes forces and bonds for s and
-// prepares the snapshot of s+1 (h->st2).  Collisions, llist updates and the
-// snapshot buffers (two, by step parity) are ordered by events.  eoff is the
-// step's draw-epoch offset from the current base; last: the step ends a
-// call or a captured sequence (the next step's half-kick is not fused into
-// this one).  dry: advance the host counters only (the launches are in a
-// captured sequence being replayed).
-static int step_one(irbc_handle* h, int64_t eoff, bool last, bool dry) {
+// the counters of the reference's loop at the start of a timestep
+// (maincode.cpp:463-479); whether it collides
+static bool step_begins(irbc_handle* h) {
   const irbc_params& p = h->P;
-  cudaStream_t ms = h->st, ss = h->st2;
-  const int64_t s = h->step;
-  h->dp.wallspeed = (s < p.warm_steps) ? p.warm_speed : p.walls;
+  h->dp.wallspeed = (h->step < p.warm_steps) ? p.warm_speed : p.walls;
   h->colsteps += 1; h->bbi += 1; h->upd += 1;
-  if (s > 0) h->filecc += 1;
-  const int buf = (int)(s & 1);
-  if (h->colsteps == h->csteps) {
+  if (h->step > 0) h->filecc += 1;
+  if (h->colsteps != h->csteps) return false;
+  h->colsteps = 0;
+  return true;
+}
+// ... and at its end
+static void step_ends(irbc_handle* h) {
+  if (h->filecc == h->P.out_every) { h->filec += 1; h->filecc = 0; }
+  h->step += 1;
+}
+
+// the steps of the stretch that has begun at h->step: up to the next
+// collision, list update, change of the wall speed or kSegMax
+static int64_t stretch_steps(const irbc_handle* h, int64_t left) {
+  int64_t H = std::min<int64_t>(left, kSegMax);
+  const int64_t coll = (int64_t)h->csteps - h->colsteps, list = (int64_t)h->uplist - h->upd;
+  const int64_t warm = h->P.warm_steps - h->step;
+  if (coll > 0) H = std::min(H, coll);
+  if (list > 0) H = std::min(H, list);
+  if (warm > 0) H = std::min(H, warm);
+  return H;
+}
+
+// A stretch of timesteps: a collision and a list update when its first step
+// has them, then the membrane of all its steps in one launch on the side
+// stream (h->st2) and the streaming of each step on the main one (h->st).
+// Between two collisions the membrane does not depend on the solvent, so it
+// runs ahead.  eoff is the first step's draw-epoch offset from the current
+// base; at most `left` steps.  dry: advance the host counters only (the
+// launches are in a captured sequence being replayed).  Returns the steps
+// taken, negative on an error.
+static int64_t stretch(irbc_handle* h, int64_t eoff, int64_t left, bool dry) {
+  cudaStream_t ms = h->st, ss = h->st2;
+  if (step_begins(h)) {
     if (dry) {
       h->s.ncoll += 1;
     } else {
-      {
-        ProfScope ps(h, PROF_COLLIDE, ms);
-        g_launches += collide_any(h, (uint64_t)eoff, ms, ss);
-      }
-      CK(cudaEventRecord(h->ev_coll, ms));
-      CK(cudaStreamWaitEvent(ss, h->ev_coll, 0));
+      ProfScope ps(h, PROF_COLLIDE, ms);
+      g_launches += collide_any(h, (uint64_t)eoff, ms, ss);
     }
-    h->colsteps = 0;
-    h->snap_ready = false;
-  }
-  if (!h->snap_ready && !dry) {
-    CK(cudaStreamWaitEvent(ss, h->ev_str[buf], 0));
-    ProfScope ps(h, PROF_MEMBRANE, ss);
-    g_launches += fast_kick_prep(h->dp, h->m, h->fb, buf, ss);
   }
   if (h->upd == h->uplist) {
-    // never inside a captured sequence.  Positions of step s are final once
-    // the side stream reaches here; its drift of step s waits for the update
-    CK(cudaEventRecord(h->ev_snap, ss));
-    CK(cudaStreamWaitEvent(ms, h->ev_snap, 0));
+    // never inside a captured sequence; the membrane's positions are those
+    // of the side stream's last launch
+    CK(cudaStreamWaitEvent(ms, h->ev_mem, 0));
     int rc = do_llist(h);
     if (rc) return rc;
     h->upd = 0;
+  }
+  const int64_t H = stretch_steps(h, left);
+  if (!dry) {
+    // the membrane follows the collision (which rotates vertex velocities)
+    // and the streaming that last read the snapshots
     CK(cudaEventRecord(h->ev_coll, ms));
     CK(cudaStreamWaitEvent(ss, h->ev_coll, 0));
-  }
-  // the next step's snapshot goes to the other buffer, read by the
-  // previous step's streaming
-  const bool next_collides = (h->colsteps + 1 == h->csteps);
-  const int next_kick = (!last && !next_collides) ? 1 : 0;
-  if (!dry) {
-    // The streams meet only where they share data.  The bulk streaming
-    // kernel reads no membrane data and starts at once; the near-membrane
-    // kernel waits for the snapshot `buf` (ev_snap: the side stream so far).
-    // The membrane step runs on, and only its writing of the next snapshot
-    // (buf ^ 1) waits for the streaming that last read that buffer.
-    CK(cudaEventRecord(h->ev_snap, ss));
-    {
-      ProfScope ps(h, PROF_STREAM, ms);
-      g_launches += stream_any(h, buf, ms, h->ev_snap);
-    }
-    CK(cudaEventRecord(h->ev_str[buf], ms));
     {
       ProfScope ps(h, PROF_MEMBRANE, ss);
-      g_launches += fast_membrane_step(h->dp, h->m, h->fb, (uint64_t)eoff, next_kick, buf ^ 1, ss,
-                                       h->ev_str[buf ^ 1]);
+      g_launches += launch_membrane(h->dp, h->m, h->fb, (uint64_t)eoff, (int)H, SEG_WHOLE, ss);
     }
     CK(cudaEventRecord(h->ev_mem, ss));
+    {
+      // the bulk streaming reads no membrane data and starts at once
+      ProfScope ps(h, PROF_STREAM, ms);
+      g_launches += stream_any(h, (int)H, ms, h->ev_mem);
+    }
   }
-  h->snap_ready = next_kick != 0;
-  if (h->filecc == p.out_every) { h->filec += 1; h->filecc = 0; }
-  h->step = s + 1;
-  return 0;
+  step_ends(h);
+  for (int64_t k = 1; k < H; ++k) {
+    step_begins(h);
+    step_ends(h);
+  }
+  return H;
 }
 
 constexpr int kGraphSteps = 24;  // two collision cycles per captured sequence
@@ -1297,7 +1503,7 @@ constexpr int kGraphSteps = 24;  // two collision cycles per captured sequence
 // (whose records belong to the graph) and after each graph launch, so that
 // later waits refer to work outside any graph and follow the launch
 static cudaError_t rearm_events(irbc_handle* h) {
-  for (cudaEvent_t e : {h->ev_str[0], h->ev_str[1], h->ev_snap, h->ev_mem, h->ev_coll, h->ev_vbin}) {
+  for (cudaEvent_t e : {h->ev_mem, h->ev_coll, h->ev_vbin}) {
     cudaError_t r = cudaEventRecord(e, h->st);
     if (r != cudaSuccess) return r;
   }
@@ -1305,10 +1511,9 @@ static cudaError_t rearm_events(irbc_handle* h) {
 }
 
 // a captured sequence can stand for the next kGraphSteps steps when no list
-// update falls inside them, the wall speed is the same throughout, and the
-// previous step did not fuse this step's half-kick
+// update falls inside them and the wall speed is the same throughout
 static bool graph_fits(const irbc_handle* h, int64_t remaining) {
-  if (!h->graphs_on || remaining < kGraphSteps || h->snap_ready) return false;
+  if (!h->graphs_on || remaining < kGraphSteps) return false;
   if (h->upd + kGraphSteps >= h->uplist) return false;
   const int64_t s = h->step, w = h->P.warm_steps;
   return (s + kGraphSteps <= w) || (s >= w);
@@ -1318,29 +1523,27 @@ static bool graph_fits(const irbc_handle* h, int64_t remaining) {
 // host counters are left where they were
 static irbc_handle::StepGraph* graph_for(irbc_handle* h) {
   const double ws = (h->step < h->P.warm_steps) ? h->P.warm_speed : h->P.walls;
-  const int parity = (int)(h->step & 1);
   for (auto& g : h->graphs)
-    if (g.colsteps0 == h->colsteps && g.parity == parity && g.wallspeed == ws) return &g;
+    if (g.colsteps0 == h->colsteps && g.wallspeed == ws) return &g;
   cudaStream_t ms = h->st, ss = h->st2;
   // counters to restore after the capture
   const int64_t step = h->step, ncoll = h->s.ncoll, resorted = h->s.resorted;
   const int colsteps = h->colsteps, bbi = h->bbi, upd = h->upd, filecc = h->filecc, filec = h->filec;
-  const bool snap = h->snap_ready;
   const double wsp = h->dp.wallspeed;
   const int64_t l0 = g_launches.load();
   h->capturing = true;
   cudaGraph_t graph = nullptr;
   bool ok = cudaStreamBeginCapture(ms, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
-  int rc = 0;
   if (ok) {
     // every event the steps wait on is first recorded inside the capture,
     // so no wait reaches outside it; then the side stream forks off
-    for (cudaEvent_t e : {h->ev_str[0], h->ev_str[1], h->ev_snap, h->ev_mem, h->ev_coll})
+    for (cudaEvent_t e : {h->ev_mem, h->ev_coll})
       ok = ok && cudaEventRecord(e, ms) == cudaSuccess;
     ok = ok && cudaStreamWaitEvent(ss, h->ev_coll, 0) == cudaSuccess;
-    for (int k = 0; ok && k < kGraphSteps; ++k) {
-      rc = step_one(h, k, k == kGraphSteps - 1, false);
-      ok = rc == 0;
+    for (int64_t k = 0; ok && k < kGraphSteps;) {
+      const int64_t took = stretch(h, k, kGraphSteps - k, false);
+      ok = took > 0;
+      k += took;
     }
     if (ok) ok = cudaStreamWaitEvent(ms, h->ev_mem, 0) == cudaSuccess;
     cudaError_t e = cudaStreamEndCapture(ms, &graph);
@@ -1354,7 +1557,7 @@ static irbc_handle::StepGraph* graph_for(irbc_handle* h) {
   g_launches -= launches;
   h->step = step; h->s.ncoll = ncoll; h->s.resorted = resorted;
   h->colsteps = colsteps; h->bbi = bbi; h->upd = upd; h->filecc = filecc; h->filec = filec;
-  h->snap_ready = snap; h->dp.wallspeed = wsp;
+  h->dp.wallspeed = wsp;
   if (ok) {
     // the side stream's priority does not travel into the graph by itself:
     // give the membrane chain's kernel nodes the high priority explicitly
@@ -1386,7 +1589,7 @@ static irbc_handle::StepGraph* graph_for(irbc_handle* h) {
     return nullptr;
   }
   irbc_handle::StepGraph g;
-  g.exec = exec; g.colsteps0 = colsteps; g.parity = parity; g.wallspeed = ws;
+  g.exec = exec; g.colsteps0 = colsteps; g.wallspeed = ws;
   g.launches = launches; g.collisions = collisions;
   h->graphs.push_back(g);
   return &h->graphs.back();
@@ -1419,7 +1622,7 @@ extern "C" int irbc_step(irbc_handle* h, int64_t n) {
         CK(set_epoch_base(h, (uint64_t)h->step));
         CK(cudaGraphLaunch(g->exec, ms));
         g_launches += g->launches;
-        for (int j = 0; j < kGraphSteps; ++j) step_one(h, j, j == kGraphSteps - 1, true);
+        for (int64_t j = 0; j < kGraphSteps;) j += stretch(h, j, kGraphSteps - j, true);
         if (h->s.ncoll - h->s.resorted >= kResortEvery) g_launches += resort_any(h, ms);
         CK(rearm_events(h));
         CK(cudaStreamWaitEvent(ss, h->ev_coll, 0));
@@ -1427,11 +1630,9 @@ extern "C" int irbc_step(irbc_handle* h, int64_t n) {
         continue;
       }
     }
-    // a plain step; the step before a collision never fuses the next
-    // half-kick, so captured sequences start at collision steps
-    int rc = step_one(h, h->step - h->ebase_val, k == n - 1, false);
-    if (rc) return rc;
-    k += 1;
+    const int64_t took = stretch(h, h->step - h->ebase_val, n - k, false);
+    if (took < 0) return (int)took;
+    k += took;
   }
   CK(cudaStreamWaitEvent(ms, h->ev_mem, 0));
   CK(cudaMemcpyAsync(h->health_host, h->health, sizeof(int), cudaMemcpyDeviceToHost, ms));
@@ -1462,9 +1663,10 @@ extern "C" int irbc_set_membrane_kernels(irbc_handle* h, int32_t mode) {
   if (h->have_mesh) {
     const bool ob = mode == 2, cl = mode == 3;
     if (ob && !one_block_fits(h->dp)) return fail(h, IRBC_ERR_CAPACITY, "mesh too large for the one-block membrane step");
-    if (ob != h->fb.one_block || cl != h->fb.cluster) invalidate_graphs(h);
+    invalidate_graphs(h);
     h->fb.one_block = ob;
     h->fb.cluster = cl;
+    return upload_patches(h);
   }
   return 0;
 }
@@ -1482,8 +1684,7 @@ namespace irbc {
 struct Cohort {
   int device = 0;
   cudaStream_t ms = nullptr, ss = nullptr;  // solvent phases / membrane phases, as a handle's two streams
-  cudaEvent_t ev_snap = nullptr, ev_mem = nullptr, ev_coll = nullptr, ev_str[2] = {nullptr, nullptr};
-  cudaEvent_t ev_join = nullptr;
+  cudaEvent_t ev_mem = nullptr, ev_coll = nullptr, ev_join = nullptr;
   MultiPlan plan;                       // device tables of `members`
   std::vector<irbc_handle*> members;    // the plan's members, in order
   std::vector<uint64_t> uids;           // their handles' unique ids
@@ -1491,6 +1692,7 @@ struct Cohort {
   size_t cap = 0;                       // members the device tables have room for
   size_t tab_cap = 0;                   // block-table entries they have room for
   int64_t ncoll = 0;                    // collisions of this cohort: a physical re-sort every kResortEvery
+  int64_t stretches = 0;                // stretches taken: their parity picks the members' queue counter
   bool ok = false;
 };
 
@@ -1502,7 +1704,7 @@ Cohort* cohort_create(int device) {
   cudaDeviceGetStreamPriorityRange(&lo, &hi);
   bool ok = cudaStreamCreateWithFlags(&c->ms, cudaStreamNonBlocking) == cudaSuccess &&
             cudaStreamCreateWithPriority(&c->ss, cudaStreamNonBlocking, hi) == cudaSuccess;
-  for (cudaEvent_t* e : {&c->ev_snap, &c->ev_mem, &c->ev_coll, &c->ev_str[0], &c->ev_str[1], &c->ev_join})
+  for (cudaEvent_t* e : {&c->ev_mem, &c->ev_coll, &c->ev_join})
     ok = ok && cudaEventCreateWithFlags(e, cudaEventDisableTiming) == cudaSuccess;
   c->ok = ok;
   return c;
@@ -1513,7 +1715,7 @@ void cohort_destroy(Cohort* c) {
   cudaSetDevice(c->device);
   if (c->ms) cudaStreamSynchronize(c->ms);
   if (c->ss) cudaStreamSynchronize(c->ss);
-  for (cudaEvent_t e : {c->ev_snap, c->ev_mem, c->ev_coll, c->ev_str[0], c->ev_str[1], c->ev_join})
+  for (cudaEvent_t e : {c->ev_mem, c->ev_coll, c->ev_join})
     if (e) cudaEventDestroy(e);
   if (c->ms) cudaStreamDestroy(c->ms);
   if (c->ss) cudaStreamDestroy(c->ss);
@@ -1528,7 +1730,6 @@ int64_t cohort_key(const irbc_handle* h) {
   k = k * 4096 + h->csteps;
   k = k * 4096 + (h->colsteps + 1);
   k = k * 2 + (h->step & 1);
-  k = k * 2 + (h->snap_ready ? 1 : 0);
   return k;
 }
 
@@ -1562,23 +1763,31 @@ static int cohort_upload(Cohort* c) {
   c->uids.resize(n);
   std::vector<std::array<int, MP_NPHASE>> nbk(n);
   int64_t tot[MP_NPHASE] = {};
-  P.vbin_smem = P.sum_smem = 0;
+  P.vbin_smem = 0;
   P.cells_short = 0;
-  P.cells_cap = 1;
   std::vector<int> cls(n);  // the near-membrane class of each member: 0 short lists, 1 long lists
   for (size_t r = 0; r < n; ++r) {
     c->host[r] = member_of(c->members[r]);
     c->uids[r] = c->members[r]->uid;
-    int sm[2];
     multi_blocks(c->host[r], nbk[r].data());
-    multi_smem(c->host[r], sm);
     for (int k = 0; k < MP_NPHASE; ++k) tot[k] += nbk[r][k];
     const int hcap = c->host[r].fb.hcap;
     cls[r] = short_lists(hcap) ? 0 : 1;
     if (cls[r] == 0) P.cells_short += nbk[r][MP_CELLS];
-    else P.cells_cap = std::max(P.cells_cap, stage_cap(hcap));
-    P.vbin_smem = std::max(P.vbin_smem, sm[0]);
-    P.sum_smem = std::max(P.sum_smem, sm[1]);
+    P.vbin_smem = std::max(P.vbin_smem, multi_vbin_smem(c->host[r]));
+  }
+  // the membrane's launches: members by the size of their cluster
+  P.seg.clear();
+  std::vector<int> scls(n);
+  for (size_t r = 0; r < n; ++r) {
+    int smem = 0;
+    const int nc = multi_segment(c->host[r], &smem);
+    size_t k = 0;
+    while (k < P.seg.size() && P.seg[k].nc != nc) ++k;
+    if (k == P.seg.size()) P.seg.push_back({nc, 0, 0});
+    P.seg[k].members += 1;
+    P.seg[k].smem = std::max(P.seg[k].smem, smem);
+    scls[r] = (int)k;
   }
   // the block tables: phase by phase, member by member
   int64_t all = 0;
@@ -1591,10 +1800,13 @@ static int cohort_upload(Cohort* c) {
   std::vector<int2> tab((size_t)all);
   for (int k = 0; k < MP_NPHASE; ++k) {
     int64_t q = P.off[k];
-    // the near-membrane blocks class by class (one launch per class)
-    for (int pass = 0; pass < (k == MP_CELLS ? 2 : 1); ++pass)
+    // the near-membrane and the membrane blocks class by class (one launch
+    // per class)
+    const int classes = k == MP_CELLS ? 2 : (k == MP_MEMBRANE ? (int)P.seg.size() : 1);
+    for (int pass = 0; pass < classes; ++pass)
       for (size_t r = 0; r < n; ++r) {
         if (k == MP_CELLS && cls[r] != pass) continue;
+        if (k == MP_MEMBRANE && scls[r] != pass) continue;
         for (int b = 0; b < nbk[r][k]; ++b) tab[(size_t)q++] = make_int2((int)r, b);
       }
   }
@@ -1670,58 +1882,40 @@ int cohort_step(Cohort* c, const std::vector<irbc_handle*>& all, int64_t n, std:
     int rc = cohort_upload(c);
     if (rc) return rc;
   }
-  irbc_handle* h0 = hs[0];
-  const int csteps = h0->csteps;
-  for (int64_t k = 0; k < n; ++k) {
-    const int buf = (int)(h0->step & 1);
-    bool moved = false;
+  for (int64_t k = 0; k < n;) {
+    // a stretch of every member (as stretch()): the members collide together
+    bool moved = false, collide = false;
     for (irbc_handle* h : hs) {
-      const irbc_params& p = h->P;
-      const double ws = (h->step < p.warm_steps) ? p.warm_speed : p.walls;
-      if (ws != h->dp.wallspeed) { h->dp.wallspeed = ws; moved = true; }
-      h->colsteps += 1; h->bbi += 1; h->upd += 1;
-      if (h->step > 0) h->filecc += 1;
+      const double ws = h->dp.wallspeed;
+      collide = step_begins(h);
+      moved = moved || ws != h->dp.wallspeed;
     }
     if (moved) {
       int rc = cohort_upload(c);
       if (rc) return rc;
     }
-    const bool collide = h0->colsteps == csteps;
     if (collide) {
       c->ncoll += 1;
       const bool resort = c->ncoll % kResortEvery == 0;
       for (irbc_handle* h : hs) {
         h->s.ncoll += 1;
         if (resort) h->s.resorted = h->s.ncoll;
-        h->colsteps = 0;
-        h->snap_ready = false;
       }
       // the vertex binning reads the positions, and the tiles rotate the
-      // vertex velocities, of the previous step's membrane step (side
-      // stream): the collision waits for it (step_one bins on the side
-      // stream for the same reason)
+      // vertex velocities, of the previous stretch's membrane launch (side
+      // stream): the collision waits for it
       if (cudaStreamWaitEvent(ms, c->ev_mem, 0) != cudaSuccess) return IRBC_ERR_CUDA;
       launched += multi_collide_front(c->plan, (uint64_t)k, ms);
       launched += multi_collide_count(c->plan, (uint64_t)k, ms);
       launched += multi_collide_scan(c->plan, ms);
       launched += multi_collide_back(c->plan, (uint64_t)k, resort, ms);
-      if (cudaEventRecord(c->ev_coll, ms) != cudaSuccess || cudaStreamWaitEvent(ss, c->ev_coll, 0) != cudaSuccess)
-        return IRBC_ERR_CUDA;
     }
-    if (!h0->snap_ready) {
-      if (cudaStreamWaitEvent(ss, c->ev_str[buf], 0) != cudaSuccess) return IRBC_ERR_CUDA;
-      launched += multi_kick(c->plan, buf, ss);
-    }
-    // list updates (rare, per member, with host waits): positions of this
-    // step are final once the side stream reaches here
+    // list updates (rare, per member, with host waits)
     bool listed = false;
     for (irbc_handle* h : hs) {
       if (h->upd != h->uplist) continue;
-      if (!listed) {
-        if (cudaEventRecord(c->ev_snap, ss) != cudaSuccess || cudaStreamWaitEvent(ms, c->ev_snap, 0) != cudaSuccess)
-          return IRBC_ERR_CUDA;
-        listed = true;
-      }
+      if (!listed && cudaStreamWaitEvent(ms, c->ev_mem, 0) != cudaSuccess) return IRBC_ERR_CUDA;
+      listed = true;
       if (cudaEventRecord(c->ev_join, ms) != cudaSuccess || cudaStreamWaitEvent(h->st, c->ev_join, 0) != cudaSuccess)
         return IRBC_ERR_CUDA;
       int rc = do_llist(h);
@@ -1734,25 +1928,23 @@ int cohort_step(Cohort* c, const std::vector<irbc_handle*>& all, int64_t n, std:
       int rc = cohort_upload(c);  // lists, buckets and staging may have moved or grown
       if (rc) return rc;
     }
-    const bool next_collides = h0->colsteps + 1 == csteps;
-    const bool next_kick = k != n - 1 && !next_collides;
-    // as step_one: the bulk streaming starts at once, the near-membrane
-    // kernel waits for the snapshot, the membrane step runs beside them and
-    // writes the next snapshot only after the streaming that read it
-    if (cudaEventRecord(c->ev_snap, ss) != cudaSuccess) return IRBC_ERR_CUDA;
-    launched += multi_stream(c->plan, buf, ms, c->ev_snap);
-    if (cudaEventRecord(c->ev_str[buf], ms) != cudaSuccess) return IRBC_ERR_CUDA;
-    launched += multi_membrane(c->plan, (uint64_t)k, ss);
-    if (next_kick) {
-      if (cudaStreamWaitEvent(ss, c->ev_str[buf ^ 1], 0) != cudaSuccess) return IRBC_ERR_CUDA;
-      launched += multi_kick(c->plan, buf ^ 1, ss);
-    }
+    int64_t H = n - k;
+    for (irbc_handle* h : hs) H = std::min(H, stretch_steps(h, H));
+    // the membranes of the stretch on the side stream, the streaming of each
+    // step on the main one
+    if (cudaEventRecord(c->ev_coll, ms) != cudaSuccess || cudaStreamWaitEvent(ss, c->ev_coll, 0) != cudaSuccess)
+      return IRBC_ERR_CUDA;
+    launched += multi_membrane(c->plan, (uint64_t)k, (int)H, ss);
     if (cudaEventRecord(c->ev_mem, ss) != cudaSuccess) return IRBC_ERR_CUDA;
+    launched += multi_stream(c->plan, (int)H, (int)(c->stretches++ & 1), ms, c->ev_mem);
     for (irbc_handle* h : hs) {
-      h->snap_ready = next_kick;
-      if (h->filecc == h->P.out_every) { h->filec += 1; h->filecc = 0; }
-      h->step += 1;
+      step_ends(h);
+      for (int64_t q = 1; q < H; ++q) {
+        step_begins(h);
+        step_ends(h);
+      }
     }
+    k += H;
   }
   // each member's own stream follows the cohort's work; its health word
   // is copied for the next irbc_step (as at the end of irbc_step)

@@ -9,93 +9,141 @@ struct TriPre {
   double X[3], Xdt[3], A1[3], A2[3];
 };
 
-// vertex positions/velocities as seen by one streaming step
+// vertex positions/velocities as seen by the streaming of one step of a
+// stretch (the arrays hold kSegMax steps, nv entries each)
 struct Snap {
   double *x, *y, *z, *vx, *vy, *vz;
   const int *t1, *t2, *t3;
 };
+// the most steps a stretch has: a stretch lies between two collisions (10 to
+// 12 steps apart at the configured dtcd / dtmd); longer ones are cut, for the
+// room that the snapshots take (kSegMax x 96 bytes per triangle)
+constexpr int kSegMax = 16;
+constexpr int kSegT = 512;  // threads per block of the membrane kernel
+// triangles whose area and volume terms the summing blocks of the membrane
+// kernel stage in shared memory (what is left of 227 KB); more stay in global
+// memory.  seg_terms(nt): the doubles staged for nt triangles, the warp tree's
+// padding included
+constexpr int kSegTerms = 20000;
+__host__ __device__ constexpr int seg_terms(int nt) { return (nt + 32 + 15) / 16 * 16; }
 
 // near-membrane streaming: particles per listed cell taken by the cell's
-// block, the longest list staged in its shared memory, and the blocks that
-// walk the overflow queue
+// warps, and the longest list they take; the others go to the queue
 constexpr int kBucket = 32;
 constexpr int kHeavyList = 1024;
-constexpr int kOverflowBlocks = 8;
-// Lists of up to kShortList entries (staging capacity hcap) take the
-// short-list path: one warp per listed cell, its lanes shared among the
-// cell's particles, from a staging of kLanePiece entries per warp
-// (kShortWarps such warps per block), then the overflow queue's walk.
-// Longer lists: the near-membrane kernel stages a listed cell's TriPre
-// records in shared memory a piece at a time, eight warps per block
-// (kStageLong entries per piece).  The kernel's registers allow two
-// eight-warp blocks per SM, which a whole 1024-entry list per block also
-// allows, so a bucketed list (at most kHeavyList entries) is one piece.
-constexpr int kShortList = 128, kStageLong = kHeavyList;
-constexpr int kShortWarps = 4, kLanePiece = 64;
-// blocks of eight warps that walk the overflow queue after the short-list
-// kernel: per simulation alone, and per member of a cohort
-constexpr int kQueueBlocks = 64, kQueueBlocksMember = 32;
-// the short-list kernel runs without the full test's registers: 64 per
-// thread, eight blocks (32 warps) per SM
-constexpr int kShortMinBlocks = 8;
+// Lists of up to kShortList entries (capacity hcap) take one warp per listed
+// cell, kShortWarps of them to a block, at 64 registers a thread (eight blocks,
+// 32 warps, per SM); longer ones kLongWarps warps per cell.
+constexpr int kShortList = 128, kShortWarps = 4, kShortMinBlocks = 8;
+constexpr int kLongWarps = 4, kLongMinBlocks = 4;
+// blocks of eight warps that walk the queue: per simulation alone, and per
+// member of a cohort
+constexpr int kQueueBlocks = 148, kQueueBlocksMember = 32;
 inline bool short_lists(int hcap) { return hcap <= kShortList; }
-// the staging piece of the long-list kernel
-inline int stage_cap(int hcap) { return hcap < kStageLong ? (hcap > 0 ? hcap : 1) : kStageLong; }
-inline int stage_bytes(int cap) { return cap * (int)(sizeof(TriPre) + sizeof(int)); }
+// the side-wall bands (3a) that a triangle's corners lie in: tri_record
+enum : int { BAND_LX = 1, BAND_HX = 2, BAND_LY = 4, BAND_HY = 8 };
+
+// A mesh split into one patch of vertices per block of the membrane's cluster
+// (build_patches in api.cu; segment.cuh): where block b's tables lie.
+struct PatchHdr {
+  int no, nl, ntri, ned, ndih, nsend;  // own vertices, vertices touched, items, coordinates sent
+  int base;                            // first own vertex in the snapshots
+  int own, tri, edge, dih, ent, eend, send;  // offsets of the tables in the block's part of the blob
+  int blob, bytes;                     // that part
+  int ne, nt, nd;                      // edge, triangle and bending entries of its vertices
+  int o_tab, o_e, o_d, o_t, o_s;       // shared memory: tables, entries, vertex state
+};
+struct PatchPlan {
+  PatchHdr* hdr = nullptr;
+  unsigned char* blob = nullptr;
+  int nc = 0;                          // blocks; 0: no patches (the state stays in global memory)
+  int sw = 0;                          // summing warps of blocks 0 and 1
+  int nl = 0;                          // the most vertices a block touches
+  int o_misc = 0, o_c = 0, o_terms = 0, o_sum = 0, o_tail = 0, smem = 0;  // shared memory
+};
+constexpr unsigned short kNoEntry = 0xffff;
+struct PatchTri {
+  unsigned short v[3], d[3];  // corners; where their entries go (kNoEntry: another block's vertex)
+  int g;                      // >= 0: the triangle whose area and volume terms this block writes
+  double tarea;
+};
+struct PatchEdge {
+  unsigned short v[2], pad[2];
+  double l0, kp;
+};
+struct PatchDih {
+  unsigned short v[4], d[4];  // l1, l4, l2, l3
+};
+struct PatchSend {
+  unsigned short own, slot, cta, pad;
+};
+// whether the device runs a cluster of nc membrane blocks with smem bytes each
+bool cluster_fits(int nc, int smem);
+// where everything lies in the blocks' shared memory (host)
+void patch_layout(PatchPlan& P, PatchHdr* hdr, int nt);
+// the most shared memory the membrane kernel takes, its most vertices per block
+constexpr int kSegSmemMax = 224 * 1024, kPatchOwn = 256;
 
 struct FastBufs {
-  Snap snap[2];
-  TriPre* pre[2] = {nullptr, nullptr};
-  int* queue = nullptr;   // overflow: particles of full buckets or over-long lists (capacity Ns)
-  int* qn = nullptr;
-  int* bcnt = nullptr;    // particles handed to each listed cell this step (reset by k_stream_cells)
-  int* bucket = nullptr;  // kBucket particle slots per listed cell
+  PatchPlan patch;
+  int* pidx = nullptr;      // place of each vertex in the snapshots
+  int *st1 = nullptr, *st2 = nullptr, *st3 = nullptr;  // the triangles' corners by that place
+  Snap snap{};
+  TriPre* pre = nullptr;  // kSegMax x nt
+  unsigned char* bands = nullptr;  // kSegMax x nt: BAND_* of each record's corners
+  int* queue = nullptr;   // particles the near-membrane cells' warps do not take (capacity Ns)
+  unsigned char* qk = nullptr;  // the step of the stretch from which on
+  int* qn = nullptr;      // their number
+  int* bcnt = nullptr;    // particles handed to each listed cell in this stretch (reset by its warps)
+  int2* bucket = nullptr; // kBucket (particle, first step) per listed cell
   int64_t bcap = 0;       // listed cells the buckets have room for
-  int* border = nullptr;  // the listed cell (rank) of each k_stream_cells block: longest lists first
+  int* border = nullptr;  // listed cells (ranks), longest lists first
   int2* arng = nullptr;   // (first entry, length) of each listed cell's list, by rank (bcap of them)
-  bool one_block = false; // the membrane step as one block per launch (small meshes)
-  bool cluster = false;   // the membrane step as one launch of a thread-block cluster (any mesh)
-  int hcap = kHeavyList;  // list entries k_stream_cells stages (its shared memory); longer lists go
-                          // to the overflow queue
+  bool one_block = false; // the membrane kernel as one block (meshes that fit, one_block_fits)
+  bool cluster = false;   // ... as a cluster of eight blocks whatever the mesh
+  int hcap = kHeavyList;  // longest list taken by a cell's warps
   double* slot = nullptr; // force terms: 3 doubles per slot, 4E + 9T + 4E slots
-  int* gstart = nullptr;  // per-vertex slot lists in the reference's order
-  int* gidx = nullptr;
-  int* vd = nullptr;      // bond draws per vertex this step
-  int* vw = nullptr;      // vertex within the parasite's WCA cutoff
-  double* vX = nullptr;   // its WCA force (3 per vertex)
+  double* a4 = nullptr;   // 4 x area of each triangle
+  double* fac = nullptr;  // factors of the global area and volume forces
+  double *ux = nullptr, *uy = nullptr;  // unwrapped vertex coordinates
+  int* gstart = nullptr;  // per vertex: where its edge, triangle and bending entries of gidx start
+  int* gidx = nullptr;    // its slots in the reference's order
+  int* vd = nullptr;      // bond draws per vertex this step, VF_* flags
+  double* vX = nullptr;   // the parasite's WCA force on it (3 per vertex)
+  double* vS = nullptr;   // its bond spring's force (3 per vertex)
 };
 
-// these return the number of kernels they launched
-int fast_kick_prep(const DevParams& p, Membrane& m, FastBufs& f, int buf, cudaStream_t st);
-void fast_snap_prep(const DevParams& p, Membrane& m, FastBufs& f, int buf, cudaStream_t st);
+__host__ __device__ inline Snap snap_of(const FastBufs& f, int step, int nv) {
+  Snap s = f.snap;
+  const int64_t o = (int64_t)step * nv;
+  s.x += o; s.y += o; s.z += o; s.vx += o; s.vy += o; s.vz += o;
+  return s;
+}
+// snapshot and triangle records of the membrane as it is, as step 0
+void fast_snap_prep(const DevParams& p, Membrane& m, FastBufs& f, cudaStream_t st);
 // list length of each listed cell (rank a < nact) into len[a], and its
 // (first entry, length) into rng[a]
 void launch_rank_lengths(const Cells& c, int* len, int2* rng, cudaStream_t st);
-// the staging capacity for lists of at most lmax entries: lmax rounded up
-// to 64, at least 64, at most kHeavyList
+// the capacity for lists of at most lmax entries: lmax rounded up to 64, at
+// least 64, at most kHeavyList
 inline int heavy_cap(int lmax) {
   int c = ((lmax + 63) / 64) * 64;
   return c < 64 ? 64 : (c > kHeavyList ? kHeavyList : c);
 }
-// ev0/ev1 (optional) are recorded around the bulk kernel k_stream_fast.  The
-// bulk kernel reads no membrane data; the near-membrane kernels read the
-// snapshot `buf` and first wait for `snap` (optional: its producer).
-// Returns the number of kernels it launched.
-int fast_stream(const DevParams& p, Solvent& s, const Cells& c, FastBufs& f, int buf, cudaStream_t st,
-                cudaEvent_t ev0 = nullptr, cudaEvent_t ev1 = nullptr, cudaEvent_t snap = nullptr);
-// these return the number of kernels they launched
-int fast_drift_va(const DevParams& p, Membrane& m, cudaStream_t st, bool with_sum);
+// the streaming of a stretch of H steps; sf: the FP32-bulk solvent, or null.
+// ev0/ev1 (optional) are recorded around the bulk kernel.  The bulk kernel
+// reads no membrane data; the near-membrane kernels read the snapshots and
+// records and first wait for `snap` (optional: their producer).  Returns the
+// number of kernels it launched.
+struct SolventF;
+int fast_stream(const DevParams& p, const Solvent& s, const SolventF* sf, const Cells& c, FastBufs& f, int H,
+                cudaStream_t st, cudaEvent_t ev0 = nullptr, cudaEvent_t ev1 = nullptr, cudaEvent_t snap = nullptr);
 bool is_membrane_kernel(const void* fn);
-// next_kick: also the next step's half-kick and snapshot into next_buf,
-// after waiting for `readers` (optional: the last streaming that read it)
-int fast_forces_tail(const DevParams& p, Membrane& m, FastBufs& f, uint64_t epoch, int next_kick, int next_buf,
-                     cudaStream_t st, bool sum_pending, cudaEvent_t readers = nullptr);
-// the whole membrane step of irbc_step (drift .. bond_dynamics, then the
-// next half-kick and snapshot as fast_forces_tail): in one launch of a
-// thread-block cluster when f.cluster, in one block per launch when
-// f.one_block, else fast_drift_va + fast_forces_tail
-int fast_membrane_step(const DevParams& p, Membrane& m, FastBufs& f, uint64_t epoch, int next_kick, int next_buf,
-                       cudaStream_t st, cudaEvent_t readers = nullptr);
+// the membrane of H <= kSegMax steps in one launch (segment.cuh); parts:
+// SEG_FIRST | SEG_SECOND, or one of them with H = 1.  Returns the number of
+// kernels launched.
+enum : int { SEG_FIRST = 1, SEG_SECOND = 2, SEG_WHOLE = 3 };
+int launch_membrane(const DevParams& p, Membrane& m, FastBufs& f, uint64_t eoff, int H, int parts, cudaStream_t st);
 // whether a mesh suits the one-block membrane step
 bool one_block_fits(const DevParams& p);
 // every kernel's dynamic shared-memory limit on the current device (before

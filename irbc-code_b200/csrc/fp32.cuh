@@ -133,78 +133,4 @@ void launch_resort_f(SolventF& f, Solvent& s, cudaStream_t st) {
   }
 }
 
-// ---- streaming ------------------------------------------------------------------
-// free flight, walls and wrap in float (maincode.cpp:516-560); particles in
-// cells with triangles are handed to the near-membrane kernels (double
-// precision)
-// the shifted-free cell of a position (the list lookup of the streaming)
-__device__ __forceinline__ int stream_cell_f(const DevParams& p, float4 q, float Lx, float Ly) {
-  int fx = (int)floorf(bbound(q.x, Lx));
-  int fy = (int)floorf(bbound(q.y, Ly));
-  int fz = (int)floorf(q.z + 1.0f);
-  return cell_of(p, fx, fy, fz);
-}
-
-// free flight, walls and wrap of particle i, loaded as (q, v), whose cell
-// pid has the list [l0, l1): particles in cells with triangles are handed
-// to the near-membrane kernels (double precision)
-__device__ __forceinline__ void stream_f_apply(const DevParams& p, const SolventF& f, const int* __restrict__ lrank,
-                                               int* bcnt, int* bucket, int* queue, int* qn, int hcap, int64_t i,
-                                               float4 q, float4 v, int pid, int l0, int l1) {
-  const float Lx = (float)p.Lx, Ly = (float)p.Ly, Lz = (float)p.Lz, dt = (float)p.dtmd;
-  if (l1 > l0) {
-    hand_off(lrank, pid, l1 - l0, hcap, (int)i, bcnt, bucket, queue, qn);
-    return;
-  }
-  float X = q.x + v.x * dt, Y = q.y + v.y * dt, Z = q.z + v.z * dt;
-  if (Z > Lz || Z < 0.0f) {
-    const float wall = Z > Lz ? Lz : 0.0f;
-    float ax = X - v.x * dt, ay = Y - v.y * dt, az = Z - v.z * dt;
-    float sp = (wall - az) / (Z - az);
-    float bx = ax + sp * (X - ax), by = ay + sp * (Y - ay), bz = az + sp * (Z - az);
-    float dist = sqrtf((bx - ax) * (bx - ax) + (by - ay) * (by - ay) + (bz - az) * (bz - az));
-    float dtt = dist / sqrtf(v.x * v.x + v.y * v.y + v.z * v.z);
-    if (Z > Lz) { v.x = (float)p.wallspeed; v.y = 0.0f; v.z = 0.0f; }
-    else { v.x = -v.x; v.y = -v.y; v.z = -v.z; }
-    X = bx + v.x * (dt - dtt); Y = by + v.y * (dt - dtt); Z = bz + v.z * (dt - dtt);
-    f.vel[i] = v;
-  }
-  X = bbound(X, Lx);
-  Y = bbound(Y, Ly);
-  raise_health(p, solvent_bad(p, X, Y, Z, v.x, v.y, v.z), HEALTH_SOLVENT);
-  f.pos[i] = make_float4(X, Y, Z, q.w);
-}
-
-__device__ __forceinline__ void stream_f_item(const DevParams& p, const SolventF& f, const int* __restrict__ lstart,
-                                              const int* __restrict__ lrank, int* bcnt, int* bucket, int* queue,
-                                              int* qn, int hcap, int64_t i) {
-  if (i >= f.n) return;
-  const float4 q = f.pos[i], v = f.vel[i];
-  const int pid = stream_cell_f(p, q, (float)p.Lx, (float)p.Ly);
-  const int l0 = __ldg(lstart + pid), l1 = __ldg(lstart + pid + 1);
-  stream_f_apply(p, f, lrank, bcnt, bucket, queue, qn, hcap, i, q, v, pid, l0, l1);
-}
-
-__global__ void __launch_bounds__(256) k_stream_f(DevParams p, SolventF f, const int* __restrict__ lstart,
-                                                  const int* __restrict__ lrank, int* bcnt, int* bucket,
-                                                  int* queue, int* qn, int hcap) {
-  stream_f_item(p, f, lstart, lrank, bcnt, bucket, queue, qn, hcap, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
-}
-
-int fast_stream_f(const DevParams& p, SolventF& f, const Cells& c, FastBufs& fb, int buf, cudaStream_t st,
-                  cudaEvent_t ev0, cudaEvent_t ev1, cudaEvent_t snap) {
-  cudaMemsetAsync(fb.qn, 0, sizeof(int), st);
-  if (f.n) {
-    if (ev0) cudaEventRecord(ev0, st);
-    k_stream_f<<<nbf(f.n, 256), 256, 0, st>>>(p, f, c.lstart, c.lrank, fb.bcnt, fb.bucket, fb.queue, fb.qn,
-                                              fb.hcap);
-    if (ev1) cudaEventRecord(ev1, st);
-    if (snap) cudaStreamWaitEvent(st, snap, 0);
-    Solvent none;
-    none.n = f.n;
-    return 1 + launch_stream_cells<true>(p, none, f, c, fb, buf, st);
-  }
-  return 0;
-}
-
 }  // namespace irbc

@@ -470,177 +470,6 @@ void launch_resort(Solvent& s, cudaStream_t st) {
   }
 }
 
-// ============================================================== stream =====
-// Streaming with bounce-back: reflectionFed(i, 0) (Src/solfuncs.cpp:400-598)
-// then the wall treatment and wrap of maincode.cpp:515-560.  The cubic
-// contact-time solver solve_p3_tt is in common.cuh.
-struct VertexView {
-  const double *x, *y, *z, *vx, *vy, *vz;
-};
-
-__device__ double reflection(const DevParams& p, const int* lstart, const int* lidx, const Membrane& m,
-                             double& X_, double& Y_, double& Z_, double& VX, double& VY, double& VZ, int indio) {
-  const double rstep = 0.0, dtmd = p.dtmd, a = p.a, Lx = p.Lx, Ly = p.Ly;
-  double fulldt = rstep;
-  int fx = (int)floor(bbound(X_, Lx));
-  int fy = (int)floor(bbound(Y_, Ly));
-  int fz = (int)floor(Z_ + 1.0);
-  int pid = cell_of(p, fx, fy, fz);
-  const int l0 = lstart[pid], l1 = lstart[pid + 1];
-  for (int j = l0; j < l1; ++j) {
-    int flg = 0;
-    int jj = lidx[j];
-    int p1 = m.t1[jj], p2 = m.t2[jj], p3 = m.t3[jj];
-    const int xx = 0, yy = 0, p1modx = 0, p2modx = 0, p3modx = 0, p1mody = 0, p2mody = 0, p3mody = 0;
-    double solvx = X_ + xx * Lx;
-    double solvy = Y_ + yy * Ly;
-    double solvz = Z_;
-    double v1x = (m.x[p1] + p1modx * Lx) + m.vx[p1] * rstep;
-    double v1y = (m.y[p1] + p1mody * Ly) + m.vy[p1] * rstep;
-    double v1z = m.z[p1] + m.vz[p1] * rstep;
-    double v2x = (m.x[p2] + p2modx * Lx) + m.vx[p2] * rstep;
-    double v2y = (m.y[p2] + p2mody * Ly) + m.vy[p2] * rstep;
-    double v2z = m.z[p2] + m.vz[p2] * rstep;
-    double v3x = (m.x[p3] + p3modx * Lx) + m.vx[p3] * rstep;
-    double v3y = (m.y[p3] + p3mody * Ly) + m.vy[p3] * rstep;
-    double v3z = m.z[p3] + m.vz[p3] * rstep;
-    double rstencilx = Lx - (3.0 * a), lstencilx = 3.0 * a;
-    double rstencily = Ly - (3.0 * a), lstencily = 3.0 * a;
-    if (solvx < lstencilx) {
-      v1x -= (v1x > rstencilx) ? Lx : 0;
-      v2x -= (v2x > rstencilx) ? Lx : 0;
-      v3x -= (v3x > rstencilx) ? Lx : 0;
-    } else if (solvx > rstencilx) {
-      v1x += (v1x < lstencilx) ? Lx : 0;
-      v2x += (v2x < lstencilx) ? Lx : 0;
-      v3x += (v3x < lstencilx) ? Lx : 0;
-    }
-    if (solvy < lstencily) {
-      v1y -= (v1y > rstencily) ? Ly : 0;
-      v2y -= (v2y > rstencily) ? Ly : 0;
-      v3y -= (v3y > rstencily) ? Ly : 0;
-    } else if (solvy > rstencily) {
-      v1y += (v1y < lstencily) ? Ly : 0;
-      v2y += (v2y < lstencily) ? Ly : 0;
-      v3y += (v3y < lstencily) ? Ly : 0;
-    }
-    const double mvx1 = m.vx[p1], mvy1 = m.vy[p1], mvz1 = m.vz[p1];
-    const double mvx2 = m.vx[p2], mvy2 = m.vy[p2], mvz2 = m.vz[p2];
-    const double mvx3 = m.vx[p3], mvy3 = m.vy[p3], mvz3 = m.vz[p3];
-    double w1x = v1x + mvx1 * (dtmd - rstep), w1y = v1y + mvy1 * (dtmd - rstep), w1z = v1z + mvz1 * (dtmd - rstep);
-    double w2x = v2x + mvx2 * (dtmd - rstep), w2y = v2y + mvy2 * (dtmd - rstep), w2z = v2z + mvz2 * (dtmd - rstep);
-    double w3x = v3x + mvx3 * (dtmd - rstep), w3y = v3y + mvy3 * (dtmd - rstep), w3z = v3z + mvz3 * (dtmd - rstep);
-    double X[3], Xdt[3], t0[3], t1v[3];
-    t0[0] = v2x - v1x; t0[1] = v2y - v1y; t0[2] = v2z - v1z;
-    t1v[0] = v3x - v1x; t1v[1] = v3y - v1y; t1v[2] = v3z - v1z;
-    cp(t0, t1v, X);
-    t0[0] = w2x - w1x; t0[1] = w2y - w1y; t0[2] = w2z - w1z;
-    t1v[0] = w3x - w1x; t1v[1] = w3y - w1y; t1v[2] = w3z - w1z;
-    cp(t0, t1v, Xdt);
-    double PSt[3], PSdt[3];
-    PSt[0] = solvx - v1x; PSt[1] = solvy - v1y; PSt[2] = solvz - v1z;
-    PSdt[0] = (solvx + VX * (dtmd - rstep)) - w1x;
-    PSdt[1] = (solvy + VY * (dtmd - rstep)) - w1y;
-    PSdt[2] = (solvz + VZ * (dtmd - rstep)) - w1z;
-    double bt = X[0] * PSt[0] + X[1] * PSt[1] + X[2] * PSt[2];
-    double bdt = Xdt[0] * PSdt[0] + Xdt[1] * PSdt[1] + Xdt[2] * PSdt[2];
-    if ((indio == 1) && (bt < 0)) flg = 1;
-    if ((indio == 0) && (bt > 0)) flg = 1;
-    if ((bt * bdt <= 0) && (flg == 0)) {
-      double a10[3], a20[3], d1[3], d2[3], a2v[3], b1[3], b2[3], b3[3], d11[3], d22[3];
-      a10[0] = v2x - v1x; a10[1] = v2y - v1y; a10[2] = v2z - v1z;
-      a20[0] = v3x - v1x; a20[1] = v3y - v1y; a20[2] = v3z - v1z;
-      d1[0] = mvx2 - mvx1; d1[1] = mvy2 - mvy1; d1[2] = mvz2 - mvz1;
-      d2[0] = mvx3 - mvx1; d2[1] = mvy3 - mvy1; d2[2] = mvz3 - mvz1;
-      const double* a1v = PSt;
-      a2v[0] = VX - mvx1; a2v[1] = VY - mvy1; a2v[2] = VZ - mvz1;
-      cp(a10, a20, b1);
-      cp(a10, d2, d11);
-      cp(d1, a20, d22);
-      cp(d1, d2, b3);
-      for (int k = 0; k < 3; ++k) b2[k] = d11[k] + d22[k];
-      double a2b3 = a2v[0] * b3[0] + a2v[1] * b3[1] + a2v[2] * b3[2];
-      double a1b3 = a1v[0] * b3[0] + a1v[1] * b3[1] + a1v[2] * b3[2];
-      double a2b2 = a2v[0] * b2[0] + a2v[1] * b2[1] + a2v[2] * b2[2];
-      double a1b2 = a1v[0] * b2[0] + a1v[1] * b2[1] + a1v[2] * b2[2];
-      double a2b1 = a2v[0] * b1[0] + a2v[1] * b1[1] + a2v[2] * b1[2];
-      double a1b1 = a1v[0] * b1[0] + a1v[1] * b1[1] + a1v[2] * b1[2];
-      double tt = solve_p3_tt((a1b3 + a2b2) / a2b3, (a1b2 + a2b1) / a2b3, a1b1 / a2b3, dtmd);
-      double pd[3], vd[3], PS2[3];
-      PS2[0] = (solvx + VX * tt) - (v1x + mvx1 * tt);
-      PS2[1] = (solvy + VY * tt) - (v1y + mvy1 * tt);
-      PS2[2] = (solvz + VZ * tt) - (v1z + mvz1 * tt);
-      pd[0] = (solvx + VX * tt);
-      pd[1] = (solvy + VY * tt);
-      pd[2] = (solvz + VZ * tt);
-      a10[0] = (v2x + mvx2 * tt) - (v1x + mvx1 * tt);
-      a10[1] = (v2y + mvy2 * tt) - (v1y + mvy1 * tt);
-      a10[2] = (v2z + mvz2 * tt) - (v1z + mvz1 * tt);
-      a20[0] = (v3x + mvx3 * tt) - (v1x + mvx1 * tt);
-      a20[1] = (v3y + mvy3 * tt) - (v1y + mvy1 * tt);
-      a20[2] = (v3z + mvz3 * tt) - (v1z + mvz1 * tt);
-      double pa1 = PS2[0] * a10[0] + PS2[1] * a10[1] + PS2[2] * a10[2];
-      double pa2 = PS2[0] * a20[0] + PS2[1] * a20[1] + PS2[2] * a20[2];
-      double a1a2 = a10[0] * a20[0] + a10[1] * a20[1] + a10[2] * a20[2];
-      double a12 = a10[0] * a10[0] + a10[1] * a10[1] + a10[2] * a10[2];
-      double a22 = a20[0] * a20[0] + a20[1] * a20[1] + a20[2] * a20[2];
-      double den = (a12 * a22) - (a1a2 * a1a2);
-      double eta = ((pa1 * a22) - (pa2 * a1a2)) / den;
-      double zeta = ((pa2 * a12) - (pa1 * a1a2)) / den;
-      if ((eta >= 0) && (zeta >= 0) && (eta + zeta <= 1) && (tt < (dtmd - rstep))) {
-        fulldt += tt;
-        vd[0] = (1.0 - eta - zeta) * mvx1 + eta * mvx2 + zeta * mvx3;
-        vd[1] = (1.0 - eta - zeta) * mvy1 + eta * mvy2 + zeta * mvy3;
-        vd[2] = (1.0 - eta - zeta) * mvz1 + eta * mvz2 + zeta * mvz3;
-        VX = 2.0 * vd[0] - VX;
-        VY = 2.0 * vd[1] - VY;
-        VZ = 2.0 * vd[2] - VZ;
-        X_ = pd[0]; Y_ = pd[1]; Z_ = pd[2];
-      }
-    }
-  }
-  return fulldt;
-}
-
-__global__ void k_stream(DevParams p, Solvent s, const int* lstart, const int* lidx, Membrane m) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= s.n) return;
-  const SolVel r = s.v[i];
-  double X = s.x[i], Y = s.y[i], Z = s.z[i], VX = r.vx, VY = r.vy, VZ = r.vz;
-  const double VX0 = VX, VY0 = VY, VZ0 = VZ;
-  const double dtmd = p.dtmd;
-  double fullts = reflection(p, lstart, lidx, m, X, Y, Z, VX, VY, VZ, s.indio[i]);
-  X += VX * (dtmd - fullts);
-  Y += VY * (dtmd - fullts);
-  Z += VZ * (dtmd - fullts);
-  const double ul = p.Lz, ll = 0;
-  if (Z > ul || Z < ll) {
-    double A[3], B[3];
-    const double wall = Z > ul ? ul : ll;
-    A[0] = X - VX * (dtmd - fullts); A[1] = Y - VY * (dtmd - fullts); A[2] = Z - VZ * (dtmd - fullts);
-    double sp = (wall - A[2]) / (Z - A[2]);
-    B[0] = A[0] + sp * (X - A[0]); B[1] = A[1] + sp * (Y - A[1]); B[2] = A[2] + sp * (Z - A[2]);
-    double dist = sqrt(((B[0] - A[0]) * (B[0] - A[0])) + ((B[1] - A[1]) * (B[1] - A[1])) + ((B[2] - A[2]) * (B[2] - A[2])));
-    double dtt = dist / sqrt((VX * VX) + (VY * VY) + (VZ * VZ));
-    if (Z > ul) {  // moving top wall: v = (wallspeed, 0, 0)
-      VX = p.wallspeed; VY = 0; VZ = 0;
-    } else {       // bounce-back bottom wall
-      VX *= -1.0; VY *= -1.0; VZ *= -1.0;
-    }
-    X = B[0] + VX * ((dtmd - fullts) - dtt);
-    Y = B[1] + VY * ((dtmd - fullts) - dtt);
-    Z = B[2] + VZ * ((dtmd - fullts) - dtt);
-  }
-  X = bbound(X, p.Lx);
-  Y = bbound(Y, p.Ly);
-  s.x[i] = X; s.y[i] = Y; s.z[i] = Z;
-  if (VX != VX0 || VY != VY0 || VZ != VZ0 || VX0 != VX0) { s.v[i].vx = VX; s.v[i].vy = VY; s.v[i].vz = VZ; }
-}
-
-void launch_stream(const DevParams& p, Solvent& s, const Cells& c, const Membrane& m, cudaStream_t st) {
-  if (s.n) k_stream<<<nblk(s.n, 256), 256, 0, st>>>(p, s, c.lstart, c.lidx, m);
-}
-
 // ============================================================== llist ======
 // llistupdate (Src/solfuncs.cpp:326-365): triangles whose centroid lies
 // within 2a of the cell centre, with the list never shrinking (entries past
@@ -778,17 +607,34 @@ __global__ void k_acell(DevParams p, Cells cl) {
   if (c >= p.ncell) return;
   if (cl.lstart[c + 1] > cl.lstart[c]) cl.acell[cl.lrank[c]] = (int)c;
 }
+// what the streaming wants to know of a cell without reading its list (Cells::flag)
+__global__ void k_cell_flags(DevParams p, Cells cl) {
+  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= p.ncell) return;
+  auto listed = [&](int64_t q) { return cl.lstart[q + 1] > cl.lstart[q]; };
+  const int k = (int)(c % p.nz), j = (int)((c / p.nz) % p.ny), i = (int)(c / ((int64_t)p.nz * p.ny));
+  // (a position off the grid counts as cell 0: cell_of)
+  bool meets = i == 0 || i >= p.nx - 1 || j == 0 || j >= p.ny - 1 || (listed(0) && (k <= 1 || k >= p.nz - 2));
+  for (int a = -1; a <= 1 && !meets; ++a)
+    for (int b = -1; b <= 1 && !meets; ++b) {
+      const int64_t row = ((int64_t)(i + a) * p.ny + j + b) * p.nz;
+      // the list starts ascend: any entry between two of them is theirs
+      meets = cl.lstart[row + min(k + 1, p.nz - 1) + 1] > cl.lstart[row + max(k - 1, 0)];
+    }
+  cl.flag[c] = (unsigned char)((listed(c) ? 1 : 0) | (meets ? 2 : 0));
+}
 int launch_llist_ranks(const DevParams& p, Cells& c, cudaStream_t st) {
   cudaMemsetAsync(c.totals + 7, 0, sizeof(int), st);
   k_lflags<<<nblk(c.n, 256), 256, 0, st>>>(p, c);
   launch_scan3(c.lrank, nullptr, nullptr, c.lrank, nullptr, nullptr, c.totals + 4, c.n, c.scan_part, st);
   k_acell<<<nblk(c.n, 256), 256, 0, st>>>(p, c);
+  k_cell_flags<<<nblk(c.n, 256), 256, 0, st>>>(p, c);
   int h[4] = {0, 0, 0, 0};
   cudaMemcpyAsync(h, c.totals + 4, sizeof(h), cudaMemcpyDeviceToHost, st);
   if (cudaStreamSynchronize(st) != cudaSuccess) return -1;
   c.nact = h[0];
   c.lmax = h[3];
-  return 5;
+  return 6;
 }
 
 // ============================================================ membrane =====

@@ -8,184 +8,138 @@
 namespace irbc {
 
 // ---- streaming -------------------------------------------------------------
-__global__ void __launch_bounds__(256, 8) km_stream_f(Member* __restrict__ mem, const int2* __restrict__ tab,
-                                                   int par) {
+__global__ void __launch_bounds__(256, 6) km_stream_bulk(Member* __restrict__ mem, const int2* __restrict__ tab, int H,
+                                                        int par) {
   KM_MEMBER;
   // copies: the descriptor is not reloaded after the stores below
   const DevParams p = M.p;
-  const SolventF f = M.f;
-  const int* __restrict__ lstart = M.c.lstart;
-  const int* __restrict__ lrank = M.c.lrank;
-  int* const bcnt = M.fb.bcnt;
-  int* const bucket = M.fb.bucket;
-  int* const queue = M.fb.queue;
-  int* const qn = M.fb.qn + par;
-  const int hcap = M.fb.hcap;
-  const int64_t n = f.n;
-  const float Lx = (float)p.Lx, Ly = (float)p.Ly;
-  constexpr int K = kMultiStreamPer;
+  const SolventArrays s = arrays_of(M.s, M.f);
+  const HandOff h = hand_off_of(M.c, M.fb, par);
+  const unsigned char* __restrict__ cflag = M.c.flag;
+  const int64_t n = M.f.n;
+  // the queue of the next stretch starts empty
+  if (b == 0 && threadIdx.x == 0) M.fb.qn[par ^ 1] = 0;
   for (int pass = 0; pass < kMultiStreamPasses; ++pass) {
-    const int64_t i0 = ((int64_t)b * kMultiStreamPasses + pass) * blockDim.x * K + threadIdx.x;
-    if (i0 >= n) break;
-    // every load of the thread's particles first, then their cells' list
-    // bounds, then the updates: the latencies overlap
-    float4 q[K], v[K];
-    int pid[K], l0[K], l1[K];
-#pragma unroll
-    for (int u = 0; u < K; ++u) {
-      const int64_t i = i0 + (int64_t)u * blockDim.x;
-      if (i < n) { q[u] = f.pos[i]; v[u] = f.vel[i]; }
-    }
-#pragma unroll
-    for (int u = 0; u < K; ++u) {
-      const int64_t i = i0 + (int64_t)u * blockDim.x;
-      if (i < n) {
-        pid[u] = stream_cell_f(p, q[u], Lx, Ly);
-        l0[u] = __ldg(lstart + pid[u]);
-        l1[u] = __ldg(lstart + pid[u] + 1);
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < K; ++u) {
-      const int64_t i = i0 + (int64_t)u * blockDim.x;
-      if (i < n) stream_f_apply(p, f, lrank, bcnt, bucket, queue, qn, hcap, i, q[u], v[u], pid[u], l0[u], l1[u]);
-    }
+    const int64_t i = ((int64_t)b * kMultiStreamPasses + pass) * blockDim.x + threadIdx.x;
+    if (i >= n) break;
+    bulk_f_item(p, s, cflag, h, H, i, s.pos[i], s.vel[i]);
   }
 }
 
-// members with long lists: a block per listed cell (and the overflow
-// blocks) of the single-simulation long-list kernel
-__global__ void __launch_bounds__(256, 2) km_stream_cells(Member* __restrict__ mem, const int2* __restrict__ tab,
-                                                       int par, int cap) {
-  KM_MEMBER;
-  // copies: the descriptor is not reloaded after the walk's stores; the
-  // snapshot buffer of this parity chosen without indexing the descriptor
-  DevParams p = M.p;
-  Solvent s = M.s;
-  SolventF f = M.f;
-  const Snap sn = par ? M.fb.snap[1] : M.fb.snap[0];
-  const TriPre* const pre = par ? M.fb.pre[1] : M.fb.pre[0];
-  int* const qn = M.fb.qn;
-  // the overflow counter of the next step starts at zero
-  if (b == 0 && threadIdx.x == 0) qn[par ^ 1] = 0;
-  const int nblk = (int)M.fb.bcap + kOverflowBlocks;
-  stream_cells_block<true>(p, s, f, M.c.lstart, M.c.lidx, M.c.acell, M.fb.bcnt, M.fb.bucket, sn, pre, M.fb.queue,
-                           qn + par, M.c.totals + 4, M.fb.border, b, nblk, cap);
+// a block's copy of what the near-membrane kernels read of its member
+struct NearMember {
+  DevParams p;
+  SolventArrays s;
+  NearArgs A;
+  const unsigned char* cflag;
+  const int* border;
+  int nact;
+};
+__device__ __forceinline__ void near_member(const Member& M, int par, NearMember& N) {
+  if (threadIdx.x == 0) {
+    N.s = arrays_of(M.s, M.f);
+    N.A = near_of(M.p, M.c, M.fb, par);
+    N.cflag = M.c.flag;
+    N.border = M.fb.border;
+    N.nact = M.c.totals[4];
+  }
+  for (int i = threadIdx.x; i < (int)sizeof(DevParams) / 4; i += blockDim.x) ((int*)&N.p)[i] = ((const int*)&M.p)[i];
+  __syncthreads();
 }
+#define KM_NEAR                                               \
+  __shared__ __align__(16) unsigned char raw[sizeof(NearMember)]; \
+  NearMember& N = *reinterpret_cast<NearMember*>(raw);        \
+  const int2 e_ = __ldg(tab + blockIdx.x);                    \
+  const int b = e_.y;                                         \
+  near_member(mem[e_.x], par, N)
 
-// members with short lists: kMultiCellsPer (= kShortWarps) warps per block,
-// each one listed cell of the single-simulation short-list kernel
+// members with long lists, with short lists, then the queues of all
+__global__ void __launch_bounds__(32 * kLongWarps, kLongMinBlocks)
+    km_near_long(const Member* __restrict__ mem, const int2* __restrict__ tab, int H, int par) {
+  KM_NEAR;
+  __shared__ NearCell S;
+  near_long_block<float>(N.p, N.s, N.A, b, N.border, N.nact, H, S);
+}
 __global__ void __launch_bounds__(32 * kShortWarps, kShortMinBlocks)
-    km_stream_cells_short(Member* __restrict__ mem, const int2* __restrict__ tab, int par) {
-  KM_MEMBER;
-  DevParams p = M.p;
-  Solvent s = M.s;
-  SolventF f = M.f;
-  const TriPre* const pre = par ? M.fb.pre[1] : M.fb.pre[0];
-  int* const qn = M.fb.qn;
-  // the overflow counter of the next step starts at zero
-  if (b == 0 && threadIdx.x == 0) qn[par ^ 1] = 0;
-  __shared__ LaneStage stage[kMultiCellsPer];
+    km_near_short(const Member* __restrict__ mem, const int2* __restrict__ tab, int H, int par) {
+  KM_NEAR;
+  __shared__ NearCell S[kShortWarps];
   const int w = (int)(threadIdx.x >> 5);
-  const int a = b * kMultiCellsPer + w;
-  if (a >= (int)M.fb.bcap) return;
-  stream_cells_warp<true>(p, s, f, M.c.lidx, M.fb.arng, M.fb.bcnt, M.fb.bucket, pre, M.fb.queue, qn + par,
-                          M.c.totals + 4, a, stage[w]);
+  near_short_warp<float>(N.p, N.s, N.A, b * kShortWarps + w, N.nact, H, S[w]);
+}
+__global__ void __launch_bounds__(256, 2) km_near_queue(const Member* __restrict__ mem, const int2* __restrict__ tab,
+                                                       int H, int par) {
+  KM_NEAR;
+  queue_walk<float>(N.p, N.s, N.A, N.cflag, H, (int64_t)b * 8 + (threadIdx.x >> 5), (int64_t)kQueueBlocksMember * 8);
 }
 
-// then their queues (the bulk kernel's overflow and the particles the
-// short-list kernel handed on): kQueueBlocksMember blocks per member
-__global__ void __launch_bounds__(256, 2) km_stream_queue(Member* __restrict__ mem, const int2* __restrict__ tab,
-                                                       int par) {
-  KM_MEMBER;
-  DevParams p = M.p;
-  Solvent s = M.s;
-  SolventF f = M.f;
-  const Snap sn = par ? M.fb.snap[1] : M.fb.snap[0];
-  const TriPre* const pre = par ? M.fb.pre[1] : M.fb.pre[0];
-  const int64_t gw = (int64_t)b * 8 + (threadIdx.x >> 5);
-  overflow_walk<true>(p, s, f, M.c.lstart, M.c.lidx, sn, pre, M.fb.queue, M.fb.qn + par, gw,
-                      (int64_t)kQueueBlocksMember * 8, threadIdx.x & 31);
-}
-
-int multi_stream(const MultiPlan& P, int par, cudaStream_t st, cudaEvent_t snap) {
-  km_stream_f<<<P.blocks[MP_STREAM], 256, 0, st>>>(P.mem, P.table(MP_STREAM), par);
+int multi_stream(const MultiPlan& P, int H, int par, cudaStream_t st, cudaEvent_t snap) {
+  km_stream_bulk<<<P.blocks[MP_STREAM], 256, 0, st>>>(P.mem, P.table(MP_STREAM), H, par);
   if (snap) cudaStreamWaitEvent(st, snap, 0);
-  // as the plain launch (launch_stream_cells): one warp per listed cell and
-  // one lane per particle for the members with short lists, eight warps per
-  // cell for the others, one launch per class
   const int n0 = P.cells_short, n1 = P.blocks[MP_CELLS] - P.cells_short;
-  int k = 1;
+  int k = 2;
   if (n0 > 0) {
-    km_stream_cells_short<<<n0, 32 * kShortWarps, 0, st>>>(P.mem, P.table(MP_CELLS), par);
-    ++k;
-  }
-  if (P.blocks[MP_QUEUE] > 0) {
-    km_stream_queue<<<P.blocks[MP_QUEUE], 256, 0, st>>>(P.mem, P.table(MP_QUEUE), par);
+    km_near_short<<<n0, 32 * kShortWarps, 0, st>>>(P.mem, P.table(MP_CELLS), H, par);
     ++k;
   }
   if (n1 > 0) {
-    km_stream_cells<<<n1, 256, stage_bytes(P.cells_cap), st>>>(P.mem, P.table(MP_CELLS) + n0, par, P.cells_cap);
+    km_near_long<<<n1, 32 * kLongWarps, 0, st>>>(P.mem, P.table(MP_CELLS) + n0, H, par);
     ++k;
   }
+  km_near_queue<<<P.blocks[MP_QUEUE], 256, 0, st>>>(P.mem, P.table(MP_QUEUE), H, par);
   return k;
 }
 
-// ---- membrane chain (the wide kernels' phases) --------------------------------
-__global__ void __launch_bounds__(128) km_drift(Member* __restrict__ mem, const int2* __restrict__ tab) {
-  KM_MEMBER;
-  m_drift_item(M.p, M.m, b * blockDim.x + threadIdx.x);
+// ---- membrane ----------------------------------------------------------------
+// a cluster per member; the descriptor's parts are copied to shared memory,
+// so that they are not read again from global memory after the kernel's stores
+struct SegMember {
+  DevParams p;
+  Membrane m;
+  FastBufs f;
+};
+__global__ void __launch_bounds__(kSegT) km_membrane(const Member* __restrict__ mem, const int2* __restrict__ tab,
+                                                     uint64_t eoff, int H) {
+  extern __shared__ __align__(16) unsigned char seg_sh[];
+  __shared__ __align__(16) unsigned char raw[sizeof(SegMember)];
+  SegMember& S = *reinterpret_cast<SegMember*>(raw);
+  const Member& M = mem[__ldg(tab + blockIdx.x).x];
+  auto copy = [](void* d, const void* s, int bytes) {
+    for (int i = threadIdx.x; i < bytes / 4; i += kSegT) ((int*)d)[i] = ((const int*)s)[i];
+  };
+  copy(&S.p, &M.p, sizeof(DevParams));
+  copy(&S.m, &M.m, sizeof(Membrane));
+  copy(&S.f, &M.fb, sizeof(FastBufs));
+  __syncthreads();
+  membrane_segment(S.p, S.m, S.f, epoch_of(S.p, eoff), H, SEG_WHOLE, seg_sh);
 }
-__global__ void __launch_bounds__(128) km_av(Member* __restrict__ mem, const int2* __restrict__ tab) {
-  KM_MEMBER;
-  m_av_item(M.p, M.m, b * blockDim.x + threadIdx.x);
-}
-__global__ void __launch_bounds__(256) km_sum_edges(Member* __restrict__ mem, const int2* __restrict__ tab) {
-  KM_MEMBER;
-  sum_edges_block(M.p, M.m, M.fb.slot, 1, M.fb.vd, M.fb.vw, M.fb.vX, b);
-}
-__global__ void __launch_bounds__(128) km_force_tri(Member* __restrict__ mem, const int2* __restrict__ tab) {
-  KM_MEMBER;
-  const int k = b * blockDim.x + threadIdx.x;
-  if (k < M.p.nt) force_item(M.p, M.m, M.fb.slot, M.p.ne + k);
-}
-__global__ void __launch_bounds__(32 * kGW) km_gather(Member* __restrict__ mem, const int2* __restrict__ tab) {
-  KM_MEMBER;
-  gather_block(M.p, M.m, M.fb.slot, M.fb.gstart, M.fb.gidx, b);
-}
-__global__ void __launch_bounds__(kTailT) km_tail(Member* __restrict__ mem, const int2* __restrict__ tab,
-                                                  uint64_t eoff) {
-  KM_MEMBER;
-  __shared__ TailSmem S;
-  tail_b_block(M.p, M.m, M.fb.vd, M.fb.vw, M.fb.vX, epoch_of(M.p, eoff), S);
-}
-
-int multi_membrane(const MultiPlan& P, uint64_t eoff, cudaStream_t st) {
-  km_drift<<<P.blocks[MP_DRIFT], 128, 0, st>>>(P.mem, P.table(MP_DRIFT));
-  km_av<<<P.blocks[MP_AV], 128, 0, st>>>(P.mem, P.table(MP_AV));
-  km_sum_edges<<<P.blocks[MP_SUM_EDGES], 256, P.sum_smem, st>>>(P.mem, P.table(MP_SUM_EDGES));
-  km_force_tri<<<P.blocks[MP_FORCE_TRI], 128, 0, st>>>(P.mem, P.table(MP_FORCE_TRI));
-  km_gather<<<P.blocks[MP_GATHER], 32 * kGW, 0, st>>>(P.mem, P.table(MP_GATHER));
-  km_tail<<<P.blocks[MP_TAIL], kTailT, 0, st>>>(P.mem, P.table(MP_TAIL), eoff);
-  return 6;
+__global__ void __launch_bounds__(128) km_tri_records(const Member* __restrict__ mem, const int2* __restrict__ tab,
+                                                      int H) {
+  const int2 e = __ldg(tab + blockIdx.x);
+  const Member& M = mem[e.x];
+  records_item(M.p, M.fb, H, (int64_t)e.y * blockDim.x + threadIdx.x);
 }
 
-// next half-kick, snapshot `buf` and its triangle records
-__global__ void __launch_bounds__(128) km_kick(Member* __restrict__ mem, const int2* __restrict__ tab, int buf) {
-  KM_MEMBER;
-  kick_snap_item(M.p, M.m, M.fb.snap[buf], b * blockDim.x + threadIdx.x);
-}
-__global__ void __launch_bounds__(128) km_tri_prep(Member* __restrict__ mem, const int2* __restrict__ tab,
-                                                   int buf) {
-  KM_MEMBER;
-  const int j = b * blockDim.x + threadIdx.x;
-  if (j < M.p.nt) tri_prep_one(M.p, M.m, j, M.m.vx, M.m.vy, M.m.vz, M.fb.pre[buf]);
-}
-
-int multi_kick(const MultiPlan& P, int buf, cudaStream_t st) {
-  km_kick<<<P.blocks[MP_KICK], 128, 0, st>>>(P.mem, P.table(MP_KICK), buf);
-  km_tri_prep<<<P.blocks[MP_TRI_PREP], 128, 0, st>>>(P.mem, P.table(MP_TRI_PREP), buf);
-  return 2;
+int multi_membrane(const MultiPlan& P, uint64_t eoff, int H, cudaStream_t st) {
+  const int2* tab = P.table(MP_MEMBRANE);
+  for (const MultiPlan::Seg& s : P.seg) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(s.members * s.nc);
+    cfg.blockDim = dim3(kSegT);
+    cfg.dynamicSmemBytes = s.smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = s.nc;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, km_membrane, (const Member*)P.mem, tab, eoff, H);
+    tab += s.members * s.nc;
+  }
+  km_tri_records<<<P.blocks[MP_RECORDS], 128, 0, st>>>(P.mem, P.table(MP_RECORDS), H);
+  return (int)P.seg.size() + 1;
 }
 
 // ---- collision: particle phases ---------------------------------------------------
@@ -237,45 +191,24 @@ int multi_collide_back(const MultiPlan& P, uint64_t eoff, bool resort, cudaStrea
 // launch attribute call (the request server sets new simulations up on
 // threads of their own while others step).
 void set_kernel_limits() {
-  const int cells = stage_bytes(kStageLong);
-  const int sums = 2 * kSumSmemT * (int)sizeof(double);
   const auto dyn = cudaFuncAttributeMaxDynamicSharedMemorySize;
-  cudaFuncSetAttribute(k_stream_cells<true>, dyn, cells);
-  cudaFuncSetAttribute(k_stream_cells<false>, dyn, cells);
-  cudaFuncSetAttribute(km_stream_cells, dyn, cells);
-  // eight blocks of the short-list kernels (24 KB of staging each) per SM
-  const auto carve = cudaFuncAttributePreferredSharedMemoryCarveout;
-  cudaFuncSetAttribute(k_stream_cells_short<true>, carve, (int)cudaSharedmemCarveoutMaxShared);
-  cudaFuncSetAttribute(k_stream_cells_short<false>, carve, (int)cudaSharedmemCarveoutMaxShared);
-  cudaFuncSetAttribute(km_stream_cells_short, carve, (int)cudaSharedmemCarveoutMaxShared);
-  cudaFuncSetAttribute(k_m_sum, dyn, sums);
-  cudaFuncSetAttribute(k_sum_edges, dyn, sums);
-  cudaFuncSetAttribute(km_sum_edges, dyn, sums);
-  cudaFuncSetAttribute(k_membrane_block, dyn, 96 * 1024);
-  cudaFuncSetAttribute(k_membrane_cluster, dyn, 200 * 1024);
+  cudaFuncSetAttribute(k_membrane, dyn, kSegSmemMax);
+  cudaFuncSetAttribute(km_membrane, dyn, kSegSmemMax);
+  // clusters of sixteen blocks (the discocyte's)
+  cudaFuncSetAttribute(k_membrane, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  cudaFuncSetAttribute(km_membrane, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   set_collide_kernel_limits();
 }
 
 // ---- the tables' sizes (host) -------------------------------------------------------
 void multi_blocks(const Member& M, int out[MP_NPHASE]) {
-  const DevParams& p = M.p;
   const int64_t ns = M.f.n, nc = M.c.n;
-  out[MP_STREAM] = (int)nbf(ns, 256 * kMultiStreamPer * kMultiStreamPasses);
-  {
-    // short lists: kMultiCellsPer listed cells per block, then the queue
-    // walk; long lists: a block per listed cell and the overflow blocks
-    const bool shrt = short_lists(M.fb.hcap);
-    out[MP_CELLS] = (int)(shrt ? (M.fb.bcap + kMultiCellsPer - 1) / kMultiCellsPer : M.fb.bcap + kOverflowBlocks);
-    out[MP_QUEUE] = shrt ? kQueueBlocksMember : 0;
-  }
-  out[MP_DRIFT] = (int)nb(p.nv, 128);
-  out[MP_AV] = (int)nb(p.nt, 128);
-  out[MP_SUM_EDGES] = 1 + (int)nb(2 * p.ne + p.nv, 256);
-  out[MP_FORCE_TRI] = (int)nb(p.nt, 128);
-  out[MP_GATHER] = (int)nb(p.nv, kGW);
-  out[MP_TAIL] = 1;
-  out[MP_KICK] = (int)nb(p.nv, 128);
-  out[MP_TRI_PREP] = (int)nb(p.nt, 128);
+  out[MP_STREAM] = (int)nbf(ns, 256 * kMultiStreamPasses);
+  // short lists: kShortWarps listed cells per block; long lists: one
+  out[MP_CELLS] = (int)(short_lists(M.fb.hcap) ? (M.fb.bcap + kShortWarps - 1) / kShortWarps : M.fb.bcap);
+  out[MP_QUEUE] = kQueueBlocksMember;
+  out[MP_MEMBRANE] = segment_blocks(M.p, M.fb);
+  out[MP_RECORDS] = (int)nbf((int64_t)kSegMax * M.p.nt, 128);
   out[MP_ZERO] = (int)nb(nc, 256);
   out[MP_VBIN] = 1;
   out[MP_COUNT] = (int)nbf(ns, 256 * kCountPer);
@@ -287,12 +220,16 @@ void multi_blocks(const Member& M, int out[MP_NPHASE]) {
   out[MP_MOVE] = (int)nbf(ns, 256);
 }
 
-void multi_smem(const Member& M, int out[2]) {
-  const DevParams& p = M.p;
+int multi_vbin_smem(const Member& M) {
   int n2 = 1;
-  while (n2 < p.nv) n2 <<= 1;
-  out[0] = (int)sizeof(uint64_t) * n2;
-  out[1] = p.nt <= kSumSmemT ? 2 * p.nt * (int)sizeof(double) : 0;
+  while (n2 < M.p.nv) n2 <<= 1;
+  return (int)sizeof(uint64_t) * n2;
+}
+
+int multi_segment(const Member& M, int* smem) {
+  const int nc = segment_blocks(M.p, M.fb);
+  *smem = (int)seg_smem(M.p, M.fb, nc);
+  return nc;
 }
 
 }  // namespace irbc

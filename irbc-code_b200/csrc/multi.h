@@ -10,6 +10,7 @@
 // member's buffers, with its block index within the member.  A member
 // therefore computes bit for bit what it computes alone.
 #pragma once
+#include <vector>
 #include "fp32.h"
 
 namespace irbc {
@@ -27,8 +28,7 @@ struct Member {
 
 enum MultiPhase : int {
   MP_STREAM, MP_CELLS, MP_QUEUE,                                  // streaming
-  MP_DRIFT, MP_AV, MP_SUM_EDGES, MP_FORCE_TRI, MP_GATHER, MP_TAIL,  // membrane
-  MP_KICK, MP_TRI_PREP,                                           // next half-kick and snapshot
+  MP_MEMBRANE, MP_RECORDS,                                        // membrane of a stretch
   MP_ZERO, MP_VBIN, MP_COUNT, MP_GHOST, MP_SCAN, MP_SCAN_TOP, MP_PERM, MP_TILE, MP_MOVE,  // collision
   MP_NPHASE
 };
@@ -43,38 +43,35 @@ struct MultiPlan {
   int n = 0;
   int blocks[MP_NPHASE] = {};    // each phase's grid
   // near-membrane streaming: phase MP_CELLS's table lists the blocks of the
-  // members with short lists first (cells_short of them), then the others;
-  // cells_cap: the staging piece of the long-list launch.  MP_QUEUE: the
-  // queue walk after the short-list kernel (short-list members only)
+  // members with short lists first (cells_short of them), then the others
   int cells_short = 0;
-  int cells_cap = 1;
   int vbin_smem = 0;             // vertex binning: the largest member's sort
-  int sum_smem = 0;              // ordered Sarea / Volume sums: the largest member's staging
+  // membrane: a launch per cluster size, its members' blocks in this order in
+  // phase MP_MEMBRANE's table; smem: the largest member's
+  struct Seg { int nc, members, smem; };
+  std::vector<Seg> seg;
   const int2* table(int k) const { return blk + off[k]; }
 };
 
-// the fused bulk streaming kernel: particles per thread in flight at once,
-// and passes per block (a block covers 256 * kMultiStreamPer *
+// the fused bulk streaming kernel: passes per block (a block covers 256 *
 // kMultiStreamPasses particles of its member, so that reading the member's
 // descriptor is paid once per that many)
-constexpr int kMultiStreamPer = 1, kMultiStreamPasses = 8;
-// listed cells (one warp each) per block of the fused short-list
-// near-membrane kernel
-constexpr int kMultiCellsPer = kShortWarps;
+constexpr int kMultiStreamPasses = 8;
 
 // blocks of each phase for one member (host)
 void multi_blocks(const Member& M, int out[MP_NPHASE]);
-// dynamic shared memory of the phases for one member (host): vbin, sum
-void multi_smem(const Member& M, int out[2]);
+// dynamic shared memory of the vertex binning for one member (host)
+int multi_vbin_smem(const Member& M);
+// the blocks of one member's membrane cluster and their shared memory (host)
+int multi_segment(const Member& M, int* smem);
 
-// fused launches; par = the step's parity: the snapshot buffer the
-// streaming reads and the overflow counter it uses (fb.qn[par]; the
-// near-membrane kernel clears fb.qn[par ^ 1] for the next step).  snap
-// (optional): the event the near-membrane kernel waits for (the snapshot's
-// producer).  Each returns the number of kernels it launched.
-int multi_stream(const MultiPlan& P, int par, cudaStream_t st, cudaEvent_t snap);
-int multi_membrane(const MultiPlan& P, uint64_t eoff, cudaStream_t st);
-int multi_kick(const MultiPlan& P, int buf, cudaStream_t st);
+// fused launches of a stretch of H steps; par = the stretch's parity: the queue
+// counter it uses (fb.qn[par]; the bulk kernel clears fb.qn[par ^ 1] for the
+// next one).  snap (optional): the event the near-membrane kernels wait for
+// (the records' producer).  Each returns the number of kernels it launched.
+int multi_stream(const MultiPlan& P, int H, int par, cudaStream_t st, cudaEvent_t snap);
+// the membrane of H steps, a cluster per member
+int multi_membrane(const MultiPlan& P, uint64_t eoff, int H, cudaStream_t st);
 // A collision, in this order: multi_collide_front (kernels.cu: the cell
 // counters cleared, the vertices binned), multi_collide_count (fast.cu: the
 // particles counted into their shifted cells), multi_collide_scan

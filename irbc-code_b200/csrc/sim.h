@@ -50,6 +50,8 @@ struct Cells {
   int64_t lcap = 0, lcap2 = 0;
   int *lrank = nullptr;         // rank among the cells with a non-empty list
   int *acell = nullptr;         // the cell of each such rank
+  unsigned char* flag = nullptr;  // 1: listed; 2: a flight of less than a cell from it may meet a listed
+                                // cell, a side wall or the grid's edge
   int nact = 0, lmax = 0;       // (host) their number and the longest list
   int *scan_part = nullptr;     // scan scratch: 3 ints per block
   int64_t scan_blocks = 0;
@@ -116,7 +118,6 @@ void launch_collide_finish(const DevParams& p, Solvent& s, Cells& c, Membrane& m
 // physical re-sort by the cells of the latest collision (any time after it)
 void launch_resort(Solvent& s, cudaStream_t st);
 void launch_ghost_flags(const DevParams& p, Cells& c, const Membrane& m, cudaStream_t st);
-void launch_stream(const DevParams& p, Solvent& s, const Cells& c, const Membrane& m, cudaStream_t st);
 // returns the total list length the update needs (host sync inside)
 int64_t launch_llist_count(const DevParams& p, Cells& c, const Membrane& m, cudaStream_t st);
 // total: the entry count launch_llist_count returned (both list buffers hold it)
