@@ -300,6 +300,7 @@ void free_fast(FastBufs& f) {
   for (int** q : {&f.gstart, &f.gidx, &f.vd, &f.pidx, &f.st1, &f.st2, &f.st3}) dfree(*q);
   dfree(f.pre);
   dfree(f.bands);
+  dfree(f.cull);
   dfree(f.patch.hdr);
   dfree(f.patch.blob);
   f.patch = PatchPlan{};
@@ -560,6 +561,7 @@ int upload_mesh(irbc_handle* h, const HostMesh& M) {
       CK(dalloc(q, (int64_t)kSegMax * M.nv));
     CK(dalloc(&f.pre, (int64_t)kSegMax * M.nt));
     CK(dalloc(&f.bands, (int64_t)kSegMax * M.nt));
+    CK(dalloc(&f.cull, 3 * (int64_t)M.nt));
     CK(dalloc(&f.pidx, M.nv));
     for (int** q : {&f.st1, &f.st2, &f.st3}) CK(dalloc(q, M.nt));
     f.snap.t1 = f.st1; f.snap.t2 = f.st2; f.snap.t3 = f.st3;
@@ -699,9 +701,6 @@ int stream_any(irbc_handle* h, int H, cudaStream_t st, cudaEvent_t snap = nullpt
     e0 = next_event(h);
     e1 = next_event(h);
   }
-  // the capacity follows the longest list; captured steps keep the largest, so
-  // that a replay stays valid after the lists grow
-  h->fb.hcap = (h->graphs_on || h->capturing) ? kHeavyList : heavy_cap(h->c.lmax);
   return fast_stream(h->dp, h->s, h->fp32 ? &h->sf : nullptr, h->c, h->fb, H, st, e0, e1, snap);
 }
 
@@ -727,9 +726,9 @@ extern "C" int64_t irbc_footprint_bytes(const irbc_params* p, int32_t nv, int32_
   int64_t ns = p->Ns;
   int64_t b = ns * (2 * (3 * 8 + 32 + 2 * 4) + 4 * 4 + 1);  // two buffer sets + key/slot/perm/stream queue
   if (p->precision == IRBC_FP32) b += ns * (2 * 32 + 2 * 4);  // float4 sets + cell ids
-  b += C * (7 * 4 + 1) + (C + 1) * 4 * 3;            // cell counts/ranks/flags + cell and llist starts
+  b += C * (5 * 4 + 1) + (C + 1) * 4 * 3;            // cell counts/ranks/flags + cell and llist starts
   b += (int64_t)nv * (12 * 8 + 8 * 4 + kMaxPairs * 12) + (int64_t)ne * 40 + (int64_t)nt * 80;
-  b += kSegMax * ((int64_t)nv * 48 + (int64_t)nt * 97);  // a stretch's snapshots and triangle records
+  b += kSegMax * ((int64_t)nv * 48 + (int64_t)nt * 100);  // a stretch's snapshots and triangle records
   b += 2 * (int64_t)(4 * p->Lx * 4 * p->Ly) * 16;    // ligands
   b += 2 * C * 4 * 8;                                 // llist entries (typical)
   return b;
@@ -800,7 +799,7 @@ extern "C" int irbc_create(const irbc_params* p, irbc_handle** out) {
   A(dalloc(&s.v, s.n));
   A(dalloc(&s.v2, s.n));
   for (int** q : {&s.indio, &s.pid, &s.indio2, &s.pid2, &s.key, &s.slot, &s.perm}) A(dalloc(q, s.n));
-  for (int** q : {&c.cnt, &c.ncm, &c.wrank, &c.mrank, &c.lcnt, &c.lrank, &c.acell}) A(dalloc(q, c.n));
+  for (int** q : {&c.cnt, &c.ncm, &c.wrank, &c.mrank, &c.lcnt}) A(dalloc(q, c.n));
   A(dalloc(&c.start, c.n + 1));
   A(dalloc(&c.lstart, c.n + 1));
   A(dalloc(&c.lstart2, c.n + 1));
@@ -823,7 +822,7 @@ extern "C" int irbc_create(const irbc_params* p, irbc_handle** out) {
   A(dalloc(&h->fb.queue, s.n));
   A(dalloc(&h->fb.qk, s.n));
   A(dalloc(&c.flag, c.n));
-  A(dalloc(&h->fb.qn, 4));
+  A(dalloc(&h->fb.qn, 8));
   if (p->precision == IRBC_FP32) {
     h->fp32 = true;
     h->sf.n = s.n;
@@ -833,7 +832,7 @@ extern "C" int irbc_create(const irbc_params* p, irbc_handle** out) {
   }
   if (rc) { irbc_destroy(h); return create_failed(rc, "device allocation"); }
   cudaMemsetAsync(c.lstart, 0, sizeof(int) * (c.n + 1), h->st);
-  cudaMemsetAsync(c.flag, 2, c.n, h->st);
+  cudaMemsetAsync(c.flag, CF_MEETS, c.n, h->st);
   cudaMemsetAsync(h->m.ligi, 0, sizeof(int) * h->dp.nlig, h->st);
   cudaMemsetAsync(h->m.sc, 0, sizeof(MemScalars), h->st);
   cudaMemsetAsync(h->ebase, 0, sizeof(uint64_t), h->st);
@@ -856,8 +855,7 @@ extern "C" void irbc_destroy(irbc_handle* h) {
   if (h->st2_own) cudaStreamSynchronize(h->st2_own);
   invalidate_graphs(h);
   free_fast(h->fb);
-  dfree(h->fb.queue); dfree(h->fb.qk); dfree(h->c.flag); dfree(h->fb.qn); dfree(h->fb.bcnt); dfree(h->fb.bucket); dfree(h->fb.border);
-  dfree(h->fb.arng);
+  dfree(h->fb.queue); dfree(h->fb.qk); dfree(h->c.flag); dfree(h->fb.qn);
   if (h->rec) cudaFree(h->rec);
   for (float4** q : {&h->sf.pos, &h->sf.vel, &h->sf.pos2, &h->sf.vel2}) dfree(*q);
   dfree(h->sf.pid); dfree(h->sf.pid2);
@@ -872,7 +870,7 @@ extern "C" void irbc_destroy(irbc_handle* h) {
   dfree(s.v);
   dfree(s.v2);
   for (int** q : {&s.indio, &s.pid, &s.indio2, &s.pid2, &s.key, &s.slot, &s.perm}) dfree(*q);
-  for (int** q : {&c.cnt, &c.ncm, &c.wrank, &c.mrank, &c.lcnt, &c.lrank, &c.acell, &c.start, &c.lstart,
+  for (int** q : {&c.cnt, &c.ncm, &c.wrank, &c.mrank, &c.lcnt, &c.start, &c.lstart,
                   &c.lstart2, &c.totals,
                   &c.scan_part, &c.lidx, &c.lidx2})
     dfree(*q);
@@ -912,40 +910,12 @@ extern "C" int irbc_health(irbc_handle* h, int32_t* flags) {
 }
 
 // ---- llist -----------------------------------------------------------------
-// ranks of the cells with a list, and room for them in the near-membrane
-// streaming buckets
+// what the streaming reads of new lists besides their entries
 static int refresh_listed(irbc_handle* h) {
-  Cells& c = h->c;
-  const int k = launch_llist_ranks(h->dp, c, h->st);
+  const int k = launch_llist_flags(h->dp, h->c, h->st);
   if (k < 0) return fail(h, IRBC_ERR_CUDA, cudaGetErrorString(cudaGetLastError()));
   g_launches += k;
-  FastBufs& f = h->fb;
-  if (c.nact > f.bcap) {
-    invalidate_graphs(h);  // the buckets move
-    dfree(f.bcnt);
-    dfree(f.bucket);
-    dfree(f.border);
-    dfree(f.arng);
-    f.bcap = c.nact + c.nact / 2 + 64;
-    CK(dalloc(&f.bcnt, f.bcap));
-    CK(dalloc(&f.bucket, f.bcap * kBucket));
-    CK(dalloc(&f.border, f.bcap));
-    CK(dalloc(&f.arng, f.bcap));
-    CK(cudaMemsetAsync(f.bcnt, 0, sizeof(int) * f.bcap, h->st));
-  }
-  // the near-membrane streaming takes the listed cells longest list first,
-  // so that the heaviest blocks do not start last (order of work only)
-  if (c.nact > 0) {
-    std::vector<int> len(c.nact), order(c.nact);
-    launch_rank_lengths(c, f.border, f.arng, h->st);
-    g_launches += 1;
-    CK(cudaMemcpyAsync(len.data(), f.border, sizeof(int) * c.nact, cudaMemcpyDeviceToHost, h->st));
-    CK(cudaStreamSynchronize(h->st));
-    for (int a = 0; a < c.nact; ++a) order[a] = a;
-    std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return len[x] > len[y]; });
-    CK(cudaMemcpyAsync(f.border, order.data(), sizeof(int) * c.nact, cudaMemcpyHostToDevice, h->st));
-    CK(cudaStreamSynchronize(h->st));
-  }
+  h->fb.lmax = h->c.lmax;
   return 0;
 }
 
@@ -1743,9 +1713,6 @@ static Member member_of(irbc_handle* h) {
   M.c = h->c;
   M.m = h->m;
   M.fb = h->fb;
-  // the staging capacity follows the longest list (as stream_any does for
-  // plain launches)
-  M.fb.hcap = heavy_cap(h->c.lmax);
   // host-only counters that no kernel reads
   M.s.ncoll = M.s.resorted = 0;
   return M;
@@ -1764,16 +1731,11 @@ static int cohort_upload(Cohort* c) {
   std::vector<std::array<int, MP_NPHASE>> nbk(n);
   int64_t tot[MP_NPHASE] = {};
   P.vbin_smem = 0;
-  P.cells_short = 0;
-  std::vector<int> cls(n);  // the near-membrane class of each member: 0 short lists, 1 long lists
   for (size_t r = 0; r < n; ++r) {
     c->host[r] = member_of(c->members[r]);
     c->uids[r] = c->members[r]->uid;
     multi_blocks(c->host[r], nbk[r].data());
     for (int k = 0; k < MP_NPHASE; ++k) tot[k] += nbk[r][k];
-    const int hcap = c->host[r].fb.hcap;
-    cls[r] = short_lists(hcap) ? 0 : 1;
-    if (cls[r] == 0) P.cells_short += nbk[r][MP_CELLS];
     P.vbin_smem = std::max(P.vbin_smem, multi_vbin_smem(c->host[r]));
   }
   // the membrane's launches: members by the size of their cluster
@@ -1800,12 +1762,10 @@ static int cohort_upload(Cohort* c) {
   std::vector<int2> tab((size_t)all);
   for (int k = 0; k < MP_NPHASE; ++k) {
     int64_t q = P.off[k];
-    // the near-membrane and the membrane blocks class by class (one launch
-    // per class)
-    const int classes = k == MP_CELLS ? 2 : (k == MP_MEMBRANE ? (int)P.seg.size() : 1);
+    // the membrane blocks class by class (one launch per class)
+    const int classes = k == MP_MEMBRANE ? (int)P.seg.size() : 1;
     for (int pass = 0; pass < classes; ++pass)
       for (size_t r = 0; r < n; ++r) {
-        if (k == MP_CELLS && cls[r] != pass) continue;
         if (k == MP_MEMBRANE && scls[r] != pass) continue;
         for (int b = 0; b < nbk[r][k]; ++b) tab[(size_t)q++] = make_int2((int)r, b);
       }
@@ -1867,7 +1827,7 @@ int cohort_step(Cohort* c, const std::vector<irbc_handle*>& all, int64_t n, std:
       return IRBC_ERR_CUDA;
     h->ebase_val = h->step;
     launch_set_u64(h->ebase, (uint64_t)h->step, ms);
-    if (cudaMemsetAsync(h->fb.qn, 0, 2 * sizeof(int), ms) != cudaSuccess) return IRBC_ERR_CUDA;
+    if (cudaMemsetAsync(h->fb.qn, 0, 8 * sizeof(int), ms) != cudaSuccess) return IRBC_ERR_CUDA;
     launched += 1;
   }
   if (cudaEventRecord(c->ev_coll, ms) != cudaSuccess || cudaStreamWaitEvent(ss, c->ev_coll, 0) != cudaSuccess)

@@ -194,12 +194,20 @@ template <typename R>
 struct Flight {
   R X, Y, Z, VX, VY, VZ;
 };
+// its cell; on: whether that is where it lies (positions off the grid count as
+// cell 0, and positions beyond a side as their image's cell)
 template <typename R>
-__device__ __forceinline__ int cell_at(const DevParams& p, R X, R Y, R Z) {
+__device__ __forceinline__ int cell_at(const DevParams& p, R X, R Y, R Z, bool& on) {
   const int fx = (int)floor(bbound(X, (R)p.Lx));
   const int fy = (int)floor(bbound(Y, (R)p.Ly));
   const int fz = (int)floor(Z + R(1));
+  on = X >= R(0) && X <= (R)p.Lx && fx < p.nx && Y >= R(0) && Y <= (R)p.Ly && fy < p.ny && fz >= 0 && fz < p.nz;
   return cell_of(p, fx, fy, fz);
+}
+template <typename R>
+__device__ __forceinline__ int cell_at(const DevParams& p, R X, R Y, R Z) {
+  bool on;
+  return cell_at(p, X, Y, Z, on);
 }
 // one step of free flight
 __device__ __forceinline__ void free_step(const DevParams& p, Flight<double>& q) {
@@ -249,35 +257,18 @@ __device__ __forceinline__ void flight_store(const SolventArrays& s, int64_t i, 
   s.vel[i] = make_float4(q.VX, q.VY, q.VZ, s.vel[i].w);
 }
 
-// ---- hand-off to the near-membrane kernels -------------------------------------------
-// Particle i, in a listed cell from step k of the stretch on: into the bucket of
-// that cell (rank lrank among the listed cells) when the list fits the kernels'
-// capacity hcap and the bucket has room, else onto the queue.
-struct HandOff {
-  const int* lstart;
-  const int* lrank;
-  int* bcnt;
-  int2* bucket;
-  int* queue;
-  unsigned char* qk;
-  int* qn;
-  int hcap;
+// ---- hand-over to the near-membrane kernel -------------------------------------------
+// particle i, in a listed cell from step k of the stretch on, onto the queue
+struct NearQueue {
+  int* i;
+  unsigned char* k;
+  int* n;  // their number; n[4]: those taken
 };
-inline __host__ __device__ HandOff hand_off_of(const Cells& c, const FastBufs& f, int par) {
-  return HandOff{c.lstart, c.lrank, f.bcnt, f.bucket, f.queue, f.qk, f.qn + par, f.hcap};
-}
-__device__ __forceinline__ void enqueue(const HandOff& h, int i, int k) {
-  const int q = atomicAdd(h.qn, 1);
-  h.queue[q] = i;
-  h.qk[q] = (unsigned char)k;
-}
-__device__ __forceinline__ void hand_off(const HandOff& h, int pid, int i, int k) {
-  if (h.lstart[pid + 1] - h.lstart[pid] <= h.hcap) {
-    const int a = h.lrank[pid];
-    const int slot = atomicAdd(h.bcnt + a, 1);
-    if (slot < kBucket) { h.bucket[(int64_t)a * kBucket + slot] = make_int2(i, k); return; }
-  }
-  enqueue(h, i, k);
+inline __host__ __device__ NearQueue queue_of(const FastBufs& f, int par) { return NearQueue{f.queue, f.qk, f.qn + par}; }
+__device__ __forceinline__ void enqueue(const NearQueue& h, int i, int k) {
+  const int q = atomicAdd(h.n, 1);
+  h.i[q] = i;
+  h.k[q] = (unsigned char)k;
 }
 
 // ---- the bulk of a stretch --------------------------------------------------------------
@@ -285,92 +276,96 @@ __device__ __forceinline__ void hand_off(const HandOff& h, int pid, int i, int k
 // pass takes each particle through all H steps of the stretch: its state is
 // read and written once instead of H times.  The arithmetic is the steps', one
 // after the other.  A particle that a step finds in a listed cell is handed over
-// at that step, with its state.  `cflag` tells per cell whether it is listed
-// (1), and whether a particle in it that flies less than a cell may meet a
-// listed cell, a side wall or the grid's edge (2): the others need no look at
-// the cells on their way.  Bound by HBM: FP64 80 bytes a particle (the 32-byte
-// record carries the index), FP32 48.
+// at that step, with its state.  The cell flags (CF_*, launch_llist_ranks) tell
+// what a particle that flies less than a cell can meet from each cell: most need
+// neither a look at the cells on their way nor wraps nor walls, and 36 additions
+// are all the 12 steps cost.  Bound by HBM: FP64 80 bytes a particle (the
+// 32-byte record carries the index), FP32 48.
 template <typename R>
 __device__ __forceinline__ bool flies_free(const DevParams& p, const Flight<R>& q, unsigned char cf, int H) {
   // (a moving top wall gives its speed to what it reflects)
   const R reach = fmax(fmax(fabs(q.VX), fabs(q.VY)), fmax(fabs(q.VZ), fabs((R)p.wallspeed))) * (R)(H * p.dtmd);
-  return !(cf & 2) && reach < R(0.99);
+  return !(cf & CF_MEETS) && reach < R(0.99);
 }
-// through steps k .. H-1; returns H, or the step that finds it in a listed cell
-// (pid)
-__device__ __forceinline__ void fly_free(const DevParams& p, Flight<double>& q, int H) {
-  double dx = q.VX * p.dtmd, dy = q.VY * p.dtmd, dz = q.VZ * p.dtmd;
-  for (int k = 0; k < H; ++k) {
-    q.X += dx; q.Y += dy; q.Z += dz;
-    if (q.Z > p.Lz || q.Z < 0) {
-      wall_step(p, p.dtmd, q.X, q.Y, q.Z, q.VX, q.VY, q.VZ);
-      dx = q.VX * p.dtmd; dy = q.VY * p.dtmd; dz = q.VZ * p.dtmd;
-    }
+__device__ __forceinline__ void wall_of(const DevParams& p, Flight<double>& q) {
+  wall_step(p, p.dtmd, q.X, q.Y, q.Z, q.VX, q.VY, q.VZ);
+}
+__device__ __forceinline__ void wall_of(const DevParams& p, Flight<float>& q) {
+  wall_step_f((float)p.wallspeed, (float)p.Lz, (float)p.dtmd, q.X, q.Y, q.Z, q.VX, q.VY, q.VZ);
+}
+// H steps away from every listed cell
+template <typename R>
+__device__ __forceinline__ void fly_free(const DevParams& p, Flight<R>& q, unsigned char cf, int H) {
+  const R dt = (R)p.dtmd;
+  R dx = q.VX * dt, dy = q.VY * dt, dz = q.VZ * dt;
+  if (!(cf & (CF_SIDE | CF_WALL))) {
+    for (int k = 0; k < H; ++k) { q.X += dx; q.Y += dy; q.Z += dz; }
+    return;
   }
-}
-__device__ __forceinline__ void fly_free(const DevParams& p, Flight<float>& q, int H) {
-  const float Lz = (float)p.Lz, dt = (float)p.dtmd;
-  float dx = q.VX * dt, dy = q.VY * dt, dz = q.VZ * dt;
+  const R Lx = (R)p.Lx, Ly = (R)p.Ly, Lz = (R)p.Lz;
   for (int k = 0; k < H; ++k) {
     q.X += dx; q.Y += dy; q.Z += dz;
-    if (q.Z > Lz || q.Z < 0.0f) {
-      wall_step_f((float)p.wallspeed, Lz, dt, q.X, q.Y, q.Z, q.VX, q.VY, q.VZ);
+    if (q.Z > Lz || q.Z < R(0)) {
+      wall_of(p, q);
       dx = q.VX * dt; dy = q.VY * dt; dz = q.VZ * dt;
     }
+    // (bbound: less than a period away)
+    if (q.X > Lx) q.X -= Lx;
+    if (q.X < R(0)) q.X += Lx;
+    if (q.Y > Ly) q.Y -= Ly;
+    if (q.Y < R(0)) q.Y += Ly;
   }
 }
+// through the stretch; returns H, or the step that finds the particle in a
+// listed cell
 template <typename R>
-__device__ __forceinline__ int fly(const DevParams& p, Flight<R>& q, const unsigned char* __restrict__ cflag, int H,
-                                   int& pid) {
-  pid = cell_at(p, q.X, q.Y, q.Z);
-  unsigned char cf = __ldg(cflag + pid);
-  if (flies_free(p, q, cf, H)) {
-    fly_free(p, q, H);
+__device__ __forceinline__ int fly(const DevParams& p, Flight<R>& q, const unsigned char* __restrict__ cflag, int H) {
+  bool on;
+  unsigned char cf = __ldg(cflag + cell_at(p, q.X, q.Y, q.Z, on));
+  if (on && flies_free(p, q, cf, H)) {
+    fly_free(p, q, cf, H);
     raise_health(p, solvent_bad(p, q.X, q.Y, q.Z, q.VX, q.VY, q.VZ), HEALTH_SOLVENT);
     return H;
   }
   for (int k = 0;;) {
-    if (cf & 1) return k;
+    if (cf & CF_LISTED) return k;
     free_step(p, q);
     raise_health(p, solvent_bad(p, q.X, q.Y, q.Z, q.VX, q.VY, q.VZ), HEALTH_SOLVENT);
     if (++k == H) return H;
-    pid = cell_at(p, q.X, q.Y, q.Z);
-    cf = __ldg(cflag + pid);
+    cf = __ldg(cflag + cell_at(p, q.X, q.Y, q.Z));
   }
 }
 
 __global__ void __launch_bounds__(256) k_stream_bulk(DevParams p, SolventArrays s, int64_t n,
-                                                     const unsigned char* __restrict__ cflag, HandOff h, int H) {
+                                                     const unsigned char* __restrict__ cflag, NearQueue h, int H) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const double X = s.x[i], Y = s.y[i], Z = s.z[i];
   const SolVel r = s.v[i];
   Flight<double> q{X, Y, Z, r.vx, r.vy, r.vz};
-  int pid;
-  const int k = fly(p, q, cflag, H, pid);
+  const int k = fly(p, q, cflag, H);
   if (k > 0) {
     s.x[i] = q.X; s.y[i] = q.Y; s.z[i] = q.Z;
     if (q.VX != r.vx || q.VY != r.vy || q.VZ != r.vz || r.vx != r.vx) {
       s.v[i].vx = q.VX; s.v[i].vy = q.VY; s.v[i].vz = q.VZ;
     }
   }
-  if (k < H) hand_off(h, pid, (int)i, k);
+  if (k < H) enqueue(h, (int)i, k);
 }
 // one particle of the FP32-bulk solvent, loaded as (a, b)
 __device__ __forceinline__ void bulk_f_item(const DevParams& p, const SolventArrays& s,
-                                            const unsigned char* __restrict__ cflag, const HandOff& h, int H, int64_t i,
+                                            const unsigned char* __restrict__ cflag, const NearQueue& h, int H, int64_t i,
                                             float4 a, float4 b) {
   Flight<float> q{a.x, a.y, a.z, b.x, b.y, b.z};
-  int pid;
-  const int k = fly(p, q, cflag, H, pid);
+  const int k = fly(p, q, cflag, H);
   if (k > 0) {
     s.pos[i] = make_float4(q.X, q.Y, q.Z, a.w);
     if (q.VX != b.x || q.VY != b.y || q.VZ != b.z || b.x != b.x) s.vel[i] = make_float4(q.VX, q.VY, q.VZ, b.w);
   }
-  if (k < H) hand_off(h, pid, (int)i, k);
+  if (k < H) enqueue(h, (int)i, k);
 }
 __global__ void __launch_bounds__(256) k_stream_bulk_f(DevParams p, SolventArrays s, int64_t n,
-                                                       const unsigned char* __restrict__ cflag, HandOff h, int H) {
+                                                       const unsigned char* __restrict__ cflag, NearQueue h, int H) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) bulk_f_item(p, s, cflag, h, H, i, s.pos[i], s.vel[i]);
 }
@@ -416,60 +411,73 @@ __device__ __forceinline__ int band_of(const DevParams& p, double x, double y) {
   return (x < l ? BAND_HX : (x > rx ? BAND_LX : 0)) | (y < l ? BAND_HY : (y > ry ? BAND_LY : 0));
 }
 
-// The triangle walk of reflectionFed for one particle, by a whole warp:
-// lanes run the crossing test on 32 list entries at a time, and every
-// crossing candidate gets the full test (contact time, barycentric test) on
-// its own lane, all from the same particle state.  The reference's loop
-// changes the state only at a hit, so up to and including the first hit of
-// the 32 these are exactly its tests: the lowest hit is applied and the walk
-// resumes after it with the updated state -- the same sequence of states as
-// the sequential loop.  L: the list's triangles, len of them; pre, bands: this
-// step's records.
-__device__ __forceinline__ void heavy_walk(const DevParams& p, const Snap& sn, const TriPre* __restrict__ pre,
-                                           const unsigned char* __restrict__ bands, const int* __restrict__ L, int len,
-                                           int lane, int indio, double& X, double& Y, double& Z, double& VX, double& VY,
-                                           double& VZ, double& fulldt) {
-  for (int cur = 0; cur < len;) {
-    const int band = band_of(p, X, Y);
-    const int e = cur + lane;
-    double x = X, y = Y, z = Z, vx = VX, vy = VY, vz = VZ, fd = 0.0;
-    bool hit = false;
-    if (e < len) {
-      const int jj = __ldg(L + e);
-      const TriPre t = ldg_tri(pre + jj);
-      const bool plain = !(__ldg(bands + jj) & band);
-      if (!plain || tri_crossing(t, X, Y, Z, X + VX * p.dtmd, Y + VY * p.dtmd, Z + VZ * p.dtmd, indio))
-        hit = tri_visit(p, sn, t, jj, x, y, z, vx, vy, vz, indio, fd, plain);
-    }
-    const unsigned hb = __ballot_sync(0xffffffffu, hit);
-    if (hb == 0u) {
-      cur += 32;
-      continue;
-    }
-    const int src = __ffs(hb) - 1;
-    X = __shfl_sync(0xffffffffu, x, src);
-    Y = __shfl_sync(0xffffffffu, y, src);
-    Z = __shfl_sync(0xffffffffu, z, src);
-    VX = __shfl_sync(0xffffffffu, vx, src);
-    VY = __shfl_sync(0xffffffffu, vy, src);
-    VZ = __shfl_sync(0xffffffffu, vz, src);
-    fulldt += __shfl_sync(0xffffffffu, fd, src);
-    cur += src + 1;
+// What no step of a stretch can make a crossing candidate, found once per
+// particle and stretch instead of in every step.  A candidate crosses the
+// triangle's plane: b_t = X_t . (P_t - A_t) changes sign, X_t the normal and A_t
+// the corner at step t, P_t the particle.  With the triangle's largest changes
+// over the stretch, dX of the normal and dA of the corner, and the particle's
+// path dP (speed x time left),
+//   |b_t - X_0 . (P - A_0)| <= dX (|P - A_0| + dP + dA) + |X_0| (dP + dA),
+// so an entry whose plane is farther away needs no test.  About 5% of the
+// 600-vertex mesh's entries and 10% of the discocyte's are left.  TriCull holds
+// what that takes in float; m covers the rounding: the coordinates' is at most
+// L 2^-24 each in a box of length L, that of the differences, products and sums
+// 4 parts in 2^24 of theirs, with differences up to L, and (L + 16) 2^-21 of the
+// normal's 1-norm covers both twice.  (NaN and infinities fail the comparison
+// and are kept.)  bands: of the triangle's corners in any of the steps.
+struct TriCull {
+  float X[3], nX, A[3], dX, dA, m;
+  int bands;
+};
+__device__ __forceinline__ TriCull ldg_cull(const float4* __restrict__ r) {
+  const float4 a = __ldg(r), b = __ldg(r + 1), c = __ldg(r + 2);
+  return TriCull{{a.x, a.y, a.z}, a.w, {b.x, b.y, b.z}, b.w, c.x, c.y, __float_as_int(c.z)};
+}
+__device__ __forceinline__ bool cull_keeps(const TriCull& c, float X, float Y, float Z, float dP, int band) {
+  const float x = X - c.A[0], y = Y - c.A[1], z = Z - c.A[2];
+  const float b = fabsf(c.X[0] * x + c.X[1] * y + c.X[2] * z);
+  const float d = sqrtf(x * x + y * y + z * z), move = dP + c.dA;
+  return (c.bands & band) || !(b > 1.0001f * (c.dX * (d + move) + c.nX * move) + c.m);
+}
+// triangle j's over H steps
+__device__ __forceinline__ void cull_item(const DevParams& p, const FastBufs& f, int H, int j) {
+  if (j >= p.nt) return;
+  const TriPre t0 = f.pre[j];
+  double dX = 0.0, dA = 0.0;
+  int bands = 0;
+  auto norm = [](double x, double y, double z) { return sqrt(x * x + y * y + z * z); };
+  for (int s = 0; s < H; ++s) {
+    const TriPre t = f.pre[(int64_t)s * p.nt + j];
+    dX = fmax(dX, fmax(norm(t.X[0] - t0.X[0], t.X[1] - t0.X[1], t.X[2] - t0.X[2]),
+                       norm(t.Xdt[0] - t0.X[0], t.Xdt[1] - t0.X[1], t.Xdt[2] - t0.X[2])));
+    dA = fmax(dA, fmax(norm(t.A1[0] - t0.A1[0], t.A1[1] - t0.A1[1], t.A1[2] - t0.A1[2]),
+                       norm(t.A2[0] - t0.A1[0], t.A2[1] - t0.A1[1], t.A2[2] - t0.A1[2])));
+    // a record that is not finite stays in every test
+    if (!isfinite(t.X[0] + t.X[1] + t.X[2] + t.Xdt[0] + t.Xdt[1] + t.Xdt[2] + t.A1[0] + t.A1[1] + t.A1[2] + t.A2[0] +
+                  t.A2[1] + t.A2[2]))
+      dX = dA = __longlong_as_double(0x7ff0000000000000ll);
+    bands |= f.bands[(int64_t)s * p.nt + j];
   }
+  const double L = fmax(p.Lx, fmax(p.Ly, p.Lz));
+  const double n1 = fabs(t0.X[0]) + fabs(t0.X[1]) + fabs(t0.X[2]) + dX;
+  float4* to = f.cull + 3 * (int64_t)j;
+  to[0] = make_float4((float)t0.X[0], (float)t0.X[1], (float)t0.X[2], (float)norm(t0.X[0], t0.X[1], t0.X[2]) * 1.00001f);
+  to[1] = make_float4((float)t0.A1[0], (float)t0.A1[1], (float)t0.A1[2], (float)dX * 1.00001f);
+  to[2] = make_float4((float)dA * 1.00001f, (float)(n1 * (L + 16.0) * (1.0 / 2097152.0)), __int_as_float(bands), 0.0f);
 }
 
-// what the near-membrane kernels read of one simulation
+// what the near-membrane kernel reads of one simulation
 struct NearArgs {
-  const int *lstart, *lidx, *acell;
-  const int2* arng;
+  const int *lstart, *lidx;
+  const unsigned char *flag, *bands;
   const TriPre* pre;
-  const unsigned char* bands;
+  const float4* cull;
   int64_t nt, nv;
   Snap snap;
-  HandOff h;
+  NearQueue q;
 };
 inline __host__ __device__ NearArgs near_of(const DevParams& p, const Cells& c, const FastBufs& f, int par) {
-  return NearArgs{c.lstart, c.lidx, c.acell, f.arng, f.pre, f.bands, p.nt, p.nv, f.snap, hand_off_of(c, f, par)};
+  return NearArgs{c.lstart, c.lidx, c.flag, f.bands, f.pre, f.cull, p.nt, p.nv, f.snap, queue_of(f, par)};
 }
 __device__ __forceinline__ Snap near_snap(const NearArgs& a, int t) {
   Snap s = a.snap;
@@ -478,229 +486,183 @@ __device__ __forceinline__ Snap near_snap(const NearArgs& a, int t) {
   return s;
 }
 
-// The particles of one listed cell through the rest of the stretch, by W warps
-// (reflectionFed, :400-598, then the walls and wrap).  Each thread holds the
-// record of a list entry in registers and runs the crossing test on the cell's
-// particles, whose states lie in shared memory.  Nothing is staged, and the particles' states
-// stay here between the steps.  Then
-//   FULL (long lists; about 0.4 candidates per particle and step, most of them
-//   crossing the plane of a triangle elsewhere): every candidate gets the full
-//   test by a thread of its own; a particle that hits something walks the list
-//   as the reference does (heavy_walk).
-//   otherwise (short lists, 0.6% of particles have a candidate): a particle with
-//   a candidate goes onto the queue, for the rest of the stretch, so that the
-//   full test's registers stay out of this kernel.
-// A particle that leaves the cell goes onto the queue too.
-constexpr int kCand = 128;
-struct NearCell {
-  double st[6][kBucket], to[3][kBucket];
-  int id[kBucket], k0[kBucket], indio[kBucket], band[kBucket], hit[kBucket];
-  unsigned cand[kCand];
-  int nc, done;
-  unsigned act, leave;
-};
-template <int W>
-__device__ __forceinline__ void near_sync() {
-  if (W == 1) __syncwarp();
-  else __syncthreads();
+// reflectionFed's test of entry e (triangle jj) at step t for a particle:
+// whether it hits; then the state after it and the time fd to it
+__device__ __forceinline__ bool near_hit(const DevParams& p, const NearArgs& A, int t, int jj, int band, int indio,
+                                         double& x, double& y, double& z, double& vx, double& vy, double& vz,
+                                         double& fd) {
+  const int64_t at = (int64_t)t * A.nt + jj;
+  const TriPre r = ldg_tri(A.pre + at);
+  const bool plain = !(__ldg(A.bands + at) & band);
+  if (plain && !tri_crossing(r, x, y, z, x + vx * p.dtmd, y + vy * p.dtmd, z + vz * p.dtmd, indio)) return false;
+  return tri_visit(p, near_snap(A, t), r, jj, x, y, z, vx, vy, vz, indio, fd, plain);
 }
-template <typename R, int W, bool FULL>
-__device__ __forceinline__ void near_cell(const DevParams& p, const SolventArrays& s, const NearArgs& A, int a, int n,
-                                          int H, NearCell& S) {
-  const int tid = W == 1 ? (threadIdx.x & 31) : threadIdx.x, lane = threadIdx.x & 31;
-  constexpr int T = 32 * W;
-  const int2 rg = __ldg(A.arng + a);
-  const int l0 = rg.x, len = rg.y, home = __ldg(A.acell + a);
-  // thread j < n looks after particle j
-  Flight<R> q{};
-  int me = -1, from = 0;
-  if (tid < n) {
-    const int2 b = A.h.bucket[(int64_t)a * kBucket + tid];
-    me = b.x;
-    from = b.y;
-    S.indio[tid] = flight_load(s, me, q);
-    S.id[tid] = me;
-  }
-  const int jj0 = tid < len ? __ldg(A.lidx + l0 + tid) : 0;
-  TriPre next{};
-  int nband = 0;
-  if (FULL && tid < len) { next = ldg_tri(A.pre + jj0); nband = __ldg(A.bands + jj0); }
-  bool here = me >= 0;
-  for (int t = 0; t < H; ++t) {
-    if (tid < 32) {
-      const bool on = here && t >= from;
-      if (on) {
-        S.st[0][tid] = q.X; S.st[1][tid] = q.Y; S.st[2][tid] = q.Z;
-        if (FULL) { S.st[3][tid] = q.VX; S.st[4][tid] = q.VY; S.st[5][tid] = q.VZ; S.hit[tid] = 0x7fffffff; }
-        S.to[0][tid] = (double)q.X + (double)q.VX * p.dtmd;
-        S.to[1][tid] = (double)q.Y + (double)q.VY * p.dtmd;
-        S.to[2][tid] = (double)q.Z + (double)q.VZ * p.dtmd;
-        S.band[tid] = band_of(p, q.X, q.Y);
-      }
-      const unsigned act = __ballot_sync(0xffffffffu, on), any = __ballot_sync(0xffffffffu, here);
-      if (lane == 0) { S.act = act; S.leave = 0u; S.nc = 0; S.done = any == 0u; }
+
+// The triangle walk of reflectionFed for one particle, by G lanes (mask): the
+// lanes test G list entries at a time, all from the same particle state.  The
+// reference's loop changes the state only at a hit, so up to and including the
+// first hit of the G these are exactly its tests: the lowest hit is applied and
+// the walk resumes after it with the updated state -- the same sequence of
+// states as the sequential loop.  From entry cur on.
+template <int G>
+__device__ void near_walk(const DevParams& p, const NearArgs& A, int t, int l0, int cur, int len, int g, unsigned mask,
+                          int indio, double& X, double& Y, double& Z, double& VX, double& VY, double& VZ,
+                          double& fulldt) {
+  while (cur < len) {
+    double x = X, y = Y, z = Z, vx = VX, vy = VY, vz = VZ, fd = 0.0;
+    const bool hit = cur + g < len && near_hit(p, A, t, __ldg(A.lidx + l0 + cur + g), band_of(p, X, Y), indio, x, y, z,
+                                               vx, vy, vz, fd);
+    const unsigned hb = __ballot_sync(mask, hit) & mask;
+    if (hb == 0u) {
+      cur += G;
+      continue;
     }
-    near_sync<W>();
-    if (S.done) return;  // every particle has left
-    const unsigned act = S.act;
-    const TriPre* pre = A.pre + (int64_t)t * A.nt;
-    const unsigned char* bands = A.bands + (int64_t)t * A.nt;
-    for (int e = tid; e < len; e += T) {
-      TriPre r;
-      int rb;
-      if (FULL && e == tid) {
-        r = next;
-        rb = nband;
-        if (t + 1 < H) { next = ldg_tri(pre + A.nt + jj0); nband = __ldg(bands + A.nt + jj0); }
-      } else {
-        const int jj = e == tid ? jj0 : __ldg(A.lidx + l0 + e);
-        r = ldg_tri(pre + jj);
-        rb = __ldg(bands + jj);
-      }
-      for (unsigned todo = act; todo; todo &= todo - 1) {
-        const int j = __ffs(todo) - 1;
-        if ((rb & S.band[j]) || tri_crossing(r, S.st[0][j], S.st[1][j], S.st[2][j], S.to[0][j], S.to[1][j], S.to[2][j],
-                                             S.indio[j])) {
-          if (FULL) {
-            const int c = atomicAdd(&S.nc, 1);
-            if (c < kCand) S.cand[c] = (unsigned)e | ((unsigned)j << 16);
-            else atomicMin(&S.hit[j], e);  // no room: the particle walks the list
-          } else {
-            atomicOr(&S.leave, 1u << j);
-          }
-        }
-      }
-    }
-    near_sync<W>();
-    if (FULL) {
-      const int nc = min(S.nc, kCand);
-      if (nc > 0) {
-        const Snap sn = near_snap(A, t);
-        for (int c = tid; c < nc; c += T) {
-          const int e = (int)(S.cand[c] & 0xffffu), j = (int)(S.cand[c] >> 16);
-          const int jj = __ldg(A.lidx + l0 + e);
-          double x = S.st[0][j], y = S.st[1][j], z = S.st[2][j], vx = S.st[3][j], vy = S.st[4][j], vz = S.st[5][j], fd = 0.0;
-          if (tri_visit(p, sn, ldg_tri(pre + jj), jj, x, y, z, vx, vy, vz, S.indio[j], fd,
-                        !(__ldg(bands + jj) & S.band[j])))
-            atomicMin(&S.hit[j], e);
-        }
-        near_sync<W>();
-        // particles that hit something, a warp each
-        for (int j = tid >> 5; j < n; j += W) {
-          if (!((act >> j) & 1) || S.hit[j] == 0x7fffffff) continue;
-          double x = S.st[0][j], y = S.st[1][j], z = S.st[2][j], vx = S.st[3][j], vy = S.st[4][j], vz = S.st[5][j], fd = 0.0;
-          heavy_walk(p, sn, pre, bands, A.lidx + l0, len, lane, S.indio[j], x, y, z, vx, vy, vz, fd);
-          if (lane == 0) {
-            S.st[0][j] = x; S.st[1][j] = y; S.st[2][j] = z; S.st[3][j] = vx; S.st[4][j] = vy; S.st[5][j] = vz;
-            S.to[0][j] = fd;
-          }
-        }
-        near_sync<W>();
-      }
-    }
-    if (here && t >= from) {
-      if (!FULL && ((S.leave >> tid) & 1)) {
-        flight_store(s, me, q);
-        enqueue(A.h, me, t);
-        here = false;
-      } else {
-        if (FULL && S.hit[tid] != 0x7fffffff) {
-          double X = S.st[0][tid], Y = S.st[1][tid], Z = S.st[2][tid], VX = S.st[3][tid], VY = S.st[4][tid],
-                 VZ = S.st[5][tid];
-          finish_stream(p, S.to[0][tid], X, Y, Z, VX, VY, VZ);
-          raise_health(p, solvent_bad(p, X, Y, Z, VX, VY, VZ), HEALTH_SOLVENT);
-          q = {(R)X, (R)Y, (R)Z, (R)VX, (R)VY, (R)VZ};
-        } else {
-          end_step(p, 0.0, q);
-        }
-        if (t + 1 == H) {
-          flight_store(s, me, q);
-        } else if (cell_at(p, q.X, q.Y, q.Z) != home) {
-          flight_store(s, me, q);
-          enqueue(A.h, me, t + 1);
-          here = false;
-        }
-      }
-    }
-    near_sync<W>();  // the shared state is written again
+    const int src = __ffs(hb) - 1;
+    X = __shfl_sync(mask, x, src);
+    Y = __shfl_sync(mask, y, src);
+    Z = __shfl_sync(mask, z, src);
+    VX = __shfl_sync(mask, vx, src);
+    VY = __shfl_sync(mask, vy, src);
+    VZ = __shfl_sync(mask, vz, src);
+    fulldt += __shfl_sync(mask, fd, src);
+    cur += (src & (G - 1)) + 1;
   }
 }
 
-// the cells with short lists: a warp each, four to a block.  64 registers:
-// eight blocks (32 warps) per SM
-template <typename R>
-__device__ __forceinline__ void near_short_warp(const DevParams& p, const SolventArrays& s, const NearArgs& A, int a,
-                                                int nact, int H, NearCell& S) {
-  if (a >= nact) return;
-  int n = 0;
-  if ((threadIdx.x & 31) == 0) {
-    n = A.h.bcnt[a];
-    if (n) A.h.bcnt[a] = 0;  // for the next stretch
-  }
-  n = min(__shfl_sync(0xffffffffu, n, 0), kBucket);
-  if (n) near_cell<R, 1, false>(p, s, A, a, n, H, S);
-}
-template <typename R>
-__global__ void __launch_bounds__(32 * kShortWarps, kShortMinBlocks)
-    k_near_short(DevParams p, SolventArrays s, NearArgs A, const int* __restrict__ nactp, int H) {
-  __shared__ NearCell S[kShortWarps];
-  const int w = (int)(threadIdx.x >> 5);
-  near_short_warp<R>(p, s, A, (int)blockIdx.x * kShortWarps + w, *nactp, H, S[w]);
-}
-// the cells with long lists: kLongWarps warps each, longest list first
-template <typename R>
-__device__ __forceinline__ void near_long_block(const DevParams& p, const SolventArrays& s, const NearArgs& A, int b,
-                                                const int* __restrict__ border, int nact, int H, NearCell& S) {
-  if (b >= nact) return;
-  const int a = border[b], n = min(A.h.bcnt[a], kBucket);
-  __syncthreads();
-  if (threadIdx.x == 0 && n) A.h.bcnt[a] = 0;
-  if (n) near_cell<R, kLongWarps, true>(p, s, A, a, n, H, S);
-}
-template <typename R>
-__global__ void __launch_bounds__(32 * kLongWarps, kLongMinBlocks)
-    k_near_long(DevParams p, SolventArrays s, NearArgs A, const int* __restrict__ border, const int* __restrict__ nactp,
-                int H) {
-  __shared__ NearCell S;
-  near_long_block<R>(p, s, A, (int)blockIdx.x, border, *nactp, H, S);
-}
-
-// The queue: particles that left their cell or (short lists) have a crossing
-// candidate, of full buckets, and in lists longer than the capacity; warp gw
-// of tw takes particles gw, gw + tw, ... through the rest of the stretch.
-template <typename R>
-__device__ __forceinline__ void queue_walk(const DevParams& p, const SolventArrays& s, const NearArgs& A,
-                                           const unsigned char* __restrict__ cflag, int H, int64_t gw, int64_t tw) {
-  const int lane = threadIdx.x & 31;
-  const int nq = *A.h.qn;
-  for (int64_t w = gw; w < nq; w += tw) {
-    const int64_t i = A.h.queue[w];
-    Flight<R> q;
-    const int indio = flight_load(s, i, q);
-    for (int t = A.h.qk[w]; t < H; ++t) {
-      const int pid = cell_at(p, q.X, q.Y, q.Z);
-      if (!(__ldg(cflag + pid) & 1)) {
-        free_step(p, q);
-        raise_health(p, solvent_bad(p, q.X, q.Y, q.Z, q.VX, q.VY, q.VZ), HEALTH_SOLVENT);
-        continue;
-      }
-      const int l0 = __ldg(A.lstart + pid), len = __ldg(A.lstart + pid + 1) - l0;
-      double x = q.X, y = q.Y, z = q.Z, vx = q.VX, vy = q.VY, vz = q.VZ, fd = 0.0;
-      heavy_walk(p, near_snap(A, t), A.pre + (int64_t)t * A.nt, A.bands + (int64_t)t * A.nt, A.lidx + l0, len, lane,
-                 indio, x, y, z, vx, vy, vz, fd);
-      finish_stream(p, fd, x, y, z, vx, vy, vz);
-      raise_health(p, solvent_bad(p, x, y, z, vx, vy, vz), HEALTH_SOLVENT);
-      q = {(R)x, (R)y, (R)z, (R)vx, (R)vy, (R)vz};
+// One particle near the membrane from step `from` to the end of the stretch
+// (reflectionFed, :400-598, then the walls and wrap), by G lanes (g of mask) that
+// all keep its state.  On entering a cell the lanes go through its list once and
+// keep the entries that the cull leaves (kept: room for KEEP of them); each step
+// then tests those, a lane each, all from the same state.  The reference's loop
+// changes the state only at a hit, so the lowest entry that hits is its first
+// one: it is applied, the list is culled again with the new velocity, and the
+// entries after it are tested from there.
+template <typename R, int G, int KEEP>
+__device__ __forceinline__ void near_particle(const DevParams& p, const SolventArrays& s, const NearArgs& A, int H,
+                                              int64_t i, int from, int g, unsigned mask, unsigned short* kept) {
+  Flight<R> q;
+  const int indio = flight_load(s, i, q);
+  int cell = -1, l0 = 0, len = 0, nk = 0, mine = 0;  // mine: this lane's first kept triangle
+  for (int t = from; t < H; ++t) {
+    // the record of the first kept triangle, wanted if the cell is still the same
+    bool early = cell >= 0 && g < nk;
+    TriPre first{};
+    int fband = 0;
+    if (early) {
+      const int64_t at = (int64_t)t * A.nt + mine;
+      first = ldg_tri(A.pre + at);
+      fband = __ldg(A.bands + at);
     }
-    if (lane == 0) flight_store(s, i, q);
+    bool on;
+    const int pid = cell_at(p, q.X, q.Y, q.Z, on);
+    if (!(__ldg(A.flag + pid) & CF_LISTED)) {
+      free_step(p, q);
+      raise_health(p, solvent_bad(p, q.X, q.Y, q.Z, q.VX, q.VY, q.VZ), HEALTH_SOLVENT);
+      cell = -1;
+      continue;
+    }
+    double x = q.X, y = q.Y, z = q.Z, vx = q.VX, vy = q.VY, vz = q.VZ, fd = 0.0;
+    bool fresh = pid != cell;  // the list is to be culled
+    if (fresh) {
+      cell = on ? pid : -1;
+      l0 = __ldg(A.lstart + pid);
+      len = __ldg(A.lstart + pid + 1) - l0;
+    }
+    for (int after = -1;;) {  // the last entry that hit in this step
+      const int band = band_of(p, x, y);
+      if (fresh) {
+        nk = 0;
+        // (the top wall gives its speed to what it reflects; a band ends inside a
+        // cell only in a box that is no whole number of cells; a wrap ends in
+        // another cell, except in a box of one)
+        float dP = (float)(fmax(sqrt(vx * vx + vy * vy + vz * vz), fabs(p.wallspeed)) * p.dtmd * (H - t)) * 1.0001f;
+        if (p.nx < 2 || p.ny < 2) dP = __int_as_float(0x7f800000);
+        const int wide = band | band_of(p, x - dP, y - dP) | band_of(p, x + dP, y + dP);
+        constexpr int U = 4;  // entries in flight per lane
+        for (int e0 = 0; e0 < len; e0 += U * G) {
+          int jj[U];
+#pragma unroll
+          for (int u = 0; u < U; ++u) jj[u] = e0 + u * G + g < len ? __ldg(A.lidx + l0 + e0 + u * G + g) : -1;
+          TriCull c[U];
+#pragma unroll
+          for (int u = 0; u < U; ++u) c[u] = ldg_cull(A.cull + 3 * (int64_t)max(jj[u], 0));
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            const bool keep = jj[u] >= 0 && cull_keeps(c[u], (float)x, (float)y, (float)z, dP, wide);
+            const unsigned kb = (__ballot_sync(mask, keep) & mask) >> (threadIdx.x & 31 & ~(G - 1));
+            const int at = nk + __popc(kb & ((1u << g) - 1u));
+            if (keep && at < KEEP) kept[at] = (unsigned short)(e0 + u * G + g);
+            nk += __popc(kb);
+          }
+        }
+        if (len > 65535) nk = KEEP + 1;
+        __syncwarp(mask);
+        if (g < min(nk, KEEP)) mine = __ldg(A.lidx + l0 + kept[g]);
+        early = false;
+        fresh = false;
+      }
+      if (nk > KEEP) {  // more than there is room for: the whole list
+        near_walk<G>(p, A, t, l0, after + 1, len, g, mask, indio, x, y, z, vx, vy, vz, fd);
+        break;
+      }
+      const double U = x + vx * p.dtmd, V = y + vy * p.dtmd, W = z + vz * p.dtmd;
+      double hx = x, hy = y, hz = z, hvx = vx, hvy = vy, hvz = vz, hfd = 0.0;
+      int hit = 0x7fffffff;
+      for (int u = g; u < nk && hit == 0x7fffffff; u += G) {
+        const int e = kept[u];
+        if (e <= after) continue;
+        const int jj = u == g ? mine : __ldg(A.lidx + l0 + e);
+        TriPre r = first;
+        int rb = fband;
+        if (u != g || !early) {
+          const int64_t at = (int64_t)t * A.nt + jj;
+          r = ldg_tri(A.pre + at);
+          rb = __ldg(A.bands + at);
+        }
+        const bool plain = !(rb & band);
+        if (plain && !tri_crossing(r, x, y, z, U, V, W, indio)) continue;
+        if (tri_visit(p, near_snap(A, t), r, jj, hx, hy, hz, hvx, hvy, hvz, indio, hfd, plain)) hit = e;
+      }
+      const unsigned hb = __ballot_sync(mask, hit != 0x7fffffff) & mask;
+      if (hb == 0u) break;
+      const int lowest = (int)__reduce_min_sync(mask, (unsigned)hit);
+      const int src = __ffs(__ballot_sync(mask, hit == lowest) & mask) - 1;
+      x = __shfl_sync(mask, hx, src);
+      y = __shfl_sync(mask, hy, src);
+      z = __shfl_sync(mask, hz, src);
+      vx = __shfl_sync(mask, hvx, src);
+      vy = __shfl_sync(mask, hvy, src);
+      vz = __shfl_sync(mask, hvz, src);
+      fd += __shfl_sync(mask, hfd, src);
+      after = lowest;
+      fresh = true;
+    }
+    finish_stream(p, fd, x, y, z, vx, vy, vz);
+    raise_health(p, solvent_bad(p, x, y, z, vx, vy, vz), HEALTH_SOLVENT);
+    q = {(R)x, (R)y, (R)z, (R)vx, (R)vy, (R)vz};
+  }
+  if (g == 0) flight_store(s, i, q);
+}
+// the queue's particles, each by the next group of G lanes that is free
+template <typename R, int G, int KEEP>
+__device__ __forceinline__ void near_groups(const DevParams& p, const SolventArrays& s, const NearArgs& A, int H,
+                                            unsigned short* kept) {
+  const int lane = threadIdx.x & 31, g = lane & (G - 1), lead = lane & ~(G - 1);
+  const unsigned mask = G == 32 ? 0xffffffffu : ((1u << G) - 1u) << lead;
+  const int nq = *A.q.n;
+  while (true) {
+    int w = 0;
+    if (g == 0) w = atomicAdd(A.q.n + 4, 1);
+    w = __shfl_sync(mask, w, lead);
+    if (w >= nq) break;
+    near_particle<R, G, KEEP>(p, s, A, H, A.q.i[w], A.q.k[w], g, mask, kept);
+    __syncwarp(mask);
   }
 }
-template <typename R>
-__global__ void __launch_bounds__(256, 2) k_near_queue(DevParams p, SolventArrays s, NearArgs A,
-                                                      const unsigned char* __restrict__ cflag, int H) {
-  const int64_t tw = (int64_t)gridDim.x * (blockDim.x >> 5);
-  const int64_t gw = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  queue_walk<R>(p, s, A, cflag, H, gw, tw);
+template <typename R, int G, int KEEP>
+__global__ void __launch_bounds__(kNearT, kNearMinBlocks) k_near(DevParams p, SolventArrays s, NearArgs A, int H) {
+  __shared__ unsigned short kept[kNearT / G][KEEP];
+  near_groups<R, G, KEEP>(p, s, A, H, kept[threadIdx.x / G]);
 }
 
 }  // namespace irbc
@@ -713,19 +675,8 @@ namespace irbc {
 // ================================================================ launch ======
 // the side stream's work: a captured graph gives it the side stream's high
 // priority
-bool is_membrane_kernel(const void* fn) { return fn == (const void*)k_membrane || fn == (const void*)k_tri_records; }
-
-__global__ void k_rank_lengths(Cells c, int nact, int* len, int2* rng) {
-  const int a = blockIdx.x * blockDim.x + threadIdx.x;
-  if (a >= nact) return;
-  const int cell = c.acell[a];
-  const int l0 = c.lstart[cell];
-  len[a] = c.lstart[cell + 1] - l0;
-  rng[a] = make_int2(l0, c.lstart[cell + 1] - l0);
-}
-void launch_rank_lengths(const Cells& c, int* len, int2* rng, cudaStream_t st) {
-  if (c.nact > 0) k_rank_lengths<<<nb(c.nact, 256), 256, 0, st>>>(c, c.nact, len, rng);
-}
+bool is_membrane_kernel(const void* fn) { return fn == (const void*)k_membrane || fn == (const void*)k_tri_records ||
+         fn == (const void*)k_tri_cull; }
 
 // snapshot and triangle records of the membrane as it is (irbc_stream), as
 // step 0 of a stretch
@@ -740,31 +691,14 @@ __global__ void k_snap(DevParams p, Membrane m, FastBufs f) {
 void fast_snap_prep(const DevParams& p, Membrane& m, FastBufs& f, cudaStream_t st) {
   k_snap<<<nb(p.nv, 128), 128, 0, st>>>(p, m, f);
   k_tri_records<<<nb(p.nt, 128), 128, 0, st>>>(p, f, 1);
-}
-
-// the near-membrane kernels of a stretch; returns the number launched
-template <typename R>
-static int launch_near(const DevParams& p, const Solvent& s, const SolventF& sf, const Cells& c, const FastBufs& f,
-                       int H, cudaStream_t st) {
-  const SolventArrays arr = arrays_of(s, sf);
-  const NearArgs A = near_of(p, c, f, 0);
-  int n = 1;
-  if (f.bcap > 0) {
-    if (short_lists(f.hcap))
-      k_near_short<R><<<nb(f.bcap, kShortWarps), 32 * kShortWarps, 0, st>>>(p, arr, A, c.totals + 4, H);
-    else
-      k_near_long<R><<<(unsigned)f.bcap, 32 * kLongWarps, 0, st>>>(p, arr, A, f.border, c.totals + 4, H);
-    ++n;
-  }
-  k_near_queue<R><<<kQueueBlocks, 256, 0, st>>>(p, arr, A, c.flag, H);
-  return n;
+  k_tri_cull<<<nb(p.nt, 64), 64, 0, st>>>(p, f, 1);
 }
 
 int fast_stream(const DevParams& p, const Solvent& s, const SolventF* sf, const Cells& c, FastBufs& f, int H,
                 cudaStream_t st, cudaEvent_t ev0, cudaEvent_t ev1, cudaEvent_t snap) {
-  cudaMemsetAsync(f.qn, 0, sizeof(int), st);
+  cudaMemsetAsync(f.qn, 0, 8 * sizeof(int), st);
   if (!s.n) return 0;
-  const HandOff h = hand_off_of(c, f, 0);
+  const NearQueue h = queue_of(f, 0);
   const SolventF none;
   const SolventArrays arr = arrays_of(s, sf ? *sf : none);
   if (ev0) cudaEventRecord(ev0, st);
@@ -772,7 +706,16 @@ int fast_stream(const DevParams& p, const Solvent& s, const SolventF* sf, const 
   else k_stream_bulk<<<nb(s.n, 256), 256, 0, st>>>(p, arr, s.n, c.flag, h, H);
   if (ev1) cudaEventRecord(ev1, st);
   if (snap) cudaStreamWaitEvent(st, snap, 0);
-  return 1 + (sf ? launch_near<float>(p, s, *sf, c, f, H, st) : launch_near<double>(p, s, none, c, f, H, st));
+  const NearArgs A = near_of(p, c, f, 0);
+  const bool few = short_lists(f.lmax);
+  if (sf) {
+    if (few) k_near<float, kShortG, kShortKeep><<<kNearBlocks, kNearT, 0, st>>>(p, arr, A, H);
+    else k_near<float, kLongG, kLongKeep><<<kNearBlocks, kNearT, 0, st>>>(p, arr, A, H);
+  } else {
+    if (few) k_near<double, kShortG, kShortKeep><<<kNearBlocks, kNearT, 0, st>>>(p, arr, A, H);
+    else k_near<double, kLongG, kLongKeep><<<kNearBlocks, kNearT, 0, st>>>(p, arr, A, H);
+  }
+  return 2;
 }
 
 }  // namespace irbc

@@ -27,19 +27,12 @@ constexpr int kSegT = 512;  // threads per block of the membrane kernel
 constexpr int kSegTerms = 20000;
 __host__ __device__ constexpr int seg_terms(int nt) { return (nt + 32 + 15) / 16 * 16; }
 
-// near-membrane streaming: particles per listed cell taken by the cell's
-// warps, and the longest list they take; the others go to the queue
-constexpr int kBucket = 32;
-constexpr int kHeavyList = 1024;
-// Lists of up to kShortList entries (capacity hcap) take one warp per listed
-// cell, kShortWarps of them to a block, at 64 registers a thread (eight blocks,
-// 32 warps, per SM); longer ones kLongWarps warps per cell.
-constexpr int kShortList = 128, kShortWarps = 4, kShortMinBlocks = 8;
-constexpr int kLongWarps = 4, kLongMinBlocks = 4;
-// blocks of eight warps that walk the queue: per simulation alone, and per
-// member of a cohort
-constexpr int kQueueBlocks = 148, kQueueBlocksMember = 32;
-inline bool short_lists(int hcap) { return hcap <= kShortList; }
+// near-membrane streaming: lanes per particle and room for kept entries, for
+// lists of up to kShortList entries and for longer ones; threads per block,
+// blocks per SM, blocks per simulation alone and per member of a cohort
+constexpr int kShortList = 128, kShortG = 8, kShortKeep = 64, kLongG = 32, kLongKeep = 512;
+constexpr int kNearT = 128, kNearMinBlocks = 4, kNearBlocks = 148 * kNearMinBlocks, kNearBlocksMember = 148;
+inline bool short_lists(int lmax) { return lmax <= kShortList; }
 // the side-wall bands (3a) that a triangle's corners lie in: tri_record
 enum : int { BAND_LX = 1, BAND_HX = 2, BAND_LY = 4, BAND_HY = 8 };
 
@@ -91,17 +84,13 @@ struct FastBufs {
   Snap snap{};
   TriPre* pre = nullptr;  // kSegMax x nt
   unsigned char* bands = nullptr;  // kSegMax x nt: BAND_* of each record's corners
-  int* queue = nullptr;   // particles the near-membrane cells' warps do not take (capacity Ns)
+  float4* cull = nullptr; // 3 x nt: what no step of the stretch needs to test (TriCull)
+  int* queue = nullptr;   // particles near the membrane (capacity Ns)
   unsigned char* qk = nullptr;  // the step of the stretch from which on
-  int* qn = nullptr;      // their number
-  int* bcnt = nullptr;    // particles handed to each listed cell in this stretch (reset by its warps)
-  int2* bucket = nullptr; // kBucket (particle, first step) per listed cell
-  int64_t bcap = 0;       // listed cells the buckets have room for
-  int* border = nullptr;  // listed cells (ranks), longest lists first
-  int2* arng = nullptr;   // (first entry, length) of each listed cell's list, by rank (bcap of them)
+  int* qn = nullptr;      // [par] their number, [4 + par] those taken (two parities: cohorts)
   bool one_block = false; // the membrane kernel as one block (meshes that fit, one_block_fits)
   bool cluster = false;   // ... as a cluster of eight blocks whatever the mesh
-  int hcap = kHeavyList;  // longest list taken by a cell's warps
+  int lmax = 0;           // (host) longest list
   double* slot = nullptr; // force terms: 3 doubles per slot, 4E + 9T + 4E slots
   double* a4 = nullptr;   // 4 x area of each triangle
   double* fac = nullptr;  // factors of the global area and volume forces
@@ -121,15 +110,6 @@ __host__ __device__ inline Snap snap_of(const FastBufs& f, int step, int nv) {
 }
 // snapshot and triangle records of the membrane as it is, as step 0
 void fast_snap_prep(const DevParams& p, Membrane& m, FastBufs& f, cudaStream_t st);
-// list length of each listed cell (rank a < nact) into len[a], and its
-// (first entry, length) into rng[a]
-void launch_rank_lengths(const Cells& c, int* len, int2* rng, cudaStream_t st);
-// the capacity for lists of at most lmax entries: lmax rounded up to 64, at
-// least 64, at most kHeavyList
-inline int heavy_cap(int lmax) {
-  int c = ((lmax + 63) / 64) * 64;
-  return c < 64 ? 64 : (c > kHeavyList ? kHeavyList : c);
-}
 // the streaming of a stretch of H steps; sf: the FP32-bulk solvent, or null.
 // ev0/ev1 (optional) are recorded around the bulk kernel.  The bulk kernel
 // reads no membrane data; the near-membrane kernels read the snapshots and

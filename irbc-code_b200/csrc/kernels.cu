@@ -593,48 +593,35 @@ void launch_llist_fill(const DevParams& p, Cells& c, const Membrane& m, int64_t 
   if (total > 0) cudaMemcpyAsync(c.lidx, c.lidx2, sizeof(int) * total, cudaMemcpyDeviceToDevice, st);
 }
 
-// cells with a non-empty list: their rank (lrank), the cell of each rank
-// (acell), their number and the longest list (host copies nact, lmax)
-__global__ void k_lflags(DevParams p, Cells cl) {
-  int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= p.ncell) return;
-  const int len = cl.lstart[c + 1] - cl.lstart[c];
-  cl.lrank[c] = len > 0 ? 1 : 0;
-  if (len > 0) atomicMax(cl.totals + 7, len);
-}
-__global__ void k_acell(DevParams p, Cells cl) {
-  int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= p.ncell) return;
-  if (cl.lstart[c + 1] > cl.lstart[c]) cl.acell[cl.lrank[c]] = (int)c;
-}
-// what the streaming wants to know of a cell without reading its list (Cells::flag)
+// Cells::flag of every cell
 __global__ void k_cell_flags(DevParams p, Cells cl) {
   const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= p.ncell) return;
-  auto listed = [&](int64_t q) { return cl.lstart[q + 1] > cl.lstart[q]; };
   const int k = (int)(c % p.nz), j = (int)((c / p.nz) % p.ny), i = (int)(c / ((int64_t)p.nz * p.ny));
-  // (a position off the grid counts as cell 0: cell_of)
-  bool meets = i == 0 || i >= p.nx - 1 || j == 0 || j >= p.ny - 1 || (listed(0) && (k <= 1 || k >= p.nz - 2));
+  const bool side = i == 0 || i >= p.nx - 1 || j == 0 || j >= p.ny - 1, wall = k <= 1 || k >= p.nz - 2;
+  // a position off the grid counts as cell 0 (cell_of): one exactly on the upper
+  // sides or on the top wall, or beyond the cells of a box that is no whole
+  // number of them; such boxes' outer cells are left to the general path
+  bool meets = (side || wall) && cl.lstart[1] > cl.lstart[0];
+  meets = meets || (side && (p.nx * p.a != p.Lx || p.ny * p.a != p.Ly || p.nx < 3 || p.ny < 3));
+  meets = meets || (wall && (p.nz - 1) * p.a != p.Lz);
   for (int a = -1; a <= 1 && !meets; ++a)
     for (int b = -1; b <= 1 && !meets; ++b) {
-      const int64_t row = ((int64_t)(i + a) * p.ny + j + b) * p.nz;
+      const int ia = (i + a + p.nx) % p.nx, jb = (j + b + p.ny) % p.ny;
+      const int64_t row = ((int64_t)ia * p.ny + jb) * p.nz;
       // the list starts ascend: any entry between two of them is theirs
       meets = cl.lstart[row + min(k + 1, p.nz - 1) + 1] > cl.lstart[row + max(k - 1, 0)];
     }
-  cl.flag[c] = (unsigned char)((listed(c) ? 1 : 0) | (meets ? 2 : 0));
+  const int len = cl.lstart[c + 1] - cl.lstart[c];
+  if (len > 0) atomicMax(cl.totals + 7, len);
+  cl.flag[c] = (unsigned char)((len > 0 ? CF_LISTED : 0) | (meets ? CF_MEETS : 0) |
+                               (side ? CF_SIDE : 0) | (wall ? CF_WALL : 0));
 }
-int launch_llist_ranks(const DevParams& p, Cells& c, cudaStream_t st) {
+int launch_llist_flags(const DevParams& p, Cells& c, cudaStream_t st) {
   cudaMemsetAsync(c.totals + 7, 0, sizeof(int), st);
-  k_lflags<<<nblk(c.n, 256), 256, 0, st>>>(p, c);
-  launch_scan3(c.lrank, nullptr, nullptr, c.lrank, nullptr, nullptr, c.totals + 4, c.n, c.scan_part, st);
-  k_acell<<<nblk(c.n, 256), 256, 0, st>>>(p, c);
   k_cell_flags<<<nblk(c.n, 256), 256, 0, st>>>(p, c);
-  int h[4] = {0, 0, 0, 0};
-  cudaMemcpyAsync(h, c.totals + 4, sizeof(h), cudaMemcpyDeviceToHost, st);
-  if (cudaStreamSynchronize(st) != cudaSuccess) return -1;
-  c.nact = h[0];
-  c.lmax = h[3];
-  return 6;
+  cudaMemcpyAsync(&c.lmax, c.totals + 7, sizeof(int), cudaMemcpyDeviceToHost, st);
+  return cudaStreamSynchronize(st) == cudaSuccess ? 1 : -1;
 }
 
 // ============================================================ membrane =====

@@ -14,11 +14,11 @@ __global__ void __launch_bounds__(256, 6) km_stream_bulk(Member* __restrict__ me
   // copies: the descriptor is not reloaded after the stores below
   const DevParams p = M.p;
   const SolventArrays s = arrays_of(M.s, M.f);
-  const HandOff h = hand_off_of(M.c, M.fb, par);
+  const NearQueue h = queue_of(M.fb, par);
   const unsigned char* __restrict__ cflag = M.c.flag;
   const int64_t n = M.f.n;
   // the queue of the next stretch starts empty
-  if (b == 0 && threadIdx.x == 0) M.fb.qn[par ^ 1] = 0;
+  if (b == 0 && threadIdx.x == 0) M.fb.qn[par ^ 1] = M.fb.qn[4 + (par ^ 1)] = 0;
   for (int pass = 0; pass < kMultiStreamPasses; ++pass) {
     const int64_t i = ((int64_t)b * kMultiStreamPasses + pass) * blockDim.x + threadIdx.x;
     if (i >= n) break;
@@ -26,68 +26,35 @@ __global__ void __launch_bounds__(256, 6) km_stream_bulk(Member* __restrict__ me
   }
 }
 
-// a block's copy of what the near-membrane kernels read of its member
+// a block's copy of what the near-membrane kernel reads of its member
 struct NearMember {
   DevParams p;
   SolventArrays s;
   NearArgs A;
-  const unsigned char* cflag;
-  const int* border;
-  int nact;
 };
-__device__ __forceinline__ void near_member(const Member& M, int par, NearMember& N) {
+template <int G, int KEEP>
+__global__ void __launch_bounds__(kNearT, kNearMinBlocks)
+    km_near(const Member* __restrict__ mem, const int2* __restrict__ tab, int H, int par) {
+  __shared__ __align__(16) unsigned char raw[sizeof(NearMember)];
+  __shared__ unsigned short kept[kNearT / G][KEEP];
+  NearMember& N = *reinterpret_cast<NearMember*>(raw);
+  const Member& M = mem[__ldg(tab + blockIdx.x).x];
   if (threadIdx.x == 0) {
     N.s = arrays_of(M.s, M.f);
     N.A = near_of(M.p, M.c, M.fb, par);
-    N.cflag = M.c.flag;
-    N.border = M.fb.border;
-    N.nact = M.c.totals[4];
   }
   for (int i = threadIdx.x; i < (int)sizeof(DevParams) / 4; i += blockDim.x) ((int*)&N.p)[i] = ((const int*)&M.p)[i];
   __syncthreads();
-}
-#define KM_NEAR                                               \
-  __shared__ __align__(16) unsigned char raw[sizeof(NearMember)]; \
-  NearMember& N = *reinterpret_cast<NearMember*>(raw);        \
-  const int2 e_ = __ldg(tab + blockIdx.x);                    \
-  const int b = e_.y;                                         \
-  near_member(mem[e_.x], par, N)
-
-// members with long lists, with short lists, then the queues of all
-__global__ void __launch_bounds__(32 * kLongWarps, kLongMinBlocks)
-    km_near_long(const Member* __restrict__ mem, const int2* __restrict__ tab, int H, int par) {
-  KM_NEAR;
-  __shared__ NearCell S;
-  near_long_block<float>(N.p, N.s, N.A, b, N.border, N.nact, H, S);
-}
-__global__ void __launch_bounds__(32 * kShortWarps, kShortMinBlocks)
-    km_near_short(const Member* __restrict__ mem, const int2* __restrict__ tab, int H, int par) {
-  KM_NEAR;
-  __shared__ NearCell S[kShortWarps];
-  const int w = (int)(threadIdx.x >> 5);
-  near_short_warp<float>(N.p, N.s, N.A, b * kShortWarps + w, N.nact, H, S[w]);
-}
-__global__ void __launch_bounds__(256, 2) km_near_queue(const Member* __restrict__ mem, const int2* __restrict__ tab,
-                                                       int H, int par) {
-  KM_NEAR;
-  queue_walk<float>(N.p, N.s, N.A, N.cflag, H, (int64_t)b * 8 + (threadIdx.x >> 5), (int64_t)kQueueBlocksMember * 8);
+  near_groups<float, G, KEEP>(N.p, N.s, N.A, H, kept[threadIdx.x / G]);
 }
 
 int multi_stream(const MultiPlan& P, int H, int par, cudaStream_t st, cudaEvent_t snap) {
   km_stream_bulk<<<P.blocks[MP_STREAM], 256, 0, st>>>(P.mem, P.table(MP_STREAM), H, par);
   if (snap) cudaStreamWaitEvent(st, snap, 0);
-  const int n0 = P.cells_short, n1 = P.blocks[MP_CELLS] - P.cells_short;
-  int k = 2;
-  if (n0 > 0) {
-    km_near_short<<<n0, 32 * kShortWarps, 0, st>>>(P.mem, P.table(MP_CELLS), H, par);
-    ++k;
-  }
-  if (n1 > 0) {
-    km_near_long<<<n1, 32 * kLongWarps, 0, st>>>(P.mem, P.table(MP_CELLS) + n0, H, par);
-    ++k;
-  }
-  km_near_queue<<<P.blocks[MP_QUEUE], 256, 0, st>>>(P.mem, P.table(MP_QUEUE), H, par);
-  return k;
+  const int n0 = P.blocks[MP_NEAR_SHORT], n1 = P.blocks[MP_NEAR_LONG];
+  if (n0 > 0) km_near<kShortG, kShortKeep><<<n0, kNearT, 0, st>>>(P.mem, P.table(MP_NEAR_SHORT), H, par);
+  if (n1 > 0) km_near<kLongG, kLongKeep><<<n1, kNearT, 0, st>>>(P.mem, P.table(MP_NEAR_LONG), H, par);
+  return 1 + (n0 > 0) + (n1 > 0);
 }
 
 // ---- membrane ----------------------------------------------------------------
@@ -120,6 +87,11 @@ __global__ void __launch_bounds__(128) km_tri_records(const Member* __restrict__
   records_item(M.p, M.fb, H, (int64_t)e.y * blockDim.x + threadIdx.x);
 }
 
+__global__ void __launch_bounds__(64) km_tri_cull(const Member* __restrict__ mem, const int2* __restrict__ tab, int H) {
+  const int2 e = __ldg(tab + blockIdx.x);
+  cull_item(mem[e.x].p, mem[e.x].fb, H, e.y * blockDim.x + threadIdx.x);
+}
+
 int multi_membrane(const MultiPlan& P, uint64_t eoff, int H, cudaStream_t st) {
   const int2* tab = P.table(MP_MEMBRANE);
   for (const MultiPlan::Seg& s : P.seg) {
@@ -139,7 +111,8 @@ int multi_membrane(const MultiPlan& P, uint64_t eoff, int H, cudaStream_t st) {
     tab += s.members * s.nc;
   }
   km_tri_records<<<P.blocks[MP_RECORDS], 128, 0, st>>>(P.mem, P.table(MP_RECORDS), H);
-  return (int)P.seg.size() + 1;
+  km_tri_cull<<<P.blocks[MP_CULL], 64, 0, st>>>(P.mem, P.table(MP_CULL), H);
+  return (int)P.seg.size() + 2;
 }
 
 // ---- collision: particle phases ---------------------------------------------------
@@ -204,11 +177,11 @@ void set_kernel_limits() {
 void multi_blocks(const Member& M, int out[MP_NPHASE]) {
   const int64_t ns = M.f.n, nc = M.c.n;
   out[MP_STREAM] = (int)nbf(ns, 256 * kMultiStreamPasses);
-  // short lists: kShortWarps listed cells per block; long lists: one
-  out[MP_CELLS] = (int)(short_lists(M.fb.hcap) ? (M.fb.bcap + kShortWarps - 1) / kShortWarps : M.fb.bcap);
-  out[MP_QUEUE] = kQueueBlocksMember;
+  out[MP_NEAR_SHORT] = short_lists(M.fb.lmax) ? kNearBlocksMember : 0;
+  out[MP_NEAR_LONG] = short_lists(M.fb.lmax) ? 0 : kNearBlocksMember;
   out[MP_MEMBRANE] = segment_blocks(M.p, M.fb);
   out[MP_RECORDS] = (int)nbf((int64_t)kSegMax * M.p.nt, 128);
+  out[MP_CULL] = (int)nb(M.p.nt, 64);
   out[MP_ZERO] = (int)nb(nc, 256);
   out[MP_VBIN] = 1;
   out[MP_COUNT] = (int)nbf(ns, 256 * kCountPer);

@@ -1408,6 +1408,10 @@ __global__ void __launch_bounds__(128) k_tri_records(DevParams p, FastBufs f, in
   records_item(p, f, H, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
+__global__ void __launch_bounds__(64) k_tri_cull(DevParams p, FastBufs f, int H) {
+  cull_item(p, f, H, blockIdx.x * blockDim.x + threadIdx.x);
+}
+
 // blocks of the membrane's cluster
 int segment_blocks(const DevParams& p, const FastBufs& f) {
   if (f.patch.nc > 0) return f.patch.nc;
@@ -1453,8 +1457,9 @@ int launch_membrane(const DevParams& p, Membrane& m, FastBufs& f, uint64_t eoff,
   cfg.numAttrs = 1;
   cudaLaunchKernelEx(&cfg, k_membrane, p, m, f, eoff, H, parts);
   if (!(parts & SEG_FIRST)) return 1;
-  k_tri_records<<<(unsigned)((int64_t)H * p.nt + 127) / 128, 128, 0, st>>>(p, f, H);
-  return 2;
+  k_tri_records<<<(unsigned)(((int64_t)H * p.nt + 127) / 128), 128, 0, st>>>(p, f, H);
+  k_tri_cull<<<(unsigned)((p.nt + 63) / 64), 64, 0, st>>>(p, f, H);
+  return 3;
 }
 
 }  // namespace irbc

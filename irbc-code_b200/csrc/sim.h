@@ -40,19 +40,21 @@ struct Solvent {
 // physically by cell; in between the cells read their particles through perm
 constexpr int kResortEvery = 16;
 
+// what the streaming wants to know of a cell without reading its list: it has
+// one; a flight of less than a cell from it may meet a listed cell, a periodic
+// side, the top or bottom wall
+enum : unsigned char { CF_LISTED = 1, CF_MEETS = 2, CF_SIDE = 4, CF_WALL = 8 };
+
 struct Cells {
   int64_t n = 0;
   int *cnt = nullptr, *start = nullptr, *ncm = nullptr, *wrank = nullptr, *mrank = nullptr;
   int *totals = nullptr;        // [0] particles, [1] wall ghost cells, [2] membrane ghost cells,
-                                // [4] cells with a list, [7] longest list, [8] llist entries,
+                                // [7] longest list, [8] llist entries,
                                 // [11] bad particle ids seen by get_state
   int *lstart = nullptr, *lidx = nullptr, *lstart2 = nullptr, *lidx2 = nullptr, *lcnt = nullptr;
   int64_t lcap = 0, lcap2 = 0;
-  int *lrank = nullptr;         // rank among the cells with a non-empty list
-  int *acell = nullptr;         // the cell of each such rank
-  unsigned char* flag = nullptr;  // 1: listed; 2: a flight of less than a cell from it may meet a listed
-                                // cell, a side wall or the grid's edge
-  int nact = 0, lmax = 0;       // (host) their number and the longest list
+  unsigned char* flag = nullptr;  // CF_* of each cell
+  int lmax = 0;                 // (host) the longest list
   int *scan_part = nullptr;     // scan scratch: 3 ints per block
   int64_t scan_blocks = 0;
 };
@@ -122,9 +124,9 @@ void launch_ghost_flags(const DevParams& p, Cells& c, const Membrane& m, cudaStr
 int64_t launch_llist_count(const DevParams& p, Cells& c, const Membrane& m, cudaStream_t st);
 // total: the entry count launch_llist_count returned (both list buffers hold it)
 void launch_llist_fill(const DevParams& p, Cells& c, const Membrane& m, int64_t total, cudaStream_t st);
-// lrank / acell / nact / lmax of the current lists (host sync inside);
-// returns the kernels launched, -1 on a CUDA error
-int launch_llist_ranks(const DevParams& p, Cells& c, cudaStream_t st);
+// flag / lmax of the current lists (host sync inside); returns the kernels
+// launched, -1 on a CUDA error
+int launch_llist_flags(const DevParams& p, Cells& c, cudaStream_t st);
 void launch_half_kick(const DevParams& p, Membrane& m, cudaStream_t st);
 void launch_drift(const DevParams& p, Membrane& m, cudaStream_t st);
 void launch_total_va(const DevParams& p, Membrane& m, cudaStream_t st);
