@@ -639,8 +639,8 @@ int resort_any(irbc_handle* h, cudaStream_t st) {
   return h->s.n ? 2 : 0;
 }
 
-// returns the number of kernels launched: vbin, count, ghost flags, three
-// scan kernels, perm, cells, and the physical re-sort when due (never while
+// returns the number of kernels launched: vbin, count, two scan kernels,
+// perm, cells, and the physical re-sort when due (never while
 // a step sequence is being captured; irbc_step re-sorts between captured
 // sequences).  With a side stream the vertex binning runs there (after
 // whatever the side stream already holds: the membrane of the previous
@@ -658,7 +658,7 @@ int collide_any(irbc_handle* h, uint64_t epoch, cudaStream_t st, cudaStream_t si
   }
   if (h->fp32) launch_collide_finish_f(h->dp, h->sf, h->s, h->c, h->m, epoch, st, resort);
   else launch_collide_finish(h->dp, h->s, h->c, h->m, epoch, st, resort);
-  return 8 + (resort && h->s.n ? 2 : 0);
+  return 6 + (resort && h->s.n ? 2 : 0);
 }
 
 // profiling: a pair of events around a launch group of a category
@@ -922,7 +922,7 @@ static int refresh_listed(irbc_handle* h) {
 static int do_llist(irbc_handle* h) {
   Cells& c = h->c;
   int64_t need = launch_llist_count(h->dp, c, h->m, h->st);
-  g_launches += 3 + 3;
+  g_launches += 2 + 2;
   if (need > c.lcap2) {
     dfree(c.lidx2);
     c.lcap2 = need + need / 4 + 1024;
@@ -1207,9 +1207,8 @@ extern "C" int irbc_set_state(irbc_handle* h, const irbc_view* v) {
     }
     // list starts: the lengths scanned on the device
     if (up(h, c.lcnt, v->llen, c.n) || up(h, c.lidx, v->lidx, tot)) return IRBC_ERR_CUDA;
-    launch_scan3(c.lcnt, nullptr, nullptr, c.lstart, nullptr, nullptr, c.totals + 8, c.n, c.scan_part, h->st);
-    CK(cudaMemcpyAsync(c.lstart + c.n, c.totals + 8, sizeof(int), cudaMemcpyDeviceToDevice, h->st));
-    g_launches += 3;
+    launch_scan3(c.lcnt, nullptr, nullptr, c.lstart, nullptr, nullptr, c.totals + 8, c.n, c.scan_part, h->st, true);
+    g_launches += 2;
     int rc = refresh_listed(h);
     if (rc) return rc;
   }

@@ -59,8 +59,7 @@ void bin_particles(const DevParams& p, const double* x, const double* y, const d
                    int* part, int* totals, cudaStream_t st) {
   cudaMemsetAsync(cnt, 0, sizeof(int) * p.ncell, st);
   if (n) k_bin_cell<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(p, x, y, z, n, rx, ry, rz, cell, slot, cnt);
-  launch_scan3(cnt, nullptr, nullptr, start, nullptr, nullptr, totals, p.ncell, part, st);
-  cudaMemcpyAsync(start + p.ncell, totals, sizeof(int), cudaMemcpyDeviceToDevice, st);
+  launch_scan3(cnt, nullptr, nullptr, start, nullptr, nullptr, totals, p.ncell, part, st, true);
   if (n) k_bin_scatter<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(cell, slot, start, n, order);
   k_bin_segsort<<<(unsigned)((p.ncell + 255) / 256), 256, 0, st>>>(start, p.ncell, order);
 }

@@ -110,9 +110,7 @@ extern "C" int irbc_bin_particles_noalloc(const irbc_params* p, const double* x,
   // the array keeps the previous call's contents: clear the counters
   if (cudaMemsetAsync(cnt, 0, sizeof(int) * d.ncell, st) != cudaSuccess) return IRBC_ERR_CUDA;
   if (n) k_na_count<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(d, x, y, z, n, rx, ry, rz, cell, cnt);
-  launch_scan3(cnt, nullptr, nullptr, start, nullptr, nullptr, totals, d.ncell, part, st);
-  if (cudaMemcpyAsync(start + d.ncell, totals, sizeof(int), cudaMemcpyDeviceToDevice, st) != cudaSuccess)
-    return IRBC_ERR_CUDA;
+  launch_scan3(cnt, nullptr, nullptr, start, nullptr, nullptr, totals, d.ncell, part, st, true);
   if (cudaMemsetAsync(cnt, 0, sizeof(int) * d.ncell, st) != cudaSuccess) return IRBC_ERR_CUDA;
   if (n) k_na_fill<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(cell, start, n, cnt, order);
   k_na_segsort<<<(unsigned)((d.ncell + 255) / 256), 256, 0, st>>>(start, d.ncell, order);

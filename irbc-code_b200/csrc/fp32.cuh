@@ -118,9 +118,7 @@ void launch_collide_count_f(const DevParams& p, SolventF& f, Solvent& s, Cells& 
 // float rotation: k_cells_tile<true> (cells_tile.cuh)
 void launch_collide_finish_f(const DevParams& p, SolventF& f, Solvent& s, Cells& c, Membrane& m, uint64_t epoch,
                              cudaStream_t st, bool resort) {
-  launch_ghost_flags(p, c, m, st);
-  launch_scan3(c.cnt, c.wrank, c.mrank, c.start, c.wrank, c.mrank, c.totals, c.n, c.scan_part, st);
-  cudaMemcpyAsync(c.start + c.n, c.totals + 0, sizeof(int), cudaMemcpyDeviceToDevice, st);
+  launch_collide_scan(p, c, m, st);
   if (f.n) k_perm_f<<<nbf(f.n, 256), 256, 0, st>>>(f.pid, s.slot, c.start, f.n, s.perm);
   k_cells_tile<true><<<cells_tile_blocks(c.n), 32 * kTileWarps, 0, st>>>(p, s, f, c, m, epoch);
   if (resort) launch_resort_f(f, s, st);

@@ -174,83 +174,58 @@ void launch_classify(const DevParams& p, Solvent& s, const Membrane& m, cudaStre
 
 // ================================================================ scan ======
 // Exclusive scan of up to three int arrays at once (null input = zeros):
-// per-block sums, one block scanning the block sums, then the per-block
-// rescan with offsets.  totals[k] receives the sum of array k.
+// per-block sums, then the per-block rescan, each block adding up the sums of
+// the blocks before it.  totals[k] receives the sum of array k, and so does the
+// entry behind oa's last one where `end` asks for it.
 constexpr int kScanT = 256, kScanItems = 4, kScanTile = kScanT * kScanItems;
 
 int64_t scan_part_blocks(int64_t n) { return (n + kScanTile - 1) / kScanTile; }
 
 __device__ __forceinline__ int ld0(const int* a, int64_t i) { return a ? a[i] : 0; }
 
-__device__ __forceinline__ void scan_part_block(const int* a, const int* b, const int* c, int64_t n, int* part,
-                                                int64_t bid) {
-  int64_t base = bid * kScanTile + threadIdx.x * kScanItems;
-  int s[3] = {0, 0, 0};
-  for (int q = 0; q < kScanItems; ++q) {
-    int64_t i = base + q;
-    if (i < n) { s[0] += ld0(a, i); s[1] += ld0(b, i); s[2] += ld0(c, i); }
-  }
+// the block's sums of s[0..2] over its threads, in thread k < 3
+__device__ __forceinline__ void block_sums3(const int s[3], int out[3]) {
+  __shared__ int ws[3][kScanT / 32];
   for (int k = 0; k < 3; ++k) {
     int x = s[k];
     for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-    s[k] = x;
+    if ((threadIdx.x & 31) == 0) ws[k][threadIdx.x >> 5] = x;
   }
-  __shared__ int ws[3][kScanT / 32];
-  if ((threadIdx.x & 31) == 0)
-    for (int k = 0; k < 3; ++k) ws[k][threadIdx.x >> 5] = s[k];
   __syncthreads();
-  if (threadIdx.x < 3) {
+  for (int k = 0; k < 3; ++k) {
     int t = 0;
-    for (int q = 0; q < kScanT / 32; ++q) t += ws[threadIdx.x][q];
-    part[bid * 3 + threadIdx.x] = t;
+    for (int q = 0; q < kScanT / 32; ++q) t += ws[k][q];
+    out[k] = t;
   }
 }
-__global__ void k_scan_part(const int* a, const int* b, const int* c, int64_t n, int* part) {
-  scan_part_block(a, b, c, n, part, blockIdx.x);
-}
-
-// one block: exclusive scan of the block sums in place, totals out
-__device__ __forceinline__ void scan_top_block(int* part, int64_t nb, int* totals) {
-  __shared__ int carry[3];
-  if (threadIdx.x < 3) carry[threadIdx.x] = 0;
-  __syncthreads();
-  for (int64_t b0 = 0; b0 < nb; b0 += blockDim.x) {
-    int64_t b = b0 + threadIdx.x;
-    for (int k = 0; k < 3; ++k) {
-      int x = b < nb ? part[b * 3 + k] : 0;
-      int orig = x;
-      const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-      for (int o = 1; o < 32; o <<= 1) {
-        int y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
-      }
-      __shared__ int ws[32];
-      if (lane == 31) ws[w] = x;
-      __syncthreads();
-      if (w == 0) {
-        int y = lane < (int)(blockDim.x >> 5) ? ws[lane] : 0;
-        int yo = y;
-        for (int o = 1; o < 32; o <<= 1) {
-          int z = __shfl_up_sync(0xffffffffu, y, o);
-          if (lane >= o) y += z;
-        }
-        if (lane < (int)(blockDim.x >> 5)) ws[lane] = y - yo;
-      }
-      __syncthreads();
-      int excl = x - orig + ws[w] + carry[k];
-      if (b < nb) part[b * 3 + k] = excl;
-      __syncthreads();
-      if (threadIdx.x == blockDim.x - 1) carry[k] = excl + orig;
-      __syncthreads();
-    }
+// item(i, v): the three values at i
+template <class Item>
+__device__ __forceinline__ void scan_part_block(int64_t n, int* part, int64_t bid, Item item) {
+  const int64_t base = bid * kScanTile + threadIdx.x * kScanItems;
+  int s[3] = {0, 0, 0}, t[3];
+  for (int q = 0; q < kScanItems; ++q) {
+    const int64_t i = base + q;
+    if (i >= n) break;
+    int v[3];
+    item(i, v);
+    s[0] += v[0]; s[1] += v[1]; s[2] += v[2];
   }
-  if (threadIdx.x < 3 && totals) totals[threadIdx.x] = carry[threadIdx.x];
+  block_sums3(s, t);
+  if (threadIdx.x < 3) part[bid * 3 + threadIdx.x] = t[threadIdx.x];
 }
-__global__ void k_scan_top(int* part, int64_t nb, int* totals) { scan_top_block(part, nb, totals); }
+__global__ void __launch_bounds__(kScanT) k_scan_part(const int* a, const int* b, const int* c, int64_t n, int* part) {
+  scan_part_block(n, part, blockIdx.x, [&](int64_t i, int v[3]) { v[0] = ld0(a, i); v[1] = ld0(b, i); v[2] = ld0(c, i); });
+}
 
 __device__ __forceinline__ void scan_final_block(const int* a, const int* b, const int* c, int* oa, int* ob, int* oc,
-                                                 int64_t n, const int* part, int64_t bid) {
-  int64_t base = bid * kScanTile + threadIdx.x * kScanItems;
+                                                 int64_t n, const int* part, int64_t bid, int64_t nblk, int* totals,
+                                                 int end) {
+  // the sums of the blocks before this one
+  int before[3], mine[3] = {0, 0, 0};
+  for (int64_t q = threadIdx.x; q < bid; q += kScanT)
+    for (int k = 0; k < 3; ++k) mine[k] += part[q * 3 + k];
+  block_sums3(mine, before);
+  const int64_t base = bid * kScanTile + threadIdx.x * kScanItems;
   int loc[3][kScanItems];
   int s[3] = {0, 0, 0};
   for (int q = 0; q < kScanItems; ++q) {
@@ -273,12 +248,11 @@ __device__ __forceinline__ void scan_final_block(const int* a, const int* b, con
     ex[k] = x - s[k];
   }
   __syncthreads();
-  if (threadIdx.x < 3) {
+  for (int k = 0; k < 3; ++k) {
     int acc = 0;
-    for (int q = 0; q < kScanT / 32; ++q) { int t = ws[threadIdx.x][q]; ws[threadIdx.x][q] = acc; acc += t; }
+    for (int q = 0; q < w; ++q) acc += ws[k][q];
+    ex[k] += acc + before[k];
   }
-  __syncthreads();
-  for (int k = 0; k < 3; ++k) ex[k] += ws[k][w] + part[bid * 3 + k];
   for (int q = 0; q < kScanItems; ++q) {
     int64_t i = base + q;
     if (i < n) {
@@ -287,19 +261,23 @@ __device__ __forceinline__ void scan_final_block(const int* a, const int* b, con
       if (oc) oc[i] = ex[2] + loc[2][q];
     }
   }
+  if (bid == nblk - 1 && threadIdx.x == kScanT - 1) {
+    if (totals)
+      for (int k = 0; k < 3; ++k) totals[k] = ex[k] + s[k];
+    if (end) oa[n] = ex[0] + s[0];
+  }
 }
-__global__ void k_scan_final(const int* a, const int* b, const int* c, int* oa, int* ob, int* oc,
-                             int64_t n, const int* part) {
-  scan_final_block(a, b, c, oa, ob, oc, n, part, blockIdx.x);
+__global__ void __launch_bounds__(kScanT) k_scan_final(const int* a, const int* b, const int* c, int* oa, int* ob,
+                                                       int* oc, int64_t n, const int* part, int* totals, int end) {
+  scan_final_block(a, b, c, oa, ob, oc, n, part, blockIdx.x, gridDim.x, totals, end);
 }
 
 void launch_scan3(const int* a, const int* b, const int* c, int* oa, int* ob, int* oc, int* totals,
-                  int64_t n, int* part, cudaStream_t st) {
+                  int64_t n, int* part, cudaStream_t st, bool end) {
   int64_t nb = scan_part_blocks(n);
   if (nb == 0) return;
   k_scan_part<<<(unsigned)nb, kScanT, 0, st>>>(a, b, c, n, part);
-  k_scan_top<<<1, 1024, 0, st>>>(part, nb, totals);
-  k_scan_final<<<(unsigned)nb, kScanT, 0, st>>>(a, b, c, oa, ob, oc, n, part);
+  k_scan_final<<<(unsigned)nb, kScanT, 0, st>>>(a, b, c, oa, ob, oc, n, part, totals, end ? 1 : 0);
 }
 
 // ============================================================== collide =====
@@ -315,46 +293,41 @@ __device__ __forceinline__ int shifted_cell(const DevParams& p, double x, double
   return cell_of(p, fx, fy, fz);
 }
 
-// vertices and parasite into the shifted grid (:149-162); vertex keys sorted
-// by (cell, vertex) with a bitonic sort in shared memory
-__device__ __forceinline__ void vbin_block(const DevParams& p, const Membrane& m, int* ncm, uint64_t eoff) {
-  const uint64_t epoch = epoch_of(p, eoff);
+// vertices and parasite into the shifted grid (:149-162); vertex keys sorted by
+// (cell, vertex).  Every block makes all keys (they are distinct) and places
+// kVbinPer of them: a key's place is the number of smaller ones, counted by
+// eight lanes.  (2562 vertices, alone 13 us and beside the count 31; a bitonic
+// sort in one block took 50, of which a small box's collision waited for 45.)
+constexpr int kVbinT = 256, kVbinPer = kVbinT / 8;
+__device__ __forceinline__ void vbin_block(const DevParams& p, const Membrane& m, int* ncm, uint64_t eoff, int bid) {
   extern __shared__ uint64_t sk[];
-  double r[3];
-  grid_shift(p, epoch, r);
-  int n2 = 1;
-  while (n2 < p.nv) n2 <<= 1;
-  for (int i = threadIdx.x; i < n2; i += blockDim.x) {
-    if (i < p.nv) {
-      int c = shifted_cell(p, m.x[i], m.y[i], m.z[i], r);
-      m.pid[i] = c;
-      atomicAdd(&ncm[c], 1);
-      sk[i] = ((uint64_t)(uint32_t)c << 32) | (uint32_t)i;
-    } else {
-      sk[i] = ~0ull;
-    }
-  }
-  if (threadIdx.x == 0) {
+  __shared__ double sr[3];
+  if (threadIdx.x == 0) grid_shift(p, epoch_of(p, eoff), sr);
+  __syncthreads();
+  const double r[3] = {sr[0], sr[1], sr[2]};
+  for (int i = threadIdx.x; i < p.nv; i += kVbinT)
+    sk[i] = ((uint64_t)(uint32_t)shifted_cell(p, m.x[i], m.y[i], m.z[i], r) << 32) | (uint32_t)i;
+  if (bid == 0 && threadIdx.x == 0) {
     MemScalars* sc = m.sc;
     sc->paraid = shifted_cell(p, sc->para[0], sc->para[1], sc->para[2], r);
   }
   __syncthreads();
-  for (int k = 2; k <= n2; k <<= 1) {
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      for (int i = threadIdx.x; i < n2; i += blockDim.x) {
-        int l = i ^ j;
-        if (l > i) {
-          uint64_t a = sk[i], b = sk[l];
-          bool up = ((i & k) == 0);
-          if ((a > b) == up) { sk[i] = b; sk[l] = a; }
-        }
-      }
-      __syncthreads();
-    }
+  const int v = bid * kVbinPer + (int)(threadIdx.x >> 3), sub = threadIdx.x & 7;
+  const uint64_t key = v < p.nv ? sk[v] : 0;
+  int below = 0;
+#pragma unroll 4
+  for (int u = sub; u < p.nv; u += 8) below += sk[u] < key ? 1 : 0;
+  for (int o = 4; o > 0; o >>= 1) below += __shfl_xor_sync(0xffffffffu, below, o);
+  if (v < p.nv && sub == 0) {
+    const int c = (int)(key >> 32);
+    m.vkey[below] = key;
+    m.pid[v] = c;
+    atomicAdd(&ncm[c], 1);
   }
-  for (int i = threadIdx.x; i < p.nv; i += blockDim.x) m.vkey[i] = sk[i];
 }
-__global__ void k_vbin(DevParams p, Membrane m, int* ncm, uint64_t eoff) { vbin_block(p, m, ncm, eoff); }
+__global__ void __launch_bounds__(kVbinT) k_vbin(DevParams p, Membrane m, int* ncm, uint64_t eoff) {
+  vbin_block(p, m, ncm, eoff, blockIdx.x);
+}
 
 // cell of each particle in the shifted grid; warp-aggregated slot counters
 __global__ void __launch_bounds__(256) k_count(DevParams p, Solvent s, int* cnt, uint64_t eoff) {
@@ -386,24 +359,35 @@ __global__ void __launch_bounds__(256) k_count(DevParams p, Solvent s, int* cnt,
   }
 }
 
-// ghost flags for the scan: wall cells (zmax >= Lz or zmin <= 0) with fewer
-// than navg solvent particles (:185-204), and membrane cells with fewer
-// than navg particles of any kind (:236-244)
-__device__ __forceinline__ void ghost_flags_item(const DevParams& p, const int* cnt, const int* ncm,
-                                                 const MemScalars* sc, int* wflag, int* mflag, int64_t c) {
-  if (c >= p.ncell) return;
-  int k = (int)(c % p.nz);
-  double zmin = -1.0 + (double)k * p.a, zmax = -1.0 + (double)k * p.a + p.a;
-  int nn = cnt[c];
-  int wall = ((zmax >= p.Lz) || (zmin <= 0)) && (nn < p.navg);
-  int nt = nn + ncm[c] + (c == sc->paraid ? 1 : 0);
-  int mem = (ncm[c] > 0) && (nt < p.navg);
-  wflag[c] = wall;
-  mflag[c] = mem;
+// what a collision scans over the cells: the particle counts and the ghost
+// flags, wall cells (zmax >= Lz or zmin <= 0) with fewer than navg solvent
+// particles (:185-204) and membrane cells with fewer than navg particles of any
+// kind (:236-244)
+__device__ __forceinline__ void collide_part_block(const DevParams& p, const int* cnt, const int* ncm,
+                                                   const MemScalars* sc, int* wflag, int* mflag, int* part,
+                                                   int64_t bid) {
+  const int paraid = sc->paraid;
+  scan_part_block(p.ncell, part, bid, [&](int64_t c, int v[3]) {
+    int k = (int)(c % p.nz);
+    double zmin = -1.0 + (double)k * p.a, zmax = -1.0 + (double)k * p.a + p.a;
+    int nn = cnt[c], nm = ncm[c];
+    int wall = ((zmax >= p.Lz) || (zmin <= 0)) && (nn < p.navg);
+    int nt = nn + nm + (c == paraid ? 1 : 0);
+    int mem = (nm > 0) && (nt < p.navg);
+    wflag[c] = wall;
+    mflag[c] = mem;
+    v[0] = nn; v[1] = wall; v[2] = mem;
+  });
 }
-__global__ void k_ghost_flags(DevParams p, const int* cnt, const int* ncm, const MemScalars* sc,
-                              int* wflag, int* mflag) {
-  ghost_flags_item(p, cnt, ncm, sc, wflag, mflag, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
+__global__ void __launch_bounds__(kScanT) k_collide_part(DevParams p, const int* cnt, const int* ncm,
+                                                         const MemScalars* sc, int* wflag, int* mflag, int* part) {
+  collide_part_block(p, cnt, ncm, sc, wflag, mflag, part, blockIdx.x);
+}
+// wrank/mrank hold the flags first, then their exclusive scans
+void launch_collide_scan(const DevParams& p, Cells& c, const Membrane& m, cudaStream_t st) {
+  const unsigned nb = (unsigned)scan_part_blocks(c.n);
+  k_collide_part<<<nb, kScanT, 0, st>>>(p, c.cnt, c.ncm, m.sc, c.wrank, c.mrank, c.scan_part);
+  k_scan_final<<<nb, kScanT, 0, st>>>(c.cnt, c.wrank, c.mrank, c.start, c.wrank, c.mrank, c.n, c.scan_part, c.totals, 1);
 }
 
 // counting sort of particle indices: perm[start[cell] + slot] = i
@@ -436,14 +420,8 @@ __global__ void k_copy_back(Solvent s) {
 
 
 void launch_vbin(const DevParams& p, Membrane& m, Cells& c, uint64_t epoch, cudaStream_t st) {
-  int n2 = 1;
-  while (n2 < p.nv) n2 <<= 1;
   cudaMemsetAsync(c.ncm, 0, sizeof(int) * c.n, st);
-  k_vbin<<<1, 1024, sizeof(uint64_t) * n2, st>>>(p, m, c.ncm, epoch);
-}
-
-void launch_ghost_flags(const DevParams& p, Cells& c, const Membrane& m, cudaStream_t st) {
-  k_ghost_flags<<<nblk(c.n, 256), 256, 0, st>>>(p, c.cnt, c.ncm, m.sc, c.wrank, c.mrank);
+  k_vbin<<<nblk(p.nv, kVbinPer), kVbinT, sizeof(uint64_t) * p.nv, st>>>(p, m, c.ncm, epoch);
 }
 
 void launch_collide_count(const DevParams& p, Solvent& s, Cells& c, uint64_t epoch, cudaStream_t st) {
@@ -453,11 +431,7 @@ void launch_collide_count(const DevParams& p, Solvent& s, Cells& c, uint64_t epo
 
 void launch_collide_finish(const DevParams& p, Solvent& s, Cells& c, Membrane& m, uint64_t epoch,
                            cudaStream_t st, bool resort) {
-  // wrank/mrank hold the flags first, then their exclusive scans
-  k_ghost_flags<<<nblk(c.n, 256), 256, 0, st>>>(p, c.cnt, c.ncm, m.sc, c.wrank, c.mrank);
-  launch_scan3(c.cnt, c.wrank, c.mrank, c.start, c.wrank, c.mrank, c.totals, c.n, c.scan_part, st);
-  // start[C] = Ns
-  cudaMemcpyAsync(c.start + c.n, c.totals + 0, sizeof(int), cudaMemcpyDeviceToDevice, st);
+  launch_collide_scan(p, c, m, st);
   if (s.n) k_perm<<<nblk(s.n, 256), 256, 0, st>>>(s.pid, s.slot, c.start, s.n, s.perm);
   k_cells_tile<false><<<cells_tile_blocks(c.n), 32 * kTileWarps, 0, st>>>(p, s, SolventF{}, c, m, epoch);
   if (resort) launch_resort(s, st);
@@ -577,11 +551,10 @@ __global__ void __launch_bounds__(kLTile) k_llist(DevParams p, Cells cl, Membran
 int64_t launch_llist_count(const DevParams& p, Cells& c, const Membrane& m, cudaStream_t st) {
   k_tri_centroid<<<nblk(p.nt, 128), 128, 0, st>>>(p, m);
   k_llist<false><<<nblk(c.n, kLTile), kLTile, 0, st>>>(p, c, m);
-  launch_scan3(c.lcnt, nullptr, nullptr, c.lstart2, nullptr, nullptr, c.totals + 8, c.n, c.scan_part, st);
+  launch_scan3(c.lcnt, nullptr, nullptr, c.lstart2, nullptr, nullptr, c.totals + 8, c.n, c.scan_part, st, true);
   int tot = 0;
   cudaMemcpyAsync(&tot, c.totals + 8, sizeof(int), cudaMemcpyDeviceToHost, st);
   cudaStreamSynchronize(st);
-  cudaMemcpyAsync(c.lstart2 + c.n, c.totals + 8, sizeof(int), cudaMemcpyDeviceToDevice, st);
   return tot;
 }
 
@@ -1102,30 +1075,21 @@ __global__ void __launch_bounds__(256) km_zero(Member* __restrict__ mem, const i
   const int64_t c = (int64_t)b * blockDim.x + threadIdx.x;
   if (c < M.c.n) { M.c.cnt[c] = 0; M.c.ncm[c] = 0; }
 }
-__global__ void __launch_bounds__(1024) km_vbin(Member* __restrict__ mem, const int2* __restrict__ tab,
+__global__ void __launch_bounds__(kVbinT) km_vbin(Member* __restrict__ mem, const int2* __restrict__ tab,
                                                 uint64_t eoff) {
   KM_MEMBER;
-  vbin_block(M.p, M.m, M.c.ncm, eoff);
+  vbin_block(M.p, M.m, M.c.ncm, eoff, b);
 }
-__global__ void __launch_bounds__(256) km_ghost(Member* __restrict__ mem, const int2* __restrict__ tab) {
+// the scans of (cnt, wrank, mrank) into (start, wrank, mrank), as
+// launch_collide_scan
+__global__ void __launch_bounds__(kScanT) km_collide_part(Member* __restrict__ mem, const int2* __restrict__ tab) {
   KM_MEMBER;
-  ghost_flags_item(M.p, M.c.cnt, M.c.ncm, M.m.sc, M.c.wrank, M.c.mrank, (int64_t)b * blockDim.x + threadIdx.x);
-}
-// the scans of (cnt, wrank, mrank) into (start, wrank, mrank), as launch_scan3
-__global__ void __launch_bounds__(kScanT) km_scan_part(Member* __restrict__ mem, const int2* __restrict__ tab) {
-  KM_MEMBER;
-  scan_part_block(M.c.cnt, M.c.wrank, M.c.mrank, M.c.n, M.c.scan_part, b);
-}
-// one block per member; also start[C] = the particle total
-__global__ void __launch_bounds__(1024) km_scan_top(Member* __restrict__ mem, const int2* __restrict__ tab) {
-  KM_MEMBER;
-  scan_top_block(M.c.scan_part, (M.c.n + kScanTile - 1) / kScanTile, M.c.totals);
-  __syncthreads();
-  if (threadIdx.x == 0) M.c.start[M.c.n] = M.c.totals[0];
+  collide_part_block(M.p, M.c.cnt, M.c.ncm, M.m.sc, M.c.wrank, M.c.mrank, M.c.scan_part, b);
 }
 __global__ void __launch_bounds__(kScanT) km_scan_final(Member* __restrict__ mem, const int2* __restrict__ tab) {
   KM_MEMBER;
-  scan_final_block(M.c.cnt, M.c.wrank, M.c.mrank, M.c.start, M.c.wrank, M.c.mrank, M.c.n, M.c.scan_part, b);
+  scan_final_block(M.c.cnt, M.c.wrank, M.c.mrank, M.c.start, M.c.wrank, M.c.mrank, M.c.n, M.c.scan_part, b,
+                   (M.c.n + kScanTile - 1) / kScanTile, M.c.totals, 1);
 }
 
 void set_collide_kernel_limits() {
@@ -1135,16 +1099,14 @@ void set_collide_kernel_limits() {
 
 int multi_collide_front(const MultiPlan& P, uint64_t eoff, cudaStream_t st) {
   km_zero<<<P.blocks[MP_ZERO], 256, 0, st>>>(P.mem, P.table(MP_ZERO));
-  km_vbin<<<P.blocks[MP_VBIN], 1024, P.vbin_smem, st>>>(P.mem, P.table(MP_VBIN), eoff);
+  km_vbin<<<P.blocks[MP_VBIN], kVbinT, P.vbin_smem, st>>>(P.mem, P.table(MP_VBIN), eoff);
   return 2;
 }
 
 int multi_collide_scan(const MultiPlan& P, cudaStream_t st) {
-  km_ghost<<<P.blocks[MP_GHOST], 256, 0, st>>>(P.mem, P.table(MP_GHOST));
-  km_scan_part<<<P.blocks[MP_SCAN], kScanT, 0, st>>>(P.mem, P.table(MP_SCAN));
-  km_scan_top<<<P.blocks[MP_SCAN_TOP], 1024, 0, st>>>(P.mem, P.table(MP_SCAN_TOP));
+  km_collide_part<<<P.blocks[MP_SCAN], kScanT, 0, st>>>(P.mem, P.table(MP_SCAN));
   km_scan_final<<<P.blocks[MP_SCAN], kScanT, 0, st>>>(P.mem, P.table(MP_SCAN));
-  return 4;
+  return 2;
 }
 
 }  // namespace irbc

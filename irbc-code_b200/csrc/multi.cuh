@@ -183,20 +183,16 @@ void multi_blocks(const Member& M, int out[MP_NPHASE]) {
   out[MP_RECORDS] = (int)nbf((int64_t)kSegMax * M.p.nt, 128);
   out[MP_CULL] = (int)nb(M.p.nt, 64);
   out[MP_ZERO] = (int)nb(nc, 256);
-  out[MP_VBIN] = 1;
+  out[MP_VBIN] = (int)nb(M.p.nv, 32);
   out[MP_COUNT] = (int)nbf(ns, 256 * kCountPer);
-  out[MP_GHOST] = (int)nb(nc, 256);
   out[MP_SCAN] = (int)scan_part_blocks(nc);
-  out[MP_SCAN_TOP] = 1;
   out[MP_PERM] = (int)nbf(ns, 256);
   out[MP_TILE] = (int)cells_tile_blocks(nc);
   out[MP_MOVE] = (int)nbf(ns, 256);
 }
 
 int multi_vbin_smem(const Member& M) {
-  int n2 = 1;
-  while (n2 < M.p.nv) n2 <<= 1;
-  return (int)sizeof(uint64_t) * n2;
+  return (int)sizeof(uint64_t) * M.p.nv;
 }
 
 int multi_segment(const Member& M, int* smem) {

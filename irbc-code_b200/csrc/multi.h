@@ -29,7 +29,7 @@ struct Member {
 enum MultiPhase : int {
   MP_STREAM, MP_NEAR_SHORT, MP_NEAR_LONG,                         // streaming
   MP_MEMBRANE, MP_RECORDS, MP_CULL,                                     // membrane of a stretch
-  MP_ZERO, MP_VBIN, MP_COUNT, MP_GHOST, MP_SCAN, MP_SCAN_TOP, MP_PERM, MP_TILE, MP_MOVE,  // collision
+  MP_ZERO, MP_VBIN, MP_COUNT, MP_SCAN, MP_PERM, MP_TILE, MP_MOVE,  // collision
   MP_NPHASE
 };
 
@@ -42,7 +42,7 @@ struct MultiPlan {
   int64_t off[MP_NPHASE] = {};   // where phase k's table starts
   int n = 0;
   int blocks[MP_NPHASE] = {};    // each phase's grid
-  int vbin_smem = 0;             // vertex binning: the largest member's sort
+  int vbin_smem = 0;             // vertex binning: the largest member's keys
   // membrane: a launch per cluster size, its members' blocks in this order in
   // phase MP_MEMBRANE's table; smem: the largest member's
   struct Seg { int nc, members, smem; };

@@ -119,7 +119,8 @@ void launch_collide_finish(const DevParams& p, Solvent& s, Cells& c, Membrane& m
                            cudaStream_t st, bool resort);
 // physical re-sort by the cells of the latest collision (any time after it)
 void launch_resort(Solvent& s, cudaStream_t st);
-void launch_ghost_flags(const DevParams& p, Cells& c, const Membrane& m, cudaStream_t st);
+// the collision's scans over the cells (counts and ghost flags)
+void launch_collide_scan(const DevParams& p, Cells& c, const Membrane& m, cudaStream_t st);
 // returns the total list length the update needs (host sync inside)
 int64_t launch_llist_count(const DevParams& p, Cells& c, const Membrane& m, cudaStream_t st);
 // total: the entry count launch_llist_count returned (both list buffers hold it)
@@ -134,8 +135,9 @@ void launch_pfdt_forces(const DevParams& p, Membrane& m, int do_pfdt, int do_for
                         cudaStream_t st);
 void launch_bonds(const DevParams& p, Membrane& m, uint64_t epoch, cudaStream_t st);
 void launch_kick2(const DevParams& p, Membrane& m, cudaStream_t st);
+// end: oa[n] receives the total too
 void launch_scan3(const int* a, const int* b, const int* c, int* oa, int* ob, int* oc, int* totals,
-                  int64_t n, int* part, cudaStream_t st);
+                  int64_t n, int* part, cudaStream_t st, bool end = false);
 // obs: the kObsDoubles scratch; nbins > 0 also fills the velocity profile
 // (obs + 64, nbins <= kObsMaxBins)
 void launch_observables(const DevParams& p, const Solvent& s, const Membrane& m, double* obs, int nbins,
