@@ -2019,8 +2019,7 @@ extern "C" int irbc_write_stl(irbc_handle* h, const char* path) {
 
 extern "C" int irbc_observables(irbc_handle* h, double* out, int32_t nout) {
   if (!h || !out || nout <= 0) return IRBC_ERR_ARG;
-  if (h->fp32) f32_to_f64(h->sf, h->s, h->st);
-  launch_observables(h->dp, h->s, h->m, h->obs, 0, h->st);
+  launch_observables(h->dp, h->s, h->fp32 ? &h->sf : nullptr, h->m, h->obs, 0, h->st);
   g_launches += 2;
   double buf[16] = {0};
   CK(cudaMemcpyAsync(buf, h->obs, sizeof(double) * 16, cudaMemcpyDeviceToHost, h->st));
@@ -2031,8 +2030,7 @@ extern "C" int irbc_observables(irbc_handle* h, double* out, int32_t nout) {
 
 extern "C" int irbc_velocity_profile(irbc_handle* h, double* out, int32_t nbins) {
   if (!h || !out || nbins <= 0 || nbins > kObsMaxBins) return IRBC_ERR_ARG;
-  if (h->fp32) f32_to_f64(h->sf, h->s, h->st);
-  launch_observables(h->dp, h->s, h->m, h->obs, nbins, h->st);
+  launch_observables(h->dp, h->s, h->fp32 ? &h->sf : nullptr, h->m, h->obs, nbins, h->st);
   g_launches += 2;
   std::vector<double> buf(2 * nbins);
   CK(cudaMemcpyAsync(buf.data(), h->obs + 64, sizeof(double) * 2 * nbins, cudaMemcpyDeviceToHost, h->st));

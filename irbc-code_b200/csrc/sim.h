@@ -22,6 +22,8 @@ struct __align__(16) SolVel {
   int id, pad;
 };
 
+struct SolventF;  // fp32.h
+
 struct Solvent {
   int64_t n = 0;
   double *x = nullptr, *y = nullptr, *z = nullptr;
@@ -138,10 +140,10 @@ void launch_kick2(const DevParams& p, Membrane& m, cudaStream_t st);
 // end: oa[n] receives the total too
 void launch_scan3(const int* a, const int* b, const int* c, int* oa, int* ob, int* oc, int* totals,
                   int64_t n, int* part, cudaStream_t st, bool end = false);
-// obs: the kObsDoubles scratch; nbins > 0 also fills the velocity profile
+// sf: the FP32-bulk solvent, or null.  obs: the kObsDoubles scratch; nbins > 0 also fills the velocity profile
 // (obs + 64, nbins <= kObsMaxBins)
-void launch_observables(const DevParams& p, const Solvent& s, const Membrane& m, double* obs, int nbins,
-                        cudaStream_t st);
+void launch_observables(const DevParams& p, const Solvent& s, const SolventF* sf, const Membrane& m, double* obs,
+                        int nbins, cudaStream_t st);
 
 int64_t scan_part_blocks(int64_t n);
 
