@@ -29,8 +29,12 @@ __host__ __device__ constexpr int seg_terms(int nt) { return (nt + 32 + 15) / 16
 
 // near-membrane streaming: lanes per particle and room for kept entries, for
 // lists of up to kShortList entries and for longer ones; threads per block,
-// blocks per SM, blocks per simulation alone and per member of a cohort
-constexpr int kShortList = 128, kShortG = 8, kShortKeep = 64, kLongG = 32, kLongKeep = 512;
+// blocks per SM, blocks per simulation alone and per member of a cohort.  A
+// simulation alone has few particles near the membrane (some 10 000), so more
+// lanes each finish sooner: 8 lanes 93 us a stretch, 1 and 2 lanes 199 and 154
+// (600 vertices); 32 lanes 242 us, 16 and 8 lanes 316 and 534 (2562).  Sixteen
+// members fill the GPU, where idle lanes cost: 4 lanes 911 us, 8 lanes 1063.
+constexpr int kShortList = 128, kShortG = 8, kShortGMember = 4, kShortKeep = 64, kLongG = 32, kLongKeep = 512;
 constexpr int kNearT = 128, kNearMinBlocks = 4, kNearBlocks = 148 * kNearMinBlocks, kNearBlocksMember = 148;
 inline bool short_lists(int lmax) { return lmax <= kShortList; }
 // the side-wall bands (3a) that a triangle's corners lie in: tri_record

@@ -52,7 +52,7 @@ int multi_stream(const MultiPlan& P, int H, int par, cudaStream_t st, cudaEvent_
   km_stream_bulk<<<P.blocks[MP_STREAM], 256, 0, st>>>(P.mem, P.table(MP_STREAM), H, par);
   if (snap) cudaStreamWaitEvent(st, snap, 0);
   const int n0 = P.blocks[MP_NEAR_SHORT], n1 = P.blocks[MP_NEAR_LONG];
-  if (n0 > 0) km_near<kShortG, kShortKeep><<<n0, kNearT, 0, st>>>(P.mem, P.table(MP_NEAR_SHORT), H, par);
+  if (n0 > 0) km_near<kShortGMember, kShortKeep><<<n0, kNearT, 0, st>>>(P.mem, P.table(MP_NEAR_SHORT), H, par);
   if (n1 > 0) km_near<kLongG, kLongKeep><<<n1, kNearT, 0, st>>>(P.mem, P.table(MP_NEAR_LONG), H, par);
   return 1 + (n0 > 0) + (n1 > 0);
 }
