@@ -54,7 +54,7 @@ struct irbc_handle {
   FastBufs fb;
   bool fp32 = false;           // solvent held in sf (float4) between exchanges
   SolventF sf;
-  cudaEvent_t ev_mem = nullptr, ev_coll = nullptr;
+  cudaEvent_t ev_mem = nullptr, ev_coll = nullptr, ev_part = nullptr;
   cudaEvent_t ev_vbin = nullptr;
   uint64_t* ebase = nullptr;   // device: the draw epoch base of the current call (DevParams::ebase)
   int64_t ebase_val = 0;       // its value as last written
@@ -561,7 +561,7 @@ int upload_mesh(irbc_handle* h, const HostMesh& M) {
       CK(dalloc(q, (int64_t)kSegMax * M.nv));
     CK(dalloc(&f.pre, (int64_t)kSegMax * M.nt));
     CK(dalloc(&f.bands, (int64_t)kSegMax * M.nt));
-    CK(dalloc(&f.cull, 3 * (int64_t)M.nt));
+    CK(dalloc(&f.cull, 6 * (int64_t)M.nt));
     CK(dalloc(&f.pidx, M.nv));
     for (int** q : {&f.st1, &f.st2, &f.st3}) CK(dalloc(q, M.nt));
     f.snap.t1 = f.st1; f.snap.t2 = f.st2; f.snap.t3 = f.st3;
@@ -694,14 +694,15 @@ struct ProfScope {
 // the streaming kernels; in a profiling window the bulk kernel alone is
 // bracketed by a pair of events of its own
 // returns the number of kernels it launched
-int stream_any(irbc_handle* h, int H, cudaStream_t st, cudaEvent_t snap = nullptr) {
+int stream_any(irbc_handle* h, int H, cudaStream_t st, cudaEvent_t snap = nullptr, int first = 0,
+               cudaEvent_t snap1 = nullptr) {
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (h->prof && !h->capturing) {
     h->ev_marks.push_back({PROF_STREAM_BULK, h->ev_used, h->ev_used + 1});
     e0 = next_event(h);
     e1 = next_event(h);
   }
-  return fast_stream(h->dp, h->s, h->fp32 ? &h->sf : nullptr, h->c, h->fb, H, st, e0, e1, snap);
+  return fast_stream(h->dp, h->s, h->fp32 ? &h->sf : nullptr, h->c, h->fb, H, st, e0, e1, snap, first, snap1);
 }
 
 }  // namespace
@@ -774,7 +775,7 @@ extern "C" int irbc_create(const irbc_params* p, irbc_handle** out) {
       return IRBC_ERR_CUDA;
     }
     h->st2_own = h->st2;
-    for (cudaEvent_t* e : {&h->ev_mem, &h->ev_coll, &h->ev_vbin, &h->ev_health})
+    for (cudaEvent_t* e : {&h->ev_mem, &h->ev_coll, &h->ev_part, &h->ev_vbin, &h->ev_health})
       cudaEventCreateWithFlags(e, cudaEventDisableTiming);
   }
   {
@@ -859,7 +860,7 @@ extern "C" void irbc_destroy(irbc_handle* h) {
   if (h->rec) cudaFree(h->rec);
   for (float4** q : {&h->sf.pos, &h->sf.vel, &h->sf.pos2, &h->sf.vel2}) dfree(*q);
   dfree(h->sf.pid); dfree(h->sf.pid2);
-  for (cudaEvent_t e : {h->ev_mem, h->ev_coll, h->ev_vbin, h->ev_health})
+  for (cudaEvent_t e : {h->ev_mem, h->ev_coll, h->ev_part, h->ev_vbin, h->ev_health})
     if (e) cudaEventDestroy(e);
   dfree(h->health);
   if (h->health_host) cudaFreeHost(h->health_host);
@@ -1304,7 +1305,7 @@ extern "C" int irbc_collide(irbc_handle* h, int64_t epoch) {
 extern "C" int irbc_stream(irbc_handle* h) {
   if (!h || !h->have_mesh) return IRBC_ERR_ARG;
   fast_snap_prep(h->dp, h->m, h->fb, h->st);
-  g_launches += 2 + stream_any(h, 1, h->st);
+  g_launches += 1 + stream_any(h, 1, h->st);
   CK(cudaGetLastError());
   return 0;
 }
@@ -1360,7 +1361,7 @@ extern "C" int irbc_step_part1(irbc_handle* h) {
   }
   {
     ProfScope ps(h, PROF_MEMBRANE);
-    g_launches += launch_membrane(h->dp, h->m, h->fb, 0, 1, SEG_FIRST, h->st);
+    g_launches += launch_membrane(h->dp, h->m, h->fb, 0, 0, 1, SEG_FIRST, h->st);
   }
   {
     ProfScope ps(h, PROF_STREAM);
@@ -1378,7 +1379,7 @@ extern "C" int irbc_step_part2(irbc_handle* h) {
   CK(set_epoch_base(h, (uint64_t)s));
   {
     ProfScope ps(h, PROF_MEMBRANE);
-    g_launches += launch_membrane(h->dp, h->m, h->fb, 0, 1, SEG_SECOND, h->st);
+    g_launches += launch_membrane(h->dp, h->m, h->fb, 0, 0, 1, SEG_SECOND, h->st);
   }
   if (h->filecc == h->P.out_every) { h->filec += 1; h->filecc = 0; }
   h->step = s + 1;
@@ -1415,11 +1416,20 @@ static int64_t stretch_steps(const irbc_handle* h, int64_t left) {
   return H;
 }
 
+// The steps of a stretch's first part (0: one part).  The near-membrane
+// streaming needs the membrane's snapshots of its steps only, so it takes the
+// first 3/5 of them while the membrane, alone on its few SMs, does the others
+// (it takes 1.5 to 2 times as long per step).  A second membrane launch costs
+// some 20 us of start and end, which shorter stretches do not earn back; 12 steps:
+// 43.7 -> 37.6 us a step (2562 vertices, 30 x 30 x 40), 76 -> 67 (120 x 120 x 36),
+// 27.5 -> 24.6 (600 vertices, FP32); half and 7/10 of them in the first part
+// were up to 1 us slower.
+static int first_part(int H) { return H >= 8 ? H * 3 / 5 : 0; }
+
 // A stretch of timesteps: a collision and a list update when its first step
-// has them, then the membrane of all its steps in one launch on the side
-// stream (h->st2) and the streaming of each step on the main one (h->st).
-// Between two collisions the membrane does not depend on the solvent, so it
-// runs ahead.  eoff is the first step's draw-epoch offset from the current
+// has them, then the membrane of its steps on the side stream (h->st2), in one
+// launch or two, and their streaming on the main one (h->st).  Between two
+// collisions the membrane does not depend on the solvent, so it runs ahead.  eoff is the first step's draw-epoch offset from the current
 // base; at most `left` steps.  dry: advance the host counters only (the
 // launches are in a captured sequence being replayed).  Returns the steps
 // taken, negative on an error.
@@ -1447,15 +1457,20 @@ static int64_t stretch(irbc_handle* h, int64_t eoff, int64_t left, bool dry) {
     // and the streaming that last read the snapshots
     CK(cudaEventRecord(h->ev_coll, ms));
     CK(cudaStreamWaitEvent(ss, h->ev_coll, 0));
+    const int first = first_part((int)H);
     {
       ProfScope ps(h, PROF_MEMBRANE, ss);
-      g_launches += launch_membrane(h->dp, h->m, h->fb, (uint64_t)eoff, (int)H, SEG_WHOLE, ss);
+      if (first > 0) {
+        g_launches += launch_membrane(h->dp, h->m, h->fb, (uint64_t)eoff, 0, first, SEG_WHOLE, ss);
+        CK(cudaEventRecord(h->ev_part, ss));
+      }
+      g_launches += launch_membrane(h->dp, h->m, h->fb, (uint64_t)eoff, first, (int)H - first, SEG_WHOLE, ss);
     }
     CK(cudaEventRecord(h->ev_mem, ss));
     {
       // the bulk streaming reads no membrane data and starts at once
       ProfScope ps(h, PROF_STREAM, ms);
-      g_launches += stream_any(h, (int)H, ms, h->ev_mem);
+      g_launches += stream_any(h, (int)H, ms, h->ev_mem, first, h->ev_part);
     }
   }
   step_ends(h);
@@ -1472,7 +1487,7 @@ constexpr int kGraphSteps = 24;  // two collision cycles per captured sequence
 // (whose records belong to the graph) and after each graph launch, so that
 // later waits refer to work outside any graph and follow the launch
 static cudaError_t rearm_events(irbc_handle* h) {
-  for (cudaEvent_t e : {h->ev_mem, h->ev_coll, h->ev_vbin}) {
+  for (cudaEvent_t e : {h->ev_mem, h->ev_coll, h->ev_part, h->ev_vbin}) {
     cudaError_t r = cudaEventRecord(e, h->st);
     if (r != cudaSuccess) return r;
   }

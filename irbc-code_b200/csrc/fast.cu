@@ -262,7 +262,7 @@ __device__ __forceinline__ void flight_store(const SolventArrays& s, int64_t i, 
 struct NearQueue {
   int* i;
   unsigned char* k;
-  int* n;  // their number; n[4]: those taken
+  int* n;  // their number
 };
 inline __host__ __device__ NearQueue queue_of(const FastBufs& f, int par) { return NearQueue{f.queue, f.qk, f.qn + par}; }
 __device__ __forceinline__ void enqueue(const NearQueue& h, int i, int k) {
@@ -439,31 +439,29 @@ __device__ __forceinline__ bool cull_keeps(const TriCull& c, float X, float Y, f
   const float d = sqrtf(x * x + y * y + z * z), move = dP + c.dA;
   return (c.bands & band) || !(b > 1.0001f * (c.dX * (d + move) + c.nX * move) + c.m);
 }
-// triangle j's over H steps
-__device__ __forceinline__ void cull_item(const DevParams& p, const FastBufs& f, int H, int j) {
-  if (j >= p.nt) return;
-  const TriPre t0 = f.pre[j];
-  double dX = 0.0, dA = 0.0;
-  int bands = 0;
-  auto norm = [](double x, double y, double z) { return sqrt(x * x + y * y + z * z); };
-  for (int s = 0; s < H; ++s) {
-    const TriPre t = f.pre[(int64_t)s * p.nt + j];
-    dX = fmax(dX, fmax(norm(t.X[0] - t0.X[0], t.X[1] - t0.X[1], t.X[2] - t0.X[2]),
-                       norm(t.Xdt[0] - t0.X[0], t.Xdt[1] - t0.X[1], t.Xdt[2] - t0.X[2])));
-    dA = fmax(dA, fmax(norm(t.A1[0] - t0.A1[0], t.A1[1] - t0.A1[1], t.A1[2] - t0.A1[2]),
-                       norm(t.A2[0] - t0.A1[0], t.A2[1] - t0.A1[1], t.A2[2] - t0.A1[2])));
-    // a record that is not finite stays in every test
-    if (!isfinite(t.X[0] + t.X[1] + t.X[2] + t.Xdt[0] + t.Xdt[1] + t.Xdt[2] + t.A1[0] + t.A1[1] + t.A1[2] + t.A2[0] +
-                  t.A2[1] + t.A2[2]))
-      dX = dA = __longlong_as_double(0x7ff0000000000000ll);
-    bands |= f.bands[(int64_t)s * p.nt + j];
-  }
+// a step's record against that of the first one
+struct CullMove {
+  double dX, dA;
+  int bands;
+};
+__device__ __forceinline__ double norm3(double x, double y, double z) { return sqrt(x * x + y * y + z * z); }
+__device__ __forceinline__ void cull_fold(CullMove& c, const TriPre& t0, const TriPre& t, int bands) {
+  c.dX = fmax(c.dX, fmax(norm3(t.X[0] - t0.X[0], t.X[1] - t0.X[1], t.X[2] - t0.X[2]),
+                         norm3(t.Xdt[0] - t0.X[0], t.Xdt[1] - t0.X[1], t.Xdt[2] - t0.X[2])));
+  c.dA = fmax(c.dA, fmax(norm3(t.A1[0] - t0.A1[0], t.A1[1] - t0.A1[1], t.A1[2] - t0.A1[2]),
+                         norm3(t.A2[0] - t0.A1[0], t.A2[1] - t0.A1[1], t.A2[2] - t0.A1[2])));
+  // a record that is not finite stays in every test
+  if (!isfinite(t.X[0] + t.X[1] + t.X[2] + t.Xdt[0] + t.Xdt[1] + t.Xdt[2] + t.A1[0] + t.A1[1] + t.A1[2] + t.A2[0] +
+                t.A2[1] + t.A2[2]))
+    c.dX = c.dA = __longlong_as_double(0x7ff0000000000000ll);
+  c.bands |= bands;
+}
+__device__ __forceinline__ void cull_store(const DevParams& p, float4* to, const TriPre& t0, const CullMove& c) {
   const double L = fmax(p.Lx, fmax(p.Ly, p.Lz));
-  const double n1 = fabs(t0.X[0]) + fabs(t0.X[1]) + fabs(t0.X[2]) + dX;
-  float4* to = f.cull + 3 * (int64_t)j;
-  to[0] = make_float4((float)t0.X[0], (float)t0.X[1], (float)t0.X[2], (float)norm(t0.X[0], t0.X[1], t0.X[2]) * 1.00001f);
-  to[1] = make_float4((float)t0.A1[0], (float)t0.A1[1], (float)t0.A1[2], (float)dX * 1.00001f);
-  to[2] = make_float4((float)dA * 1.00001f, (float)(n1 * (L + 16.0) * (1.0 / 2097152.0)), __int_as_float(bands), 0.0f);
+  const double n1 = fabs(t0.X[0]) + fabs(t0.X[1]) + fabs(t0.X[2]) + c.dX;
+  to[0] = make_float4((float)t0.X[0], (float)t0.X[1], (float)t0.X[2], (float)norm3(t0.X[0], t0.X[1], t0.X[2]) * 1.00001f);
+  to[1] = make_float4((float)t0.A1[0], (float)t0.A1[1], (float)t0.A1[2], (float)c.dX * 1.00001f);
+  to[2] = make_float4((float)c.dA * 1.00001f, (float)(n1 * (L + 16.0) * (1.0 / 2097152.0)), __int_as_float(c.bands), 0.0f);
 }
 
 // what the near-membrane kernel reads of one simulation
@@ -475,9 +473,14 @@ struct NearArgs {
   int64_t nt, nv;
   Snap snap;
   NearQueue q;
+  int first;   // the part's first step
+  int* taken;  // particles taken from the queue
 };
-inline __host__ __device__ NearArgs near_of(const DevParams& p, const Cells& c, const FastBufs& f, int par) {
-  return NearArgs{c.lstart, c.lidx, c.flag, f.bands, f.pre, f.cull, p.nt, p.nv, f.snap, queue_of(f, par)};
+// part: of a stretch in two parts (k_near runs once for each)
+inline __host__ __device__ NearArgs near_of(const DevParams& p, const Cells& c, const FastBufs& f, int par, int first,
+                                            int part) {
+  return NearArgs{c.lstart, c.lidx, c.flag, f.bands, f.pre, f.cull + (int64_t)part * 3 * p.nt, p.nt, p.nv, f.snap,
+                  queue_of(f, par), first, f.qn + 4 - 2 * part + par};
 }
 __device__ __forceinline__ Snap near_snap(const NearArgs& a, int t) {
   Snap s = a.snap;
@@ -643,7 +646,8 @@ __device__ __forceinline__ void near_particle(const DevParams& p, const SolventA
   }
   if (g == 0) flight_store(s, i, q);
 }
-// the queue's particles, each by the next group of G lanes that is free
+// the queue's particles through the steps before H, each by the next group of G
+// lanes that is free
 template <typename R, int G, int KEEP>
 __device__ __forceinline__ void near_groups(const DevParams& p, const SolventArrays& s, const NearArgs& A, int H,
                                             unsigned short* kept) {
@@ -652,10 +656,12 @@ __device__ __forceinline__ void near_groups(const DevParams& p, const SolventArr
   const int nq = *A.q.n;
   while (true) {
     int w = 0;
-    if (g == 0) w = atomicAdd(A.q.n + 4, 1);
+    if (g == 0) w = atomicAdd(A.taken, 1);
     w = __shfl_sync(mask, w, lead);
     if (w >= nq) break;
-    near_particle<R, G, KEEP>(p, s, A, H, A.q.i[w], A.q.k[w], g, mask, kept);
+    const int from = max((int)A.q.k[w], A.first);
+    if (from >= H) continue;
+    near_particle<R, G, KEEP>(p, s, A, H, A.q.i[w], from, g, mask, kept);
     __syncwarp(mask);
   }
 }
@@ -675,11 +681,9 @@ namespace irbc {
 // ================================================================ launch ======
 // the side stream's work: a captured graph gives it the side stream's high
 // priority
-bool is_membrane_kernel(const void* fn) { return fn == (const void*)k_membrane || fn == (const void*)k_tri_records ||
-         fn == (const void*)k_tri_cull; }
+bool is_membrane_kernel(const void* fn) { return fn == (const void*)k_membrane; }
 
-// snapshot and triangle records of the membrane as it is (irbc_stream), as
-// step 0 of a stretch
+// snapshot of the membrane as it is (irbc_stream), as step 0 of a stretch
 __global__ void k_snap(DevParams p, Membrane m, FastBufs f) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= p.nv) return;
@@ -690,12 +694,10 @@ __global__ void k_snap(DevParams p, Membrane m, FastBufs f) {
 }
 void fast_snap_prep(const DevParams& p, Membrane& m, FastBufs& f, cudaStream_t st) {
   k_snap<<<nb(p.nv, 128), 128, 0, st>>>(p, m, f);
-  k_tri_records<<<nb(p.nt, 128), 128, 0, st>>>(p, f, 1);
-  k_tri_cull<<<nb(p.nt, 64), 64, 0, st>>>(p, f, 1);
 }
 
 int fast_stream(const DevParams& p, const Solvent& s, const SolventF* sf, const Cells& c, FastBufs& f, int H,
-                cudaStream_t st, cudaEvent_t ev0, cudaEvent_t ev1, cudaEvent_t snap) {
+                cudaStream_t st, cudaEvent_t ev0, cudaEvent_t ev1, cudaEvent_t snap, int first, cudaEvent_t snap1) {
   cudaMemsetAsync(f.qn, 0, 8 * sizeof(int), st);
   if (!s.n) return 0;
   const NearQueue h = queue_of(f, 0);
@@ -705,17 +707,23 @@ int fast_stream(const DevParams& p, const Solvent& s, const SolventF* sf, const 
   if (sf) k_stream_bulk_f<<<nb(s.n, 256), 256, 0, st>>>(p, arr, s.n, c.flag, h, H);
   else k_stream_bulk<<<nb(s.n, 256), 256, 0, st>>>(p, arr, s.n, c.flag, h, H);
   if (ev1) cudaEventRecord(ev1, st);
-  if (snap) cudaStreamWaitEvent(st, snap, 0);
-  const NearArgs A = near_of(p, c, f, 0);
   const bool few = short_lists(f.lmax);
-  if (sf) {
-    if (few) k_near<float, kShortG, kShortKeep><<<kNearBlocks, kNearT, 0, st>>>(p, arr, A, H);
-    else k_near<float, kLongG, kLongKeep><<<kNearBlocks, kNearT, 0, st>>>(p, arr, A, H);
-  } else {
-    if (few) k_near<double, kShortG, kShortKeep><<<kNearBlocks, kNearT, 0, st>>>(p, arr, A, H);
-    else k_near<double, kLongG, kLongKeep><<<kNearBlocks, kNearT, 0, st>>>(p, arr, A, H);
+  const int parts = first > 0 ? 2 : 1;
+  for (int part = 0; part < parts; ++part) {
+    const int s0 = part ? first : 0, s1 = part + 1 < parts ? first : H;
+    const cudaEvent_t ready = part + 1 < parts ? snap1 : snap;
+    if (ready) cudaStreamWaitEvent(st, ready, 0);
+    k_tri_records<<<nb(p.nt, kRecordTris), kRecordT, 0, st>>>(p, f, s0, s1, part);
+    const NearArgs A = near_of(p, c, f, 0, s0, part);
+    if (sf) {
+      if (few) k_near<float, kShortG, kShortKeep><<<kNearBlocks, kNearT, 0, st>>>(p, arr, A, s1);
+      else k_near<float, kLongG, kLongKeep><<<kNearBlocks, kNearT, 0, st>>>(p, arr, A, s1);
+    } else {
+      if (few) k_near<double, kShortG, kShortKeep><<<kNearBlocks, kNearT, 0, st>>>(p, arr, A, s1);
+      else k_near<double, kLongG, kLongKeep><<<kNearBlocks, kNearT, 0, st>>>(p, arr, A, s1);
+    }
   }
-  return 2;
+  return 1 + 2 * parts;
 }
 
 }  // namespace irbc

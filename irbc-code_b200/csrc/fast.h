@@ -88,10 +88,10 @@ struct FastBufs {
   Snap snap{};
   TriPre* pre = nullptr;  // kSegMax x nt
   unsigned char* bands = nullptr;  // kSegMax x nt: BAND_* of each record's corners
-  float4* cull = nullptr; // 3 x nt: what no step of the stretch needs to test (TriCull)
+  float4* cull = nullptr; // 2 x 3 x nt: what no step of a stretch's part needs to test (TriCull)
   int* queue = nullptr;   // particles near the membrane (capacity Ns)
   unsigned char* qk = nullptr;  // the step of the stretch from which on
-  int* qn = nullptr;      // [par] their number, [4 + par] those taken (two parities: cohorts)
+  int* qn = nullptr;      // [par] their number, [4 + par] those taken, in the second part [2 + par] (two parities: cohorts)
   bool one_block = false; // the membrane kernel as one block (meshes that fit, one_block_fits)
   bool cluster = false;   // ... as a cluster of eight blocks whatever the mesh
   int lmax = 0;           // (host) longest list
@@ -112,22 +112,25 @@ __host__ __device__ inline Snap snap_of(const FastBufs& f, int step, int nv) {
   s.x += o; s.y += o; s.z += o; s.vx += o; s.vy += o; s.vz += o;
   return s;
 }
-// snapshot and triangle records of the membrane as it is, as step 0
+// snapshot of the membrane as it is, as step 0
 void fast_snap_prep(const DevParams& p, Membrane& m, FastBufs& f, cudaStream_t st);
 // the streaming of a stretch of H steps; sf: the FP32-bulk solvent, or null.
 // ev0/ev1 (optional) are recorded around the bulk kernel.  The bulk kernel
-// reads no membrane data; the near-membrane kernels read the snapshots and
-// records and first wait for `snap` (optional: their producer).  Returns the
-// number of kernels it launched.
+// reads no membrane data; the triangle records and the near-membrane kernel
+// read the snapshots and first wait for `snap` (optional: their producer).
+// first > 0: they run in two parts, the first `first` steps after snap1 and the
+// others after snap.  Returns the number of kernels it launched.
 struct SolventF;
 int fast_stream(const DevParams& p, const Solvent& s, const SolventF* sf, const Cells& c, FastBufs& f, int H,
-                cudaStream_t st, cudaEvent_t ev0 = nullptr, cudaEvent_t ev1 = nullptr, cudaEvent_t snap = nullptr);
+                cudaStream_t st, cudaEvent_t ev0 = nullptr, cudaEvent_t ev1 = nullptr, cudaEvent_t snap = nullptr,
+                int first = 0, cudaEvent_t snap1 = nullptr);
 bool is_membrane_kernel(const void* fn);
-// the membrane of H <= kSegMax steps in one launch (segment.cuh); parts:
-// SEG_FIRST | SEG_SECOND, or one of them with H = 1.  Returns the number of
-// kernels launched.
+// the membrane of the H steps from step s0 of a stretch (s0 + H <= kSegMax) in
+// one launch (segment.cuh); eoff: the stretch's; parts: SEG_FIRST | SEG_SECOND,
+// or one of them with H = 1.  Returns the number of kernels launched.
 enum : int { SEG_FIRST = 1, SEG_SECOND = 2, SEG_WHOLE = 3 };
-int launch_membrane(const DevParams& p, Membrane& m, FastBufs& f, uint64_t eoff, int H, int parts, cudaStream_t st);
+int launch_membrane(const DevParams& p, Membrane& m, const FastBufs& fb, uint64_t eoff, int s0, int H, int parts,
+                    cudaStream_t st);
 // whether a mesh suits the one-block membrane step
 bool one_block_fits(const DevParams& p);
 // every kernel's dynamic shared-memory limit on the current device (before

@@ -41,7 +41,7 @@ __global__ void __launch_bounds__(kNearT, kNearMinBlocks)
   const Member& M = mem[__ldg(tab + blockIdx.x).x];
   if (threadIdx.x == 0) {
     N.s = arrays_of(M.s, M.f);
-    N.A = near_of(M.p, M.c, M.fb, par);
+    N.A = near_of(M.p, M.c, M.fb, par, 0, 0);
   }
   for (int i = threadIdx.x; i < (int)sizeof(DevParams) / 4; i += blockDim.x) ((int*)&N.p)[i] = ((const int*)&M.p)[i];
   __syncthreads();
@@ -80,16 +80,12 @@ __global__ void __launch_bounds__(kSegT) km_membrane(const Member* __restrict__ 
   __syncthreads();
   membrane_segment(S.p, S.m, S.f, epoch_of(S.p, eoff), H, SEG_WHOLE, seg_sh);
 }
-__global__ void __launch_bounds__(128) km_tri_records(const Member* __restrict__ mem, const int2* __restrict__ tab,
-                                                      int H) {
+__global__ void __launch_bounds__(kRecordT) km_tri_records(const Member* __restrict__ mem, const int2* __restrict__ tab,
+                                                           int H) {
+  __shared__ RecordSmem S;
   const int2 e = __ldg(tab + blockIdx.x);
   const Member& M = mem[e.x];
-  records_item(M.p, M.fb, H, (int64_t)e.y * blockDim.x + threadIdx.x);
-}
-
-__global__ void __launch_bounds__(64) km_tri_cull(const Member* __restrict__ mem, const int2* __restrict__ tab, int H) {
-  const int2 e = __ldg(tab + blockIdx.x);
-  cull_item(mem[e.x].p, mem[e.x].fb, H, e.y * blockDim.x + threadIdx.x);
+  records_block(M.p, M.fb, 0, H, 0, e.y, S);
 }
 
 int multi_membrane(const MultiPlan& P, uint64_t eoff, int H, cudaStream_t st) {
@@ -110,9 +106,8 @@ int multi_membrane(const MultiPlan& P, uint64_t eoff, int H, cudaStream_t st) {
     cudaLaunchKernelEx(&cfg, km_membrane, (const Member*)P.mem, tab, eoff, H);
     tab += s.members * s.nc;
   }
-  km_tri_records<<<P.blocks[MP_RECORDS], 128, 0, st>>>(P.mem, P.table(MP_RECORDS), H);
-  km_tri_cull<<<P.blocks[MP_CULL], 64, 0, st>>>(P.mem, P.table(MP_CULL), H);
-  return (int)P.seg.size() + 2;
+  km_tri_records<<<P.blocks[MP_RECORDS], kRecordT, 0, st>>>(P.mem, P.table(MP_RECORDS), H);
+  return (int)P.seg.size() + 1;
 }
 
 // ---- collision: particle phases ---------------------------------------------------
@@ -180,8 +175,7 @@ void multi_blocks(const Member& M, int out[MP_NPHASE]) {
   out[MP_NEAR_SHORT] = short_lists(M.fb.lmax) ? kNearBlocksMember : 0;
   out[MP_NEAR_LONG] = short_lists(M.fb.lmax) ? 0 : kNearBlocksMember;
   out[MP_MEMBRANE] = segment_blocks(M.p, M.fb);
-  out[MP_RECORDS] = (int)nbf((int64_t)kSegMax * M.p.nt, 128);
-  out[MP_CULL] = (int)nb(M.p.nt, 64);
+  out[MP_RECORDS] = (int)nb(M.p.nt, kRecordTris);
   out[MP_ZERO] = (int)nb(nc, 256);
   out[MP_VBIN] = (int)nb(M.p.nv, 32);
   out[MP_COUNT] = (int)nbf(ns, 256 * kCountPer);

@@ -28,7 +28,7 @@ struct Member {
 
 enum MultiPhase : int {
   MP_STREAM, MP_NEAR_SHORT, MP_NEAR_LONG,                         // streaming
-  MP_MEMBRANE, MP_RECORDS, MP_CULL,                                     // membrane of a stretch
+  MP_MEMBRANE, MP_RECORDS,                                        // membrane of a stretch
   MP_ZERO, MP_VBIN, MP_COUNT, MP_SCAN, MP_PERM, MP_TILE, MP_MOVE,  // collision
   MP_NPHASE
 };

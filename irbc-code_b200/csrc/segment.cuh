@@ -1387,29 +1387,71 @@ static size_t seg_smem(const DevParams& p, const FastBufs& f, int nc) {
   return fixed + (p.nt <= kSegTerms ? (nc > 1 ? 1 : 2) * (size_t)seg_terms(p.nt) * sizeof(double) : 0);
 }
 
-// the streaming's records of every triangle and step of a stretch.  A kernel of
-// its own: in the membrane kernel their scattered loads and 96-byte stores
-// bound the few blocks it has
-__device__ __forceinline__ void records_item(const DevParams& p, const FastBufs& f, int H, int64_t q) {
-  if (q >= (int64_t)H * p.nt) return;
-  const int s = (int)(q / p.nt), j = (int)(q - (int64_t)s * p.nt);
-  const Snap sn = snap_of(f, s, p.nv);
-  const int c[3] = {f.st1[j], f.st2[j], f.st3[j]};
-  f.pre[q] = tri_record(p, sn, c[0], c[1], c[2]);
+// the streaming's records of every triangle for the steps [s0, s1) of a stretch
+// and what none of them needs to test (TriCull), by a lane per triangle and
+// kRecordRows rows of steps.  A kernel of its own: in the membrane kernel their
+// scattered loads and 96-byte stores bound the few blocks it has.  Latency
+// bound: 5 to 7 us (a kernel for the records and one for the cull took 7 + 12,
+// the latter a serial loop over the steps; 16 members 29 + 13 -> 21).
+constexpr int kRecordTris = 32, kRecordRows = 8, kRecordT = kRecordTris * kRecordRows;
+struct RecordSmem {
+  double first[12][kRecordTris];
+  double dX[kRecordRows][kRecordTris], dA[kRecordRows][kRecordTris];
+  int bands[kRecordRows][kRecordTris];
+};
+__device__ __forceinline__ void records_block(const DevParams& p, const FastBufs& f, int s0, int s1, int part, int64_t bid,
+                                              RecordSmem& S) {
+  const int lane = threadIdx.x % kRecordTris, row = threadIdx.x / kRecordTris;
+  const int64_t j = bid * kRecordTris + lane;
+  const bool on = j < p.nt;
+  const int c[3] = {on ? f.st1[j] : 0, on ? f.st2[j] : 0, on ? f.st3[j] : 0};
   const double rx = p.Lx - (3.0 * p.a), ry = p.Ly - (3.0 * p.a), l = 3.0 * p.a;
-  int b = 0;
-  for (int k = 0; k < 3; ++k) {
-    const double x = sn.x[c[k]], y = sn.y[c[k]];
-    b |= (x < l ? BAND_LX : 0) | (x > rx ? BAND_HX : 0) | (y < l ? BAND_LY : 0) | (y > ry ? BAND_HY : 0);
+  CullMove mv{0.0, 0.0, 0};
+  TriPre t0{};
+  for (int base = s0; base < s1; base += kRecordRows) {
+    const int s = base + row;
+    TriPre t{};
+    int b = 0;
+    if (on && s < s1) {
+      const Snap sn = snap_of(f, s, p.nv);
+      t = tri_record(p, sn, c[0], c[1], c[2]);
+      for (int k = 0; k < 3; ++k) {
+        const double x = sn.x[c[k]], y = sn.y[c[k]];
+        b |= (x < l ? BAND_LX : 0) | (x > rx ? BAND_HX : 0) | (y < l ? BAND_LY : 0) | (y > ry ? BAND_HY : 0);
+      }
+      const int64_t q = (int64_t)s * p.nt + j;
+      f.pre[q] = t;
+      f.bands[q] = (unsigned char)b;
+    }
+    if (base == s0) {
+      if (row == 0)
+        for (int k = 0; k < 3; ++k) {
+          S.first[k][lane] = t.X[k]; S.first[3 + k][lane] = t.Xdt[k];
+          S.first[6 + k][lane] = t.A1[k]; S.first[9 + k][lane] = t.A2[k];
+        }
+      __syncthreads();
+      for (int k = 0; k < 3; ++k) {
+        t0.X[k] = S.first[k][lane]; t0.Xdt[k] = S.first[3 + k][lane];
+        t0.A1[k] = S.first[6 + k][lane]; t0.A2[k] = S.first[9 + k][lane];
+      }
+    }
+    if (on && s < s1) cull_fold(mv, t0, t, b);
   }
-  f.bands[q] = (unsigned char)b;
+  S.dX[row][lane] = mv.dX;
+  S.dA[row][lane] = mv.dA;
+  S.bands[row][lane] = mv.bands;
+  __syncthreads();
+  if (row != 0 || !on) return;
+  for (int r = 1; r < kRecordRows; ++r) {
+    mv.dX = fmax(mv.dX, S.dX[r][lane]);
+    mv.dA = fmax(mv.dA, S.dA[r][lane]);
+    mv.bands |= S.bands[r][lane];
+  }
+  cull_store(p, f.cull + 3 * ((int64_t)part * p.nt + j), t0, mv);
 }
-__global__ void __launch_bounds__(128) k_tri_records(DevParams p, FastBufs f, int H) {
-  records_item(p, f, H, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
-}
-
-__global__ void __launch_bounds__(64) k_tri_cull(DevParams p, FastBufs f, int H) {
-  cull_item(p, f, H, blockIdx.x * blockDim.x + threadIdx.x);
+__global__ void __launch_bounds__(kRecordT) k_tri_records(DevParams p, FastBufs f, int s0, int s1, int part) {
+  __shared__ RecordSmem S;
+  records_block(p, f, s0, s1, part, blockIdx.x, S);
 }
 
 // blocks of the membrane's cluster
@@ -1441,7 +1483,10 @@ bool cluster_fits(int nc, int smem) {
   return ok;
 }
 
-int launch_membrane(const DevParams& p, Membrane& m, FastBufs& f, uint64_t eoff, int H, int parts, cudaStream_t st) {
+int launch_membrane(const DevParams& p, Membrane& m, const FastBufs& fb, uint64_t eoff, int s0, int H, int parts,
+                    cudaStream_t st) {
+  FastBufs f = fb;
+  f.snap = snap_of(fb, s0, p.nv);
   const int nc = segment_blocks(p, f);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(nc);
@@ -1455,11 +1500,8 @@ int launch_membrane(const DevParams& p, Membrane& m, FastBufs& f, uint64_t eoff,
   at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, k_membrane, p, m, f, eoff, H, parts);
-  if (!(parts & SEG_FIRST)) return 1;
-  k_tri_records<<<(unsigned)(((int64_t)H * p.nt + 127) / 128), 128, 0, st>>>(p, f, H);
-  k_tri_cull<<<(unsigned)((p.nt + 63) / 64), 64, 0, st>>>(p, f, H);
-  return 3;
+  cudaLaunchKernelEx(&cfg, k_membrane, p, m, f, eoff + (uint64_t)s0, H, parts);
+  return 1;
 }
 
 }  // namespace irbc
