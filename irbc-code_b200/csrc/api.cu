@@ -341,9 +341,11 @@ void build_gather(const HostMesh& M, const std::vector<int>& start, const std::v
 
 // the vertices ordered so that every run of them is a connected patch where
 // the mesh allows it: each half of a bisection is the nearer half, by edges,
-// to a vertex far from the others; `part` weights of the runs
+// to a vertex far from the others; w: the runs' weights, cap: the most vertices
+// of each, where all of them fit
 void bisect(const std::vector<std::vector<int>>& nb, std::vector<int>& v, size_t lo, size_t hi,
-            const std::vector<double>& w, size_t p0, size_t p1, std::vector<size_t>& cut) {
+            const std::vector<double>& w, const std::vector<size_t>& cap, size_t p0, size_t p1,
+            std::vector<size_t>& cut) {
   if (p1 - p0 < 2) return;
   std::vector<int> at(nb.size(), -1);
   auto bfs = [&](int from) {
@@ -370,10 +372,14 @@ void bisect(const std::vector<std::vector<int>>& nb, std::vector<int>& v, size_t
   const size_t pm = (p0 + p1) / 2;
   double wl = 0, wa = 0;
   for (size_t q = p0; q < p1; ++q) { wa += w[q]; if (q < pm) wl += w[q]; }
-  const size_t mid = lo + (size_t)std::llround((double)(hi - lo) * (wa > 0 ? wl / wa : 0.5));
+  size_t left = (size_t)std::llround((double)(hi - lo) * (wa > 0 ? wl / wa : 0.5));
+  size_t cl = 0, cr = 0;
+  for (size_t q = p0; q < p1; ++q) (q < pm ? cl : cr) += cap[q];
+  if (hi - lo <= cl + cr) left = std::max(std::min(left, cl), hi - lo > cr ? hi - lo - cr : 0);
+  const size_t mid = lo + left;
   cut[pm] = mid;
-  bisect(nb, v, lo, mid, w, p0, pm, cut);
-  bisect(nb, v, mid, hi, w, pm, p1, cut);
+  bisect(nb, v, lo, mid, w, cap, p0, pm, cut);
+  bisect(nb, v, mid, hi, w, cap, pm, p1, cut);
 }
 
 // The mesh split into patches for a cluster of nc blocks, the tables of each
@@ -383,19 +389,25 @@ bool build_patches(const HostMesh& M, const std::vector<int>& start, const std::
                    PatchPlan& P, std::vector<PatchHdr>& hdr, std::vector<unsigned char>& blob, std::vector<int>& own) {
   // The summing warps: in reference order the sums take half of two blocks'
   // warps, the warp tree one of four (the others for the tail); those blocks'
-  // patches are smaller by as much (and by the room that many terms take).
+  // patches are smaller by as much (and by the room that many terms take; block
+  // 1 has no tail and all its warps in phase C).  cap: a component of a vertex
+  // per thread in phase C, where one more costs a second round (10 000 cycles
+  // instead of 7 600 for 171 vertices instead of 170).
   P = PatchPlan{};
   P.nc = nc;
   P.sw = tree ? 4 : 8;
   std::vector<double> w(nc, 1.0);
-  w[0] = w[1] = tree && M.nt <= 2048 ? 0.85 : 0.5;
+  w[0] = tree && M.nt <= 2048 ? 0.85 : 0.5;
+  w[1] = tree && M.nt <= 2048 ? 0.85 : 0.62;
+  std::vector<size_t> cap(nc, kSegT / 3);
+  cap[0] = (kSegT - 32 * P.sw) / 3;
   std::vector<std::vector<int>> nb(M.nv);
   for (int i = 0; i < M.ne; ++i) { nb[M.e1[i]].push_back(M.e2[i]); nb[M.e2[i]].push_back(M.e1[i]); }
   own.resize(M.nv);
   for (int v = 0; v < M.nv; ++v) own[v] = v;
   std::vector<size_t> cut(nc + 1, 0);
   cut[nc] = M.nv;
-  bisect(nb, own, 0, M.nv, w, 0, nc, cut);
+  bisect(nb, own, 0, M.nv, w, cap, 0, nc, cut);
   std::vector<int> place(M.nv), owner(M.nv);
   for (int b = 0; b < nc; ++b) {
     for (size_t q = cut[b]; q < cut[b + 1]; ++q) { place[own[q]] = (int)(q - cut[b]); owner[own[q]] = b; }

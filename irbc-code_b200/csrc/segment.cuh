@@ -13,15 +13,19 @@
 //      memory) and every force term up to the factors that need Sarea and
 //      Volume
 //   B  blocks 0 and 1: the ordered sums Sarea and Volume (TotalVA); the
-//      others: edge and bending terms, bond preparation, triangle records
+//      others: edge and bending terms, beside them the bond preparation
 //   C  per vertex component: the gather of its force terms in the reference's
 //      order, external forces, second half-kick, and the next step's first
 //      half-kick, snapshot and drift; the last block: bond events and the
 //      parasite
 // A step's chain of eight dependent launches (at least 2 us apart from the
 // host, each cold) took 67 us on the 600-vertex mesh and 128 us on the
-// 2562-vertex discocyte; what is left is latency: L2 reads after each
-// barrier, and the 8-cycle FP64 additions of the ordered sums.
+// 2562-vertex discocyte, this 12 and 21.  What is left is latency, in cycles of
+// a step of 24 000 (600 vertices) and 43 000 (2562): the triangles 3 000 and
+// 4 700, the ordered sums 10 000 and 19 000 (the other blocks' terms and bonds
+// end before them), phase C 8 000 and 11 000, the three barriers with what they
+// wait for of stores to other blocks some 5 000.  A quarter of the vertices a
+// block hardly changes them.
 #include <cooperative_groups.h>
 
 namespace irbc {
@@ -847,13 +851,17 @@ struct PatchTail {
   int nw, ndr, nev;
   MemScalars sc;
 };
-// half-warps of a block that look for bond candidates
-constexpr int kBondHalves = 16;
+// warps of a block that do the bond preparation, half-warps of them that look
+// for bond candidates
+constexpr int kBondWarps = 8, kBondHalves = 2 * kBondWarps;
 struct PatchMisc {
   double fac[2], para[3];
   int paradx, parady;
   int nb;                                // free knobs of the block near the wall
+  int next;                              // chunk of edges or bending terms to be taken next
   unsigned short bond[kPatchOwn];
+  unsigned char pn[kPatchOwn];           // their candidates
+  int bpid[kPatchOwn];                   // their cells
   double pd[kBondHalves][kMaxPairs];
   int pj[kBondHalves][kMaxPairs];
 };
@@ -883,6 +891,11 @@ __device__ __forceinline__ void patch_tail(const DevParams& p, const Membrane& m
                                            PatchTail& S, int tid, int tn) {
   const int nw = S.nw, nd = S.ndr, words = (p.nv + 31) / 32;
   const bool wfits = nw <= kTailWca, dfits = nd <= kTailDraw;
+  if (wfits)
+    for (int e = tid; e < nw; e += tn) atomicOr(&S.wbits[S.wid[e] >> 5], 1u << (S.wid[e] & 31));
+  if (dfits)
+    for (int e = tid; e < nd; e += tn) atomicOr(&S.dbits[S.did[e] >> 5], 1u << (S.did[e] & 31));
+  bar_named(4, tn);
   if (tid < 32) bit_prefix(S.wbits, S.wpre, words, tid);
   else if (tid < 64) bit_prefix(S.dbits, S.dpre, words, tid - 32);
   bar_named(4, tn);
@@ -980,13 +993,22 @@ __device__ __forceinline__ void patch_tail(const DevParams& p, const Membrane& m
   if (tid == 0) S.nw = 0;
 }
 
-// a vertex's bond draws onto the tail's list
-__device__ __forceinline__ void patch_draws(cooperative_groups::cluster_group& cl, PatchTail& tail, int i, int val,
-                                            double pr) {
-  PatchTail* T = cl.map_shared_rank(&tail, 0);
-  const int e = atomicAdd(&T->ndr, 1);
-  if (e < kTailDraw) { T->did[e] = i; T->dval[e] = val; T->dpr[e] = pr; }
-  atomicOr(&T->dbits[i >> 5], 1u << (i & 31));
+// room for a warp's entries on a list of the tail, its place taken with one
+// atomic (block 0's shared memory serves them one at a time: with one per entry
+// the discocyte's bond preparation took 16 000 cycles, most of it waiting);
+// this lane's entry
+__device__ __forceinline__ int tail_room(int* count, bool on) {
+  const unsigned b = __ballot_sync(0xffffffffu, on);
+  if (b == 0u) return 0;
+  const int lane = threadIdx.x & 31, first = __ffs(b) - 1;
+  int at = 0;
+  if (lane == first) at = atomicAdd(count, __popc(b));
+  return __shfl_sync(0xffffffffu, at, first) + __popc(b & ((1u << lane) - 1u));
+}
+// vertices' bond draws onto the tail's list, by a whole warp
+__device__ __forceinline__ void patch_draws(PatchTail* T, bool on, int i, int val, double pr) {
+  const int e = tail_room(&T->ndr, on);
+  if (on && e < kTailDraw) { T->did[e] = i; T->dval[e] = val; T->dpr[e] = pr; }
 }
 
 // the parasite's position to every block
@@ -1034,8 +1056,12 @@ __device__ __forceinline__ void membrane_patch(const DevParams& p, const Membran
   // blocks 0 and 1 give their first sw warps to the sums (Sarea, Volume);
   // block 0's also run the tail
   const int busy = cta < 2 ? 32 * P.sw : 0;
-  const int wt = t - busy, nwk = kSegT - busy, no3 = 3 * hd.no;
+  const int wt = t - busy, nwk = kSegT - busy, no3 = 3 * hd.no, lane = t & 31;
   const bool summing = wt < 0;
+  // block 1's summing warps help with phase C (block 0's run the tail then)
+  const int cw = cta == 1 ? t : wt, ncw = cta == 1 ? kSegT : nwk;
+  const double pon = 1.0 - exp(-p.onrate * p.dtmd);
+  PatchTail* T = cl.map_shared_rank(&tail, 0);
   const bool pad = p.tree_sums != 0;
   const int run = tree_run(p.nt);
   // f dt / (2 m) of a half-kick
@@ -1065,9 +1091,9 @@ __device__ __forceinline__ void membrane_patch(const DevParams& p, const Membran
     cx[k * P.nl + v] = u;
   };
   // the seam's coordinates to the blocks that read them
-  auto publish = [&]() {
-    bar_named(3, nwk);
-    for (int q = wt; q < hd.nsend; q += nwk) {
+  auto publish = [&](int me, int n) {
+    bar_named(3, n);
+    for (int q = me; q < hd.nsend; q += n) {
       const PatchSend e = send[q];
       double* to = cl.map_shared_rank(cx, e.cta) + e.slot;
       to[0] = cx[e.own]; to[P.nl] = cx[P.nl + e.own]; to[2 * P.nl] = cx[2 * P.nl + e.own];
@@ -1090,8 +1116,8 @@ __device__ __forceinline__ void membrane_patch(const DevParams& p, const Membran
   }
   cluster_arrive();  // every block has started: its shared memory may be written
   cluster_wait();
-  if (!summing) publish();
-  if (t == 0) misc->nb = 0;
+  if (!summing) publish(wt, nwk);
+  if (t == 0) misc->nb = misc->next = 0;
   if (cta == 0 && t < 32) {
     if (t == 0) {
       tail.sc = *m.sc;
@@ -1124,9 +1150,7 @@ __device__ __forceinline__ void membrane_patch(const DevParams& p, const Membran
       cluster_arrive();
       cluster_wait();
       if (!(parts & SEG_SECOND)) break;
-      // the tail beside the next step's first phase: the bond preparation, which
-      // needs it, waits for this block's next arrival
-      cluster_arrive();
+      // the tail beside phase C
       if (cta == 0) {
         patch_tail(p, m, f, epoch + s, tail, t, 32 * P.sw);
         if (t < 32 && more) {
@@ -1134,34 +1158,13 @@ __device__ __forceinline__ void membrane_patch(const DevParams& p, const Membran
           __syncwarp();
           patch_para(cl, misc, tail.sc, t, nc);
         }
-      }
-      cluster_wait();
-      continue;
-    }
-    // A: triangles and edges, the triangles first (the sums wait for them)
-    const int nab = hd.ntri + ((parts & SEG_SECOND) ? hd.ned : 0);
-    for (int q = wt; q < nab; q += nwk) {
-      if (q >= hd.ntri) {
-        const PatchEdge e = edge[q - hd.ntri];
-        double A[3];
-        A[0] = cx[e.v[0]] - cx[e.v[1]];
-        A[1] = cx[P.nl + e.v[0]] - cx[P.nl + e.v[1]];
-        A[2] = cx[2 * P.nl + e.v[0]] - cx[2 * P.nl + e.v[1]];
-        const double aa = sqrt(A[0] * A[0] + A[1] * A[1] + A[2] * A[2]);
-        A[0] /= aa; A[1] /= aa; A[2] /= aa;
-        const double xx = aa / (2.5 * e.l0);
-        const double xxx = 1.0 / (4.0 * (1.0 - xx) * (1.0 - xx));
-        // the terms on the second end (wl A, pk); those on the first are their
-        // negatives
-        double* to = E + (q - hd.ntri);
-        to[0] = rlap * (xxx - 0.25 + xx);
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-          to[(1 + k) * hd.ned] = A[k];
-          to[(4 + k) * hd.ned] = -e.kp * A[k] / (aa * aa);
-        }
+        cluster_arrive();
+        cluster_wait();
         continue;
       }
+    } else {
+    // A: triangles
+    for (int q = wt; q < hd.ntri; q += nwk) {
       const PatchTri e = tri[q];
       const double x1 = cx[e.v[0]], y1 = cx[P.nl + e.v[0]], z1 = cx[2 * P.nl + e.v[0]];
       const double x2 = cx[e.v[1]], y2 = cx[P.nl + e.v[1]], z2 = cx[2 * P.nl + e.v[1]];
@@ -1198,87 +1201,134 @@ __device__ __forceinline__ void membrane_patch(const DevParams& p, const Membran
       }
     }
     cluster_arrive();
-    // B: bending terms
-    for (int q = wt; q < ((parts & SEG_SECOND) ? hd.ndih : 0); q += nwk) {
-      const PatchDih e = dih[q];
-      const double *c1 = cx + e.v[0], *c4 = cx + e.v[1], *c2 = cx + e.v[2], *c3 = cx + e.v[3];
-      double r[4][3];
-      dih_terms(p, c1[0], c1[P.nl], c1[2 * P.nl], c2[0], c2[P.nl], c2[2 * P.nl], c3[0], c3[P.nl], c3[2 * P.nl], c4[0],
-                c4[P.nl], c4[2 * P.nl], r);
-#pragma unroll
-      for (int c = 0; c < 4; ++c)
-        if (e.d[c] != kNoEntry)
-          for (int k = 0; k < 3; ++k) D[k * hd.nd + e.d[c]] = r[c][k];
-    }
-    // (the tail of the step before has ended: bond states and the parasite)
-    cluster_wait();
     if (parts & SEG_SECOND) {
-      // bond preparation, bond springs and the parasite's force
-      for (int v = wt; v < hd.no; v += nwk) {
-        const int i = own[v];
-        const double u[3] = {cx[v], cx[P.nl + v], cx[2 * P.nl + v]};
-        int flags = 0;
-        const int bondi = m.bondi[i];
-        if (bondi == 1) {
-          double pr, sp[3];
-          flags = bonded_prep(p, m, i, sx[3 * v], sx[3 * v + 1], u[2], sim[2 * v], sim[2 * v + 1], pr, sp);
-          if (flags & VF_SPRING)
-            for (int k = 0; k < 3; ++k) f.vS[3 * i + k] = sp[k];
-          patch_draws(cl, tail, i, 1 | flags, pr);
-          flags |= 1;
-        } else if ((u[2] < p.dthr) && (bondi == 0) && (m.knob[i] == 1)) {
-          misc->bond[atomicAdd(&misc->nb, 1)] = (unsigned short)v;
+      // B: the first warps prepare the bonds (a chain of dependent reads and few
+      // operations) beside the others' edge and bending terms, then join them
+      if (wt < 32 * kBondWarps) {
+        for (int v0 = wt - lane; v0 < hd.no; v0 += 32 * kBondWarps) {
+          const int v = v0 + lane;
+          const bool on = v < hd.no;
+          const int i = on ? own[v] : 0;
+          int flags = 0, bondi = -1, knob = 0, pid = 0;
+          double pr = 0.0, w[3];
+          bool wca = false;
+          if (on) {
+            bondi = m.bondi[i];
+            knob = m.knob[i];
+            pid = m.pid[i];
+            const double u[3] = {cx[v], cx[P.nl + v], cx[2 * P.nl + v]};
+            const double pp[3] = {(misc->para[0] + misc->paradx * p.Lx), (misc->para[1] + misc->parady * p.Ly),
+                                  misc->para[2]};
+            wca = wca_at(p, pp, u[0], u[1], u[2], w);
+            if (wca)
+              for (int k = 0; k < 3; ++k) f.vX[3 * i + k] = w[k];
+            if (bondi == 1) {
+              double sp[3];
+              flags = bonded_prep(p, m, i, sx[3 * v], sx[3 * v + 1], u[2], sim[2 * v], sim[2 * v + 1], pr, sp);
+              if (flags & VF_SPRING)
+                for (int k = 0; k < 3; ++k) f.vS[3 * i + k] = sp[k];
+              flags |= 1;
+            } else if ((u[2] < p.dthr) && (bondi == 0) && (knob == 1)) {
+              const int at = atomicAdd(&misc->nb, 1);
+              misc->bond[at] = (unsigned short)v;
+              misc->bpid[at] = pid;
+            }
+          }
+          patch_draws(T, bondi == 1, i, flags, pr);
+          const int e = tail_room(&T->nw, wca);
+          if (wca) {
+            if (e < kTailWca) { T->wid[e] = i; T->wX[0][e] = w[0]; T->wX[1][e] = w[1]; T->wX[2][e] = w[2]; }
+            flags |= VF_WCA;
+          }
+          if (on) f.vd[i] = sfl[v] = flags;
         }
-        double w[3];
-        const double pp[3] = {(misc->para[0] + misc->paradx * p.Lx), (misc->para[1] + misc->parady * p.Ly), misc->para[2]};
-        if (wca_at(p, pp, u[0], u[1], u[2], w)) {
-          flags |= VF_WCA;
-          for (int k = 0; k < 3; ++k) f.vX[3 * i + k] = w[k];
-          PatchTail* T = cl.map_shared_rank(&tail, 0);
-          const int e = atomicAdd(&T->nw, 1);
-          if (e < kTailWca) { T->wid[e] = i; T->wX[0][e] = w[0]; T->wX[1][e] = w[1]; T->wX[2][e] = w[2]; }
-          atomicOr(&T->wbits[i >> 5], 1u << (i & 31));
-        }
-        sfl[v] = flags;
-        f.vd[i] = flags;
-      }
-      bar_named(3, nwk);
-      // free knobs near the wall, half a warp each: candidates and their order
-      const int nb = misc->nb, half = wt >> 4, halves = min(kBondHalves, nwk >> 4);
-      if (half < kBondHalves)
-        for (int e0 = half & ~1; e0 < nb; e0 += halves) {
+        bar_named(6, 32 * kBondWarps);
+        // free knobs near the wall, half a warp each: candidates and their order
+        const int nb = misc->nb, half = wt >> 4;
+        for (int e0 = half & ~1; e0 < nb; e0 += kBondHalves) {
           const int e = e0 + (half & 1);
           const bool on = e < nb;
           const int v = on ? misc->bond[e] : 0, i = on ? own[v] : 0;
           const int n = bond_pairs(p, m, on, i, sx[3 * v], sx[3 * v + 1], cx[2 * P.nl + v], sim[2 * v], sim[2 * v + 1],
-                                   on ? m.pid[i] : 0, misc->pd[half], misc->pj[half]);
+                                   on ? misc->bpid[e] : 0, misc->pd[half], misc->pj[half]);
           if (on && (wt & 15) == 0) {
-            const double pon = 1.0 - exp(-p.onrate * p.dtmd);
             m.pon[i] = pon;
             m.npair[i] = n;
             f.vd[i] = sfl[v] |= n;
-            if (n > 0) patch_draws(cl, tail, i, n, pon);
+            misc->pn[e] = (unsigned char)n;
           }
         }
+        if (nb > 0) {
+          bar_named(6, 32 * kBondWarps);
+          for (int e0 = wt - lane; e0 < nb; e0 += 32 * kBondWarps) {
+            const int e = e0 + lane, n = e < nb ? misc->pn[e] : 0;
+            patch_draws(T, n > 0, e < nb ? own[misc->bond[e]] : 0, n, pon);
+          }
+        }
+      }
+      // chunks of 32 bending terms, then edges, each by the next free warp
+      const int nd = (hd.ndih + 31) / 32, nch = nd + (hd.ned + 31) / 32;
+      while (true) {
+        int ch = 0;
+        if (lane == 0) ch = atomicAdd(&misc->next, 1);
+        ch = __shfl_sync(0xffffffffu, ch, 0);
+        if (ch >= nch) break;
+        if (ch < nd) {
+          const int q = 32 * ch + lane;
+          if (q >= hd.ndih) continue;
+          const PatchDih e = dih[q];
+          const double *c1 = cx + e.v[0], *c4 = cx + e.v[1], *c2 = cx + e.v[2], *c3 = cx + e.v[3];
+          double r[4][3];
+          dih_terms(p, c1[0], c1[P.nl], c1[2 * P.nl], c2[0], c2[P.nl], c2[2 * P.nl], c3[0], c3[P.nl], c3[2 * P.nl],
+                    c4[0], c4[P.nl], c4[2 * P.nl], r);
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+            if (e.d[c] != kNoEntry)
+              for (int k = 0; k < 3; ++k) D[k * hd.nd + e.d[c]] = r[c][k];
+          continue;
+        }
+        const int q = 32 * (ch - nd) + lane;
+        if (q >= hd.ned) continue;
+        const PatchEdge e = edge[q];
+        double A[3];
+        A[0] = cx[e.v[0]] - cx[e.v[1]];
+        A[1] = cx[P.nl + e.v[0]] - cx[P.nl + e.v[1]];
+        A[2] = cx[2 * P.nl + e.v[0]] - cx[2 * P.nl + e.v[1]];
+        const double aa = sqrt(A[0] * A[0] + A[1] * A[1] + A[2] * A[2]);
+        A[0] /= aa; A[1] /= aa; A[2] /= aa;
+        const double xx = aa / (2.5 * e.l0);
+        const double xxx = 1.0 / (4.0 * (1.0 - xx) * (1.0 - xx));
+        // the terms on the second end (wl A, pk); those on the first are their
+        // negatives
+        double* to = E + q;
+        to[0] = rlap * (xxx - 0.25 + xx);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          to[(1 + k) * hd.ned] = A[k];
+          to[(4 + k) * hd.ned] = -e.kp * A[k] / (aa * aa);
+        }
+      }
     }
+    cluster_wait();
     cluster_arrive();
     cluster_wait();
     if (!(parts & SEG_SECOND)) break;
+    }
     // C: the triangles' factors; then each vertex component adds its terms in
     // order, external forces, kicks
     {
       const double beta = misc->fac[0], betav = misc->fac[1];
       const Divisor six{6.0, 1.0 / 6.0};
-      for (int e = wt; e < hd.nt; e += nwk) {
+      for (int e = cw; e < hd.nt; e += ncw) {
         double* q = Y + e;
         q[7 * hd.nt] = beta / q[7 * hd.nt];
 #pragma unroll
         for (int k = 3; k < 6; ++k) q[k * hd.nt] = div_by(betav * q[k * hd.nt], six);
       }
-      if (wt == 0) misc->nb = 0;
-      bar_named(3, nwk);
+      if (cw == 0) misc->nb = misc->next = 0;
+      bar_named(3, ncw);
     }
-    for (int q = wt; q < no3; q += nwk) {
+    for (int q = cw; q < no3; q += ncw) {
       const int v = q / 3, k = q - 3 * v, i = own[v];
       const unsigned short *e0 = ent + 3 * v, *e1 = e0 + 3;
       double acc = 0.0;
@@ -1325,7 +1375,7 @@ __device__ __forceinline__ void membrane_patch(const DevParams& p, const Membran
         *F = fk;
       }
     }
-    if (more) publish();
+    if (more) publish(cw, ncw);
     cluster_arrive();
     cluster_wait();
   }
@@ -1371,7 +1421,7 @@ void patch_layout(PatchPlan& P, PatchHdr* hdr, int nt) {
   const int sums = o;
   for (int b = 0; b < P.nc; ++b) {
     PatchHdr& h = hdr[b];
-    o = b < 2 ? sums : common;
+    o = b == 0 ? sums : (b == 1 ? P.o_tail : common);  // block 0 alone has a tail
     h.o_tab = take(h.bytes);
     h.o_e = take(7 * (size_t)h.ned * sizeof(double));
     h.o_d = take(3 * (size_t)h.nd * sizeof(double));
