@@ -1,0 +1,106 @@
+"""The launches that take several timesteps, or more of the box, at once, at
+the sizes where their rules and edges lie.
+
+A stretch of timesteps between two collisions equals the same timesteps one at
+a time bit for bit: stretches above the 16 steps that one launch takes, those
+in one part and in two, boxes so narrow that every particle lies in a side
+wall's band or wraps into its own cell's neighbour, sparse ones, particles fast
+enough to cross several cells in a stretch, every form of the membrane, both
+precisions."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+import helpers as H
+
+pytestmark = pytest.mark.gpu
+
+
+STRETCHES = [  # dtcd, Lx, Ly, particles, speed factor, membrane form
+    (0.02, 60.0, 30.0, 30000, 1.0, 1),     # 10 steps: parts of 6 and 4
+    (0.014, 60.0, 30.0, 30000, 1.0, 1),    # 7 steps: one part
+    (0.05, 60.0, 30.0, 30000, 1.0, 1),     # 25 steps: launches of 16 and 9
+    (0.02, 13.0, 13.0, 20000, 1.0, 1),     # the bands of 3 cells meet the membrane
+    (0.02, 13.5, 12.25, 12000, 1.0, 1),    # a box of no whole number of cells
+    (0.02, 60.0, 30.0, 900, 1.0, 1),       # few particles
+    (0.05, 40.0, 20.0, 30000, 25.0, 1),    # up to some cells a stretch
+    (0.02, 40.0, 20.0, 20000, 1.0, 2),     # the membrane in one block
+    (0.05, 40.0, 20.0, 20000, 1.0, 3),     # ... in a cluster on global memory
+]
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("case", STRETCHES, ids=lambda c: "%g-%gx%g-%d-%g-%d" % c)
+def test_stretches_equal_single_steps(case, precision):
+    dtcd, Lx, Ly, ns, fast, form = case
+    op, orc = H.make_oracle(ns=ns, seed=41, onrate=300.0, offrate=50.0, dtcd=dtcd, Lx=Lx, Ly=Ly)
+    st = orc.get_state()
+    for k in ("svx", "svy", "svz"):
+        st.a[k] = st.a[k] * fast
+    a = H.gpu_like(op, orc, 41, precision=precision, state=st)
+    b = H.gpu_like(op, orc, 41, precision=precision, state=st)
+    a.set_membrane_kernels(form)
+    b.set_membrane_kernels(form)
+    for n in (3, 30, 55):  # collisions inside and at the ends, the list update
+        a.step(n)
+        for _ in range(n):
+            b.call("step_part1")
+            b.call("step_part2")
+        assert H.compare(a.get_state(), b.get_state(), 0.0) == {}, n
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("Lz", [20.0, 300.0])  # layers in shared memory (256), beyond
+def test_layer_sums(Lz, precision):
+    """Temperature, mean velocity and profiles against sums of the state in
+    numpy: n additions in any order differ by at most n eps of the terms'
+    magnitudes."""
+    op, orc = H.make_oracle(ns=20000, seed=43, Lx=30.0, Ly=15.0, Lz=Lz)
+    sim = H.gpu_like(op, orc, 43, precision=precision)
+    sim.step(3)
+    s = sim.get_state().a
+    v, z = np.stack([s["svx"], s["svy"], s["svz"]]), s["sz"]
+    n, eps = z.size, 2.0 ** -53
+    o = sim.observables()
+    tol = n * eps
+    lay = np.clip(np.floor(z).astype(int), 0, int(Lz) - 1)
+    m = np.bincount(lay, minlength=int(Lz))
+    u = np.stack([np.bincount(lay, w, int(Lz)) for w in v]) / np.maximum(m, 1)
+    # the layers' means are subtracted from the whole, so errors are the whole's
+    whole = np.mean(v ** 2)
+    assert abs(o[0] - np.mean((v - u[:, lay]) ** 2)) <= 4 * tol * whole
+    assert abs(o[8] - whole) <= tol * whole
+    assert abs(o[7] - np.mean(v[0])) <= tol * np.mean(np.abs(v[0]))
+    for bins in (1, 20, 256, 257, 300):
+        b = np.clip(np.floor(z).astype(int), 0, bins - 1)
+        c = np.bincount(b, minlength=bins)
+        want = np.bincount(b, v[0], bins) / np.maximum(c, 1)
+        bound = tol * np.bincount(b, np.abs(v[0]), bins) / np.maximum(c, 1)
+        assert (np.abs(sim.velocity_profile(bins) - want) <= bound).all(), bins
+
+
+@pytest.mark.parametrize("box", [(16, 16, 3), (31, 11, 2), (41, 5, 4), (3, 1, 1), (128, 128, 64)])
+def test_cell_scan_at_tile_edges(box):
+    """Counting sorts over 1024, 1023, 1025, 6 and 1,064,960 cells (a tile of
+    the scan has 1024 cells; 1040 tiles are more than a block's threads)."""
+    import torch
+    import irbc_b200 as G
+    Lx, Ly, Lz = box
+    p = G.default_params(Lx=float(Lx), Ly=float(Ly), Lz=float(Lz), Ns=0)
+    ncell = Lx * Ly * (Lz + 1)
+    rng = np.random.default_rng(3)
+    for n in (0, 1, 5000):
+        pos = [torch.tensor(rng.uniform(0, L, n), device="cuda") for L in box]
+        cell = torch.zeros(max(n, 1), dtype=torch.int32, device="cuda")
+        start = torch.full((ncell + 1,), -1, dtype=torch.int32, device="cuda")
+        order = torch.zeros(max(n, 1), dtype=torch.int32, device="cuda")
+        rc = G.lib().irbc_bin_particles(C.byref(p), *[q.data_ptr() for q in pos], n, 0.25, 0.5, 0.75,
+                                        cell.data_ptr(), start.data_ptr(), order.data_ptr())
+        assert rc == 0
+        f = [np.floor((q.cpu().numpy() - r) % L) for q, r, L in zip(pos[:2], (0.25, 0.5), box)]
+        want = ((f[0] * Ly + f[1]) * (Lz + 1) + np.floor(pos[2].cpu().numpy() + 0.25)).astype(np.int64)
+        np.testing.assert_array_equal(cell.cpu().numpy()[:n], want)
+        np.testing.assert_array_equal(start.cpu().numpy(),
+                                      np.concatenate([[0], np.cumsum(np.bincount(want, minlength=ncell))]))
+        np.testing.assert_array_equal(order.cpu().numpy()[:n], np.argsort(want, kind="stable"))
