@@ -148,13 +148,14 @@ int irbc_set_graphs(irbc_handle* h, int32_t on);
  * simulations sharing a GPU (fewer streams contend for the device's
  * hardware queues); the results are the same either way. */
 int irbc_set_streams(irbc_handle* h, int32_t n);
-/* Not in the reference.  How irbc_step launches the membrane step: mode 1
- * (the default) as wide kernels over many SMs; mode 2 as one block per
- * launch, two kernels per step instead of eight, for meshes up to 1024
- * vertices (IRBC_ERR_CAPACITY for a larger mesh; a mesh set later keeps
- * the wide kernels); mode 3 as one launch of a thread-block cluster (8
- * blocks of 512 threads on one GPC, its phases separated by cluster
- * barriers), any mesh.  The results are the same in every mode. */
+/* Not in the reference.  How irbc_step launches the membrane of a stretch
+ * of timesteps: mode 1 (the default) as a thread-block cluster of 8 or 16
+ * blocks whose shared memory holds the mesh, a patch of it each (a mesh
+ * that no cluster holds runs as mode 3 does); mode 2 as one block on global
+ * memory, for meshes up to 1024 vertices (IRBC_ERR_CAPACITY for a larger
+ * mesh; a mesh set later keeps mode 1's form); mode 3 as a cluster of 8
+ * blocks on global memory, any mesh.  The results are the same in every
+ * mode. */
 int irbc_set_membrane_kernels(irbc_handle* h, int32_t mode);
 int irbc_step_part1(irbc_handle* h);
 int irbc_step_part2(irbc_handle* h);
@@ -185,7 +186,7 @@ int irbc_bin_particles(const irbc_params* p, const double* x, const double* y, c
  * allocator callback or memory-pool hook, threads that must not take the
  * driver's allocation lock, embedders with a fixed device-memory budget).
  * Same arguments and results; allocates nothing.  Its scratch is a fixed
- * static device array (4 MiB plus 12 KiB) that every GPU loading the library
+ * static device array (12 KiB) that every GPU loading the library
  * keeps until the process exits, so boxes are limited to 1,048,576 cells
  * (Lx*Ly*(Lz+1)); larger boxes return IRBC_ERR_CAPACITY.  The first call on
  * a device looks up the array's device address and keeps it for the life of
@@ -241,8 +242,9 @@ int64_t irbc_launch_count(const irbc_handle* h);
  * streaming steps, out[3] = ms in the collision kernels, out[4] =
  * collisions, out[5] = ms in the membrane kernels (side stream), out[6] =
  * membrane launch groups, out[7] = kernel launches in the window, out[8] =
- * ms in the bulk streaming kernel alone (k_stream_fast / k_stream_f),
- * out[9] = its launches; nout <= 10 values are written */
+ * ms in the bulk streaming kernel alone (k_stream_bulk, k_stream_bulk_f),
+ * out[9] = its launches (one per stretch of timesteps between collisions);
+ * nout <= 10 values are written */
 /* device time (ms) between irbc_timer_begin and irbc_timer_end: two CUDA
  * events on the handle's stream and no per-phase events in between (what
  * irbc_step queues is joined back to that stream before it returns) */
@@ -268,8 +270,8 @@ int irbc_batch_step(irbc_batch* b, int64_t n);
  * How a batch launches its members' steps.  No field changes what a member
  * computes; each is checked bit for bit against its default:
  *   streams   irbc_set_streams for every member (1 or 2; default 2)
- *   membrane  irbc_set_membrane_kernels for every member (1 wide kernels,
- *             2 one block; default 1)
+ *   membrane  irbc_set_membrane_kernels for every member (1 the cluster
+ *             on shared memory, 2 one block; default 1)
  *   graphs    irbc_set_graphs for every member (0 or 1; default 0)
  *   chunk     steps a pool thread issues to one member before it turns to
  *             its next member (a multiple of 24 in 24..2400; default 24)
@@ -361,7 +363,7 @@ double irbc_server_clock(irbc_server* s);
 /* the launch schedule (irbc_schedule) for simulations admitted from now on
  * and for the rounds' issue chunk (default {2, 1, 0, 24, 0}: the pool);
  * membrane = 2 applies only to meshes that fit the one-block form, the
- * others keep the wide kernels.  Results do not depend on it. */
+ * others keep the default form.  Results do not depend on it. */
 int irbc_server_set_schedule(irbc_server* s, const irbc_schedule* sched);
 /* destroys a kept handle (a polled result of a keep = 1 request) and frees
  * its share of the budget; IRBC_ERR_ARG for a handle the server did not hand

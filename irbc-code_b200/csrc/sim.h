@@ -137,6 +137,9 @@ void launch_pfdt_forces(const DevParams& p, Membrane& m, int do_pfdt, int do_for
                         cudaStream_t st);
 void launch_bonds(const DevParams& p, Membrane& m, uint64_t epoch, cudaStream_t st);
 void launch_kick2(const DevParams& p, Membrane& m, cudaStream_t st);
+// the counting sort of particles by shifted cell (binning.cu)
+void bin_particles(const DevParams& p, const double* x, const double* y, const double* z, int64_t n, double rx,
+                   double ry, double rz, int* cell, int* start, int* order, int* part, cudaStream_t st);
 // end: oa[n] receives the total too
 void launch_scan3(const int* a, const int* b, const int* c, int* oa, int* ob, int* oc, int* totals,
                   int64_t n, int* part, cudaStream_t st, bool end = false);
