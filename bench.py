@@ -313,10 +313,10 @@ def run_ours(args):
     bpp = 72 if precision == G.FP64 else 48
     bulk_avg_ms = kprof["bulk_ms"] / max(1, kprof["bulk_launches"])
     achieved = ns * bpp / (bulk_avg_ms * 1e-3) / 1e9
-    # the whole step against the same bound: streaming every step plus the
-    # collision's read and write once per 10-12 steps (79.2 B FP64, 52.8 B
-    # FP32 per particle-step), at the measured particle-steps/s
-    step_bpp = 79.2 if precision == G.FP64 else 52.8
+    # the whole step against the same bound: one streaming pass and the
+    # collision's read and write per stretch of 12 steps (72 + 86 B a particle
+    # FP64, 48 + 58 B FP32), at the measured particle-steps/s
+    step_bpp = 13.2 if precision == G.FP64 else 8.8
     peak, kind = peaks()
     traffic = None
     tfile = os.path.join(ROOT, "profiles", "stream_traffic.json")
@@ -458,8 +458,8 @@ def run_batched(G, nrep=64, steps=240, nthreads=8):
             "vs_plain": agg / plain,
             "fused_default_value": total * steps / dt_fused, "pool_value": total * steps / dt_pool,
             "launches_per_batch_step": launches,
-            "roofline": {"bytes_per_particle_step": 52.8, "achieved_gbs": agg * 52.8 / 1e9, "peak": peak,
-                         "peak_kind": kind, "frac": agg * 52.8 / 1e9 / peak},
+            "roofline": {"bytes_per_particle_step": 8.8, "achieved_gbs": agg * 8.8 / 1e9, "peak": peak,
+                         "peak_kind": kind, "frac": agg * 8.8 / 1e9 / peak},
             "host_threads": nthreads, "dtype": "f32-bulk", "state_finite": finite, "healthy": not any(health),
             "schedule": sched,
             "autotune": {"seconds": tune_s, "steps": tune_steps, "trial_steps": 48, "repeats": 2},

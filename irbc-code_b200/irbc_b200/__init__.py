@@ -440,7 +440,8 @@ class Simulation:
         self._ck(self.L.irbc_set_streams(self.h, int(n)), "irbc_set_streams")
 
     def set_membrane_kernels(self, mode):
-        """1: wide kernels (default); 2: one block (meshes up to 1024 vertices)"""
+        """1: a cluster on shared memory (default); 2: one block (meshes up to 1024 vertices); 3: a cluster on global
+        memory"""
         self._ck(self.L.irbc_set_membrane_kernels(self.h, int(mode)), "irbc_set_membrane_kernels")
 
     def profile_begin(self):
