@@ -707,14 +707,14 @@ struct ProfScope {
 // bracketed by a pair of events of its own
 // returns the number of kernels it launched
 int stream_any(irbc_handle* h, int H, cudaStream_t st, cudaEvent_t snap = nullptr, int first = 0,
-               cudaEvent_t snap1 = nullptr) {
+               cudaEvent_t snap1 = nullptr, bool recorded = false) {
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (h->prof && !h->capturing) {
     h->ev_marks.push_back({PROF_STREAM_BULK, h->ev_used, h->ev_used + 1});
     e0 = next_event(h);
     e1 = next_event(h);
   }
-  return fast_stream(h->dp, h->s, h->fp32 ? &h->sf : nullptr, h->c, h->fb, H, st, e0, e1, snap, first, snap1);
+  return fast_stream(h->dp, h->s, h->fp32 ? &h->sf : nullptr, h->c, h->fb, H, st, e0, e1, snap, first, snap1, recorded);
 }
 
 }  // namespace
@@ -1477,12 +1477,18 @@ static int64_t stretch(irbc_handle* h, int64_t eoff, int64_t left, bool dry) {
         CK(cudaEventRecord(h->ev_part, ss));
       }
       g_launches += launch_membrane(h->dp, h->m, h->fb, (uint64_t)eoff, first, (int)H - first, SEG_WHOLE, ss);
+      // in one part, the records do not wait for a longer bulk streaming (a
+      // single step of 5.2 M particles: 88 us beside 64 us of membrane)
+      if (first == 0) {
+        launch_records(h->dp, h->fb, 0, (int)H, 0, ss);
+        g_launches += 1;
+      }
     }
     CK(cudaEventRecord(h->ev_mem, ss));
     {
       // the bulk streaming reads no membrane data and starts at once
       ProfScope ps(h, PROF_STREAM, ms);
-      g_launches += stream_any(h, (int)H, ms, h->ev_mem, first, h->ev_part);
+      g_launches += stream_any(h, (int)H, ms, h->ev_mem, first, h->ev_part, first == 0);
     }
   }
   step_ends(h);

@@ -696,8 +696,12 @@ void fast_snap_prep(const DevParams& p, Membrane& m, FastBufs& f, cudaStream_t s
   k_snap<<<nb(p.nv, 128), 128, 0, st>>>(p, m, f);
 }
 
+void launch_records(const DevParams& p, const FastBufs& f, int s0, int s1, int part, cudaStream_t st) {
+  k_tri_records<<<nb(p.nt, kRecordTris), kRecordT, 0, st>>>(p, f, s0, s1, part);
+}
+
 int fast_stream(const DevParams& p, const Solvent& s, const SolventF* sf, const Cells& c, FastBufs& f, int H,
-                cudaStream_t st, cudaEvent_t ev0, cudaEvent_t ev1, cudaEvent_t snap, int first, cudaEvent_t snap1) {
+                cudaStream_t st, cudaEvent_t ev0, cudaEvent_t ev1, cudaEvent_t snap, int first, cudaEvent_t snap1, bool recorded) {
   cudaMemsetAsync(f.qn, 0, 8 * sizeof(int), st);
   if (!s.n) return 0;
   const NearQueue h = queue_of(f, 0);
@@ -713,7 +717,7 @@ int fast_stream(const DevParams& p, const Solvent& s, const SolventF* sf, const 
     const int s0 = part ? first : 0, s1 = part + 1 < parts ? first : H;
     const cudaEvent_t ready = part + 1 < parts ? snap1 : snap;
     if (ready) cudaStreamWaitEvent(st, ready, 0);
-    k_tri_records<<<nb(p.nt, kRecordTris), kRecordT, 0, st>>>(p, f, s0, s1, part);
+    if (!recorded) launch_records(p, f, s0, s1, part, st);
     const NearArgs A = near_of(p, c, f, 0, s0, part);
     if (sf) {
       if (few) k_near<float, kShortG, kShortKeep><<<kNearBlocks, kNearT, 0, st>>>(p, arr, A, s1);
@@ -723,7 +727,7 @@ int fast_stream(const DevParams& p, const Solvent& s, const SolventF* sf, const 
       else k_near<double, kLongG, kLongKeep><<<kNearBlocks, kNearT, 0, st>>>(p, arr, A, s1);
     }
   }
-  return 1 + 2 * parts;
+  return 1 + (recorded ? 1 : 2) * parts;
 }
 
 }  // namespace irbc

@@ -119,11 +119,14 @@ void fast_snap_prep(const DevParams& p, Membrane& m, FastBufs& f, cudaStream_t s
 // reads no membrane data; the triangle records and the near-membrane kernel
 // read the snapshots and first wait for `snap` (optional: their producer).
 // first > 0: they run in two parts, the first `first` steps after snap1 and the
-// others after snap.  Returns the number of kernels it launched.
+// others after snap.  recorded: the triangle records are made already
+// (launch_records, before snap).  Returns the number of kernels it launched.
 struct SolventF;
 int fast_stream(const DevParams& p, const Solvent& s, const SolventF* sf, const Cells& c, FastBufs& f, int H,
                 cudaStream_t st, cudaEvent_t ev0 = nullptr, cudaEvent_t ev1 = nullptr, cudaEvent_t snap = nullptr,
-                int first = 0, cudaEvent_t snap1 = nullptr);
+                int first = 0, cudaEvent_t snap1 = nullptr, bool recorded = false);
+// the triangle records of the steps [s0, s1), part `part` of a stretch
+void launch_records(const DevParams& p, const FastBufs& f, int s0, int s1, int part, cudaStream_t st);
 bool is_membrane_kernel(const void* fn);
 // the membrane of the H steps from step s0 of a stretch (s0 + H <= kSegMax) in
 // one launch (segment.cuh); eoff: the stretch's; parts: SEG_FIRST | SEG_SECOND,
