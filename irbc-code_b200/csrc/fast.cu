@@ -371,23 +371,6 @@ __global__ void __launch_bounds__(256) k_stream_bulk_f(DevParams p, SolventArray
 }
 
 // ---- near the membrane ---------------------------------------------------------------------
-// reflectionFed's crossing test on a record's precomputed normals (the use_pre
-// case of tri_visit, Src/solfuncs.cpp:461-517): whether the full test can hit.
-// (X, Y, Z): the particle; (U, V, W): where it would fly in this step
-__device__ __forceinline__ bool tri_crossing(const TriPre& q, double X, double Y, double Z, double U, double V, double W,
-                                             int indio) {
-  double PSt0 = X - q.A1[0], PSt1 = Y - q.A1[1], PSt2 = Z - q.A1[2];
-  double PD0 = U - q.A2[0];
-  double PD1 = V - q.A2[1];
-  double PD2 = W - q.A2[2];
-  const double bt = q.X[0] * PSt0 + q.X[1] * PSt1 + q.X[2] * PSt2;
-  const double bdt = q.Xdt[0] * PD0 + q.Xdt[1] * PD1 + q.Xdt[2] * PD2;
-  int flg = 0;
-  if ((indio == 1) && (bt < 0)) flg = 1;
-  if ((indio == 0) && (bt > 0)) flg = 1;
-  return (bt * bdt <= 0) && (flg == 0);
-}
-
 // one TriPre record through the read-only path as six 16-byte loads (the
 // records are 96 bytes from a 256-byte aligned base)
 __device__ __forceinline__ TriPre ldg_tri(const TriPre* __restrict__ q) {
@@ -411,57 +394,16 @@ __device__ __forceinline__ int band_of(const DevParams& p, double x, double y) {
   return (x < l ? BAND_HX : (x > rx ? BAND_LX : 0)) | (y < l ? BAND_HY : (y > ry ? BAND_LY : 0));
 }
 
-// What no step of a stretch can make a crossing candidate, found once per
-// particle and stretch instead of in every step.  A candidate crosses the
-// triangle's plane: b_t = X_t . (P_t - A_t) changes sign, X_t the normal and A_t
-// the corner at step t, P_t the particle.  With the triangle's largest changes
-// over the stretch, dX of the normal and dA of the corner, and the particle's
-// path dP (speed x time left),
-//   |b_t - X_0 . (P - A_0)| <= dX (|P - A_0| + dP + dA) + |X_0| (dP + dA),
-// so an entry whose plane is farther away needs no test.  About 5% of the
-// 600-vertex mesh's entries and 10% of the discocyte's are left.  TriCull holds
-// what that takes in float; m covers the rounding: the coordinates' is at most
-// L 2^-24 each in a box of length L, that of the differences, products and sums
-// 4 parts in 2^24 of theirs, with differences up to L, and (L + 16) 2^-21 of the
-// normal's 1-norm covers both twice.  (NaN and infinities fail the comparison
-// and are kept.)  bands: of the triangle's corners in any of the steps.
-struct TriCull {
-  float X[3], nX, A[3], dX, dA, m;
-  int bands;
-};
 __device__ __forceinline__ TriCull ldg_cull(const float4* __restrict__ r) {
   const float4 a = __ldg(r), b = __ldg(r + 1), c = __ldg(r + 2);
   return TriCull{{a.x, a.y, a.z}, a.w, {b.x, b.y, b.z}, b.w, c.x, c.y, __float_as_int(c.z)};
 }
-__device__ __forceinline__ bool cull_keeps(const TriCull& c, float X, float Y, float Z, float dP, int band) {
-  const float x = X - c.A[0], y = Y - c.A[1], z = Z - c.A[2];
-  const float b = fabsf(c.X[0] * x + c.X[1] * y + c.X[2] * z);
-  const float d = sqrtf(x * x + y * y + z * z), move = dP + c.dA;
-  return (c.bands & band) || !(b > 1.0001f * (c.dX * (d + move) + c.nX * move) + c.m);
-}
-// a step's record against that of the first one
-struct CullMove {
-  double dX, dA;
-  int bands;
-};
-__device__ __forceinline__ double norm3(double x, double y, double z) { return sqrt(x * x + y * y + z * z); }
-__device__ __forceinline__ void cull_fold(CullMove& c, const TriPre& t0, const TriPre& t, int bands) {
-  c.dX = fmax(c.dX, fmax(norm3(t.X[0] - t0.X[0], t.X[1] - t0.X[1], t.X[2] - t0.X[2]),
-                         norm3(t.Xdt[0] - t0.X[0], t.Xdt[1] - t0.X[1], t.Xdt[2] - t0.X[2])));
-  c.dA = fmax(c.dA, fmax(norm3(t.A1[0] - t0.A1[0], t.A1[1] - t0.A1[1], t.A1[2] - t0.A1[2]),
-                         norm3(t.A2[0] - t0.A1[0], t.A2[1] - t0.A1[1], t.A2[2] - t0.A1[2])));
-  // a record that is not finite stays in every test
-  if (!isfinite(t.X[0] + t.X[1] + t.X[2] + t.Xdt[0] + t.Xdt[1] + t.Xdt[2] + t.A1[0] + t.A1[1] + t.A1[2] + t.A2[0] +
-                t.A2[1] + t.A2[2]))
-    c.dX = c.dA = __longlong_as_double(0x7ff0000000000000ll);
-  c.bands |= bands;
-}
-__device__ __forceinline__ void cull_store(const DevParams& p, float4* to, const TriPre& t0, const CullMove& c) {
-  const double L = fmax(p.Lx, fmax(p.Ly, p.Lz));
-  const double n1 = fabs(t0.X[0]) + fabs(t0.X[1]) + fabs(t0.X[2]) + c.dX;
-  to[0] = make_float4((float)t0.X[0], (float)t0.X[1], (float)t0.X[2], (float)norm3(t0.X[0], t0.X[1], t0.X[2]) * 1.00001f);
-  to[1] = make_float4((float)t0.A1[0], (float)t0.A1[1], (float)t0.A1[2], (float)c.dX * 1.00001f);
-  to[2] = make_float4((float)c.dA * 1.00001f, (float)(n1 * (L + 16.0) * (1.0 / 2097152.0)), __int_as_float(c.bands), 0.0f);
+__device__ __forceinline__ double longest_side(const DevParams& p) { return fmax(p.Lx, fmax(p.Ly, p.Lz)); }
+__device__ __forceinline__ void cull_store(const DevParams& p, float4* to, const TriPre& t0, const CullMove& mv) {
+  const TriCull c = cull_of(t0, mv, longest_side(p));
+  to[0] = make_float4(c.X[0], c.X[1], c.X[2], c.nX);
+  to[1] = make_float4(c.A[0], c.A[1], c.A[2], c.dX);
+  to[2] = make_float4(c.dA, c.m, __int_as_float(c.bands), 0.0f);
 }
 
 // what the near-membrane kernel reads of one simulation
@@ -575,10 +517,9 @@ __device__ __forceinline__ void near_particle(const DevParams& p, const SolventA
       const int band = band_of(p, x, y);
       if (fresh) {
         nk = 0;
-        // (the top wall gives its speed to what it reflects; a band ends inside a
-        // cell only in a box that is no whole number of cells; a wrap ends in
-        // another cell, except in a box of one)
-        float dP = (float)(fmax(sqrt(vx * vx + vy * vy + vz * vz), fabs(p.wallspeed)) * p.dtmd * (H - t)) * 1.0001f;
+        // (a band ends inside a cell only in a box that is no whole number of
+        // cells; a wrap ends in another cell, except in a box of one)
+        float dP = cull_path<R>(vx, vy, vz, p.wallspeed, p.dtmd, longest_side(p), H - t);
         if (p.nx < 2 || p.ny < 2) dP = __int_as_float(0x7f800000);
         const int wide = band | band_of(p, x - dP, y - dP) | band_of(p, x + dP, y + dP);
         constexpr int U = 4;  // entries in flight per lane

@@ -1,13 +1,9 @@
 // fast.h -- buffers and launchers of the production step (fast.cu).
 #pragma once
+#include "cull.h"
 #include "sim.h"
 
 namespace irbc {
-
-// per-triangle data of reflectionFed at rstep = 0 (Src/solfuncs.cpp:457-517)
-struct TriPre {
-  double X[3], Xdt[3], A1[3], A2[3];
-};
 
 // vertex positions/velocities as seen by the streaming of one step of a
 // stretch (the arrays hold kSegMax steps, nv entries each)

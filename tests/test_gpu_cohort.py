@@ -113,3 +113,68 @@ def test_members_out_of_phase_form_their_own_cohorts():
     b.close()
     for s in sims:
         s.close()
+
+
+def test_cohort_reflects_what_rounding_carries_to_the_membrane():
+    """A cohort takes 16 steps in one part.  In a box longer than 256 a
+    particle at x > 256 moves in units of 2^-15; with v dt = 23.51 of them it is
+    rounded to 24 a step, so one that starts 381 to 383 units before the
+    membrane, which 16 steps of v dt do not reach, crosses it in the last step.
+    The members equal single steps bit for bit."""
+    import irbc_b200 as G
+    from irbc_b200 import mesh
+    # a cube of side 2, each face in 2 x 2 squares
+    pts, T = {}, []
+    for k in range(3):
+        for side in (-1, 1):
+            at = {}
+            for i in (-1, 0, 1):
+                for j in (-1, 0, 1):
+                    q = [i, j]
+                    q.insert(k, side)
+                    at[i, j] = pts.setdefault(tuple(q), len(pts))
+            for i in (-1, 0):
+                for j in (-1, 0):
+                    c = at[i, j], at[i + 1, j], at[i + 1, j + 1], at[i, j + 1]
+                    T += [(c[0], c[1], c[2]), (c[0], c[2], c[3])]
+    V, T = np.array(list(pts), float), np.array(T, np.int32)
+    nv = len(V)
+    T = mesh.orient_outward(V, T)
+    E = mesh.edges_of(T)
+    ulp, face = 2.0 ** -15, 261.0
+    units = np.arange(365, 395)
+    spots = [(5.3, 6.45), (6.62, 6.55), (6.4, 5.2)]  # (y, z) inside triangles of the face
+    ns = len(units) * len(spots)
+    # (a heavy membrane stays where it is)
+    p = G.default_params(Lx=276.0, Ly=12.0, Lz=12.0, Ns=ns, seed=5, precision=G.FP32, dtcd=0.05, pmass=1e12, Nt=nv)
+    ends, sims = [], []
+    for _ in range(3):
+        s = G.Simulation(p)
+        s.init(V, E, T, 0)
+        st = s.get_state()
+        a = st.a
+        a["x"], a["y"], a["z"] = V[:, 0] + face + 1.0, V[:, 1] + 6.0, V[:, 2] + 6.0
+        for k in ("vx", "vy", "vz"):
+            a[k] = np.zeros(nv)
+        st.s.update(para=np.array([20.0, 6.0, 6.0]), paraV=np.zeros(3))
+        a["sx"] = np.repeat(face - units * ulp, len(spots))
+        a["sy"], a["sz"] = np.tile(np.array(spots).T, len(units))
+        a["svx"] = np.full(ns, 23.51 * ulp / p.dtmd)
+        a["svy"], a["svz"], a["sindio"] = np.zeros(ns), np.zeros(ns), np.ones(ns, np.int32)
+        s.set_state(st)
+        s.call("llist_update")
+        sims.append(s)
+    for _ in range(16):
+        sims[2].call("step_part1")
+        sims[2].call("step_part2")
+    b = G.Batch(nthreads=1)
+    b.add(sims[0])
+    b.add(sims[1])
+    b.step(16)
+    ends = [s.get_state() for s in sims]
+    hit = (ends[2].a["svx"] < 0).reshape(len(units), len(spots))
+    late = (units >= 381) & (units <= 383)
+    assert hit[late].any() and not hit[units >= 385].any()
+    for k in (0, 1):
+        assert H.compare(ends[k], ends[2], 0.0) == {}, k
+    b.close()
