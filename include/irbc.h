@@ -151,7 +151,8 @@ int irbc_set_streams(irbc_handle* h, int32_t n);
 /* Not in the reference.  How irbc_step launches the membrane of a stretch
  * of timesteps: mode 1 (the default) as a thread-block cluster of 8 or 16
  * blocks whose shared memory holds the mesh, a patch of it each (a mesh
- * that no cluster holds runs as mode 3 does); mode 2 as one block on global
+ * that no cluster holds, from about 2600 vertices on, runs as one kernel per
+ * phase over the whole GPU); mode 2 as one block on global
  * memory, for meshes up to 1024 vertices (IRBC_ERR_CAPACITY for a larger
  * mesh; a mesh set later keeps mode 1's form); mode 3 as a cluster of 8
  * blocks on global memory, any mesh.  The results are the same in every

@@ -1762,7 +1762,7 @@ static int cohort_upload(Cohort* c) {
   c->uids.resize(n);
   std::vector<std::array<int, MP_NPHASE>> nbk(n);
   int64_t tot[MP_NPHASE] = {};
-  P.vbin_smem = 0;
+  P.vbin_smem = P.wide_smem = 0;
   for (size_t r = 0; r < n; ++r) {
     c->host[r] = member_of(c->members[r]);
     c->uids[r] = c->members[r]->uid;
@@ -1776,6 +1776,11 @@ static int cohort_upload(Cohort* c) {
   for (size_t r = 0; r < n; ++r) {
     int smem = 0;
     const int nc = multi_segment(c->host[r], &smem);
+    scls[r] = -1;
+    if (nc == 0) {
+      P.wide_smem = std::max(P.wide_smem, smem);
+      continue;
+    }
     size_t k = 0;
     while (k < P.seg.size() && P.seg[k].nc != nc) ++k;
     if (k == P.seg.size()) P.seg.push_back({nc, 0, 0});

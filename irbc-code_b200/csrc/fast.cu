@@ -622,7 +622,12 @@ namespace irbc {
 // ================================================================ launch ======
 // the side stream's work: a captured graph gives it the side stream's high
 // priority
-bool is_membrane_kernel(const void* fn) { return fn == (const void*)k_membrane; }
+bool is_membrane_kernel(const void* fn) {
+  for (const void* k : {(const void*)k_membrane, (const void*)k_wide_first, (const void*)k_wide_tri,
+                        (const void*)k_wide_terms, (const void*)k_wide_gather})
+    if (fn == k) return true;
+  return false;
+}
 
 // snapshot of the membrane as it is (irbc_stream), as step 0 of a stretch
 __global__ void k_snap(DevParams p, Membrane m, FastBufs f) {

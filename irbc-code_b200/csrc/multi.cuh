@@ -65,20 +65,44 @@ struct SegMember {
   Membrane m;
   FastBufs f;
 };
-__global__ void __launch_bounds__(kSegT) km_membrane(const Member* __restrict__ mem, const int2* __restrict__ tab,
-                                                     uint64_t eoff, int H) {
-  extern __shared__ __align__(16) unsigned char seg_sh[];
-  __shared__ __align__(16) unsigned char raw[sizeof(SegMember)];
-  SegMember& S = *reinterpret_cast<SegMember*>(raw);
-  const Member& M = mem[__ldg(tab + blockIdx.x).x];
+__device__ __forceinline__ void seg_member(const Member& M, SegMember& S) {
   auto copy = [](void* d, const void* s, int bytes) {
-    for (int i = threadIdx.x; i < bytes / 4; i += kSegT) ((int*)d)[i] = ((const int*)s)[i];
+    for (int i = threadIdx.x; i < bytes / 4; i += blockDim.x) ((int*)d)[i] = ((const int*)s)[i];
   };
   copy(&S.p, &M.p, sizeof(DevParams));
   copy(&S.m, &M.m, sizeof(Membrane));
   copy(&S.f, &M.fb, sizeof(FastBufs));
   __syncthreads();
+}
+#define KM_SEG_MEMBER                                            \
+  __shared__ __align__(16) unsigned char raw[sizeof(SegMember)]; \
+  SegMember& S = *reinterpret_cast<SegMember*>(raw);             \
+  const int2 e = __ldg(tab + blockIdx.x);                        \
+  seg_member(mem[e.x], S)
+__global__ void __launch_bounds__(kSegT) km_membrane(const Member* __restrict__ mem, const int2* __restrict__ tab,
+                                                     uint64_t eoff, int H) {
+  extern __shared__ __align__(16) unsigned char seg_sh[];
+  KM_SEG_MEMBER;
   membrane_segment(S.p, S.m, S.f, epoch_of(S.p, eoff), H, SEG_WHOLE, seg_sh);
+}
+__global__ void __launch_bounds__(kWideT) km_wide_first(const Member* __restrict__ mem, const int2* __restrict__ tab) {
+  KM_SEG_MEMBER;
+  wide_first_block(S.p, S.m, S.f, SEG_WHOLE, e.y);
+}
+__global__ void __launch_bounds__(kWideT) km_wide_tri(const Member* __restrict__ mem, const int2* __restrict__ tab) {
+  KM_SEG_MEMBER;
+  wide_tri_block(S.p, S.m, S.f, e.y);
+}
+__global__ void __launch_bounds__(kSegT) km_wide_terms(const Member* __restrict__ mem, const int2* __restrict__ tab) {
+  extern __shared__ __align__(16) unsigned char seg_sh[];
+  KM_SEG_MEMBER;
+  wide_terms_block(S.p, S.m, S.f, SEG_WHOLE, e.y, seg_sh);
+}
+__global__ void __launch_bounds__(kWideT) km_wide_gather(const Member* __restrict__ mem, const int2* __restrict__ tab,
+                                                         uint64_t eoff, int s, int more) {
+  __shared__ TailSmem tail;
+  KM_SEG_MEMBER;
+  wide_gather_block(S.p, S.m, S.f, epoch_of(S.p, eoff), s, SEG_WHOLE, more, e.y, tail);
 }
 __global__ void __launch_bounds__(kRecordT) km_tri_records(const Member* __restrict__ mem, const int2* __restrict__ tab,
                                                            int H) {
@@ -106,8 +130,15 @@ int multi_membrane(const MultiPlan& P, uint64_t eoff, int H, cudaStream_t st) {
     cudaLaunchKernelEx(&cfg, km_membrane, (const Member*)P.mem, tab, eoff, H);
     tab += s.members * s.nc;
   }
+  const int wide = P.blocks[MP_WIDE_FIRST] > 0 ? H : 0;
+  if (wide) km_wide_first<<<P.blocks[MP_WIDE_FIRST], kWideT, 0, st>>>(P.mem, P.table(MP_WIDE_FIRST));
+  for (int s = 0; s < wide; ++s) {
+    km_wide_tri<<<P.blocks[MP_WIDE_TRI], kWideT, 0, st>>>(P.mem, P.table(MP_WIDE_TRI));
+    km_wide_terms<<<P.blocks[MP_WIDE_TERMS], kSegT, P.wide_smem, st>>>(P.mem, P.table(MP_WIDE_TERMS));
+    km_wide_gather<<<P.blocks[MP_WIDE_GATHER], kWideT, 0, st>>>(P.mem, P.table(MP_WIDE_GATHER), eoff, s, s + 1 < H);
+  }
   km_tri_records<<<P.blocks[MP_RECORDS], kRecordT, 0, st>>>(P.mem, P.table(MP_RECORDS), H);
-  return (int)P.seg.size() + 1;
+  return (int)P.seg.size() + (wide ? 1 + 3 * wide : 0) + 1;
 }
 
 // ---- collision: particle phases ---------------------------------------------------
@@ -162,6 +193,8 @@ void set_kernel_limits() {
   const auto dyn = cudaFuncAttributeMaxDynamicSharedMemorySize;
   cudaFuncSetAttribute(k_membrane, dyn, kSegSmemMax);
   cudaFuncSetAttribute(km_membrane, dyn, kSegSmemMax);
+  cudaFuncSetAttribute(k_wide_terms, dyn, kSegSmemMax);
+  cudaFuncSetAttribute(km_wide_terms, dyn, kSegSmemMax);
   // clusters of sixteen blocks (the discocyte's)
   cudaFuncSetAttribute(k_membrane, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   cudaFuncSetAttribute(km_membrane, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
@@ -174,7 +207,12 @@ void multi_blocks(const Member& M, int out[MP_NPHASE]) {
   out[MP_STREAM] = (int)nbf(ns, 256 * kMultiStreamPasses);
   out[MP_NEAR_SHORT] = short_lists(M.fb.lmax) ? kNearBlocksMember : 0;
   out[MP_NEAR_LONG] = short_lists(M.fb.lmax) ? 0 : kNearBlocksMember;
-  out[MP_MEMBRANE] = segment_blocks(M.p, M.fb);
+  const bool wide = wide_membrane(M.fb);
+  out[MP_MEMBRANE] = wide ? 0 : segment_blocks(M.fb);
+  out[MP_WIDE_FIRST] = wide ? wide_first_blocks(M.p) : 0;
+  out[MP_WIDE_TRI] = wide ? wide_tri_blocks(M.p) : 0;
+  out[MP_WIDE_TERMS] = wide ? wide_terms_blocks(M.p, SEG_WHOLE) : 0;
+  out[MP_WIDE_GATHER] = wide ? wide_gather_blocks(M.p) : 0;
   out[MP_RECORDS] = (int)nb(M.p.nt, kRecordTris);
   out[MP_ZERO] = (int)nb(nc, 256);
   out[MP_VBIN] = (int)nb(M.p.nv, 32);
@@ -190,7 +228,11 @@ int multi_vbin_smem(const Member& M) {
 }
 
 int multi_segment(const Member& M, int* smem) {
-  const int nc = segment_blocks(M.p, M.fb);
+  if (wide_membrane(M.fb)) {
+    *smem = (int)wide_smem(M.p);
+    return 0;
+  }
+  const int nc = segment_blocks(M.fb);
   *smem = (int)seg_smem(M.p, M.fb, nc);
   return nc;
 }

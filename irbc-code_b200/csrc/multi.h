@@ -29,6 +29,7 @@ struct Member {
 enum MultiPhase : int {
   MP_STREAM, MP_NEAR_SHORT, MP_NEAR_LONG,                         // streaming
   MP_MEMBRANE, MP_RECORDS,                                        // membrane of a stretch
+  MP_WIDE_FIRST, MP_WIDE_TRI, MP_WIDE_TERMS, MP_WIDE_GATHER,      // ... of members without patches
   MP_ZERO, MP_VBIN, MP_COUNT, MP_SCAN, MP_PERM, MP_TILE, MP_MOVE,  // collision
   MP_NPHASE
 };
@@ -43,6 +44,7 @@ struct MultiPlan {
   int n = 0;
   int blocks[MP_NPHASE] = {};    // each phase's grid
   int vbin_smem = 0;             // vertex binning: the largest member's keys
+  int wide_smem = 0;             // MP_WIDE_TERMS: the largest member's
   // membrane: a launch per cluster size, its members' blocks in this order in
   // phase MP_MEMBRANE's table; smem: the largest member's
   struct Seg { int nc, members, smem; };
@@ -59,7 +61,8 @@ constexpr int kMultiStreamPasses = 8;
 void multi_blocks(const Member& M, int out[MP_NPHASE]);
 // dynamic shared memory of the vertex binning for one member (host)
 int multi_vbin_smem(const Member& M);
-// the blocks of one member's membrane cluster and their shared memory (host)
+// the blocks of one member's membrane cluster (0: a kernel a phase) and their
+// shared memory (MP_WIDE_TERMS's where there is no cluster) (host)
 int multi_segment(const Member& M, int* smem);
 
 // fused launches of a stretch of H steps; par = the stretch's parity: the queue
@@ -67,7 +70,7 @@ int multi_segment(const Member& M, int* smem);
 // next one).  snap (optional): the event the near-membrane kernels wait for
 // (the records' producer).  Each returns the number of kernels it launched.
 int multi_stream(const MultiPlan& P, int H, int par, cudaStream_t st, cudaEvent_t snap);
-// the membrane of H steps, a cluster per member
+// the membrane of H steps, a cluster per member or a kernel a phase
 int multi_membrane(const MultiPlan& P, uint64_t eoff, int H, cudaStream_t st);
 // A collision, in this order: multi_collide_front (kernels.cu: the cell
 // counters cleared, the vertices binned), multi_collide_count (fast.cu: the

@@ -565,11 +565,12 @@ __device__ __noinline__ void bond_events_serial(const DevParams& p, const Membra
   }
 }
 
+template <int T>
 __device__ __forceinline__ void tail_block(const DevParams& p, const Membrane& m, const FastBufs& f, uint64_t epoch,
                                            bool drift_next, TailSmem& S) {
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   MemScalars* sc = m.sc;
-  const int chunk = (p.nv + kSegT - 1) / kSegT;
+  const int chunk = (p.nv + T - 1) / T;
   const int v0 = min(tid * chunk, p.nv), v1 = min(v0 + chunk, p.nv);
   int nd = 0, nw = 0;
   for (int ii = v0; ii < v1; ++ii) {
@@ -585,7 +586,7 @@ __device__ __forceinline__ void tail_block(const DevParams& p, const Membrane& m
   if (lane == 31) { S.wd[w] = sd; S.ww[w] = sw; }
   __syncthreads();
   int od = sd - nd, ow = sw - nw, ndt = 0, nwt = 0;
-  for (int u = 0; u < kSegT / 32; ++u) {
+  for (int u = 0; u < T / 32; ++u) {
     const int a = S.wd[u], b = S.ww[u];
     if (u < w) { od += a; ow += b; }
     ndt += a; nwt += b;
@@ -679,12 +680,116 @@ __device__ __forceinline__ void kick_drift(const DevParams& p, const Membrane& m
   X[i] = x;
 }
 
+// The phases of a step with the state in global memory, by G threads numbered g.
+// The first half-kick of the first step (SEG_FIRST), or only the unwrapped
+// coordinates that the force terms read
+__device__ __forceinline__ void global_first(const DevParams& p, const Membrane& m, const FastBufs& f, int parts, int g,
+                                             int G) {
+  if (parts & SEG_FIRST) {
+    const Snap sn = snap_of(f, 0, p.nv);
+    for (int q = g; q < 3 * p.nv; q += G) {
+      const int i = q / 3, k = q - 3 * i;
+      double* F = k == 0 ? m.fx : (k == 1 ? m.fy : m.fz);
+      kick_drift(p, m, f, sn, i, k, (k == 0 ? m.vx : (k == 1 ? m.vy : m.vz))[i], F[i]);
+      F[i] = 0.0;
+    }
+    if (g == 0) para_drift(p, m.sc);
+  } else {
+    for (int i = g; i < p.nv; i += G) { f.ux[i] = m.x[i] + m.ix[i] * p.Lx; f.uy[i] = m.y[i] + m.iy[i] * p.Ly; }
+  }
+}
+// A: the triangles; their area and volume terms to a_to and v_to
+__device__ __forceinline__ void global_tri(const DevParams& p, const Membrane& m, const FastBufs& f, double* a_to,
+                                           double* v_to, bool pad, int g, int G) {
+  const int run = tree_run(p.nt);
+  for (int i = g; i < p.nt; i += G) {
+    double ar, vo;
+    tri_item(p, m, f, i, ar, vo);
+    const int at = pad ? tree_at(i, run) : i;
+    a_to[at] = ar;
+    v_to[at] = vo;
+  }
+}
+// B: Sarea or Volume from its terms by sw warps (thread st of them, named
+// barrier bar), and the factor of the global area or volume force
+__device__ __forceinline__ void global_sum(const DevParams& p, const Membrane& m, const FastBufs& f, int parts, bool area,
+                                           const double* src, bool pad, SumScratch& S, int st, int sw, int bar) {
+  double* sum = area ? &m.sc->Sarea : &m.sc->Volume;
+  if (parts & SEG_FIRST) {
+    double r;
+    if (p.tree_sums) r = tree_sum(src, p.nt, pad, st & 31);
+    else r = ordered_sum(src, p.nt, S, st, sw, bar);
+    if (st == 0) *sum = r;
+  }
+  if (st == 0) {
+    if (area) f.fac[0] = -p.kappasa * (*sum - p.Sarea0) / p.Sarea0;
+    else f.fac[1] = -p.kappav * (*sum - p.Volume0) / (p.Volume0);
+  }
+}
+// ... beside them the edge and bending terms
+__device__ __forceinline__ void global_terms(const DevParams& p, const Membrane& m, const FastBufs& f, int worker,
+                                             int workers) {
+  for (int q = worker; q < 2 * p.ne; q += workers) {
+    if (q < p.ne) dih_item(p, m, f, q);
+    else edge_item(p, m, f, q - p.ne);
+  }
+}
+// C: the gather of step s and the kicks
+__device__ __forceinline__ void global_gather(const DevParams& p, const Membrane& m, const FastBufs& f, int s, int parts,
+                                              bool more, int g, int G) {
+  const Snap sn = snap_of(f, s + 1, p.nv);
+  const double beta = f.fac[0], betav = f.fac[1];
+  const int base_t = 4 * p.ne;
+  for (int q = g; q < 3 * p.nv; q += G) {
+    const int i = q / 3, k = q - 3 * i;
+    const int q0 = f.gstart[3 * i], q1 = f.gstart[3 * i + 1], q2 = f.gstart[3 * i + 2], q3 = f.gstart[3 * i + 3];
+    const int vd = f.vd[i];
+    const double* S = f.slot + k;
+    double acc = 0.0;
+#pragma unroll 8
+    for (int e = q0; e < q1; ++e) acc += S[3 * (int64_t)f.gidx[e]];
+#pragma unroll 2
+    for (int e = q1; e < q2; e += 2) {
+      // the three terms of a triangle's corner (tri_item): slots n, n + 1
+      // and gidx[e + 1]
+      const int n = f.gidx[e];
+      acc += (beta / f.a4[(n - base_t) / 9]) * S[3 * (int64_t)n];
+      acc += S[3 * (int64_t)(n + 1)];
+      acc += betav * S[3 * (int64_t)f.gidx[e + 1]] / 6.0;
+    }
+#pragma unroll 8
+    for (int e = q2; e < q3; ++e) acc += S[3 * (int64_t)f.gidx[e]];
+    // the first half-kick has reset the force (:490)
+    double* F = k == 0 ? m.fx : (k == 1 ? m.fy : m.fz);
+    double fk = (parts & SEG_FIRST) ? 0.0 : F[i];
+    if (vd & VF_WCA) fk -= f.vX[3 * i + k];  // pfdt's -X
+    fk += acc;
+    if (k == 2) fk += -p.Fg / (double)p.nv;
+    if (vd & VF_SPRING) fk += f.vS[3 * i + k];
+    if (k == 2) {
+      double cc = m.z[i];
+      if (cc < 0.5) fk += 300.0 * exp(-50.0 * cc);
+      cc = p.Lz - m.z[i];
+      if (cc < 0.5) fk -= 300.0 * exp(-50.0 * cc);
+    }
+    // second half-kick (maincode.cpp:727-733)
+    double* V = k == 0 ? m.vx : (k == 1 ? m.vy : m.vz);
+    const double v = V[i] + (fk * p.dtmd / (2.0 * p.pmass));
+    raise_health(p, !isfinite(fk + v), HEALTH_MEMBRANE);
+    if (more) {
+      kick_drift(p, m, f, sn, i, k, v, fk);
+    } else {
+      V[i] = v;
+      F[i] = fk;
+    }
+  }
+}
+
 // The membrane of H steps by a cluster of blocks that keep its state in global
-// memory: meshes whose patches do not fit (membrane_patch), and the one-block
-// and eight-block forms of irbc_set_membrane_kernels.  Bound by the load and
-// store units: a warp's scattered 8-byte accesses take a cycle a line (the
-// discocyte on eight blocks: 92 us a step).  seg_smem() bytes of shared memory,
-// the same layout in every block.
+// memory: the one-block and eight-block forms of irbc_set_membrane_kernels.
+// Bound by the load and store units: a warp's scattered 8-byte accesses take a
+// cycle a line (the discocyte on eight blocks: 92 us a step).  seg_smem() bytes
+// of shared memory, the same layout in every block.
 __device__ __forceinline__ void membrane_global(const DevParams& p, const Membrane& m, const FastBufs& f,
                                                  uint64_t epoch, int H, int parts, unsigned char* smem) {
   namespace cg = cooperative_groups;
@@ -712,120 +817,105 @@ __device__ __forceinline__ void membrane_global(const DevParams& p, const Membra
   const int workers = G - busy0 - busy1;
   // the area and volume terms: in the summing blocks' shared memory when they
   // fit (terms of block 0 and of block 1; one after the other in a block
-  // alone), else in global memory
+  // alone), else in global memory (meshes of more triangles than a closed
+  // surface of 8192 vertices has)
   const bool staged = p.nt <= kSegTerms;
   const bool pad = staged && p.tree_sums;
-  const int run = tree_run(p.nt);
   double* a_to = staged ? (nc > 1 ? cl.map_shared_rank(terms, 0) : terms) : m.area;
   double* v_to = staged ? (nc > 1 ? cl.map_shared_rank(terms, 1) : terms + seg_terms(p.nt)) : m.vol;
   double* v_at = staged ? (nc > 1 ? terms : terms + seg_terms(p.nt)) : m.vol;
   const double* a_at = staged ? terms : m.area;
 
-  if (parts & SEG_FIRST) {
-    const Snap sn = snap_of(f, 0, p.nv);
-    for (int q = g; q < 3 * p.nv; q += G) {
-      const int i = q / 3, k = q - 3 * i;
-      double* F = k == 0 ? m.fx : (k == 1 ? m.fy : m.fz);
-      kick_drift(p, m, f, sn, i, k, (k == 0 ? m.vx : (k == 1 ? m.vy : m.vz))[i], F[i]);
-      F[i] = 0.0;
-    }
-    if (g == 0) para_drift(p, m.sc);
-  } else {
-    for (int i = g; i < p.nv; i += G) { f.ux[i] = m.x[i] + m.ix[i] * p.Lx; f.uy[i] = m.y[i] + m.iy[i] * p.Ly; }
-  }
+  global_first(p, m, f, parts, g, G);
   cl.sync();
   for (int s = 0; s < H; ++s) {
-    // A: the triangles
-    for (int i = g; i < p.nt; i += G) {
-      double ar, vo;
-      tri_item(p, m, f, i, ar, vo);
-      const int at = pad ? tree_at(i, run) : i;
-      a_to[at] = ar;
-      v_to[at] = vo;
-    }
+    global_tri(p, m, f, a_to, v_to, pad, g, G);
     cl.sync();
-    // B: sums beside the other force terms
     if (area_w || vol_w) {
-      const int st = area_w ? t : t - 32 * voff * sw;
-      if (parts & SEG_FIRST) {
-        const double* src = area_w ? a_at : v_at;
-        double r;
-        if (p.tree_sums) r = tree_sum(src, p.nt, pad, t & 31);
-        else r = ordered_sum(src, p.nt, area_w ? ss0 : ss1, st, sw, area_w ? 1 : 2);
-        if (st == 0) *(area_w ? &m.sc->Sarea : &m.sc->Volume) = r;
-      }
-      if (st == 0) {
-        // the factors of the global area and volume forces
-        if (area_w) f.fac[0] = -p.kappasa * (m.sc->Sarea - p.Sarea0) / p.Sarea0;
-        else f.fac[1] = -p.kappav * (m.sc->Volume - p.Volume0) / (p.Volume0);
-      }
-    } else {
-      const int ne = (parts & SEG_SECOND) ? p.ne : 0;
-      for (int q = worker; q < 2 * ne; q += workers) {
-        if (q < ne) dih_item(p, m, f, q);
-        else edge_item(p, m, f, q - ne);
-      }
-      if (parts & SEG_SECOND) bond_prep_all(p, m, f, worker, workers, reinterpret_cast<unsigned char*>(&tail));
+      global_sum(p, m, f, parts, area_w, area_w ? a_at : v_at, pad, area_w ? ss0 : ss1,
+                 area_w ? t : t - 32 * voff * sw, sw, area_w ? 1 : 2);
+    } else if (parts & SEG_SECOND) {
+      global_terms(p, m, f, worker, workers);
+      bond_prep_all(p, m, f, worker, workers, reinterpret_cast<unsigned char*>(&tail));
     }
     if (!(parts & SEG_SECOND)) return;
     cl.sync();
-    // C: the gather and the kicks; the tail by the last block
     const bool more = s + 1 < H;
     const int gb = nc >= 4 ? nc - 1 : nc;  // blocks that gather
-    if (cta < gb) {
-      const Snap sn = snap_of(f, s + 1, p.nv);
-      const double beta = f.fac[0], betav = f.fac[1];
-      const int base_t = 4 * p.ne;
-      for (int q = g; q < 3 * p.nv; q += gb * T) {
-        const int i = q / 3, k = q - 3 * i;
-        const int q0 = f.gstart[3 * i], q1 = f.gstart[3 * i + 1], q2 = f.gstart[3 * i + 2], q3 = f.gstart[3 * i + 3];
-        const int vd = f.vd[i];
-        const double* S = f.slot + k;
-        double acc = 0.0;
-#pragma unroll 8
-        for (int e = q0; e < q1; ++e) acc += S[3 * (int64_t)f.gidx[e]];
-#pragma unroll 2
-        for (int e = q1; e < q2; e += 2) {
-          // the three terms of a triangle's corner (tri_item): slots n, n + 1
-          // and gidx[e + 1]
-          const int n = f.gidx[e];
-          acc += (beta / f.a4[(n - base_t) / 9]) * S[3 * (int64_t)n];
-          acc += S[3 * (int64_t)(n + 1)];
-          acc += betav * S[3 * (int64_t)f.gidx[e + 1]] / 6.0;
-        }
-#pragma unroll 8
-        for (int e = q2; e < q3; ++e) acc += S[3 * (int64_t)f.gidx[e]];
-        // the first half-kick has reset the force (:490)
-        double* F = k == 0 ? m.fx : (k == 1 ? m.fy : m.fz);
-        double fk = (parts & SEG_FIRST) ? 0.0 : F[i];
-        if (vd & VF_WCA) fk -= f.vX[3 * i + k];  // pfdt's -X
-        fk += acc;
-        if (k == 2) fk += -p.Fg / (double)p.nv;
-        if (vd & VF_SPRING) fk += f.vS[3 * i + k];
-        if (k == 2) {
-          double cc = m.z[i];
-          if (cc < 0.5) fk += 300.0 * exp(-50.0 * cc);
-          cc = p.Lz - m.z[i];
-          if (cc < 0.5) fk -= 300.0 * exp(-50.0 * cc);
-        }
-        // second half-kick (maincode.cpp:727-733)
-        double* V = k == 0 ? m.vx : (k == 1 ? m.vy : m.vz);
-        const double v = V[i] + (fk * p.dtmd / (2.0 * p.pmass));
-        raise_health(p, !isfinite(fk + v), HEALTH_MEMBRANE);
-        if (more) {
-          kick_drift(p, m, f, sn, i, k, v, fk);
-        } else {
-          V[i] = v;
-          F[i] = fk;
-        }
-      }
-    }
-    if (cta == nc - 1) {
-      // (a block that also gathers reads vX and vd there, which the tail only reads)
-      tail_block(p, m, f, epoch + s, more, tail);
-    }
+    if (cta < gb) global_gather(p, m, f, s, parts, more, g, gb * T);
+    // (a block that also gathers reads vX and vd there, which the tail only reads)
+    if (cta == nc - 1) tail_block<kSegT>(p, m, f, epoch + s, more, tail);
     cl.sync();
   }
+}
+
+// The membrane of a mesh that no cluster holds in patches (from about 2600
+// vertices on): a kernel a phase over the whole GPU, three dependent
+// launches a step.  A cluster's few blocks lose to their scattered accesses, the
+// more the larger the mesh; us a step in a 64 x 32 x 32 box with 50,000
+// particles, a cluster of eight on global memory against this, FP64 and FP32:
+// 2892 vertices 97, 92 and 62, 53; 4002 vertices 114, 108 and 66, 52; 7842
+// vertices 209, 197 and 70, 59.  So do cohorts, a launch a phase over all their
+// members: 1, 2 and 16 members of 7842 vertices 220, 231, 566 and 82, 93, 380.
+constexpr int kWideT = 256;
+// blocks of each phase (a block of the terms: kSegT threads, two for the sums; the
+// gather's last one: the tail)
+__host__ __device__ inline int wide_first_blocks(const DevParams& p) { return (3 * p.nv + kWideT - 1) / kWideT; }
+__host__ __device__ inline int wide_tri_blocks(const DevParams& p) { return (p.nt + kWideT - 1) / kWideT; }
+__host__ __device__ inline int wide_bond0(const DevParams& p) { return (2 * p.ne + 31) / 32 * 32; }
+__host__ __device__ inline int wide_terms_blocks(const DevParams& p, int parts) {
+  return 2 + ((parts & SEG_SECOND) ? (wide_bond0(p) + p.nv + kSegT - 1) / kSegT : 0);
+}
+__host__ __device__ inline int wide_gather_blocks(const DevParams& p) { return wide_first_blocks(p) + 1; }
+
+__device__ __forceinline__ void wide_first_block(const DevParams& p, const Membrane& m, const FastBufs& f, int parts,
+                                                 int b) {
+  global_first(p, m, f, parts, b * kWideT + threadIdx.x, wide_first_blocks(p) * kWideT);
+}
+__device__ __forceinline__ void wide_tri_block(const DevParams& p, const Membrane& m, const FastBufs& f, int b) {
+  global_tri(p, m, f, m.area, m.vol, false, b * kWideT + threadIdx.x, wide_tri_blocks(p) * kWideT);
+}
+// blocks 0 and 1: the sums, their terms staged in shared memory first where
+// they fit; the others: a term or a vertex's bond preparation per thread
+__device__ __forceinline__ void wide_terms_block(const DevParams& p, const Membrane& m, const FastBufs& f, int parts,
+                                                 int b, unsigned char* smem) {
+  const int t = threadIdx.x;
+  if (b < 2) {
+    const bool area = b == 0, staged = p.nt <= kSegTerms, pad = staged && p.tree_sums;
+    const int run = tree_run(p.nt), sw = p.tree_sums ? 1 : kSegT / 32;
+    const double* src = area ? m.area : m.vol;
+    SumScratch& S = *reinterpret_cast<SumScratch*>(smem);
+    double* terms = reinterpret_cast<double*>(smem + sizeof(SumScratch));
+    if (staged && (parts & SEG_FIRST))
+      for (int i = t; i < p.nt; i += kSegT) terms[pad ? tree_at(i, run) : i] = src[i];
+    __syncthreads();
+    if (t < 32 * sw) global_sum(p, m, f, parts, area, staged ? terms : src, pad, S, t, sw, 1);
+    return;
+  }
+  const int worker = (b - 2) * kSegT + t, bond0 = wide_bond0(p);
+  if (worker < bond0) global_terms(p, m, f, worker, bond0);
+  else bond_prep_all(p, m, f, worker - bond0, 1 << 30, smem);
+}
+__device__ __forceinline__ void wide_gather_block(const DevParams& p, const Membrane& m, const FastBufs& f,
+                                                  uint64_t epoch, int s, int parts, bool more, int b, TailSmem& tail) {
+  const int n = wide_first_blocks(p);
+  if (b == n) tail_block<kWideT>(p, m, f, epoch + s, more, tail);
+  else global_gather(p, m, f, s, parts, more, b * kWideT + threadIdx.x, n * kWideT);
+}
+__global__ void __launch_bounds__(kWideT) k_wide_first(DevParams p, Membrane m, FastBufs f, int parts) {
+  wide_first_block(p, m, f, parts, blockIdx.x);
+}
+__global__ void __launch_bounds__(kWideT) k_wide_tri(DevParams p, Membrane m, FastBufs f) {
+  wide_tri_block(p, m, f, blockIdx.x);
+}
+__global__ void __launch_bounds__(kSegT) k_wide_terms(DevParams p, Membrane m, FastBufs f, int parts) {
+  extern __shared__ __align__(16) unsigned char seg_sh[];
+  wide_terms_block(p, m, f, parts, blockIdx.x, seg_sh);
+}
+__global__ void __launch_bounds__(kWideT) k_wide_gather(DevParams p, Membrane m, FastBufs f, uint64_t eoff, int s,
+                                                        int parts, int more) {
+  __shared__ TailSmem tail;
+  wide_gather_block(p, m, f, epoch_of(p, eoff), s, parts, more, blockIdx.x, tail);
 }
 
 // ---- the membrane in patches ---------------------------------------------------------
@@ -1437,6 +1527,12 @@ static size_t seg_smem(const DevParams& p, const FastBufs& f, int nc) {
   return fixed + (p.nt <= kSegTerms ? (nc > 1 ? 1 : 2) * (size_t)seg_terms(p.nt) * sizeof(double) : 0);
 }
 
+// k_wide_terms: the staged terms, or the bond preparation's room
+static size_t wide_smem(const DevParams& p) {
+  const size_t sum = sizeof(SumScratch) + (p.nt <= kSegTerms ? (size_t)seg_terms(p.nt) * sizeof(double) : 0);
+  return std::max(sum, (size_t)(kSegT / 16) * kMaxPairs * (sizeof(double) + sizeof(int)));
+}
+
 // the streaming's records of every triangle for the steps [s0, s1) of a stretch
 // and what none of them needs to test (TriCull), by a lane per triangle and
 // kRecordRows rows of steps.  A kernel of its own: in the membrane kernel their
@@ -1504,12 +1600,13 @@ __global__ void __launch_bounds__(kRecordT) k_tri_records(DevParams p, FastBufs 
   records_block(p, f, s0, s1, part, blockIdx.x, S);
 }
 
-// blocks of the membrane's cluster
-int segment_blocks(const DevParams& p, const FastBufs& f) {
+// whether a membrane runs as a kernel a phase
+static bool wide_membrane(const FastBufs& f) { return f.patch.nc == 0 && !f.one_block && !f.cluster; }
+
+// blocks of the membrane's cluster (not where wide_membrane)
+int segment_blocks(const FastBufs& f) {
   if (f.patch.nc > 0) return f.patch.nc;
-  if (f.one_block) return 1;
-  if (f.cluster) return 8;
-  return p.nt <= 2048 ? 4 : 8;
+  return f.one_block ? 1 : 8;
 }
 
 bool one_block_fits(const DevParams& p) { return p.nv <= 1024 && p.nt <= 6144; }
@@ -1537,7 +1634,18 @@ int launch_membrane(const DevParams& p, Membrane& m, const FastBufs& fb, uint64_
                     cudaStream_t st) {
   FastBufs f = fb;
   f.snap = snap_of(fb, s0, p.nv);
-  const int nc = segment_blocks(p, f);
+  if (wide_membrane(f)) {
+    eoff += (uint64_t)s0;
+    k_wide_first<<<wide_first_blocks(p), kWideT, 0, st>>>(p, m, f, parts);
+    for (int s = 0; s < H; ++s) {
+      k_wide_tri<<<wide_tri_blocks(p), kWideT, 0, st>>>(p, m, f);
+      k_wide_terms<<<wide_terms_blocks(p, parts), kSegT, wide_smem(p), st>>>(p, m, f, parts);
+      if (parts & SEG_SECOND)
+        k_wide_gather<<<wide_gather_blocks(p), kWideT, 0, st>>>(p, m, f, eoff, s, parts, s + 1 < H);
+    }
+    return 1 + H * ((parts & SEG_SECOND) ? 3 : 2);
+  }
+  const int nc = segment_blocks(f);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(nc);
   cfg.blockDim = dim3(kSegT);

@@ -27,6 +27,33 @@ def troph():
     return O.load_mesh_files(*O.troph_files())
 
 
+def geodesic(n, R):
+    """Geodesic sphere of radius R: 10 n^2 + 2 vertices, their edges and
+    triangles."""
+    from irbc_b200 import mesh
+    V0, F0 = mesh.icosphere(0)
+    ids, V, F = {}, [], []
+    for a, b, c in F0:
+        at = {}
+        for i in range(n + 1):
+            for j in range(n + 1 - i):
+                w = [(a, n - i - j), (b, i), (c, j)]
+                key = tuple(sorted(q for q in w if q[1]))
+                if key not in ids:
+                    ids[key] = len(V)
+                    v = sum(V0[q] * k for q, k in w)
+                    V.append(R * v / np.linalg.norm(v))
+                at[i, j] = ids[key]
+        for i in range(n):
+            for j in range(n - i):
+                F.append((at[i, j], at[i + 1, j], at[i, j + 1]))
+                if i + j < n - 1:
+                    F.append((at[i + 1, j], at[i + 1, j + 1], at[i, j + 1]))
+    V = np.array(V)
+    F = mesh.orient_outward(V, np.array(F, np.int32))
+    return V, mesh.edges_of(F), F
+
+
 def make_oracle(ns=40000, seed=11, onrate=0.005, offrate=0.015, nknobs=500, **over):
     op = O.default_params(Ns=ns, onrate=onrate, offrate=offrate, **over)
     orc = O.Oracle(op, seed)

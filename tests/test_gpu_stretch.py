@@ -50,6 +50,63 @@ def test_stretches_equal_single_steps(case, precision):
         assert H.compare(a.get_state(), b.get_state(), 0.0) == {}, n
 
 
+def _mesh_oracle(V, E, T, nknobs, **over):
+    """an oracle with a mesh of its own (elap scaled to it)"""
+    import oracle as O
+    from irbc_b200 import mesh
+    op = O.default_params(Nt=len(V), elap=mesh.scaled_elap(V, E), **over)
+    orc = O.Oracle(op, 43)
+    orc.init(V, E, T, nknobs)
+    return op, orc
+
+
+# the smallest geodesic mesh that no cluster holds in patches, the largest one
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("freq", [17, 28])
+def test_meshes_beyond_the_patches(freq, precision):
+    """Meshes above the patches' size run a kernel a phase: stretches, with
+    bonds, equal single steps, mode 3 (a cluster on global memory) and replayed
+    graphs bit for bit, and in FP64 the oracle step by step within 1e-12."""
+    V, E, T = H.geodesic(freq, 0.07 * np.sqrt(10.0 * freq * freq + 2))
+    op, orc = _mesh_oracle(V, E, T, 1500, Ns=30000, onrate=300.0, offrate=50.0, Lx=40.0, Ly=24.0, Lz=24.0)
+    st = orc.get_state()
+    sims = [H.gpu_like(op, orc, 43, precision=precision, state=st) for _ in range(4)]
+    sims[1].set_membrane_kernels(3)
+    sims[2].set_graphs(True)
+    for n in (3, 40):
+        for s in sims[:3]:
+            s.step(n)
+        for _ in range(n):
+            sims[3].call("step_part1")
+            sims[3].call("step_part2")
+        want = sims[3].get_state()
+        for k, s in enumerate(sims[:3]):
+            assert H.compare(s.get_state(), want, 0.0) == {}, (n, k)
+    assert sims[3].get_state().a["bondi"].sum() > 0
+    if precision == 1:  # members of a cohort, beside one in patches
+        import irbc_b200 as G
+        top, torc = H.make_oracle(ns=20000, seed=44, Lx=40.0, Ly=20.0)
+        b = G.Batch(nthreads=1)
+        members = [H.gpu_like(op, orc, 43, precision=1, state=st) for _ in range(2)]
+        members.append(H.gpu_like(top, torc, 44, precision=1))
+        alone = H.gpu_like(top, torc, 44, precision=1)
+        for s in members:
+            b.add(s)
+        for n in (3, 40):
+            b.step(n)
+            alone.step(n)
+        for s in members[:2]:
+            assert H.compare(s.get_state(), want, 0.0) == {}
+        assert H.compare(members[2].get_state(), alone.get_state(), 0.0) == {}
+        b.close()
+    else:
+        s = H.gpu_like(op, orc, 43, precision=0, state=st)
+        for k in range(4):
+            orc.step(1)
+            s.step(1)
+            assert H.compare(s.get_state(), orc.get_state()) == {}, k
+
+
 @pytest.mark.parametrize("precision", [0, 1])
 @pytest.mark.parametrize("Lz", [20.0, 300.0])  # layers in shared memory (256), beyond
 def test_layer_sums(Lz, precision):
