@@ -70,6 +70,7 @@ struct irbc_handle {
   bool capturing = false;
   std::string err;
   bool have_mesh = false;
+  void* mesh_mem = nullptr;        // the arrays of Membrane and FastBufs that a mesh sizes
   int64_t step = 0;
   int colsteps = -1, upd = 0, filecc = 0, filec = 0, bbi = 0;
   int csteps = 10, uplist = 83;
@@ -113,6 +114,29 @@ cudaError_t dalloc(T** p, int64_t n) {
   return cudaMalloc((void**)p, sizeof(T) * (size_t)n);
 }
 
+// Device arrays taken in one allocation.  A mesh sizes some sixty; one by one,
+// with the incidence lists made twice and the patches tried for eight blocks in
+// vain, irbc_init took 12.6 ms and irbc_destroy 3.7 with the discocyte in a 32^3
+// box, so 9.2 and 2.5 (600 vertices: 4.4 and 2.7, 3.4 and 2.1).
+struct Arrays {
+  std::vector<std::pair<void**, size_t>> want;
+  template <typename T>
+  void add(T** p, int64_t n) {
+    want.push_back({(void**)p, (sizeof(T) * (size_t)std::max<int64_t>(n, 1) + 255) / 256 * 256});
+  }
+  cudaError_t take(void** base) {
+    size_t total = 0;
+    for (auto& w : want) total += w.second;
+    cudaError_t e = cudaMalloc(base, total);
+    char* at = e == cudaSuccess ? (char*)*base : nullptr;
+    for (auto& w : want) {
+      *w.first = at;
+      if (at) at += w.second;
+    }
+    return e;
+  }
+};
+
 template <typename T>
 void dfree(T*& p) {
   if (p) cudaFree(p);
@@ -149,16 +173,6 @@ void build_ligands(irbc_handle* h) {
   h->dp.nligy = ny;
   h->dp.nlig = (int)h->xlig.size();
   h->dp.nligx = ny ? h->dp.nlig / ny : 0;
-}
-
-void free_membrane(Membrane& m) {
-  for (double** p : {&m.x, &m.y, &m.z, &m.vx, &m.vy, &m.vz, &m.fx, &m.fy, &m.fz, &m.poff, &m.pon, &m.l0,
-                     &m.kappap, &m.tarea, &m.area, &m.vol, &m.tcx, &m.tcy, &m.tcz, &m.pair_d})
-    dfree(*p);
-  for (int** p : {&m.pid, &m.ix, &m.iy, &m.bondi, &m.bondl, &m.knob, &m.e1, &m.e2, &m.es1, &m.es2, &m.iedge,
-                  &m.t1, &m.t2, &m.t3, &m.inc_start, &m.inc, &m.npair, &m.pair_j})
-    dfree(*p);
-  dfree(m.vkey);
 }
 
 inline void hcp(const double A[], const double B[], double C[]) {
@@ -245,33 +259,22 @@ void build_iedge(HostMesh& M, double Lx, double Ly, double Lz) {
 
 // per-vertex contribution lists in the order force_calculate_dt adds them
 void build_incidence(const HostMesh& M, std::vector<int>& start, std::vector<int>& inc) {
-  std::vector<std::vector<int>> L(M.nv);
-  auto enc = [](int kind, int role, int item) { return (kind << 30) | (role << 27) | item; };
-  for (int i = 0; i < M.ne; ++i) {
-    L[M.e1[i]].push_back(enc(0, 0, i));
-    L[M.e2[i]].push_back(enc(0, 1, i));
-  }
-  for (int i = 0; i < M.nt; ++i) {
-    L[M.t1[i]].push_back(enc(1, 0, i));
-    L[M.t2[i]].push_back(enc(1, 1, i));
-    L[M.t3[i]].push_back(enc(1, 2, i));
-  }
-  for (int i = 0; i < M.ne; ++i) {
-    int l2, l3;
-    if (M.iedge[i] == -1) { l3 = M.e1[i]; l2 = M.e2[i]; } else { l2 = M.e1[i]; l3 = M.e2[i]; }
-    int l1 = M.es1[i], l4 = M.es2[i];
-    L[l1].push_back(enc(2, 0, i));
-    L[l4].push_back(enc(2, 1, i));
-    L[l2].push_back(enc(2, 2, i));
-    L[l3].push_back(enc(2, 3, i));
-  }
+  // item by item (kind, role, item) to its vertices: once to count, once to place
+  auto each = [&](auto&& to) {
+    for (int i = 0; i < M.ne; ++i) { to(M.e1[i], 0, 0, i); to(M.e2[i], 0, 1, i); }
+    for (int i = 0; i < M.nt; ++i) { to(M.t1[i], 1, 0, i); to(M.t2[i], 1, 1, i); to(M.t3[i], 1, 2, i); }
+    for (int i = 0; i < M.ne; ++i) {
+      int l2, l3;
+      if (M.iedge[i] == -1) { l3 = M.e1[i]; l2 = M.e2[i]; } else { l2 = M.e1[i]; l3 = M.e2[i]; }
+      to(M.es1[i], 2, 0, i); to(M.es2[i], 2, 1, i); to(l2, 2, 2, i); to(l3, 2, 3, i);
+    }
+  };
   start.assign(M.nv + 1, 0);
-  inc.clear();
-  for (int v = 0; v < M.nv; ++v) {
-    start[v] = (int)inc.size();
-    inc.insert(inc.end(), L[v].begin(), L[v].end());
-  }
-  start[M.nv] = (int)inc.size();
+  each([&](int v, int, int, int) { start[v + 1] += 1; });
+  for (int v = 0; v < M.nv; ++v) start[v + 1] += start[v];
+  inc.resize(start[M.nv]);
+  std::vector<int> next(start.begin(), start.end() - 1);
+  each([&](int v, int kind, int role, int item) { inc[next[v]++] = (kind << 30) | (role << 27) | item; });
 }
 
 template <typename T>
@@ -293,17 +296,14 @@ int down(irbc_handle* h, T* v, const T* d, int64_t n) {
   return 0;
 }
 
-void free_fast(FastBufs& f) {
-  for (double** q : {&f.snap.x, &f.snap.y, &f.snap.z, &f.snap.vx, &f.snap.vy, &f.snap.vz, &f.slot, &f.a4, &f.fac,
-                     &f.ux, &f.uy, &f.vX, &f.vS})
-    dfree(*q);
-  for (int** q : {&f.gstart, &f.gidx, &f.vd, &f.pidx, &f.st1, &f.st2, &f.st3}) dfree(*q);
-  dfree(f.pre);
-  dfree(f.bands);
-  dfree(f.cull);
-  dfree(f.patch.hdr);
-  dfree(f.patch.blob);
-  f.patch = PatchPlan{};
+// the device memory of a mesh; the pointers into it are left behind
+void free_mesh(irbc_handle* h) {
+  h->have_mesh = false;
+  if (h->mesh_mem) cudaFree(h->mesh_mem);
+  h->mesh_mem = nullptr;
+  dfree(h->fb.patch.hdr);
+  dfree(h->fb.patch.blob);
+  h->fb.patch = PatchPlan{};
 }
 
 // per-vertex force slots in the order force_calculate_dt adds the terms:
@@ -343,21 +343,26 @@ void build_gather(const HostMesh& M, const std::vector<int>& start, const std::v
 // the mesh allows it: each half of a bisection is the nearer half, by edges,
 // to a vertex far from the others; w: the runs' weights, cap: the most vertices
 // of each, where all of them fit
-void bisect(const std::vector<std::vector<int>>& nb, std::vector<int>& v, size_t lo, size_t hi,
-            const std::vector<double>& w, const std::vector<size_t>& cap, size_t p0, size_t p1,
-            std::vector<size_t>& cut) {
+struct Neighbours {
+  std::vector<int> start, of;  // vertex v's: of[start[v]] to of[start[v + 1] - 1]
+};
+void bisect(const Neighbours& nb, std::vector<int>& v, size_t lo, size_t hi, const std::vector<double>& w,
+            const std::vector<size_t>& cap, size_t p0, size_t p1, std::vector<size_t>& cut) {
   if (p1 - p0 < 2) return;
-  std::vector<int> at(nb.size(), -1);
+  std::vector<int> at(nb.start.size() - 1, -1);
   auto bfs = [&](int from) {
     for (size_t q = lo; q < hi; ++q) at[v[q]] = 0;  // 0: in this set, not reached
     std::vector<int> out;
+    out.reserve(hi - lo);
     size_t next = lo;
     for (int start = from; out.size() < hi - lo;) {
       at[start] = 1;
       out.push_back(start);
       for (size_t q = out.size() - 1; q < out.size(); ++q)
-        for (int u : nb[out[q]])
+        for (int e = nb.start[out[q]]; e < nb.start[out[q] + 1]; ++e) {
+          const int u = nb.of[e];
           if (at[u] == 0) { at[u] = 1; out.push_back(u); }
+        }
       while (next < hi && at[v[next]] != 0) ++next;  // a part of its own
       if (next < hi) start = v[next];
     }
@@ -387,6 +392,12 @@ void bisect(const std::vector<std::vector<int>>& nb, std::vector<int>& v, size_t
 // its patch.  own: the vertices in patch order.
 bool build_patches(const HostMesh& M, const std::vector<int>& start, const std::vector<int>& inc, int nc, bool tree,
                    PatchPlan& P, std::vector<PatchHdr>& hdr, std::vector<unsigned char>& blob, std::vector<int>& own) {
+  // what the blocks hold at least, each item and entry once (patch_layout); too
+  // much for nc of them: no need to try
+  const size_t least = M.nt * (sizeof(PatchTri) + 3 * 8 * sizeof(double)) +
+                       M.ne * (sizeof(PatchEdge) + 7 * sizeof(double) + sizeof(PatchDih) + 4 * 3 * sizeof(double)) +
+                       M.nv * (6 * sizeof(double) + 3 * sizeof(int)) + seg_terms(M.nt) * 2 * sizeof(double);
+  if (least > (size_t)nc * kSegSmemMax) return false;
   // The summing warps: in reference order the sums take half of two blocks'
   // warps, the warp tree one of four (the others for the tail); those blocks'
   // patches are smaller by as much (and by the room that many terms take; block
@@ -401,8 +412,15 @@ bool build_patches(const HostMesh& M, const std::vector<int>& start, const std::
   w[1] = tree && M.nt <= 2048 ? 0.85 : 0.62;
   std::vector<size_t> cap(nc, kSegT / 3);
   cap[0] = (kSegT - 32 * P.sw) / 3;
-  std::vector<std::vector<int>> nb(M.nv);
-  for (int i = 0; i < M.ne; ++i) { nb[M.e1[i]].push_back(M.e2[i]); nb[M.e2[i]].push_back(M.e1[i]); }
+  Neighbours nb;
+  nb.start.assign(M.nv + 1, 0);
+  nb.of.resize(2 * (size_t)M.ne);
+  for (int i = 0; i < M.ne; ++i) { nb.start[M.e1[i] + 1] += 1; nb.start[M.e2[i] + 1] += 1; }
+  for (int v = 0; v < M.nv; ++v) nb.start[v + 1] += nb.start[v];
+  {
+    std::vector<int> next(nb.start.begin(), nb.start.end() - 1);
+    for (int i = 0; i < M.ne; ++i) { nb.of[next[M.e1[i]]++] = M.e2[i]; nb.of[next[M.e2[i]]++] = M.e1[i]; }
+  }
   own.resize(M.nv);
   for (int v = 0; v < M.nv; ++v) own[v] = v;
   std::vector<size_t> cut(nc + 1, 0);
@@ -423,20 +441,32 @@ bool build_patches(const HostMesh& M, const std::vector<int>& start, const std::
     std::vector<PatchSend> send;
   };
   std::vector<Tables> tab(nc);
+  // where a block has put a vertex or an item: in[] the block, at[] the place
+  struct Places {
+    std::vector<int> in, at;
+    explicit Places(size_t n) : in(n, -1), at(n) {}
+    bool has(int i, int b) const { return in[i] == b; }
+    void set(int i, int b, int p) { in[i] = b; at[i] = p; }
+  };
+  Places slot(M.nv), it(M.ne), itt(M.nt), itd(M.ne);
   for (int b = 0; b < nc; ++b) {
     PatchHdr& h = hdr[b];
     Tables& t = tab[b];
     h.base = (int)cut[b];
     h.no = (int)(cut[b + 1] - cut[b]);
-    std::vector<int> slot(M.nv, -1), it(M.ne, -1), itt(M.nt, -1), itd(M.ne, -1);
+    t.ent.reserve(3 * (size_t)h.no + 3);
+    t.eend.reserve(7 * (size_t)h.no);
+    t.edge.reserve(5 * (size_t)h.no);
+    t.tri.reserve(4 * (size_t)h.no);
+    t.dih.reserve(8 * (size_t)h.no);
     int nl = h.no;
     auto local = [&](int v) -> unsigned short {
       if (owner[v] == b) return (unsigned short)place[v];
-      if (slot[v] < 0) {
-        slot[v] = nl++;
-        tab[owner[v]].send.push_back({(unsigned short)place[v], (unsigned short)slot[v], (unsigned short)b, 0});
+      if (!slot.has(v, b)) {
+        slot.set(v, b, nl++);
+        tab[owner[v]].send.push_back({(unsigned short)place[v], (unsigned short)slot.at[v], (unsigned short)b, 0});
       }
-      return (unsigned short)slot[v];
+      return (unsigned short)slot.at[v];
     };
     int ne = 0, nt = 0, nd = 0;
     for (int q = 0; q < h.no; ++q) {
@@ -447,28 +477,28 @@ bool build_patches(const HostMesh& M, const std::vector<int>& start, const std::
       for (int u = start[v]; u < start[v + 1]; ++u) {
         const int e = inc[u], kind = (e >> 30) & 3, role = (e >> 27) & 7, item = e & ((1 << 27) - 1);
         if (kind == 0) {
-          if (it[item] < 0) {
-            it[item] = (int)t.edge.size();
+          if (!it.has(item, b)) {
+            it.set(item, b, (int)t.edge.size());
             t.edge.push_back({{local(M.e1[item]), local(M.e2[item])}, {0, 0}, M.l0[item], M.kappap[item]});
           }
-          t.eend.push_back((unsigned short)(2 * it[item] + role));
+          t.eend.push_back((unsigned short)(2 * it.at[item] + role));
           ++ne;
         } else if (kind == 1) {
-          if (itt[item] < 0) {
-            itt[item] = (int)t.tri.size();
+          if (!itt.has(item, b)) {
+            itt.set(item, b, (int)t.tri.size());
             t.tri.push_back({{local(M.t1[item]), local(M.t2[item]), local(M.t3[item])}, {kNoEntry, kNoEntry, kNoEntry},
                              owner[M.t1[item]] == b ? item : -1, M.tarea[item]});
           }
-          t.tri[itt[item]].d[role] = (unsigned short)nt++;
+          t.tri[itt.at[item]].d[role] = (unsigned short)nt++;
         } else {
-          if (itd[item] < 0) {
+          if (!itd.has(item, b)) {
             int l2, l3;
             if (M.iedge[item] == -1) { l3 = M.e1[item]; l2 = M.e2[item]; } else { l2 = M.e1[item]; l3 = M.e2[item]; }
-            itd[item] = (int)t.dih.size();
+            itd.set(item, b, (int)t.dih.size());
             t.dih.push_back({{local(M.es1[item]), local(M.es2[item]), local(l2), local(l3)},
                              {kNoEntry, kNoEntry, kNoEntry, kNoEntry}});
           }
-          t.dih[itd[item]].d[role] = (unsigned short)nd++;
+          t.dih[itd.at[item]].d[role] = (unsigned short)nd++;
         }
       }
     }
@@ -478,6 +508,11 @@ bool build_patches(const HostMesh& M, const std::vector<int>& start, const std::
     h.ne = ne; h.nt = nt; h.nd = nd;
     P.nl = std::max(P.nl, nl);
   }
+  size_t bytes = 0;
+  for (const Tables& t : tab)
+    bytes += sizeof(PatchTri) * t.tri.size() + sizeof(PatchEdge) * t.edge.size() + sizeof(PatchDih) * t.dih.size() +
+             sizeof(unsigned short) * (t.ent.size() + t.eend.size()) + sizeof(PatchSend) * t.send.size() + 7 * 16;
+  blob.reserve(bytes + sizeof(int) * M.nv);
   for (int b = 0; b < nc; ++b) {
     PatchHdr& h = hdr[b];
     const Tables& t = tab[b];
@@ -505,16 +540,15 @@ bool build_patches(const HostMesh& M, const std::vector<int>& start, const std::
 // the patches of the handle's mesh and membrane form; without them (one or
 // eight blocks asked for, or a mesh that does not fit) the snapshots keep the
 // vertices' order
-int upload_patches(irbc_handle* h) {
+int upload_patches(irbc_handle* h, const std::vector<int>& start, const std::vector<int>& inc) {
   FastBufs& f = h->fb;
   const HostMesh& M = h->host_mesh;
   dfree(f.patch.hdr);
   dfree(f.patch.blob);
   f.patch = PatchPlan{};
-  std::vector<int> start, inc, own(M.nv);
+  std::vector<int> own(M.nv);
   for (int v = 0; v < M.nv; ++v) own[v] = v;
   if (h->mem_mode == 1) {
-    build_incidence(M, start, inc);
     // eight blocks, or sixteen (a non-portable size) where eight do not hold
     // their patches and the device can run such a cluster.  Fewer blocks than
     // eight take two rounds of items a phase: 21 against 15 us a step on the
@@ -549,48 +583,44 @@ int upload_mesh(irbc_handle* h, const HostMesh& M) {
   Membrane& m = h->m;
   if (M.nv > 8192) return fail(h, IRBC_ERR_ARG, "at most 8192 membrane vertices");
   invalidate_graphs(h);
-  free_membrane(m);
-  free_fast(h->fb);
+  free_mesh(h);
   m.nv = M.nv; m.ne = M.ne; m.nt = M.nt;
-  for (double** p : {&m.x, &m.y, &m.z, &m.vx, &m.vy, &m.vz, &m.fx, &m.fy, &m.fz, &m.poff, &m.pon})
-    CK(dalloc(p, M.nv));
-  for (int** p : {&m.pid, &m.ix, &m.iy, &m.bondi, &m.bondl, &m.knob, &m.npair}) CK(dalloc(p, M.nv));
-  CK(dalloc(&m.vkey, M.nv));
-  CK(dalloc(&m.pair_d, (int64_t)M.nv * kMaxPairs));
-  CK(dalloc(&m.pair_j, (int64_t)M.nv * kMaxPairs));
-  for (int** p : {&m.e1, &m.e2, &m.es1, &m.es2, &m.iedge}) CK(dalloc(p, M.ne));
-  for (double** p : {&m.l0, &m.kappap}) CK(dalloc(p, M.ne));
-  for (int** p : {&m.t1, &m.t2, &m.t3}) CK(dalloc(p, M.nt));
-  for (double** p : {&m.tarea, &m.area, &m.vol, &m.tcx, &m.tcy, &m.tcz}) CK(dalloc(p, M.nt));
-  std::vector<int> start, inc;
+  std::vector<int> start, inc, gstart, gidx;
   build_incidence(M, start, inc);
-  CK(dalloc(&m.inc_start, M.nv + 1));
-  CK(dalloc(&m.inc, (int64_t)inc.size()));
-  if (up(h, m.inc_start, start) || up(h, m.inc, inc)) return IRBC_ERR_CUDA;
+  build_gather(M, start, inc, gstart, gidx);
+  FastBufs& f = h->fb;
   {
-    FastBufs& f = h->fb;
+    Arrays A;
+    for (double** p : {&m.x, &m.y, &m.z, &m.vx, &m.vy, &m.vz, &m.fx, &m.fy, &m.fz, &m.poff, &m.pon}) A.add(p, M.nv);
+    for (int** p : {&m.pid, &m.ix, &m.iy, &m.bondi, &m.bondl, &m.knob, &m.npair}) A.add(p, M.nv);
+    A.add(&m.vkey, M.nv);
+    A.add(&m.pair_d, (int64_t)M.nv * kMaxPairs);
+    A.add(&m.pair_j, (int64_t)M.nv * kMaxPairs);
+    for (int** p : {&m.e1, &m.e2, &m.es1, &m.es2, &m.iedge}) A.add(p, M.ne);
+    for (double** p : {&m.l0, &m.kappap}) A.add(p, M.ne);
+    for (int** p : {&m.t1, &m.t2, &m.t3}) A.add(p, M.nt);
+    for (double** p : {&m.tarea, &m.area, &m.vol, &m.tcx, &m.tcy, &m.tcz}) A.add(p, M.nt);
+    A.add(&m.inc_start, M.nv + 1);
+    A.add(&m.inc, (int64_t)inc.size());
     for (double** q : {&f.snap.x, &f.snap.y, &f.snap.z, &f.snap.vx, &f.snap.vy, &f.snap.vz})
-      CK(dalloc(q, (int64_t)kSegMax * M.nv));
-    CK(dalloc(&f.pre, (int64_t)kSegMax * M.nt));
-    CK(dalloc(&f.bands, (int64_t)kSegMax * M.nt));
-    CK(dalloc(&f.cull, 6 * (int64_t)M.nt));
-    CK(dalloc(&f.pidx, M.nv));
-    for (int** q : {&f.st1, &f.st2, &f.st3}) CK(dalloc(q, M.nt));
-    f.snap.t1 = f.st1; f.snap.t2 = f.st2; f.snap.t3 = f.st3;
-    std::vector<int> gstart, gidx;
-    build_gather(M, start, inc, gstart, gidx);
-    CK(dalloc(&f.slot, 3 * (int64_t)(8 * M.ne + 9 * M.nt)));
-    CK(dalloc(&f.a4, M.nt));
-    CK(dalloc(&f.fac, 2));
-    CK(dalloc(&f.ux, M.nv));
-    CK(dalloc(&f.uy, M.nv));
-    CK(dalloc(&f.vS, 3 * (int64_t)M.nv));
-    CK(dalloc(&f.gstart, 3 * (int64_t)M.nv + 1));
-    CK(dalloc(&f.gidx, (int64_t)gidx.size()));
-    CK(dalloc(&f.vd, M.nv));
-    CK(dalloc(&f.vX, 3 * (int64_t)M.nv));
-    if (up(h, f.gstart, gstart) || up(h, f.gidx, gidx)) return IRBC_ERR_CUDA;
+      A.add(q, (int64_t)kSegMax * M.nv);
+    A.add(&f.pre, (int64_t)kSegMax * M.nt);
+    A.add(&f.bands, (int64_t)kSegMax * M.nt);
+    A.add(&f.cull, 6 * (int64_t)M.nt);
+    for (int** q : {&f.pidx, &f.vd}) A.add(q, M.nv);
+    for (int** q : {&f.st1, &f.st2, &f.st3}) A.add(q, M.nt);
+    A.add(&f.slot, 3 * (int64_t)(8 * M.ne + 9 * M.nt));
+    A.add(&f.a4, M.nt);
+    A.add(&f.fac, 2);
+    for (double** q : {&f.ux, &f.uy}) A.add(q, M.nv);
+    for (double** q : {&f.vS, &f.vX}) A.add(q, 3 * (int64_t)M.nv);
+    A.add(&f.gstart, 3 * (int64_t)M.nv + 1);
+    A.add(&f.gidx, (int64_t)gidx.size());
+    CK(A.take(&h->mesh_mem));
   }
+  f.snap.t1 = f.st1; f.snap.t2 = f.st2; f.snap.t3 = f.st3;
+  if (up(h, m.inc_start, start) || up(h, m.inc, inc) || up(h, f.gstart, gstart) || up(h, f.gidx, gidx))
+    return IRBC_ERR_CUDA;
   if (up(h, m.e1, M.e1) || up(h, m.e2, M.e2) || up(h, m.es1, M.es1) || up(h, m.es2, M.es2) ||
       up(h, m.iedge, M.iedge) || up(h, m.l0, M.l0) || up(h, m.kappap, M.kappap) || up(h, m.t1, M.t1) ||
       up(h, m.t2, M.t2) || up(h, m.t3, M.t3) || up(h, m.tarea, M.tarea))
@@ -605,7 +635,7 @@ int upload_mesh(irbc_handle* h, const HostMesh& M) {
   h->host_mesh = M;
   h->fb.one_block = h->mem_mode == 2 && one_block_fits(h->dp);
   h->fb.cluster = h->mem_mode == 3;
-  const int rc = upload_patches(h);
+  const int rc = upload_patches(h, start, inc);
   if (rc) return rc;
   h->have_mesh = true;
   return 0;
@@ -867,7 +897,7 @@ extern "C" void irbc_destroy(irbc_handle* h) {
   if (h->st) cudaStreamSynchronize(h->st);
   if (h->st2_own) cudaStreamSynchronize(h->st2_own);
   invalidate_graphs(h);
-  free_fast(h->fb);
+  free_mesh(h);
   dfree(h->fb.queue); dfree(h->fb.qk); dfree(h->c.flag); dfree(h->fb.qn);
   if (h->rec) cudaFree(h->rec);
   for (float4** q : {&h->sf.pos, &h->sf.vel, &h->sf.pos2, &h->sf.vel2}) dfree(*q);
@@ -887,7 +917,6 @@ extern "C" void irbc_destroy(irbc_handle* h) {
                   &c.lstart2, &c.totals,
                   &c.scan_part, &c.lidx, &c.lidx2})
     dfree(*q);
-  free_membrane(h->m);
   dfree(h->m.ligi); dfree(h->m.xlig); dfree(h->m.ylig); dfree(h->ebase); dfree(h->m.sc); dfree(h->obs);
   for (cudaEvent_t e : h->ev_pool) cudaEventDestroy(e);
   if (h->ev_begin) cudaEventDestroy(h->ev_begin);
@@ -1668,7 +1697,9 @@ extern "C" int irbc_set_membrane_kernels(irbc_handle* h, int32_t mode) {
     invalidate_graphs(h);
     h->fb.one_block = ob;
     h->fb.cluster = cl;
-    return upload_patches(h);
+    std::vector<int> start, inc;
+    build_incidence(h->host_mesh, start, inc);
+    return upload_patches(h, start, inc);
   }
   return 0;
 }

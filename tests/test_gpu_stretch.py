@@ -108,6 +108,30 @@ def test_meshes_beyond_the_patches(freq, precision):
 
 
 @pytest.mark.parametrize("precision", [0, 1])
+def test_a_mesh_takes_another_ones_place(precision):
+    """Meshes set one after the other on one handle, in patches of 8 and 16
+    blocks and beyond them: each steps as on a handle of its own."""
+    import irbc_b200 as G
+    from irbc_b200 import mesh
+    box = dict(Ns=8000, Lx=40.0, Ly=20.0, Lz=20.0)
+    meshes = [H.troph(), mesh.discocyte(), H.geodesic(17, 3.0), H.geodesic(2, 3.0)]
+    sim = None
+    for V, E, T in meshes + meshes[:1]:
+        op, orc = _mesh_oracle(V, E, T, 12, **box)
+        p = H.to_irbc_params(op, 43, precision)
+        if sim is None:
+            sim = G.Simulation(p)
+            p0 = p
+        alone = G.Simulation(p0)
+        for s in (sim, alone):  # (both with the first mesh's elap)
+            s.set_mesh(orc.get_mesh())
+            s.set_state(G.State.from_other(orc.get_state()))
+            s.step(25)
+        assert H.compare(sim.get_state(), alone.get_state(), 0.0) == {}, len(V)
+        alone.close()
+
+
+@pytest.mark.parametrize("precision", [0, 1])
 @pytest.mark.parametrize("Lz", [20.0, 300.0])  # layers in shared memory (256), beyond
 def test_layer_sums(Lz, precision):
     """Temperature, mean velocity and profiles against sums of the state in
