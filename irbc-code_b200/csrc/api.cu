@@ -681,8 +681,8 @@ int resort_any(irbc_handle* h, cudaStream_t st) {
   return h->s.n ? 2 : 0;
 }
 
-// returns the number of kernels launched: vbin, count, two scan kernels,
-// perm, cells, and the physical re-sort when due (never while
+// returns the number of kernels launched: vbin, count, the scan's, perm,
+// cells, and the physical re-sort when due (never while
 // a step sequence is being captured; irbc_step re-sorts between captured
 // sequences).  With a side stream the vertex binning runs there (after
 // whatever the side stream already holds: the membrane of the previous
@@ -698,9 +698,8 @@ int collide_any(irbc_handle* h, uint64_t epoch, cudaStream_t st, cudaStream_t si
     cudaEventRecord(h->ev_vbin, side);
     cudaStreamWaitEvent(st, h->ev_vbin, 0);
   }
-  if (h->fp32) launch_collide_finish_f(h->dp, h->sf, h->s, h->c, h->m, epoch, st, resort);
-  else launch_collide_finish(h->dp, h->s, h->c, h->m, epoch, st, resort);
-  return 6 + (resort && h->s.n ? 2 : 0);
+  if (h->fp32) return 2 + launch_collide_finish_f(h->dp, h->sf, h->s, h->c, h->m, epoch, st, resort);
+  return 2 + launch_collide_finish(h->dp, h->s, h->c, h->m, epoch, st, resort);
 }
 
 // profiling: a pair of events around a launch group of a category
@@ -847,8 +846,7 @@ extern "C" int irbc_create(const irbc_params* p, irbc_handle** out) {
   A(dalloc(&c.lstart, c.n + 1));
   A(dalloc(&c.lstart2, c.n + 1));
   A(dalloc(&c.totals, 12));
-  c.scan_blocks = scan_part_blocks(c.n + 1);
-  A(dalloc(&c.scan_part, c.scan_blocks * 3 + 3));
+  A(dalloc(&c.scan_part, scan_part_ints(c.n)));
   c.lcap = c.lcap2 = std::max<int64_t>(1024, c.n / 16);
   A(dalloc(&c.lidx, c.lcap));
   A(dalloc(&c.lidx2, c.lcap2));
@@ -964,7 +962,7 @@ static int refresh_listed(irbc_handle* h) {
 static int do_llist(irbc_handle* h) {
   Cells& c = h->c;
   int64_t need = launch_llist_count(h->dp, c, h->m, h->st);
-  g_launches += 2 + 2;
+  g_launches += scan_groups(c.n) > 0 ? 5 : 4;
   if (need > c.lcap2) {
     dfree(c.lidx2);
     c.lcap2 = need + need / 4 + 1024;
@@ -1249,8 +1247,8 @@ extern "C" int irbc_set_state(irbc_handle* h, const irbc_view* v) {
     }
     // list starts: the lengths scanned on the device
     if (up(h, c.lcnt, v->llen, c.n) || up(h, c.lidx, v->lidx, tot)) return IRBC_ERR_CUDA;
-    launch_scan3(c.lcnt, nullptr, nullptr, c.lstart, nullptr, nullptr, c.totals + 8, c.n, c.scan_part, h->st, true);
-    g_launches += 2;
+    g_launches +=
+        launch_scan3(c.lcnt, nullptr, nullptr, c.lstart, nullptr, nullptr, c.totals + 8, c.n, c.scan_part, h->st, true);
     int rc = refresh_listed(h);
     if (rc) return rc;
   }
@@ -2123,13 +2121,13 @@ extern "C" int irbc_bin_particles(const irbc_params* p, const double* x, const d
   // the scan's block sums lie in order, which is written after them, or where
   // there are fewer particles in memory of their own (allocating and freeing the
   // counters, places and sums of 5.2 M particles took 0.7 ms of 2 ms)
-  const int64_t np = 3 * scan_part_blocks(d.ncell);
+  const int64_t np = scan_part_ints(d.ncell);
   int* own = nullptr;
   cudaError_t e = cudaSuccess;
   if (n > 0 && n < np) e = dalloc(&own, np);
   if (e == cudaSuccess) {
     bin_particles(d, x, y, z, n, rx, ry, rz, cell, start, order, own ? own : order, 0);
-    g_launches += n > 0 ? 5 : 0;
+    g_launches += n > 0 ? (scan_groups(d.ncell) > 0 ? 6 : 5) : 0;
     e = cudaStreamSynchronize(0);
   }
   dfree(own);

@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(256) k_bin_segsort(const int* start, int64_t n
   }
 }
 
-// The full sort; part: 3 scan_part_blocks(C) ints of scratch, which may be order.
+// The full sort; part: scan_part_ints(C) of scratch, which may be order.
 void bin_particles(const DevParams& p, const double* x, const double* y, const double* z, int64_t n,
                    double rx, double ry, double rz, int* cell, int* start, int* order, int* part, cudaStream_t st) {
   const unsigned nb = (unsigned)((n + 255) / 256);

@@ -20,6 +20,7 @@ namespace irbc {
 constexpr int64_t kNoAllocMaxCells = 1 << 20;                      // 1,048,576 cells
 constexpr int64_t kNoAllocScanBlocks = (kNoAllocMaxCells + 1024) / 1024 + 1;  // scan tiles of 1024
 constexpr int64_t kNoAllocInts = 3 * kNoAllocScanBlocks;
+static_assert(kNoAllocScanBlocks <= kScanLook, "no room for the sums of groups");
 
 // 3 ints per scan tile
 static __device__ __align__(256) int g_bin_scratch[kNoAllocInts];

@@ -116,12 +116,13 @@ void launch_collide_count_f(const DevParams& p, SolventF& f, Solvent& s, Cells& 
 
 // per-cell statistics (sums in double, reference particle order) and the
 // float rotation: k_cells_tile<true> (cells_tile.cuh)
-void launch_collide_finish_f(const DevParams& p, SolventF& f, Solvent& s, Cells& c, Membrane& m, uint64_t epoch,
-                             cudaStream_t st, bool resort) {
-  launch_collide_scan(p, c, m, st);
+int launch_collide_finish_f(const DevParams& p, SolventF& f, Solvent& s, Cells& c, Membrane& m, uint64_t epoch,
+                            cudaStream_t st, bool resort) {
+  const int scans = launch_collide_scan(p, c, m, st);
   if (f.n) k_perm_f<<<nbf(f.n, 256), 256, 0, st>>>(f.pid, s.slot, c.start, f.n, s.perm);
   k_cells_tile<true><<<cells_tile_blocks(c.n), 32 * kTileWarps, 0, st>>>(p, s, f, c, m, epoch);
   if (resort) launch_resort_f(f, s, st);
+  return scans + 1 + (f.n ? (resort ? 3 : 1) : 0);
 }
 
 void launch_resort_f(SolventF& f, Solvent& s, cudaStream_t st) {

@@ -17,7 +17,7 @@ void f32_from_f64(Solvent& s, SolventF& f, cudaStream_t st);
 void f32_to_f64(SolventF& f, Solvent& s, cudaStream_t st);
 void launch_collide_count_f(const DevParams& p, SolventF& f, Solvent& s, Cells& c, uint64_t epoch,
                             cudaStream_t st);
-void launch_collide_finish_f(const DevParams& p, SolventF& f, Solvent& s, Cells& c, Membrane& m, uint64_t epoch,
-                             cudaStream_t st, bool resort);
+int launch_collide_finish_f(const DevParams& p, SolventF& f, Solvent& s, Cells& c, Membrane& m, uint64_t epoch,
+                            cudaStream_t st, bool resort);
 void launch_resort_f(SolventF& f, Solvent& s, cudaStream_t st);
 }  // namespace irbc

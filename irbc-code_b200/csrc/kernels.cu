@@ -176,15 +176,25 @@ void launch_classify(const DevParams& p, Solvent& s, const Membrane& m, cudaStre
 // ================================================================ scan ======
 // Exclusive scan of up to three int arrays at once (null input = zeros):
 // per-block sums, then the per-block rescan, each block adding up the sums of
-// the blocks before it.  totals[k] receives the sum of array k, and so does the
-// entry behind oa's last one where `end` asks for it.
+// the blocks before it.  What that reads grows with the square of the blocks, so
+// above kScanLook of them a launch between the two scans the block sums in groups
+// of kScanTile, and a block adds up the groups before its own.  irbc_bin_particles
+// without and with that launch: 2048 blocks 188 and 192 us, 4096 258 and 260, 8192
+// 405 and 396, 16384 771 and 724, 131072 9.9 and 5.8 ms.  totals[k] receives the sum of array
+// k, and so does the entry behind oa's last one where `end` asks for it.
 constexpr int kScanT = 256, kScanItems = 4, kScanTile = kScanT * kScanItems;
 
 int64_t scan_part_blocks(int64_t n) { return (n + kScanTile - 1) / kScanTile; }
+// the launch between: its blocks, 0 where there is none
+int64_t scan_groups(int64_t n) {
+  const int64_t nb = scan_part_blocks(n);
+  return nb > kScanLook ? scan_part_blocks(nb) : 0;
+}
+int64_t scan_part_ints(int64_t n) { return 3 * (scan_part_blocks(n) + scan_groups(n)); }
 
 __device__ __forceinline__ int ld0(const int* a, int64_t i) { return a ? a[i] : 0; }
 
-// the block's sums of s[0..2] over its threads, in thread k < 3
+// the block's sums of s[0..2] over its threads
 __device__ __forceinline__ void block_sums3(const int s[3], int out[3]) {
   __shared__ int ws[3][kScanT / 32];
   for (int k = 0; k < 3; ++k) {
@@ -198,6 +208,23 @@ __device__ __forceinline__ void block_sums3(const int s[3], int out[3]) {
     for (int q = 0; q < kScanT / 32; ++q) t += ws[k][q];
     out[k] = t;
   }
+}
+// the sums of s[0..2] over the threads before this one
+__device__ __forceinline__ void block_scan3(const int s[3], int ex[3]) {
+  __shared__ int ws[3][kScanT / 32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (int k = 0; k < 3; ++k) {
+    int x = s[k];
+    for (int o = 1; o < 32; o <<= 1) {
+      int y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    if (lane == 31) ws[k][w] = x;
+    ex[k] = x - s[k];
+  }
+  __syncthreads();
+  for (int k = 0; k < 3; ++k)
+    for (int q = 0; q < w; ++q) ex[k] += ws[k][q];
 }
 // item(i, v): the three values at i
 template <class Item>
@@ -218,42 +245,50 @@ __global__ void __launch_bounds__(kScanT) k_scan_part(const int* a, const int* b
   scan_part_block(n, part, blockIdx.x, [&](int64_t i, int v[3]) { v[0] = ld0(a, i); v[1] = ld0(b, i); v[2] = ld0(c, i); });
 }
 
+// the nblk block sums of part scanned within groups of kScanTile; the groups'
+// sums behind them
+__device__ __forceinline__ void scan_sums_block(int* part, int64_t nblk, int64_t bid) {
+  const int64_t base = bid * kScanTile + threadIdx.x * kScanItems;
+  int v[kScanItems][3], s[3] = {0, 0, 0}, ex[3];
+  for (int q = 0; q < kScanItems; ++q)
+    for (int k = 0; k < 3; ++k) {
+      v[q][k] = base + q < nblk ? part[(base + q) * 3 + k] : 0;
+      s[k] += v[q][k];
+    }
+  block_scan3(s, ex);
+  if (threadIdx.x == kScanT - 1)
+    for (int k = 0; k < 3; ++k) part[(nblk + bid) * 3 + k] = ex[k] + s[k];
+  for (int q = 0; q < kScanItems; ++q)
+    for (int k = 0; k < 3; ++k) {
+      if (base + q < nblk) part[(base + q) * 3 + k] = ex[k];
+      ex[k] += v[q][k];
+    }
+}
+__global__ void __launch_bounds__(kScanT) k_scan_sums(int* part, int64_t nblk) { scan_sums_block(part, nblk, blockIdx.x); }
+
 __device__ __forceinline__ void scan_final_block(const int* a, const int* b, const int* c, int* oa, int* ob, int* oc,
                                                  int64_t n, const int* part, int64_t bid, int64_t nblk, int* totals,
                                                  int end) {
   // the sums of the blocks before this one
+  const bool grouped = nblk > kScanLook;
+  const int64_t first = grouped ? nblk : 0, last = grouped ? nblk + bid / kScanTile : bid;
   int before[3], mine[3] = {0, 0, 0};
-  for (int64_t q = threadIdx.x; q < bid; q += kScanT)
+  for (int64_t q = first + threadIdx.x; q < last; q += kScanT)
     for (int k = 0; k < 3; ++k) mine[k] += part[q * 3 + k];
   block_sums3(mine, before);
+  if (grouped)
+    for (int k = 0; k < 3; ++k) before[k] += part[bid * 3 + k];
   const int64_t base = bid * kScanTile + threadIdx.x * kScanItems;
   int loc[3][kScanItems];
   int s[3] = {0, 0, 0};
   for (int q = 0; q < kScanItems; ++q) {
     int64_t i = base + q;
-    int va = i < n ? ld0(a, i) : 0, vb = i < n ? ld0(b, i) : 0, vc = i < n ? ld0(c, i) : 0;
-    loc[0][q] = s[0]; loc[1][q] = s[1]; loc[2][q] = s[2];
-    s[0] += va; s[1] += vb; s[2] += vc;
+    int v[3] = {i < n ? ld0(a, i) : 0, i < n ? ld0(b, i) : 0, i < n ? ld0(c, i) : 0};
+    for (int k = 0; k < 3; ++k) { loc[k][q] = s[k]; s[k] += v[k]; }
   }
-  // exclusive scan of per-thread sums across the block
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  __shared__ int ws[3][kScanT / 32];
   int ex[3];
-  for (int k = 0; k < 3; ++k) {
-    int x = s[k];
-    for (int o = 1; o < 32; o <<= 1) {
-      int y = __shfl_up_sync(0xffffffffu, x, o);
-      if (lane >= o) x += y;
-    }
-    if (lane == 31) ws[k][w] = x;
-    ex[k] = x - s[k];
-  }
-  __syncthreads();
-  for (int k = 0; k < 3; ++k) {
-    int acc = 0;
-    for (int q = 0; q < w; ++q) acc += ws[k][q];
-    ex[k] += acc + before[k];
-  }
+  block_scan3(s, ex);
+  for (int k = 0; k < 3; ++k) ex[k] += before[k];
   for (int q = 0; q < kScanItems; ++q) {
     int64_t i = base + q;
     if (i < n) {
@@ -272,13 +307,21 @@ __global__ void __launch_bounds__(kScanT) k_scan_final(const int* a, const int* 
                                                        int* oc, int64_t n, const int* part, int* totals, int end) {
   scan_final_block(a, b, c, oa, ob, oc, n, part, blockIdx.x, gridDim.x, totals, end);
 }
+// what follows the block sums; returns the launches
+static int scan_finish(const int* a, const int* b, const int* c, int* oa, int* ob, int* oc, int64_t n, int* part,
+                       int* totals, int end, cudaStream_t st) {
+  const int64_t nb = scan_part_blocks(n), ng = scan_groups(n);
+  if (ng > 0) k_scan_sums<<<(unsigned)ng, kScanT, 0, st>>>(part, nb);
+  k_scan_final<<<(unsigned)nb, kScanT, 0, st>>>(a, b, c, oa, ob, oc, n, part, totals, end);
+  return ng > 0 ? 2 : 1;
+}
 
-void launch_scan3(const int* a, const int* b, const int* c, int* oa, int* ob, int* oc, int* totals,
-                  int64_t n, int* part, cudaStream_t st, bool end) {
+int launch_scan3(const int* a, const int* b, const int* c, int* oa, int* ob, int* oc, int* totals,
+                 int64_t n, int* part, cudaStream_t st, bool end) {
   int64_t nb = scan_part_blocks(n);
-  if (nb == 0) return;
+  if (nb == 0) return 0;
   k_scan_part<<<(unsigned)nb, kScanT, 0, st>>>(a, b, c, n, part);
-  k_scan_final<<<(unsigned)nb, kScanT, 0, st>>>(a, b, c, oa, ob, oc, n, part, totals, end ? 1 : 0);
+  return 1 + scan_finish(a, b, c, oa, ob, oc, n, part, totals, end ? 1 : 0, st);
 }
 
 // ============================================================== collide =====
@@ -385,10 +428,10 @@ __global__ void __launch_bounds__(kScanT) k_collide_part(DevParams p, const int*
   collide_part_block(p, cnt, ncm, sc, wflag, mflag, part, blockIdx.x);
 }
 // wrank/mrank hold the flags first, then their exclusive scans
-void launch_collide_scan(const DevParams& p, Cells& c, const Membrane& m, cudaStream_t st) {
+int launch_collide_scan(const DevParams& p, Cells& c, const Membrane& m, cudaStream_t st) {
   const unsigned nb = (unsigned)scan_part_blocks(c.n);
   k_collide_part<<<nb, kScanT, 0, st>>>(p, c.cnt, c.ncm, m.sc, c.wrank, c.mrank, c.scan_part);
-  k_scan_final<<<nb, kScanT, 0, st>>>(c.cnt, c.wrank, c.mrank, c.start, c.wrank, c.mrank, c.n, c.scan_part, c.totals, 1);
+  return 1 + scan_finish(c.cnt, c.wrank, c.mrank, c.start, c.wrank, c.mrank, c.n, c.scan_part, c.totals, 1, st);
 }
 
 // counting sort of particle indices: perm[start[cell] + slot] = i
@@ -430,12 +473,13 @@ void launch_collide_count(const DevParams& p, Solvent& s, Cells& c, uint64_t epo
   if (s.n) k_count<<<nblk(s.n, 256 * kCountPer), 256, 0, st>>>(p, s, c.cnt, epoch);
 }
 
-void launch_collide_finish(const DevParams& p, Solvent& s, Cells& c, Membrane& m, uint64_t epoch,
-                           cudaStream_t st, bool resort) {
-  launch_collide_scan(p, c, m, st);
+int launch_collide_finish(const DevParams& p, Solvent& s, Cells& c, Membrane& m, uint64_t epoch,
+                          cudaStream_t st, bool resort) {
+  const int scans = launch_collide_scan(p, c, m, st);
   if (s.n) k_perm<<<nblk(s.n, 256), 256, 0, st>>>(s.pid, s.slot, c.start, s.n, s.perm);
   k_cells_tile<false><<<cells_tile_blocks(c.n), 32 * kTileWarps, 0, st>>>(p, s, SolventF{}, c, m, epoch);
   if (resort) launch_resort(s, st);
+  return scans + 1 + (s.n ? (resort ? 3 : 1) : 0);
 }
 
 void launch_resort(Solvent& s, cudaStream_t st) {
@@ -1143,6 +1187,10 @@ __global__ void __launch_bounds__(kScanT) km_collide_part(Member* __restrict__ m
   KM_MEMBER;
   collide_part_block(M.p, M.c.cnt, M.c.ncm, M.m.sc, M.c.wrank, M.c.mrank, M.c.scan_part, b);
 }
+__global__ void __launch_bounds__(kScanT) km_scan_sums(Member* __restrict__ mem, const int2* __restrict__ tab) {
+  KM_MEMBER;
+  scan_sums_block(M.c.scan_part, (M.c.n + kScanTile - 1) / kScanTile, b);
+}
 __global__ void __launch_bounds__(kScanT) km_scan_final(Member* __restrict__ mem, const int2* __restrict__ tab) {
   KM_MEMBER;
   scan_final_block(M.c.cnt, M.c.wrank, M.c.mrank, M.c.start, M.c.wrank, M.c.mrank, M.c.n, M.c.scan_part, b,
@@ -1162,8 +1210,10 @@ int multi_collide_front(const MultiPlan& P, uint64_t eoff, cudaStream_t st) {
 
 int multi_collide_scan(const MultiPlan& P, cudaStream_t st) {
   km_collide_part<<<P.blocks[MP_SCAN], kScanT, 0, st>>>(P.mem, P.table(MP_SCAN));
+  const int sums = P.blocks[MP_SCAN_SUMS];
+  if (sums > 0) km_scan_sums<<<sums, kScanT, 0, st>>>(P.mem, P.table(MP_SCAN_SUMS));
   km_scan_final<<<P.blocks[MP_SCAN], kScanT, 0, st>>>(P.mem, P.table(MP_SCAN));
-  return 2;
+  return sums > 0 ? 3 : 2;
 }
 
 }  // namespace irbc

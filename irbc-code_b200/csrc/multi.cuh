@@ -218,6 +218,7 @@ void multi_blocks(const Member& M, int out[MP_NPHASE]) {
   out[MP_VBIN] = (int)nb(M.p.nv, 32);
   out[MP_COUNT] = (int)nbf(ns, 256 * kCountPer);
   out[MP_SCAN] = (int)scan_part_blocks(nc);
+  out[MP_SCAN_SUMS] = (int)scan_groups(nc);
   out[MP_PERM] = (int)nbf(ns, 256);
   out[MP_TILE] = (int)cells_tile_blocks(nc);
   out[MP_MOVE] = (int)nbf(ns, 256);

@@ -30,7 +30,7 @@ enum MultiPhase : int {
   MP_STREAM, MP_NEAR_SHORT, MP_NEAR_LONG,                         // streaming
   MP_MEMBRANE, MP_RECORDS,                                        // membrane of a stretch
   MP_WIDE_FIRST, MP_WIDE_TRI, MP_WIDE_TERMS, MP_WIDE_GATHER,      // ... of members without patches
-  MP_ZERO, MP_VBIN, MP_COUNT, MP_SCAN, MP_PERM, MP_TILE, MP_MOVE,  // collision
+  MP_ZERO, MP_VBIN, MP_COUNT, MP_SCAN, MP_SCAN_SUMS, MP_PERM, MP_TILE, MP_MOVE,  // collision
   MP_NPHASE
 };
 

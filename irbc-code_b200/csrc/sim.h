@@ -57,8 +57,7 @@ struct Cells {
   int64_t lcap = 0, lcap2 = 0;
   unsigned char* flag = nullptr;  // CF_* of each cell
   int lmax = 0;                 // (host) the longest list
-  int *scan_part = nullptr;     // scan scratch: 3 ints per block
-  int64_t scan_blocks = 0;
+  int *scan_part = nullptr;     // scan scratch (scan_part_ints)
 };
 
 // device scalars of the membrane / parasite (one small struct)
@@ -116,13 +115,14 @@ void launch_classify(const DevParams& p, Solvent& s, const Membrane& m, cudaStre
 void set_collide_kernel_limits();
 void launch_vbin(const DevParams& p, Membrane& m, Cells& c, uint64_t epoch, cudaStream_t st);
 void launch_collide_count(const DevParams& p, Solvent& s, Cells& c, uint64_t epoch, cudaStream_t st);
-// resort: also re-sort the arrays physically by this collision's cells
-void launch_collide_finish(const DevParams& p, Solvent& s, Cells& c, Membrane& m, uint64_t epoch,
-                           cudaStream_t st, bool resort);
+// resort: also re-sort the arrays physically by this collision's cells; returns
+// the kernels launched
+int launch_collide_finish(const DevParams& p, Solvent& s, Cells& c, Membrane& m, uint64_t epoch,
+                          cudaStream_t st, bool resort);
 // physical re-sort by the cells of the latest collision (any time after it)
 void launch_resort(Solvent& s, cudaStream_t st);
-// the collision's scans over the cells (counts and ghost flags)
-void launch_collide_scan(const DevParams& p, Cells& c, const Membrane& m, cudaStream_t st);
+// the collision's scans over the cells (counts and ghost flags); returns the kernels launched
+int launch_collide_scan(const DevParams& p, Cells& c, const Membrane& m, cudaStream_t st);
 // returns the total list length the update needs (host sync inside)
 int64_t launch_llist_count(const DevParams& p, Cells& c, const Membrane& m, cudaStream_t st);
 // total: the entry count launch_llist_count returned (both list buffers hold it)
@@ -140,14 +140,19 @@ void launch_kick2(const DevParams& p, Membrane& m, cudaStream_t st);
 // the counting sort of particles by shifted cell (binning.cu)
 void bin_particles(const DevParams& p, const double* x, const double* y, const double* z, int64_t n, double rx,
                    double ry, double rz, int* cell, int* start, int* order, int* part, cudaStream_t st);
-// end: oa[n] receives the total too
-void launch_scan3(const int* a, const int* b, const int* c, int* oa, int* ob, int* oc, int* totals,
-                  int64_t n, int* part, cudaStream_t st, bool end = false);
+// end: oa[n] receives the total too; part: scan_part_ints(n) of scratch.  Returns the kernels launched
+int launch_scan3(const int* a, const int* b, const int* c, int* oa, int* ob, int* oc, int* totals,
+                 int64_t n, int* part, cudaStream_t st, bool end = false);
 // sf: the FP32-bulk solvent, or null.  obs: the kObsDoubles scratch; nbins > 0 also fills the velocity profile
 // (obs + 64, nbins <= kObsMaxBins)
 void launch_observables(const DevParams& p, const Solvent& s, const SolventF* sf, const Membrane& m, double* obs,
                         int nbins, cudaStream_t st);
 
+// the scans' blocks, the most of them that go without a launch between (kScanLook:
+// kernels.cu, "scan"), that launch's, and the scratch of both
+constexpr int kScanLook = 4096;
 int64_t scan_part_blocks(int64_t n);
+int64_t scan_groups(int64_t n);
+int64_t scan_part_ints(int64_t n);
 
 }  // namespace irbc

@@ -161,10 +161,35 @@ def test_layer_sums(Lz, precision):
         assert (np.abs(sim.velocity_profile(bins) - want) <= bound).all(), bins
 
 
-@pytest.mark.parametrize("box", [(16, 16, 3), (31, 11, 2), (41, 5, 4), (3, 1, 1), (128, 128, 64)])
+def test_collisions_above_4096_tiles():
+    """Two collisions in a box of 4128 tiles (three arrays in one scan) against
+    the oracle, and a cohort of two such members against one alone."""
+    import irbc_b200 as G
+    V, E, T = H.geodesic(2, 3.0)
+    op, orc = _mesh_oracle(V, E, T, 12, Ns=20000, Lx=129.0, Ly=128.0, Lz=255.0, dtcd=0.004)
+    st = orc.get_state()
+    sim = H.gpu_like(op, orc, 43, state=st)
+    alone, *members = [H.gpu_like(op, orc, 43, precision=1, state=st) for _ in range(3)]
+    orc.step(4)
+    sim.step(4)
+    assert H.compare(sim.get_state(), orc.get_state()) == {}
+    b = G.Batch(nthreads=1)
+    for s in members:
+        b.add(s)
+    b.step(4)
+    alone.step(4)
+    for s in members:
+        assert H.compare(s.get_state(), alone.get_state(), 0.0) == {}
+    b.close()
+
+
+@pytest.mark.parametrize("box", [(16, 16, 3), (31, 11, 2), (41, 5, 4), (3, 1, 1), (128, 128, 64),
+                                 (128, 128, 255), (129, 128, 255)])
 def test_cell_scan_at_tile_edges(box):
     """Counting sorts over 1024, 1023, 1025, 6 and 1,064,960 cells (a tile of
-    the scan has 1024 cells; 1040 tiles are more than a block's threads)."""
+    the scan has 1024 cells; 1040 tiles are more than a block's threads), over
+    4096 tiles, the most that go without a launch for the tiles' sums, and over
+    4128, whose sums are scanned in groups of 1024."""
     import torch
     import irbc_b200 as G
     Lx, Ly, Lz = box
