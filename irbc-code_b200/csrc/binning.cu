@@ -54,6 +54,14 @@ __global__ void __launch_bounds__(256) k_bin_place(const int* cell, int64_t n, i
   if (c >= 0) order[at] = (int)i;
 }
 
+__device__ __forceinline__ void insertion_sort(int* a, int m) {
+  for (int q = 1; q < m; ++q) {
+    const int v = a[q];
+    int r = q;
+    while (r > 0 && a[r - 1] > v) { a[r] = a[r - 1]; --r; }
+    a[r] = v;
+  }
+}
 // Ascending particle index within each cell, by sixteen lanes: each holds up to
 // kSortPer of the cell's entries and counts the smaller ones.  Fuller cells are
 // sorted by insertion by one lane.  5.2 M particles, ten a cell: 55 us; with the
@@ -99,14 +107,21 @@ __global__ void __launch_bounds__(256) k_bin_segsort(const int* start, int64_t n
       if (q * kSortLanes + lane < m) a[r[q]] = v[q];
     return;
   }
-  if (lane != 0) return;
-  for (int q = 1; q < m; ++q) {
-    const int v = a[q];
-    int r = q;
-    while (r > 0 && a[r - 1] > v) { a[r] = a[r - 1]; --r; }
-    a[r] = v;
-  }
+  if (lane == 0) insertion_sort(a, m);
 }
+// The same by a thread per cell, for cells with few entries, where most of sixteen
+// lanes have none.  The whole call, sixteen lanes and this: 134 M cells with 2 M
+// particles 5.9 and 1.3 ms, 0.5 M cells with 1, 2 and 4 a cell 81 and 59, 97 and
+// 69, 120 and 94 us; 65,000 cells with 4 and 8 a cell 54 and 55, 60 and 66.  More a
+// cell depends on their order (5.2 M particles, ten a cell: in cell order 164 and
+// 194 us, in no order 199 and 181).
+__global__ void __launch_bounds__(256) k_bin_segsort_sparse(const int* start, int64_t ncell, int* order) {
+  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= ncell) return;
+  const int s0 = start[c];
+  insertion_sort(order + s0, start[c + 1] - s0);
+}
+constexpr int kSparse = 4;  // particles a cell
 
 // The full sort; part: scan_part_ints(C) of scratch, which may be order.
 void bin_particles(const DevParams& p, const double* x, const double* y, const double* z, int64_t n,
@@ -121,7 +136,10 @@ void bin_particles(const DevParams& p, const double* x, const double* y, const d
   k_bin_count<<<nb, 256, 0, st>>>(p, x, y, z, n, rx, ry, rz, cell, start + 1);
   launch_scan3(start + 1, nullptr, nullptr, start + 1, nullptr, nullptr, nullptr, p.ncell, part, st);
   k_bin_place<<<nb, 256, 0, st>>>(cell, n, start + 1, order);
-  k_bin_segsort<<<(unsigned)((p.ncell * kSortLanes + 255) / 256), 256, 0, st>>>(start, p.ncell, order);
+  if (n < kSparse * p.ncell)
+    k_bin_segsort_sparse<<<(unsigned)((p.ncell + 255) / 256), 256, 0, st>>>(start, p.ncell, order);
+  else
+    k_bin_segsort<<<(unsigned)((p.ncell * kSortLanes + 255) / 256), 256, 0, st>>>(start, p.ncell, order);
 }
 
 }  // namespace irbc

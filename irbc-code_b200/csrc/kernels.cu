@@ -179,7 +179,7 @@ void launch_classify(const DevParams& p, Solvent& s, const Membrane& m, cudaStre
 // the blocks before it.  What that reads grows with the square of the blocks, so
 // above kScanLook of them a launch between the two scans the block sums in groups
 // of kScanTile, and a block adds up the groups before its own.  irbc_bin_particles
-// without and with that launch: 2048 blocks 188 and 192 us, 4096 258 and 260, 8192
+// of 2 M particles (sixteen lanes a cell) without and with that launch: 2048 blocks 188 and 192 us, 4096 258 and 260, 8192
 // 405 and 396, 16384 771 and 724, 131072 9.9 and 5.8 ms.  totals[k] receives the sum of array
 // k, and so does the entry behind oa's last one where `end` asks for it.
 constexpr int kScanT = 256, kScanItems = 4, kScanTile = kScanT * kScanItems;

@@ -189,14 +189,15 @@ def test_cell_scan_at_tile_edges(box):
     """Counting sorts over 1024, 1023, 1025, 6 and 1,064,960 cells (a tile of
     the scan has 1024 cells; 1040 tiles are more than a block's threads), over
     4096 tiles, the most that go without a launch for the tiles' sums, and over
-    4128, whose sums are scanned in groups of 1024."""
+    4128, whose sums are scanned in groups of 1024; cells sorted by a thread
+    each below four particles a cell, by sixteen lanes from there on."""
     import torch
     import irbc_b200 as G
     Lx, Ly, Lz = box
     p = G.default_params(Lx=float(Lx), Ly=float(Ly), Lz=float(Lz), Ns=0)
     ncell = Lx * Ly * (Lz + 1)
     rng = np.random.default_rng(3)
-    for n in (0, 1, 5000):
+    for n in (0, 1, 5000) + ((4 * ncell - 1, 4 * ncell) if ncell < 2000 else ()):
         pos = [torch.tensor(rng.uniform(0, L, n), device="cuda") for L in box]
         cell = torch.zeros(max(n, 1), dtype=torch.int32, device="cuda")
         start = torch.full((ncell + 1,), -1, dtype=torch.int32, device="cuda")
