@@ -88,7 +88,8 @@ struct irbc_handle {
   cudaEvent_t ev_begin = nullptr, ev_end = nullptr;
   std::vector<cudaEvent_t> ev_pool;
   size_t ev_used = 0;
-  struct Mark { int cat; size_t start, end; };  // a timed span: pool indices of its two events
+  // a timed span: pool indices of its two events, what it counts as
+  struct Mark { int cat; size_t start, end; int units; };
   std::vector<Mark> ev_marks;
   int64_t prof_launch0 = 0;
 };
@@ -717,13 +718,14 @@ struct ProfScope {
   size_t mark;
   cudaStream_t st;
   bool on;
-  ProfScope(irbc_handle* hh, int cat, cudaStream_t s = nullptr)
+  // units: what it counts as (the steps of a stretch's streaming)
+  ProfScope(irbc_handle* hh, int cat, cudaStream_t s = nullptr, int units = 1)
       : h(hh), mark(0), st(s ? s : hh->st), on(hh->prof && !hh->capturing) {
     if (!on) return;
     const size_t idx = h->ev_used;
     cudaEventRecord(next_event(h), st);
     mark = h->ev_marks.size();
-    h->ev_marks.push_back({cat, idx, idx});
+    h->ev_marks.push_back({cat, idx, idx, units});
   }
   ~ProfScope() {
     if (!on) return;
@@ -739,7 +741,7 @@ int stream_any(irbc_handle* h, int H, cudaStream_t st, cudaEvent_t snap = nullpt
                cudaEvent_t snap1 = nullptr, bool recorded = false) {
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (h->prof && !h->capturing) {
-    h->ev_marks.push_back({PROF_STREAM_BULK, h->ev_used, h->ev_used + 1});
+    h->ev_marks.push_back({PROF_STREAM_BULK, h->ev_used, h->ev_used + 1, 1});
     e0 = next_event(h);
     e1 = next_event(h);
   }
@@ -1514,7 +1516,7 @@ static int64_t stretch(irbc_handle* h, int64_t eoff, int64_t left, bool dry) {
     CK(cudaEventRecord(h->ev_mem, ss));
     {
       // the bulk streaming reads no membrane data and starts at once
-      ProfScope ps(h, PROF_STREAM, ms);
+      ProfScope ps(h, PROF_STREAM, ms, (int)H);
       g_launches += stream_any(h, (int)H, ms, h->ev_mem, first, h->ev_part, first == 0);
     }
   }
@@ -2182,7 +2184,7 @@ extern "C" int irbc_profile_end(irbc_handle* h, double* out, int32_t nout) {
     CK(cudaEventElapsedTime(&t, h->ev_pool[mk.start], h->ev_pool[mk.end]));
     const int slot = mk.cat == PROF_STREAM_BULK ? 8 : 1 + 2 * mk.cat;
     r[slot] += t;
-    r[slot + 1] += 1;
+    r[slot + 1] += mk.units;
   }
   r[7] = (double)(g_launches.load() - h->prof_launch0);
   for (int k = 0; k < nout && k < 10; ++k) out[k] = r[k];

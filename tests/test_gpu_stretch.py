@@ -60,6 +60,21 @@ def _mesh_oracle(V, E, T, nknobs, **over):
     return op, orc
 
 
+def test_profile_counts_steps_and_launches():
+    """A profiled window counts the streamed steps, however many of them a
+    launch takes, and the launches of the bulk kernel."""
+    op, orc = H.make_oracle(ns=5000, seed=41, Lx=40.0, Ly=20.0, Lz=20.0)
+    sim = H.gpu_like(op, orc, 41)
+    sim.call("profile_begin")
+    sim.step(30)  # three stretches of ten
+    sim.call("step_part1")
+    sim.call("step_part2")
+    out = sim.profile_end()
+    assert out["stream_steps"] == 31
+    assert out["collides"] == 3
+    assert out["bulk_launches"] == 4
+
+
 # the smallest geodesic mesh that no cluster holds in patches, the largest one
 @pytest.mark.parametrize("precision", [0, 1])
 @pytest.mark.parametrize("freq", [17, 28])
