@@ -538,33 +538,30 @@ bool build_patches(const HostMesh& M, const std::vector<int>& start, const std::
   return P.smem <= kSegSmemMax;
 }
 
-// the patches of the handle's mesh and membrane form; without them (one or
-// eight blocks asked for, or a mesh that does not fit) the snapshots keep the
-// vertices' order
+// The form of the membrane (h->mem_mode) for the handle's mesh: its patches and
+// the order of the vertices in the snapshots, which without patches is their own.
+// A mesh too large for the one block keeps mode 1's form.  Where memory runs out
+// the form stays the one before.
 int upload_patches(irbc_handle* h, const std::vector<int>& start, const std::vector<int>& inc) {
   FastBufs& f = h->fb;
   const HostMesh& M = h->host_mesh;
-  dfree(f.patch.hdr);
-  dfree(f.patch.blob);
-  f.patch = PatchPlan{};
+  const bool one_block = h->mem_mode == 2 && one_block_fits(h->dp), cluster = h->mem_mode == 3;
+  PatchPlan plan;
+  std::vector<PatchHdr> hdr;
+  std::vector<unsigned char> blob;
   std::vector<int> own(M.nv);
   for (int v = 0; v < M.nv; ++v) own[v] = v;
-  if (h->mem_mode == 1) {
+  if (!one_block && !cluster) {
     // eight blocks, or sixteen (a non-portable size) where eight do not hold
     // their patches and the device can run such a cluster.  Fewer blocks than
     // eight take two rounds of items a phase: 21 against 15 us a step on the
     // 600-vertex mesh with four
     for (int nc : {8, 16}) {
       PatchPlan P;
-      std::vector<PatchHdr> hdr;
-      std::vector<unsigned char> blob;
       std::vector<int> order;
       if (!build_patches(M, start, inc, nc, h->dp.tree_sums != 0, P, hdr, blob, order)) continue;
       if (!cluster_fits(nc, P.smem)) continue;
-      CK(dalloc(&P.hdr, nc));
-      CK(dalloc(&P.blob, (int64_t)blob.size()));
-      if (up(h, P.hdr, hdr) || up(h, P.blob, blob)) return IRBC_ERR_CUDA;
-      f.patch = P;
+      plan = P;
       own = order;
       break;
     }
@@ -572,6 +569,21 @@ int upload_patches(irbc_handle* h, const std::vector<int>& start, const std::vec
   std::vector<int> place(M.nv), c1(M.nt), c2(M.nt), c3(M.nt);
   for (int q = 0; q < M.nv; ++q) place[own[q]] = q;
   for (int j = 0; j < M.nt; ++j) { c1[j] = place[M.t1[j]]; c2[j] = place[M.t2[j]]; c3[j] = place[M.t3[j]]; }
+  // everything allocated before anything of the old form goes
+  if (plan.nc > 0) {
+    CK(dalloc(&plan.hdr, plan.nc));
+    const cudaError_t e = dalloc(&plan.blob, (int64_t)blob.size());
+    if (e != cudaSuccess) {
+      dfree(plan.hdr);
+      return fail(h, IRBC_ERR_CUDA, std::string("patch tables: ") + cudaGetErrorString(e));
+    }
+  }
+  dfree(f.patch.hdr);
+  dfree(f.patch.blob);
+  f.patch = plan;
+  f.one_block = one_block;
+  f.cluster = cluster;
+  if (plan.nc > 0 && (up(h, plan.hdr, hdr) || up(h, plan.blob, blob))) return IRBC_ERR_CUDA;
   if (up(h, f.pidx, place) || up(h, f.st1, c1) || up(h, f.st2, c2) || up(h, f.st3, c3)) return IRBC_ERR_CUDA;
   CK(cudaStreamSynchronize(h->st));  // the copies' sources are local
   return 0;
@@ -634,8 +646,6 @@ int upload_mesh(irbc_handle* h, const HostMesh& M) {
   h->dp.cth0 = cos(M.theta0 * h->P.Pi / 180.0);
   h->dp.sth0 = sin(M.theta0 * h->P.Pi / 180.0);
   h->host_mesh = M;
-  h->fb.one_block = h->mem_mode == 2 && one_block_fits(h->dp);
-  h->fb.cluster = h->mem_mode == 3;
   const int rc = upload_patches(h, start, inc);
   if (rc) return rc;
   h->have_mesh = true;
@@ -1688,20 +1698,20 @@ extern "C" int irbc_set_streams(irbc_handle* h, int32_t n) {
 extern "C" int irbc_set_membrane_kernels(irbc_handle* h, int32_t mode) {
   if (!h || mode < 1 || mode > 3) return IRBC_ERR_ARG;
   cudaSetDevice(h->P.device);
+  if (h->have_mesh && mode == 2 && !one_block_fits(h->dp))
+    return fail(h, IRBC_ERR_CAPACITY, "mesh too large for the one-block membrane step");
+  if (mode == h->mem_mode) return 0;
   CK(cudaStreamSynchronize(h->st));
   CK(cudaStreamSynchronize(h->st2_own));
+  const int old = h->mem_mode;
   h->mem_mode = mode;
-  if (h->have_mesh) {
-    const bool ob = mode == 2, cl = mode == 3;
-    if (ob && !one_block_fits(h->dp)) return fail(h, IRBC_ERR_CAPACITY, "mesh too large for the one-block membrane step");
-    invalidate_graphs(h);
-    h->fb.one_block = ob;
-    h->fb.cluster = cl;
-    std::vector<int> start, inc;
-    build_incidence(h->host_mesh, start, inc);
-    return upload_patches(h, start, inc);
-  }
-  return 0;
+  if (!h->have_mesh) return 0;
+  invalidate_graphs(h);
+  std::vector<int> start, inc;
+  build_incidence(h->host_mesh, start, inc);
+  const int rc = upload_patches(h, start, inc);
+  if (rc) h->mem_mode = old;
+  return rc;
 }
 
 extern "C" int irbc_set_graphs(irbc_handle* h, int32_t on) {

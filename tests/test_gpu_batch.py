@@ -167,6 +167,34 @@ def test_cluster_membrane_equals_wide_kernels(precision, which):
     assert H.compare(out[2], out[0], 0.0) == {}
 
 
+def test_a_refused_or_unfit_mode_keeps_the_default_form():
+    """Mode 2 (one block) on the 2562-vertex mesh: refused on a handle that has
+    the mesh, which goes on as it was; set before the mesh, the handle takes the
+    default form for it.  Both launch what a handle never asked launches and
+    end in the same state."""
+    import irbc_b200 as G
+    from irbc_b200 import mesh
+    V, E, T = mesh.discocyte()
+    _, p = _small(16)
+    p.Nt, p.elap = len(V), mesh.scaled_elap(V, E)
+    out = []
+    for when in ("never", "after", "before"):
+        s = G.Simulation(p)
+        if when == "before":
+            s.set_membrane_kernels(2)
+        s.init(V, E, T, 300)
+        if when == "after":
+            with pytest.raises(G.IrbcError):
+                s.set_membrane_kernels(2)
+        n0 = s.launch_count()
+        s.step(30)
+        out.append((s.launch_count() - n0, s.get_state()))
+        s.close()
+    for launches, st in out[1:]:
+        assert launches == out[0][0]
+        assert H.compare(st, out[0][1], 0.0) == {}
+
+
 def test_server_reports_a_failed_set_up_alone():
     """A request whose set-up fails on the server's set-up thread (a knob
     count above the mesh's vertex count: irbc_init rejects it) ends with
