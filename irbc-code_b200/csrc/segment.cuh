@@ -786,12 +786,12 @@ __device__ __forceinline__ void global_gather(const DevParams& p, const Membrane
 }
 
 // The membrane of H steps by a cluster of blocks that keep its state in global
-// memory: the one-block and eight-block forms of irbc_set_membrane_kernels.
-// Bound by the load and store units: a warp's scattered 8-byte accesses take a
-// cycle a line (the discocyte on eight blocks: 92 us a step).  seg_smem() bytes
-// of shared memory, the same layout in every block.
+// memory: the one-block and eight-block forms of irbc_set_membrane_kernels, for
+// whole steps.  Bound by the load and store units: a warp's scattered 8-byte
+// accesses take a cycle a line (the discocyte on eight blocks: 92 us a step).
+// seg_smem() bytes of shared memory, the same layout in every block.
 __device__ __forceinline__ void membrane_global(const DevParams& p, const Membrane& m, const FastBufs& f,
-                                                 uint64_t epoch, int H, int parts, unsigned char* smem) {
+                                                 uint64_t epoch, int H, unsigned char* smem) {
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
   const int cta = (int)cl.block_rank(), nc = (int)cl.num_blocks();
@@ -826,23 +826,22 @@ __device__ __forceinline__ void membrane_global(const DevParams& p, const Membra
   double* v_at = staged ? (nc > 1 ? terms : terms + seg_terms(p.nt)) : m.vol;
   const double* a_at = staged ? terms : m.area;
 
-  global_first(p, m, f, parts, g, G);
+  global_first(p, m, f, SEG_WHOLE, g, G);
   cl.sync();
   for (int s = 0; s < H; ++s) {
     global_tri(p, m, f, a_to, v_to, pad, g, G);
     cl.sync();
     if (area_w || vol_w) {
-      global_sum(p, m, f, parts, area_w, area_w ? a_at : v_at, pad, area_w ? ss0 : ss1,
+      global_sum(p, m, f, SEG_WHOLE, area_w, area_w ? a_at : v_at, pad, area_w ? ss0 : ss1,
                  area_w ? t : t - 32 * voff * sw, sw, area_w ? 1 : 2);
-    } else if (parts & SEG_SECOND) {
+    } else {
       global_terms(p, m, f, worker, workers);
       bond_prep_all(p, m, f, worker, workers, reinterpret_cast<unsigned char*>(&tail));
     }
-    if (!(parts & SEG_SECOND)) return;
     cl.sync();
     const bool more = s + 1 < H;
     const int gb = nc >= 4 ? nc - 1 : nc;  // blocks that gather
-    if (cta < gb) global_gather(p, m, f, s, parts, more, g, gb * T);
+    if (cta < gb) global_gather(p, m, f, s, SEG_WHOLE, more, g, gb * T);
     // (a block that also gathers reads vX and vd there, which the tail only reads)
     if (cta == nc - 1) tail_block<kSegT>(p, m, f, epoch + s, more, tail);
     cl.sync();
@@ -1491,7 +1490,7 @@ __device__ __forceinline__ void membrane_patch(const DevParams& p, const Membran
 __device__ __forceinline__ void membrane_segment(const DevParams& p, const Membrane& m, const FastBufs& f,
                                                  uint64_t epoch, int H, int parts, unsigned char* smem) {
   if (f.patch.nc > 0) membrane_patch(p, m, f, epoch, H, parts, smem);
-  else membrane_global(p, m, f, epoch, H, parts, smem);
+  else membrane_global(p, m, f, epoch, H, smem);
 }
 
 __global__ void __launch_bounds__(kSegT) k_membrane(DevParams p, Membrane m, FastBufs f, uint64_t eoff, int H, int parts) {
