@@ -1781,7 +1781,6 @@ int64_t cohort_key(const irbc_handle* h) {
   int64_t k = h->P.device;
   k = k * 4096 + h->csteps;
   k = k * 4096 + (h->colsteps + 1);
-  k = k * 2 + (h->step & 1);
   return k;
 }
 

@@ -14,8 +14,7 @@ Cohort* cohort_create(int device);
 void cohort_destroy(Cohort* c);
 
 // Members that can share a cohort have equal keys: the same device, the
-// FP32 solvent, a mesh, the same collision interval and phase, the same
-// step parity and the same snapshot state.  A key of -1 means the handle
+// FP32 solvent, a mesh, the same collision interval and phase.  A key of -1 means the handle
 // cannot join a cohort (FP64, no mesh): it is stepped on its own.
 int64_t cohort_key(const irbc_handle* h);
 

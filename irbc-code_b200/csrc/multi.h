@@ -1,14 +1,13 @@
 // multi.h -- one launch per phase over many FP32 simulations (a cohort).
 //
-// A cohort's members advance in lock step: the same step parity, the same
-// collision phase.  Each phase of the step (bulk streaming, near-membrane
-// streaming, every membrane kernel, every collision kernel) is ONE launch
-// whose blocks are split among the members: member r owns a contiguous run
-// of each phase's blocks, each block reads (member, block index within the
-// member) from the phase's block table with one load, and then runs
-// exactly the device code the single-simulation kernel runs, on that
-// member's buffers, with its block index within the member.  A member
-// therefore computes bit for bit what it computes alone.
+// A cohort's members advance in lock step, in the same collision phase.  Each
+// phase of the step (bulk streaming, near-membrane streaming, every membrane
+// kernel, every collision kernel) is ONE launch whose blocks are split among the
+// members: member r owns a contiguous run of each phase's blocks, each block
+// reads (member, block index within the member) from the phase's block table with
+// one load, and then runs exactly the device code the single-simulation kernel
+// runs, on that member's buffers, with its block index within the member.  A
+// member therefore computes bit for bit what it computes alone.
 #pragma once
 #include <vector>
 #include "fp32.h"

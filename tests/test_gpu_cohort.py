@@ -115,6 +115,37 @@ def test_members_out_of_phase_form_their_own_cohorts():
         s.close()
 
 
+def test_members_an_odd_number_of_steps_apart_share_a_cohort():
+    """Five steps between collisions: a member five steps ahead collides on the
+    same steps as another, so both advance in one cohort (as many launches as
+    for one member), and each equals itself alone."""
+    import irbc_b200 as G
+    troph = H.troph()
+    cfgs = [(_params(910 + r, 40, 20000, dtcd=0.01), troph, 300) for r in range(3)]
+    sims = []
+    for p, (V, E, T), nk in cfgs:
+        s = G.Simulation(p)
+        s.init(V, E, T, nk)
+        sims.append(s)
+    sims[0].step(5)
+    sims[1].step(10)
+    launches = []
+    for group in ((sims[2],), sims[:2]):
+        b = G.Batch(nthreads=2)
+        for s in group:
+            b.add(s)
+        if len(group) == 1:
+            b.step(5)
+        n0 = sims[0].launch_count()
+        b.step(40)
+        launches.append(sims[0].launch_count() - n0)
+        b.close()
+    # (a launch per member sets its draw base)
+    assert launches[1] == launches[0] + 1
+    for s, c, n in zip(sims, cfgs, (45, 50, 45)):
+        _check([s], [c], n)
+
+
 def test_cohort_reflects_what_rounding_carries_to_the_membrane():
     """A cohort takes 16 steps in one part.  In a box longer than 256 a
     particle at x > 256 moves in units of 2^-15; with v dt = 23.51 of them it is
