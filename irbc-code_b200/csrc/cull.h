@@ -1,14 +1,7 @@
 // cull.h -- which triangles of a list a particle can reach in a stretch of
 // timesteps (k_near): plain C++ too, so that the bound is tested on the host.
 #pragma once
-#include <cmath>
-#include <cstdint>
-
-#ifdef __CUDACC__
-#define IRBC_HD __host__ __device__ __forceinline__
-#else
-#define IRBC_HD inline
-#endif
+#include "hd.h"
 
 namespace irbc {
 

@@ -27,24 +27,9 @@
 // wait for of stores to other blocks some 5 000.  A quarter of the vertices a
 // block hardly changes them.
 #include <cooperative_groups.h>
+#include "div.h"
 
 namespace irbc {
-
-// x / y for a divisor whose correctly rounded reciprocal r is at hand, rounded
-// as the division is (P. Markstein, IBM J. Res. Dev. 34 (1990) 111: from a
-// quotient within one ulp, q + (x - q y) r is the correctly rounded one; the
-// first correction brings it there).  Five dependent operations and no branch,
-// where a division takes about 150 cycles.  Zeros lose their sign, infinities
-// become NaN, and a quotient below 2^-1022 may differ.
-struct Divisor {
-  double y, r;
-};
-__device__ __forceinline__ double div_by(double x, Divisor d) {
-  double q = x * d.r;
-  q = __fma_rn(__fma_rn(-d.y, q, x), d.r, q);
-  return __fma_rn(__fma_rn(-d.y, q, x), d.r, q);
-}
-__device__ __forceinline__ double div3(double x) { return div_by(x, Divisor{3.0, 1.0 / 3.0}); }
 
 // ---- the ordered sums ------------------------------------------------------------
 // a[0] + a[1] + ... added left to right in double, bit for bit, by G warps
