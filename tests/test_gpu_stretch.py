@@ -30,26 +30,6 @@ STRETCHES = [  # dtcd, Lx, Ly, particles, speed factor, membrane form
 ]
 
 
-@pytest.mark.parametrize("precision", [0, 1])
-@pytest.mark.parametrize("case", STRETCHES, ids=lambda c: "%g-%gx%g-%d-%g-%d" % c)
-def test_stretches_equal_single_steps(case, precision):
-    dtcd, Lx, Ly, ns, fast, form = case
-    op, orc = H.make_oracle(ns=ns, seed=41, onrate=300.0, offrate=50.0, dtcd=dtcd, Lx=Lx, Ly=Ly)
-    st = orc.get_state()
-    for k in ("svx", "svy", "svz"):
-        st.a[k] = st.a[k] * fast
-    a = H.gpu_like(op, orc, 41, precision=precision, state=st)
-    b = H.gpu_like(op, orc, 41, precision=precision, state=st)
-    a.set_membrane_kernels(form)
-    b.set_membrane_kernels(form)
-    for n in (3, 30, 55):  # collisions inside and at the ends, the list update
-        a.step(n)
-        for _ in range(n):
-            b.call("step_part1")
-            b.call("step_part2")
-        assert H.compare(a.get_state(), b.get_state(), 0.0) == {}, n
-
-
 def _mesh_oracle(V, E, T, nknobs, **over):
     """an oracle with a mesh of its own (elap scaled to it)"""
     import oracle as O
@@ -58,6 +38,114 @@ def _mesh_oracle(V, E, T, nknobs, **over):
     orc = O.Oracle(op, 43)
     orc.init(V, E, T, nknobs)
     return op, orc
+
+
+def _against_single_steps(op, orc, seed, st, precision, form, counts):
+    """stretches of a simulation against one that takes the same steps singly"""
+    a = H.gpu_like(op, orc, seed, precision=precision, state=st)
+    b = H.gpu_like(op, orc, seed, precision=precision, state=st)
+    a.set_membrane_kernels(form)
+    b.set_membrane_kernels(form)
+    for n in counts:
+        a.step(n)
+        for _ in range(n):
+            b.call("step_part1")
+            b.call("step_part2")
+        assert H.compare(a.get_state(), b.get_state(), 0.0) == {}, n
+    return a.get_state()
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("case", STRETCHES, ids=lambda c: "%g-%gx%g-%d-%g-%d" % c)
+def test_stretches_equal_single_steps(case, precision):
+    dtcd, Lx, Ly, ns, fast, form = case
+    op, orc = H.make_oracle(ns=ns, seed=41, onrate=300.0, offrate=50.0, dtcd=dtcd, Lx=Lx, Ly=Ly)
+    st = orc.get_state()
+    for k in ("svx", "svy", "svz"):
+        st.a[k] = st.a[k] * fast
+    # collisions inside and at the ends, the list update
+    _against_single_steps(op, orc, 41, st, precision, form, (3, 30, 55))
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("dtcd", [0.025, 0.05])  # 12 steps in two parts, launches of 16 and 9
+def test_stretches_of_the_discocyte(dtcd, precision):
+    """The membrane in sixteen blocks, its long lists by 32 lanes."""
+    from irbc_b200 import mesh
+    V, E, T = mesh.discocyte()
+    op, orc = _mesh_oracle(V, E, T, 1000, Ns=30000, onrate=300.0, offrate=50.0, dtcd=dtcd, Lx=40.0, Ly=24.0, Lz=24.0)
+    st = _against_single_steps(op, orc, 43, orc.get_state(), precision, 1, (3, 30, 55))
+    assert st.a["bondi"].sum() > 0
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("freq,R,room", [(8, 4.0, 64), (15, 2.5, 512)])  # kShortKeep, kLongKeep
+def test_lists_that_keep_more_than_there_is_room_for(freq, R, room, precision):
+    """Particles whose path in a stretch is longer than three cells reach every
+    entry of their list (its centroids lie within two cells of the cell's
+    centre), so a list longer than the room is walked whole in each step; single
+    steps cull it."""
+    V, E, T = H.geodesic(freq, R)
+    op, orc = _mesh_oracle(V, E, T, 0, Ns=20000, dtcd=0.05, Lx=40.0, Ly=12.0, Lz=12.0, pmass=1e6)
+    st = orc.get_state()
+    longest = st.a["llen"].max()
+    assert room < longest and (longest <= 128) == (room == 64)
+    for k in ("svx", "svy", "svz"):
+        st.a[k] = st.a[k] * 120.0
+    v = np.sqrt(st.a["svx"] ** 2 + st.a["svy"] ** 2 + st.a["svz"] ** 2)
+    cell = (np.floor(st.a["sx"]) * 12 + np.floor(st.a["sy"])) * 13 + np.floor(st.a["sz"]) + 1
+    far = (v * 16 * op.dtmd > 3.6) & (st.a["llen"][cell.astype(int)] > room)
+    assert far.sum() > 10
+    _against_single_steps(op, orc, 43, st, precision, 1, (16, 20))
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("case", ["events", "draws", "parasite"])
+def test_more_than_the_tail_of_the_patches_holds(case, precision):
+    """More bond events in a step than its list takes (128), more vertices with
+    draws (1024) and more in the parasite's reach (768): the patches against the
+    cluster on global memory and single steps, in FP64 also against the oracle.
+    (Heavy vertices, so that forces of such reaches do not break the mesh.)"""
+    from irbc_b200 import mesh
+    V, E, T = mesh.discocyte()
+    over = dict(events=dict(dthr=0.9, onrate=1e6, offrate=1e4), draws=dict(dthr=2.0, onrate=300.0, offrate=1e4),
+                parasite=dict(paraR=6.0, PRmass=1e9))[case]
+    op, orc = _mesh_oracle(V, E, T, len(V), Ns=20000, Lx=40.0, Ly=24.0, Lz=24.0, pmass=1e7, **over)
+    st = orc.get_state()
+    if case == "parasite":
+        d2 = sum((st.a[k] - st.s["para"][i]) ** 2 for i, k in enumerate("xyz"))
+        assert (d2 < op.paraR ** 2).sum() > 768
+    else:
+        # each vertex in its own cell, as a collision without a shift leaves it,
+        # and its pairs in the first step: the ligands within dthr on that cell's
+        # list (cells below z = 2, centres within 1.5)
+        f = [np.floor(st.a["x"]), np.floor(st.a["y"]), np.floor(st.a["z"]) + 1]
+        st.a["pid"] = ((f[0] * int(op.Ly) + f[1]) * (int(op.Lz) + 1) + f[2]).astype(np.int32)
+        orc.set_state(st)
+        near = (st.a["z"] < op.dthr) & (st.a["knob"] == 1) & (f[2] <= 2)
+        g = np.stack(np.meshgrid(np.arange(0, op.Lx, 0.5), np.arange(0, op.Ly, 0.5), indexing="ij")).reshape(2, -1)
+        d = [st.a[k][near][:, None] - g[i][None] for i, k in enumerate("xy")]
+        listed = np.logical_and(*[np.abs(f[i][near][:, None] + 0.5 - g[i][None]) < 1.5 for i in (0, 1)])
+        d2 = d[0] ** 2 + d[1] ** 2 + st.a["z"][near][:, None] ** 2
+        pairs = (listed & (d2 <= op.dthr ** 2)).sum(axis=1)
+        assert pairs.max() <= 64
+        if case == "events":  # every draw succeeds
+            assert (pairs > 0).sum() <= 1024 and pairs.sum() > 128
+        else:
+            assert (pairs > 0).sum() > 1024
+    patches = _against_single_steps(op, orc, 43, st, precision, 1, (3, 22))
+    cluster = H.gpu_like(op, orc, 43, precision=precision, state=st)
+    cluster.set_membrane_kernels(3)
+    cluster.step(25)
+    assert H.compare(patches, cluster.get_state(), 0.0) == {}
+    if case != "parasite":
+        assert patches.a["bondi"].sum() > 0
+    if precision == 0:
+        s = H.gpu_like(op, orc, 43, precision=0, state=st)
+        for k in range(14):
+            orc.step(1)
+            s.step(1)
+            assert H.compare(s.get_state(), orc.get_state()) == {}, k
 
 
 def test_profile_counts_steps_and_launches():
