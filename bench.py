@@ -318,14 +318,6 @@ def run_ours(args):
     # FP64, 48 + 58 B FP32), at the measured particle-steps/s
     step_bpp = 13.2 if precision == G.FP64 else 8.8
     peak, kind = peaks()
-    traffic = None
-    tfile = os.path.join(ROOT, "profiles", "stream_traffic.json")
-    if os.path.exists(tfile):
-        try:
-            tj = json.load(open(tfile))
-            traffic = tj.get("fp64" if precision == G.FP64 else "fp32")
-        except Exception:
-            traffic = None
     # end to end through the C ABI with host buffers: the full state in from
     # page-locked memory, every step the RBCdata record out, the final state out
     e2e = None
@@ -340,8 +332,7 @@ def run_ours(args):
                        l2="state larger than L2 (no flush needed)",
                        timed="whole collision cycles: the requested steps rounded up to a multiple of 12"),
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                     "frac": achieved / peak, "traffic": traffic,
-                     "kernel": "k_stream_bulk" if precision == G.FP64 else "k_stream_bulk_f",
+                     "frac": achieved / peak, "kernel": "k_stream_bulk" if precision == G.FP64 else "k_stream_bulk_f",
                      "bytes_per_particle": bpp, "units_per_launch": ns, "peak_kind": kind,
                      "kernel_ms_avg": bulk_avg_ms,
                      "step_bytes_per_particle_step": step_bpp,

@@ -50,7 +50,7 @@ struct irbc_handle {
   cudaStream_t st2 = nullptr;  // membrane kernels, run beside the solvent ones (== st with one stream)
   cudaStream_t st2_own = nullptr;  // the side stream this handle created
   int mem_mode = 1;                // membrane: 1 patches, 2 one block, 3 one cluster on global memory
-  HostMesh host_mesh;              // topology only
+  HostMesh host_mesh;              // what the patches are built from: topology, rest lengths and areas
   FastBufs fb;
   bool fp32 = false;           // solvent held in sf (float4) between exchanges
   SolventF sf;
@@ -895,7 +895,6 @@ extern "C" int irbc_create(const irbc_params* p, irbc_handle** out) {
   cudaMemcpyAsync(h->m.xlig, h->xlig.data(), sizeof(double) * h->dp.nlig, cudaMemcpyHostToDevice, h->st);
   cudaMemcpyAsync(h->m.ylig, h->ylig.data(), sizeof(double) * h->dp.nlig, cudaMemcpyHostToDevice, h->st);
   if (cudaStreamSynchronize(h->st) != cudaSuccess) { irbc_destroy(h); return create_failed(IRBC_ERR_CUDA, "set-up copies"); }
-  // the vertex bitonic sort stages up to 8192 keys in dynamic shared memory
   h->launches0 = g_launches.load();
   *out = h;
   return 0;
@@ -1971,7 +1970,7 @@ int cohort_step(Cohort* c, const std::vector<irbc_handle*>& all, int64_t n, std:
         return IRBC_ERR_CUDA;
     }
     if (listed) {
-      int rc = cohort_upload(c);  // lists, buckets and staging may have moved or grown
+      int rc = cohort_upload(c);  // the lists may have moved or grown
       if (rc) return rc;
     }
     int64_t H = n - k;
@@ -2127,9 +2126,6 @@ extern "C" int irbc_velocity_profile(irbc_handle* h, double* out, int32_t nbins)
 }
 
 // ---- standalone binning ------------------------------------------------------------
-namespace irbc {
-}
-
 extern "C" int irbc_bin_particles(const irbc_params* p, const double* x, const double* y, const double* z,
                                   int64_t n, double rx, double ry, double rz, int32_t* cell, int32_t* start,
                                   int32_t* order) {

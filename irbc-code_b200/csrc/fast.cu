@@ -3,7 +3,8 @@
 // with triangles, and the membrane (segment.cuh) on a side stream beside the
 // bulk.
 //
-// Results equal the one-kernel-per-phase path (kernels.cu) bit for bit.
+// The membrane's and the streaming's single phases that the C ABI also offers are
+// in kernels.cu.
 #include <algorithm>
 #include <cstdio>
 #include "fast.h"
@@ -12,9 +13,6 @@
 namespace irbc {
 
 static inline unsigned nb(int64_t n, int t) { return (unsigned)((n + t - 1) / t); }
-
-#define UXm(v) (m.x[v] + m.ix[v] * p.Lx)
-#define UYm(v) (m.y[v] + m.iy[v] * p.Ly)
 
 // ================================================================ stream =====
 // reflectionFed's per-triangle test and hit, reading the vertex snapshot.
@@ -183,10 +181,6 @@ __device__ __forceinline__ void wall_step_f(float wallspeed, float Lz, float dt,
   X = bx + VX * (dt - dtt); Y = by + VY * (dt - dtt); Z = bz + VZ * (dt - dtt);
 }
 
-__device__ __forceinline__ bool in_stencil(const DevParams& p, double x, double y) {
-  return (x < 3.0 * p.a) || (x > p.Lx - (3.0 * p.a)) || (y < 3.0 * p.a) || (y > p.Ly - (3.0 * p.a));
-}
-
 // A particle's state through a stretch, in the arithmetic of the solvent's
 // precision R: double, or float for the FP32-bulk solvent, which is promoted to
 // double for reflectionFed and rounded back after every step.
@@ -219,14 +213,6 @@ __device__ __forceinline__ void free_step(const DevParams& p, Flight<float>& q) 
   if (q.Z > Lz || q.Z < 0.0f) wall_step_f((float)p.wallspeed, Lz, dt, q.X, q.Y, q.Z, q.VX, q.VY, q.VZ);
   q.X = bbound(q.X, (float)p.Lx);
   q.Y = bbound(q.Y, (float)p.Ly);
-}
-// the step of a particle that has spent fulldt of it at the membrane
-template <typename R>
-__device__ __forceinline__ void end_step(const DevParams& p, double fulldt, Flight<R>& q) {
-  double X = q.X, Y = q.Y, Z = q.Z, VX = q.VX, VY = q.VY, VZ = q.VZ;
-  finish_stream(p, fulldt, X, Y, Z, VX, VY, VZ);
-  raise_health(p, solvent_bad(p, X, Y, Z, VX, VY, VZ), HEALTH_SOLVENT);
-  q.X = (R)X; q.Y = (R)Y; q.Z = (R)Z; q.VX = (R)VX; q.VY = (R)VY; q.VZ = (R)VZ;
 }
 // the solvent's arrays
 struct SolventArrays {
@@ -276,7 +262,7 @@ __device__ __forceinline__ void enqueue(const NearQueue& h, int i, int k) {
 // pass takes each particle through all H steps of the stretch: its state is
 // read and written once instead of H times.  The arithmetic is the steps', one
 // after the other.  A particle that a step finds in a listed cell is handed over
-// at that step, with its state.  The cell flags (CF_*, launch_llist_ranks) tell
+// at that step, with its state.  The cell flags (CF_*, launch_llist_flags) tell
 // what a particle that flies less than a cell can meet from each cell: most need
 // neither a look at the cells on their way nor wraps nor walls, and 36 additions
 // are all the 12 steps cost.  Bound by HBM: FP64 80 bytes a particle (the
@@ -388,7 +374,8 @@ __device__ __forceinline__ TriPre ldg_tri(const TriPre* __restrict__ q) {
 // Inside the periodic stencil bands (3a from each side wall) reflectionFed
 // shifts a corner that lies in the opposite band by a period (:471-493).  A
 // triangle without such a corner gives what its record holds.  band_of: the
-// bands a particle's corners would be shifted from, as tri_bands reports them.
+// bands a particle's corners would be shifted from, as the records' bands
+// (records_block) report them.
 __device__ __forceinline__ int band_of(const DevParams& p, double x, double y) {
   const double rx = p.Lx - (3.0 * p.a), ry = p.Ly - (3.0 * p.a), l = 3.0 * p.a;
   return (x < l ? BAND_HX : (x > rx ? BAND_LX : 0)) | (y < l ? BAND_HY : (y > ry ? BAND_LY : 0));

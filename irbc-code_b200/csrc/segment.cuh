@@ -5,8 +5,8 @@
 // kicks, drift, forces and bonds (maincode.cpp:487-496, 566-744) of several
 // steps depend only on one another.  So one launch of a thread-block cluster
 // advances the membrane through a whole stretch (up to kSegMax steps) and
-// leaves for every step what the streaming reads: the half-kicked vertices
-// (snap) and the per-triangle records (pre).  Its phases are separated by
+// leaves for every step what the streaming reads, the half-kicked vertices
+// (snap; k_tri_records makes the per-triangle records of them).  Its phases are separated by
 // cluster barriers (barrier.cluster arrive.release / wait.acquire); three per
 // step:
 //   A  per triangle: area and volume terms (to the summing blocks' shared
@@ -904,10 +904,10 @@ __global__ void __launch_bounds__(kWideT) k_wide_gather(DevParams p, Membrane m,
 
 // ---- the membrane in patches ---------------------------------------------------------
 // The vertices are split among the cluster's blocks into connected patches
-// (host, build_patches).  A block keeps its vertices' state in registers, one
-// thread each, and in shared memory the coordinates of its vertices and of
-// those its items touch, and the force terms of its own vertices, at the place
-// where the gather reads them.  Items on a seam are computed by each block
+// (host, build_patches).  A block keeps in shared memory its vertices' state
+// (phase C: a component of a vertex per thread), the coordinates of its vertices
+// and of those its items touch, and the force terms of its own vertices, at the
+// place where the gather reads them.  Items on a seam are computed by each block
 // that owns one of their vertices (every time by the same operations), so
 // between the phases only coordinates of seam vertices, the area and volume
 // terms and the two factors cross blocks, through distributed shared memory.

@@ -117,10 +117,10 @@ def test_one_stream_equals_two(precision):
 
 
 @pytest.mark.parametrize("precision", [0, 1])
-def test_one_block_membrane_equals_wide_kernels(precision):
+def test_one_block_membrane_equals_the_default(precision):
     """The one-block membrane step (an option for meshes up to 1024
-    vertices, such as this 600-vertex one) and the wide kernels (the
-    default) give the same state, bit for bit, across collisions, bond
+    vertices, such as this 600-vertex one) and the default, a cluster that
+    holds the mesh in patches, give the same state, bit for bit, across collisions, bond
     events and a list update."""
     import irbc_b200 as G
     V, E, T = H.troph()
@@ -138,10 +138,10 @@ def test_one_block_membrane_equals_wide_kernels(precision):
 
 @pytest.mark.parametrize("precision", [0, 1])
 @pytest.mark.parametrize("which", ["troph", "disc"])
-def test_cluster_membrane_equals_wide_kernels(precision, which):
-    """The membrane step as one launch of a thread-block cluster (any mesh:
-    the 600-vertex trophozoite and the 2562-vertex discocyte) and the wide
-    kernels give the same state, bit for bit, across collisions, bond
+def test_cluster_membrane_equals_the_default(precision, which):
+    """The membrane in a cluster on global memory (mode 3, any mesh: the
+    600-vertex trophozoite and the 2562-vertex discocyte) and in patches (mode
+    1) give the same state, bit for bit, across collisions, bond
     events, list updates and captured graphs."""
     import irbc_b200 as G
     from irbc_b200 import mesh

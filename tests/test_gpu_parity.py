@@ -63,9 +63,8 @@ def test_phase_matches_oracle(base, phase):
 
 def test_stream_crowded_cell_and_long_list(base):
     """Near-membrane streaming off its usual path: 80 particles crowded into
-    one listed cell (more than a cell's bucket takes, so most go to the
-    overflow queue), and a second cell whose list is padded to 1500 entries
-    with repeats; both must follow the reference's sequential triangle walk."""
+    one listed cell, and a second cell whose list is padded to 1500 entries
+    with repeats (longer than the short lists' class); both must follow the reference's sequential triangle walk."""
     op, mesh, st = base
     st2 = st.copy()
     off, lidx = st2.llists()

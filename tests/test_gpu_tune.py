@@ -56,7 +56,7 @@ def test_autotuned_batch_equals_members_alone():
 def test_server_schedule_keeps_results():
     """A server given a launch schedule applies it to every request it
     admits; the one-block membrane form only where the mesh fits it (the
-    600-vertex mesh), the wide kernels elsewhere (the 2562-vertex
+    600-vertex mesh), the default form elsewhere (the 2562-vertex
     discocyte).  Every kept result equals the same request run alone."""
     import irbc_b200 as G
     from irbc_b200 import mesh

@@ -1,12 +1,12 @@
-"""The property the short-list near-membrane kernels rest on, checked on the
+"""The property the near-membrane streaming rests on (k_near), checked on the
 oracle (bit for bit the reference's reflectionFed, Src/solfuncs.cpp:400-598):
 a particle outside the periodic stencil bands none of whose list entries
 passes the crossing test on the triangle's normals at t and t + dtmd
 (bt * bdt <= 0 with the inside/outside flag clear) leaves the loop with its
-state unchanged and a contact time of 0.  The first launch finishes exactly
-those particles with free flight and walls; every other particle goes to the
-queue, whose walk is the loop itself.  The test also bounds how many
-particles need the queue, which is what makes the split pay."""
+state unchanged and a contact time of 0.  So k_near runs the full test of a
+triangle (tri_visit) only where the crossing test (tri_crossing) passes.  The
+test also bounds how many particles have a candidate in a step at all: few, so
+what the lanes mostly do is the crossing test."""
 import ctypes as C
 
 import numpy as np
@@ -67,5 +67,5 @@ def test_particles_without_a_crossing_candidate_leave_reflection_unchanged():
     after = orc.get_state().a
     for k in before:
         np.testing.assert_array_equal(after[k][free], before[k][free])
-    # few particles need the full walk
+    # few particles need a full test
     assert queued <= 0.05 * len(listed), (queued, len(listed))
