@@ -181,6 +181,7 @@ __device__ __forceinline__ void wall_step_f(float wallspeed, float Lz, float dt,
   X = bx + VX * (dt - dtt); Y = by + VY * (dt - dtt); Z = bz + VZ * (dt - dtt);
 }
 
+__device__ __forceinline__ double longest_side(const DevParams& p) { return fmax(p.Lx, fmax(p.Ly, p.Lz)); }
 // A particle's state through a stretch, in the arithmetic of the solvent's
 // precision R: double, or float for the FP32-bulk solvent, which is promoted to
 // double for reflectionFed and rounded back after every step.
@@ -271,7 +272,10 @@ template <typename R>
 __device__ __forceinline__ bool flies_free(const DevParams& p, const Flight<R>& q, unsigned char cf, int H) {
   // (a moving top wall gives its speed to what it reflects)
   const R reach = fmax(fmax(fabs(q.VX), fabs(q.VY)), fmax(fabs(q.VZ), fabs((R)p.wallspeed))) * (R)(H * p.dtmd);
-  return !(cf & CF_MEETS) && reach < R(0.99);
+  // (above 2^16 a float's rounding after each step can carry 0.99 of a cell
+  // beyond a whole one: 11 steps of 0.0899 are 11 of 12 / 128)
+  const bool fine = sizeof(R) > sizeof(float) || longest_side(p) <= 65536.0;
+  return !(cf & CF_MEETS) && reach < R(0.99) && fine;
 }
 __device__ __forceinline__ void wall_of(const DevParams& p, Flight<double>& q) {
   wall_step(p, p.dtmd, q.X, q.Y, q.Z, q.VX, q.VY, q.VZ);
@@ -385,7 +389,6 @@ __device__ __forceinline__ TriCull ldg_cull(const float4* __restrict__ r) {
   const float4 a = __ldg(r), b = __ldg(r + 1), c = __ldg(r + 2);
   return TriCull{{a.x, a.y, a.z}, a.w, {b.x, b.y, b.z}, b.w, c.x, c.y, __float_as_int(c.z)};
 }
-__device__ __forceinline__ double longest_side(const DevParams& p) { return fmax(p.Lx, fmax(p.Ly, p.Lz)); }
 __device__ __forceinline__ void cull_store(const DevParams& p, float4* to, const TriPre& t0, const CullMove& mv) {
   const TriCull c = cull_of(t0, mv, longest_side(p));
   to[0] = make_float4(c.X[0], c.X[1], c.X[2], c.nX);

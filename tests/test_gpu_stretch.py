@@ -148,6 +148,34 @@ def test_more_than_the_tail_of_the_patches_holds(case, precision):
             assert H.compare(s.get_state(), orc.get_state()) == {}, k
 
 
+def test_free_flight_in_a_box_longer_than_a_float_resolves():
+    """At x > 2^16 an FP32 particle moves in units of 2^-7: 11 steps of 11.51
+    units are rounded to 12 each, more than the 0.99 of a cell that its speed
+    gives, so one that starts at the end of the last cell but one leaves the box
+    in one stretch and is wrapped as by single steps."""
+    import irbc_b200 as G
+    V, E, T = H.geodesic(2, 1.0)
+    ulp = 2.0 ** -7
+    p = G.default_params(Lx=66000.0, Ly=6.0, Lz=6.0, Ns=40, seed=5, precision=G.FP32, dtcd=0.0221, Nt=len(V))
+    sims = []
+    for _ in range(2):
+        s = G.Simulation(p)
+        s.init(V, E, T, 0)
+        st = s.get_state()
+        st.a["sx"] = 65999.0 - ulp * np.arange(1, 41)
+        st.a["sy"], st.a["sz"] = np.full(40, 3.5), np.full(40, 3.5)
+        st.a["svx"], st.a["svy"], st.a["svz"] = np.full(40, 11.51 * ulp / p.dtmd), np.zeros(40), np.zeros(40)
+        s.set_state(st)
+        sims.append(s)
+    sims[0].step(11)
+    for _ in range(11):
+        sims[1].call("step_part1")
+        sims[1].call("step_part2")
+    want = sims[1].get_state()
+    assert (want.a["sx"] < 10.0).any()
+    assert H.compare(sims[0].get_state(), want, 0.0) == {}
+
+
 def test_profile_counts_steps_and_launches():
     """A profiled window counts the streamed steps, however many of them a
     launch takes, and the launches of the bulk kernel."""
