@@ -20,8 +20,10 @@
 //      parasite
 // A step's chain of eight dependent launches (at least 2 us apart from the
 // host, each cold) took 67 us on the 600-vertex mesh and 128 us on the
-// 2562-vertex discocyte, this 12 and 21.  What is left is latency, in cycles of
-// a step of 24 000 (600 vertices) and 43 000 (2562): the triangles 3 000 and
+// 2562-vertex discocyte.  A step inside a launch takes 12 and 21 us, and with some
+// 20 us for a launch's start and end, two launches to 12 steps, 14 and 31 (FP32
+// 15 and 22, whose sums take less).  What is left is latency, in cycles of a step
+// of 24 000 (600 vertices) and 43 000 (2562): the triangles 3 000 and
 // 4 700, the ordered sums 10 000 and 19 000 (the other blocks' terms and bonds
 // end before them), phase C 8 000 and 11 000, the three barriers with what they
 // wait for of stores to other blocks some 5 000.  A quarter of the vertices a
