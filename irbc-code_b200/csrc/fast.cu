@@ -307,9 +307,15 @@ __device__ __forceinline__ void fly_free(const DevParams& p, Flight<R>& q, unsig
   }
 }
 // through the stretch; returns H, or the step that finds the particle in a
-// listed cell
-template <typename R>
+// listed cell.  ONE: H is 1, where looking ahead saves nothing
+template <typename R, bool ONE>
 __device__ __forceinline__ int fly(const DevParams& p, Flight<R>& q, const unsigned char* __restrict__ cflag, int H) {
+  if (ONE) {
+    if (__ldg(cflag + cell_at(p, q.X, q.Y, q.Z)) & CF_LISTED) return 0;
+    free_step(p, q);
+    raise_health(p, solvent_bad(p, q.X, q.Y, q.Z, q.VX, q.VY, q.VZ), HEALTH_SOLVENT);
+    return 1;
+  }
   bool on;
   unsigned char cf = __ldg(cflag + cell_at(p, q.X, q.Y, q.Z, on));
   if (on && flies_free(p, q, cf, H)) {
@@ -326,14 +332,19 @@ __device__ __forceinline__ int fly(const DevParams& p, Flight<R>& q, const unsig
   }
 }
 
-__global__ void __launch_bounds__(256) k_stream_bulk(DevParams p, SolventArrays s, int64_t n,
-                                                     const unsigned char* __restrict__ cflag, NearQueue h, int H) {
+// The blocks an SM holds bound how many loads are in flight; 20 M particles, us of
+// one step and of 12: FP64 64 registers (4 blocks) 299 and 328, 40 and some spills
+// (6 blocks) 264 and 280, with ONE 248; FP32 55 registers 246 and 266, 32 (8 blocks)
+// 172 and 196, with ONE 164.
+template <bool ONE>
+__global__ void __launch_bounds__(256, 6) k_stream_bulk(DevParams p, SolventArrays s, int64_t n,
+                                                        const unsigned char* __restrict__ cflag, NearQueue h, int H) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const double X = s.x[i], Y = s.y[i], Z = s.z[i];
   const SolVel r = s.v[i];
   Flight<double> q{X, Y, Z, r.vx, r.vy, r.vz};
-  const int k = fly(p, q, cflag, H);
+  const int k = fly<double, ONE>(p, q, cflag, H);
   if (k > 0) {
     s.x[i] = q.X; s.y[i] = q.Y; s.z[i] = q.Z;
     if (q.VX != r.vx || q.VY != r.vy || q.VZ != r.vz || r.vx != r.vx) {
@@ -343,21 +354,23 @@ __global__ void __launch_bounds__(256) k_stream_bulk(DevParams p, SolventArrays 
   if (k < H) enqueue(h, (int)i, k);
 }
 // one particle of the FP32-bulk solvent, loaded as (a, b)
+template <bool ONE>
 __device__ __forceinline__ void bulk_f_item(const DevParams& p, const SolventArrays& s,
                                             const unsigned char* __restrict__ cflag, const NearQueue& h, int H, int64_t i,
                                             float4 a, float4 b) {
   Flight<float> q{a.x, a.y, a.z, b.x, b.y, b.z};
-  const int k = fly(p, q, cflag, H);
+  const int k = fly<float, ONE>(p, q, cflag, H);
   if (k > 0) {
     s.pos[i] = make_float4(q.X, q.Y, q.Z, a.w);
     if (q.VX != b.x || q.VY != b.y || q.VZ != b.z || b.x != b.x) s.vel[i] = make_float4(q.VX, q.VY, q.VZ, b.w);
   }
   if (k < H) enqueue(h, (int)i, k);
 }
-__global__ void __launch_bounds__(256) k_stream_bulk_f(DevParams p, SolventArrays s, int64_t n,
-                                                       const unsigned char* __restrict__ cflag, NearQueue h, int H) {
+template <bool ONE>
+__global__ void __launch_bounds__(256, 8) k_stream_bulk_f(DevParams p, SolventArrays s, int64_t n,
+                                                          const unsigned char* __restrict__ cflag, NearQueue h, int H) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) bulk_f_item(p, s, cflag, h, H, i, s.pos[i], s.vel[i]);
+  if (i < n) bulk_f_item<ONE>(p, s, cflag, h, H, i, s.pos[i], s.vel[i]);
 }
 
 // ---- near the membrane ---------------------------------------------------------------------
@@ -644,8 +657,9 @@ int fast_stream(const DevParams& p, const Solvent& s, const SolventF* sf, const 
   const SolventF none;
   const SolventArrays arr = arrays_of(s, sf ? *sf : none);
   if (ev0) cudaEventRecord(ev0, st);
-  if (sf) k_stream_bulk_f<<<nb(s.n, 256), 256, 0, st>>>(p, arr, s.n, c.flag, h, H);
-  else k_stream_bulk<<<nb(s.n, 256), 256, 0, st>>>(p, arr, s.n, c.flag, h, H);
+  const auto bulk = sf ? (H == 1 ? k_stream_bulk_f<true> : k_stream_bulk_f<false>)
+                       : (H == 1 ? k_stream_bulk<true> : k_stream_bulk<false>);
+  bulk<<<nb(s.n, 256), 256, 0, st>>>(p, arr, s.n, c.flag, h, H);
   if (ev1) cudaEventRecord(ev1, st);
   const bool few = short_lists(f.lmax);
   const int parts = first > 0 ? 2 : 1;

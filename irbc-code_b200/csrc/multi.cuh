@@ -22,7 +22,7 @@ __global__ void __launch_bounds__(256, 6) km_stream_bulk(Member* __restrict__ me
   for (int pass = 0; pass < kMultiStreamPasses; ++pass) {
     const int64_t i = ((int64_t)b * kMultiStreamPasses + pass) * blockDim.x + threadIdx.x;
     if (i >= n) break;
-    bulk_f_item(p, s, cflag, h, H, i, s.pos[i], s.vel[i]);
+    bulk_f_item<false>(p, s, cflag, h, H, i, s.pos[i], s.vel[i]);
   }
 }
 
