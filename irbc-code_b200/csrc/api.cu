@@ -948,7 +948,6 @@ static int check_health(irbc_handle* h) {
 extern "C" int irbc_sync(irbc_handle* h) {
   if (!h) return IRBC_ERR_ARG;
   cudaSetDevice(h->P.device);
-  CK(cudaStreamSynchronize(h->st));
   return check_health(h);
 }
 
@@ -2003,6 +2002,12 @@ int cohort_step(Cohort* c, const std::vector<irbc_handle*>& all, int64_t n, std:
   }
   g_launches += launched;
   return cudaGetLastError() == cudaSuccess ? 0 : IRBC_ERR_CUDA;
+}
+
+int cohort_wait(irbc_handle* h) {
+  cudaSetDevice(h->P.device);
+  CK(cudaStreamSynchronize(h->st));
+  return health_status(h, *h->health_host);
 }
 
 }  // namespace irbc

@@ -164,7 +164,7 @@ int step_members(StepPool& pool, std::vector<irbc::Cohort*>& cohorts, const std:
   // the cohorts' device work (and each member's health word)
   for (auto& kv : groups)
     for (size_t i : kv.second)
-      if (!status[i]) status[i] = irbc_sync(members[i]);
+      if (!status[i]) status[i] = irbc::cohort_wait(members[i]);
   for (int e : status)
     if (e) return e;
   return 0;

@@ -27,5 +27,8 @@ int64_t cohort_key(const irbc_handle* h);
 // then in an undefined state).  The kernels launched are counted in the
 // process-wide launch count that irbc_launch_count reads.
 int cohort_step(Cohort* c, const std::vector<irbc_handle*>& members, int64_t n, std::vector<int>& status);
+// waits for a member's work after cohort_step, which has queued the copy of its
+// health word already; as irbc_sync
+int cohort_wait(irbc_handle* h);
 
 }  // namespace irbc
