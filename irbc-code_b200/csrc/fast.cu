@@ -484,8 +484,9 @@ __device__ void near_walk(const DevParams& p, const NearArgs& A, int t, int l0, 
 // then tests those, a lane each, all from the same state.  The reference's loop
 // changes the state only at a hit, so the lowest entry that hits is its first
 // one: it is applied, the list is culled again with the new velocity, and the
-// entries after it are tested from there.
-template <typename R, int G, int KEEP>
+// entries after it are tested from there.  ONE: a stretch of one step with short
+// lists, where the cull costs what it saves: the list is walked as it is.
+template <typename R, int G, int KEEP, bool ONE>
 __device__ __forceinline__ void near_particle(const DevParams& p, const SolventArrays& s, const NearArgs& A, int H,
                                               int64_t i, int from, int g, unsigned mask, unsigned short* kept) {
   Flight<R> q;
@@ -516,7 +517,8 @@ __device__ __forceinline__ void near_particle(const DevParams& p, const SolventA
       l0 = __ldg(A.lstart + pid);
       len = __ldg(A.lstart + pid + 1) - l0;
     }
-    for (int after = -1;;) {  // the last entry that hit in this step
+    if (ONE) near_walk<G>(p, A, t, l0, 0, len, g, mask, indio, x, y, z, vx, vy, vz, fd);
+    for (int after = -1; !ONE;) {  // the last entry that hit in this step
       const int band = band_of(p, x, y);
       if (fresh) {
         nk = 0;
@@ -591,13 +593,21 @@ __device__ __forceinline__ void near_particle(const DevParams& p, const SolventA
   if (g == 0) flight_store(s, i, q);
 }
 // the queue's particles through the steps before H, each by the next group of G
-// lanes that is free
-template <typename R, int G, int KEEP>
+// lanes that is free; ONE: by block bid of nb in turns, as their work differs
+// little and is short against the counter's latency
+template <typename R, int G, int KEEP, bool ONE>
 __device__ __forceinline__ void near_groups(const DevParams& p, const SolventArrays& s, const NearArgs& A, int H,
-                                            unsigned short* kept) {
+                                            unsigned short* kept, int bid, int nb) {
   const int lane = threadIdx.x & 31, g = lane & (G - 1), lead = lane & ~(G - 1);
   const unsigned mask = G == 32 ? 0xffffffffu : ((1u << G) - 1u) << lead;
   const int nq = *A.q.n;
+  if (ONE) {
+    for (int w = bid * (kNearT / G) + threadIdx.x / G; w < nq; w += nb * (kNearT / G)) {
+      near_particle<R, G, KEEP, true>(p, s, A, 1, A.q.i[w], 0, g, mask, kept);
+      __syncwarp(mask);
+    }
+    return;
+  }
   while (true) {
     int w = 0;
     if (g == 0) w = atomicAdd(A.taken, 1);
@@ -605,14 +615,21 @@ __device__ __forceinline__ void near_groups(const DevParams& p, const SolventArr
     if (w >= nq) break;
     const int from = max((int)A.q.k[w], A.first);
     if (from >= H) continue;
-    near_particle<R, G, KEEP>(p, s, A, H, A.q.i[w], from, g, mask, kept);
+    near_particle<R, G, KEEP, false>(p, s, A, H, A.q.i[w], from, g, mask, kept);
     __syncwarp(mask);
   }
 }
-template <typename R, int G, int KEEP>
+template <typename R, int G, int KEEP, bool ONE>
 __global__ void __launch_bounds__(kNearT, kNearMinBlocks) k_near(DevParams p, SolventArrays s, NearArgs A, int H) {
   __shared__ unsigned short kept[kNearT / G][KEEP];
-  near_groups<R, G, KEEP>(p, s, A, H, kept[threadIdx.x / G]);
+  near_groups<R, G, KEEP, ONE>(p, s, A, H, kept[threadIdx.x / G], blockIdx.x, gridDim.x);
+}
+template <typename R>
+static void launch_near(const DevParams& p, const SolventArrays& s, const NearArgs& A, bool few, bool one, int H,
+                        cudaStream_t st) {
+  const auto k = !few ? k_near<R, kLongG, kLongKeep, false>
+                      : (one ? k_near<R, kShortGOne, kShortKeep, true> : k_near<R, kShortG, kShortKeep, false>);
+  k<<<kNearBlocks, kNearT, 0, st>>>(p, s, A, H);
 }
 
 }  // namespace irbc
@@ -669,13 +686,8 @@ int fast_stream(const DevParams& p, const Solvent& s, const SolventF* sf, const 
     if (ready) cudaStreamWaitEvent(st, ready, 0);
     if (!recorded) launch_records(p, f, s0, s1, part, st);
     const NearArgs A = near_of(p, c, f, 0, s0, part);
-    if (sf) {
-      if (few) k_near<float, kShortG, kShortKeep><<<kNearBlocks, kNearT, 0, st>>>(p, arr, A, s1);
-      else k_near<float, kLongG, kLongKeep><<<kNearBlocks, kNearT, 0, st>>>(p, arr, A, s1);
-    } else {
-      if (few) k_near<double, kShortG, kShortKeep><<<kNearBlocks, kNearT, 0, st>>>(p, arr, A, s1);
-      else k_near<double, kLongG, kLongKeep><<<kNearBlocks, kNearT, 0, st>>>(p, arr, A, s1);
-    }
+    if (sf) launch_near<float>(p, arr, A, few, H == 1, s1, st);
+    else launch_near<double>(p, arr, A, few, H == 1, s1, st);
   }
   return 1 + (recorded ? 1 : 2) * parts;
 }

@@ -30,7 +30,11 @@ __host__ __device__ constexpr int seg_terms(int nt) { return (nt + 32 + 15) / 16
 // lanes each finish sooner: 8 lanes 93 us a stretch, 1 and 2 lanes 199 and 154
 // (600 vertices); 32 lanes 242 us, 16 and 8 lanes 316 and 534 (2562).  Sixteen
 // members fill the GPU, where idle lanes cost: 4 lanes 911 us, 8 lanes 1063.
-constexpr int kShortList = 128, kShortG = 8, kShortGMember = 4, kShortKeep = 64, kLongG = 32, kLongKeep = 512;
+// Stretches of one step take short lists as they are, 4 lanes a particle
+// (kShortGOne): eight FP64 members of 600 vertices 287 us a step, with the cull
+// and the queue's counter 319; 8 lanes 295.
+constexpr int kShortList = 128, kShortG = 8, kShortGMember = 4, kShortGOne = 4, kShortKeep = 64;
+constexpr int kLongG = 32, kLongKeep = 512;
 constexpr int kNearT = 128, kNearMinBlocks = 4, kNearBlocks = 148 * kNearMinBlocks, kNearBlocksMember = 148;
 inline bool short_lists(int lmax) { return lmax <= kShortList; }
 // the side-wall bands (3a) that a triangle's corners lie in: tri_record

@@ -32,28 +32,30 @@ struct NearMember {
   SolventArrays s;
   NearArgs A;
 };
-template <int G, int KEEP>
+template <int G, int KEEP, bool ONE>
 __global__ void __launch_bounds__(kNearT, kNearMinBlocks)
     km_near(const Member* __restrict__ mem, const int2* __restrict__ tab, int H, int par) {
   __shared__ __align__(16) unsigned char raw[sizeof(NearMember)];
   __shared__ unsigned short kept[kNearT / G][KEEP];
   NearMember& N = *reinterpret_cast<NearMember*>(raw);
-  const Member& M = mem[__ldg(tab + blockIdx.x).x];
+  const int2 e = __ldg(tab + blockIdx.x);
+  const Member& M = mem[e.x];
   if (threadIdx.x == 0) {
     N.s = arrays_of(M.s, M.f);
     N.A = near_of(M.p, M.c, M.fb, par, 0, 0);
   }
   for (int i = threadIdx.x; i < (int)sizeof(DevParams) / 4; i += blockDim.x) ((int*)&N.p)[i] = ((const int*)&M.p)[i];
   __syncthreads();
-  near_groups<float, G, KEEP>(N.p, N.s, N.A, H, kept[threadIdx.x / G]);
+  near_groups<float, G, KEEP, ONE>(N.p, N.s, N.A, H, kept[threadIdx.x / G], e.y, kNearBlocksMember);
 }
 
 int multi_stream(const MultiPlan& P, int H, int par, cudaStream_t st, cudaEvent_t snap) {
   km_stream_bulk<<<P.blocks[MP_STREAM], 256, 0, st>>>(P.mem, P.table(MP_STREAM), H, par);
   if (snap) cudaStreamWaitEvent(st, snap, 0);
   const int n0 = P.blocks[MP_NEAR_SHORT], n1 = P.blocks[MP_NEAR_LONG];
-  if (n0 > 0) km_near<kShortGMember, kShortKeep><<<n0, kNearT, 0, st>>>(P.mem, P.table(MP_NEAR_SHORT), H, par);
-  if (n1 > 0) km_near<kLongG, kLongKeep><<<n1, kNearT, 0, st>>>(P.mem, P.table(MP_NEAR_LONG), H, par);
+  const auto few = H == 1 ? km_near<kShortGOne, kShortKeep, true> : km_near<kShortGMember, kShortKeep, false>;
+  if (n0 > 0) few<<<n0, kNearT, 0, st>>>(P.mem, P.table(MP_NEAR_SHORT), H, par);
+  if (n1 > 0) km_near<kLongG, kLongKeep, false><<<n1, kNearT, 0, st>>>(P.mem, P.table(MP_NEAR_LONG), H, par);
   return 1 + (n0 > 0) + (n1 > 0);
 }
 
