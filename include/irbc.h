@@ -177,7 +177,9 @@ int irbc_bond_dynamics(irbc_handle* h, int64_t epoch); /* bond prep + bond_dynam
  * index, cindex semantics), start[C+1] (exclusive scan of the per-cell
  * counts, C = Lx*Ly*(Lz+1)) and order[n] (particle indices grouped by cell,
  * ascending within a cell: the Cells[].sol lists).  Uses the box of p.
- * Scratch memory is taken with cudaMalloc and released before returning. */
+ * order serves as scratch before its result; where it is too short (fewer
+ * particles than 3 per 1024 cells) scratch memory is taken with cudaMalloc and
+ * released before returning. */
 int irbc_bin_particles(const irbc_params* p, const double* x, const double* y, const double* z,
                        int64_t n, double rx, double ry, double rz, int32_t* cell, int32_t* start,
                        int32_t* order);

@@ -332,12 +332,13 @@ __device__ __forceinline__ int fly(const DevParams& p, Flight<R>& q, const unsig
   }
 }
 
-// The blocks an SM holds bound how many loads are in flight; 20 M particles, us of
-// one step and of 12: FP64 64 registers (4 blocks) 299 and 328, 40 and some spills
-// (6 blocks) 264 and 280, with ONE 248; FP32 55 registers 246 and 266, 32 (8 blocks)
-// 172 and 196, with ONE 164.
+// The blocks an SM holds bound how many loads are in flight.  One step of 20 M
+// particles: FP64 64 registers (4 blocks) 299 us, 40 (6 blocks) 264, with ONE 248;
+// FP32 55 registers 246, 32 (8 blocks) 172, with ONE 164.  A stretch's kernel is the
+// faster for it too (12 steps 328 and 280, 266 and 196), but so many blocks keep
+// the membrane's from starting: 780 steps of 5.2 M particles 62.6 and 62.8 ms.
 template <bool ONE>
-__global__ void __launch_bounds__(256, 6) k_stream_bulk(DevParams p, SolventArrays s, int64_t n,
+__global__ void __launch_bounds__(256, ONE ? 6 : 4) k_stream_bulk(DevParams p, SolventArrays s, int64_t n,
                                                         const unsigned char* __restrict__ cflag, NearQueue h, int H) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -367,7 +368,7 @@ __device__ __forceinline__ void bulk_f_item(const DevParams& p, const SolventArr
   if (k < H) enqueue(h, (int)i, k);
 }
 template <bool ONE>
-__global__ void __launch_bounds__(256, 8) k_stream_bulk_f(DevParams p, SolventArrays s, int64_t n,
+__global__ void __launch_bounds__(256, ONE ? 8 : 4) k_stream_bulk_f(DevParams p, SolventArrays s, int64_t n,
                                                           const unsigned char* __restrict__ cflag, NearQueue h, int H) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) bulk_f_item<ONE>(p, s, cflag, h, H, i, s.pos[i], s.vel[i]);
