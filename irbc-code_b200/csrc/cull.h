@@ -39,9 +39,13 @@ IRBC_HD bool tri_crossing(const TriPre& q, double X, double Y, double Z, double 
 // normal's 1-norm, in a box whose longest side is L, it is at most L + 1 of the
 // particle's and of the corner's coordinates in float, and with differences up
 // to L another L each of the normal in float, the differences and the products
-// and 2 L of the sums: 7 L + 2, and m is 8 (L + 16).  (NaN and infinities fail
-// the comparison and are kept.)  bands: of the triangle's corners in any of the
-// steps.
+// and 2 L of the sums: 7 L + 2, and m is 8 (L + 16).  The FP32-bulk solvent is
+// also rounded to float after every step, by up to 2^-24 of each coordinate and
+// at a constant velocity always the same way, which lengthens the path: for the
+// steps of a stretch (roundings) m is sqrt(3) (L + 1) larger each.  (Without that a
+// stretch of 12 steps lost reflections in boxes longer than 128.  NaN and
+// infinities fail the comparison and are kept.)  bands: of the triangle's corners
+// in any of the steps.
 struct TriCull {
   float X[3], nX, A[3], dX, dA, m;
   int bands;
@@ -54,17 +58,9 @@ IRBC_HD bool cull_keeps(const TriCull& c, float X, float Y, float Z, float dP, i
 }
 // The longest path of a particle with velocity (vx, vy, vz) in the `left` steps
 // that a stretch still has: its speed, or the top wall's, which it gives to what
-// it reflects.  The FP32-bulk solvent is rounded to float after every step (R),
-// by up to 2^-24 of each coordinate, and at a constant velocity always the same
-// way: without that term a stretch of 12 steps lost reflections in boxes longer
-// than 128.
-template <typename R>
-IRBC_HD float cull_path(double vx, double vy, double vz, double wallspeed, double dtmd, double L, int left) {
-  const double v = sqrt(vx * vx + vy * vy + vz * vz), w = fabs(wallspeed);
-  // (the larger one; a NaN speed is kept, and the comparison keeps its entries)
-  double path = (v < w ? w : v) * dtmd * left;
-  if (sizeof(R) == sizeof(float)) path += 1.7320509 * (L + 1.0) * left * (1.0 / 16777216.0);
-  return (float)path * 1.0001f;
+// it reflects
+IRBC_HD float cull_path(double vx, double vy, double vz, double wallspeed, double dtmd, int left) {
+  return (float)(fmax(sqrt(vx * vx + vy * vy + vz * vz), fabs(wallspeed)) * dtmd * left) * 1.0001f;
 }
 // a step's record against that of the first one
 struct CullMove {
@@ -83,15 +79,15 @@ IRBC_HD void cull_fold(CullMove& c, const TriPre& t0, const TriPre& t, int bands
   if (!(fabs(s) <= 1.7976931348623157e308)) c.dX = c.dA = HUGE_VAL;
   c.bands |= bands;
 }
-// L: the box's longest side
-IRBC_HD TriCull cull_of(const TriPre& t0, const CullMove& c, double L) {
+// L: the box's longest side; roundings: see above
+IRBC_HD TriCull cull_of(const TriPre& t0, const CullMove& c, double L, int roundings) {
   const double n1 = fabs(t0.X[0]) + fabs(t0.X[1]) + fabs(t0.X[2]) + c.dX;
   return TriCull{{(float)t0.X[0], (float)t0.X[1], (float)t0.X[2]},
                  (float)norm3(t0.X[0], t0.X[1], t0.X[2]) * 1.00001f,
                  {(float)t0.A1[0], (float)t0.A1[1], (float)t0.A1[2]},
                  (float)c.dX * 1.00001f,
                  (float)c.dA * 1.00001f,
-                 (float)(n1 * (L + 16.0) * (1.0 / 2097152.0)),
+                 (float)(n1 * ((L + 16.0) * (1.0 / 2097152.0) + 1.74 * (L + 1.0) * roundings * (1.0 / 16777216.0))),
                  c.bands};
 }
 

@@ -404,7 +404,8 @@ __device__ __forceinline__ TriCull ldg_cull(const float4* __restrict__ r) {
   return TriCull{{a.x, a.y, a.z}, a.w, {b.x, b.y, b.z}, b.w, c.x, c.y, __float_as_int(c.z)};
 }
 __device__ __forceinline__ void cull_store(const DevParams& p, float4* to, const TriPre& t0, const CullMove& mv) {
-  const TriCull c = cull_of(t0, mv, longest_side(p));
+  // (tree_sums: the FP32-bulk solvent)
+  const TriCull c = cull_of(t0, mv, longest_side(p), p.tree_sums ? kSegMax : 0);
   to[0] = make_float4(c.X[0], c.X[1], c.X[2], c.nX);
   to[1] = make_float4(c.A[0], c.A[1], c.A[2], c.dX);
   to[2] = make_float4(c.dA, c.m, __int_as_float(c.bands), 0.0f);
@@ -525,7 +526,7 @@ __device__ __forceinline__ void near_particle(const DevParams& p, const SolventA
         nk = 0;
         // (a band ends inside a cell only in a box that is no whole number of
         // cells; a wrap ends in another cell, except in a box of one)
-        float dP = cull_path<R>(vx, vy, vz, p.wallspeed, p.dtmd, longest_side(p), H - t);
+        float dP = cull_path(vx, vy, vz, p.wallspeed, p.dtmd, H - t);
         if (p.nx < 2 || p.ny < 2) dP = __int_as_float(0x7f800000);
         const int wide = band | band_of(p, x - dP, y - dP) | band_of(p, x + dP, y + dP);
         constexpr int U = 4;  // entries in flight per lane
